@@ -22,6 +22,7 @@ namespace ibmk {
 // STAGE 2/3: dudt = u + f1*gradp; dudt += (f2*RHS - f3*rhs_old); stage 2
 // stores rhs_old = RHS.  The output goes straight into the forcing buffer
 // (dudtf == dudt on entry of the IBM loop, main.f90:288-306).
+// One thread per cell: the mixed forms' fields of 2^31 cells and more.
 // ---------------------------------------------------------------------------
 template <typename TU, typename T, int STAGE>
 __global__ void __launch_bounds__(256) k_predict(Geo g, const TU *__restrict__ u, const TU *__restrict__ v,
@@ -126,6 +127,175 @@ __global__ void __launch_bounds__(256) k_predict(Geo g, const TU *__restrict__ u
     ru[c] = ru_new;
     rv[c] = rv_new;
     rw[c] = rw_new;
+  }
+}
+
+// FP64 predictor: bound by FP64 issue (one warp instruction in about 18 cycles
+// per SM), so the kernel is built around the number of FP64 instructions a
+// cell takes.  Every product of interpolated velocities is a flux through one
+// face or edge and is formed once, by the cell on its lower side:
+//   xx = (u(i+1) + u)^2, yy = (v(j+1) + v)^2, zz = (w(k+1) + w)^2,
+//   uv = (u(j+1) + u)(v(i+1) + v), uw = (u(k+1) + u)(w(i+1) + w),
+//   vw = (w(j+1) + w)(v(k+1) + v);
+// the cells at i+1 and j+1 read it from shared memory, the one at k+1 keeps
+// it in registers as the block marches along z.  With the Laplacian as sums
+// of opposite neighbours that is 63 to 66 FP64 instructions a cell, against
+// about 130 for one thread per cell forming all its fluxes.  256^3, stage 2:
+// 4.39 -> 2.22 ms (0.50 T FP64 instructions/s both times).
+// A block of tx x ty cells (at most 256) holds planes k and k+1 with a
+// one-cell x/y halo (periodic) in shared memory; plane k+2 is in flight in
+// registers while k is computed.  The products on the tile's lower halo
+// column and row are formed by two of its warps.
+struct PredCoef {
+  double qx, qy, qz;          // dxi/4, dyi/4, dzi/4 (stage 3: times f2)
+  double vx, vy, vz, vc;      // visc dxi^2 .., -2 (vx + vy + vz) (stage 3: times f2)
+  double gx, gy, gz;          // -f1 dxi ..
+  double f2, mf3;             // f1 (stage 1) or f2, -f3
+  double bc;                  // buoyancy factor (stage 3: times f2)
+};
+template <int STAGE, bool BUOY>
+__global__ void __launch_bounds__(256, 2) k_predict_d(Geo g, const double *__restrict__ u, const double *__restrict__ v,
+                                                      const double *__restrict__ w, const double *__restrict__ p,
+                                                      double *__restrict__ ru, double *__restrict__ rv,
+                                                      double *__restrict__ rw, double *__restrict__ fu,
+                                                      double *__restrict__ fv, double *__restrict__ fw, PredCoef q,
+                                                      const double *__restrict__ cb, int tx, int ty, int kc) {
+  extern __shared__ __align__(16) double smd[];
+  const int hx = tx + 2, hn = hx * (ty + 2), qx = tx + 1, qn = qx * (ty + 1);
+  double *su = smd, *sv = su + 2 * hn, *sw = sv + 2 * hn, *sp = sw + 2 * hn;  // two planes each
+  double *qxx = sp + 2 * hn, *qyy = qxx + qn, *quv = qyy + qn, *quw = quv + qn, *qvw = quw + qn;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int i0 = blockIdx.x * tx, j0 = blockIdx.y * ty;
+  const int k0 = 1 + blockIdx.z * kc, k1 = min(g.K, k0 + kc - 1);
+  const long PL = g.plane;
+  // this thread's elements of a haloed plane (at most two)
+  int hoff[2];
+  bool has[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int t = tid + e * nt;
+    has[e] = t < hn;
+    const int y = has[e] ? t / hx : 0, x = has[e] ? t - y * hx : 0;
+    const int gi = (i0 - 1 + x + g.I) % g.I, gj = (j0 - 1 + y + g.J) % g.J;
+    hoff[e] = gj * g.I + gi;
+  }
+  double nu[2], nv[2], nw[2], np_[2];
+  auto fetch = [&](int kk) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      if (has[e]) {
+        const long o = (long)kk * PL + hoff[e];
+        nu[e] = u[o]; nv[e] = v[o]; nw[e] = w[o]; np_[e] = p[o];
+      }
+  };
+  auto commit = [&](int kk) {
+    const int b = (kk & 1) * hn;
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      if (has[e]) {
+        const int t = b + tid + e * nt;
+        su[t] = nu[e]; sv[t] = nv[e]; sw[t] = nw[e]; sp[t] = np_[e];
+      }
+  };
+  fetch(k0 - 1);
+  commit(k0 - 1);
+  fetch(k0);
+  commit(k0);
+  fetch(k0 + 1);
+  __syncthreads();
+  const bool cell = tid < tx * ty;
+  const int ly = cell ? tid / tx : 0, lx = cell ? tid - ly * tx : 0;
+  const int i = i0 + lx, j = j0 + ly;
+  const bool in = cell && i < g.I && j < g.J;
+  const int ch = (ly + 1) * hx + lx + 1, cq = (ly + 1) * qx + lx + 1;
+  // the fluxes through the block's lowest z faces, and the column's values
+  double Um, Vm, Wm, U0, V0, W0, uwm, vwm, zzm;
+  {
+    const int a = ((k0 - 1) & 1) * hn + ch, b = (k0 & 1) * hn + ch;
+    Um = su[a]; Vm = sv[a]; Wm = sw[a];
+    U0 = su[b]; V0 = sv[b]; W0 = sw[b];
+    uwm = (U0 + Um) * (sw[a + 1] + Wm);
+    vwm = (sw[a + hx] + Wm) * (V0 + Vm);
+    const double z = W0 + Wm;
+    zzm = z * z;
+  }
+  __syncthreads();
+  long c = (long)k0 * PL + (long)j * g.I + i;
+  for (int k = k0; k <= k1; ++k, c += PL) {
+    commit(k + 1);  // over plane k - 1, which no thread reads any more
+    __syncthreads();
+    if (k < k1) fetch(k + 2);
+    const double *uk = su + (k & 1) * hn, *vk = sv + (k & 1) * hn, *wk = sw + (k & 1) * hn, *pk = sp + (k & 1) * hn;
+    const double *ukp = su + ((k + 1) & 1) * hn, *vkp = sv + ((k + 1) & 1) * hn, *wkp = sw + ((k + 1) & 1) * hn;
+    double Up = 0., Vp = 0., Wp = 0., xx = 0., yy = 0., zz = 0., uv = 0., uw = 0., vw = 0.;
+    double au = 0., av = 0., aw = 0., du = 0., dv = 0., dw = 0.;
+    if (cell) {
+      Up = ukp[ch]; Vp = vkp[ch]; Wp = wkp[ch];
+      const double Uip = uk[ch + 1], Ujp = uk[ch + hx], Vip = vk[ch + 1], Vjp = vk[ch + hx], Wip = wk[ch + 1],
+                   Wjp = wk[ch + hx];
+      const double sx = Uip + U0, sy = Vjp + V0, sz = Wp + W0;
+      xx = sx * sx;
+      yy = sy * sy;
+      zz = sz * sz;
+      uv = (Ujp + U0) * (Vip + V0);
+      uw = (Up + U0) * (Wip + W0);
+      vw = (Wjp + W0) * (Vp + V0);
+      qxx[cq] = xx; qyy[cq] = yy; quv[cq] = uv; quw[cq] = uw; qvw[cq] = vw;
+      // velocity and pressure gradient, then (stage 3, whose right-hand side
+      // is not stored) everything added onto them, else the right-hand side
+      // starts from the Laplacian alone
+      const double P0 = pk[ch];
+      du = fma(q.gx, pk[ch + 1] - P0, U0);
+      dv = fma(q.gy, pk[ch + hx] - P0, V0);
+      dw = fma(q.gz, sp[((k + 1) & 1) * hn + ch] - P0, W0);
+      if (STAGE != 1 && in) {
+        du = fma(q.mf3, ru[c], du);
+        dv = fma(q.mf3, rv[c], dv);
+        dw = fma(q.mf3, rw[c], dw);
+      }
+      au = STAGE == 3 ? fma(q.vc, U0, du) : q.vc * U0;
+      av = STAGE == 3 ? fma(q.vc, V0, dv) : q.vc * V0;
+      aw = STAGE == 3 ? fma(q.vc, W0, dw) : q.vc * W0;
+      au = fma(q.vx, Uip + uk[ch - 1], fma(q.vy, Ujp + uk[ch - hx], fma(q.vz, Up + Um, au)));
+      av = fma(q.vx, Vip + vk[ch - 1], fma(q.vy, Vjp + vk[ch - hx], fma(q.vz, Vp + Vm, av)));
+      aw = fma(q.vx, Wip + wk[ch - 1], fma(q.vy, Wjp + wk[ch - hx], fma(q.vz, Wp + Wm, aw)));
+      if constexpr (BUOY)
+        if (in) aw = fma(q.bc, cb[c] + cb[c + PL], aw);  // momzbuoy
+    }
+    if (tid < tx) {  // row j0 - 1
+      const int a = tid + 1, b = hx + tid + 1;
+      const double s = vk[b] + vk[a];
+      qyy[tid + 1] = s * s;
+      quv[tid + 1] = (uk[b] + uk[a]) * (vk[a + 1] + vk[a]);
+      qvw[tid + 1] = (wk[b] + wk[a]) * (vkp[a] + vk[a]);
+    }
+    const int lh = nt - 1 - tid;
+    if (lh < ty) {  // column i0 - 1
+      const int a = (lh + 1) * hx, o = (lh + 1) * qx;
+      const double s = uk[a + 1] + uk[a];
+      qxx[o] = s * s;
+      quv[o] = (uk[a + hx] + uk[a]) * (vk[a + 1] + vk[a]);
+      quw[o] = (ukp[a] + uk[a]) * (wk[a + 1] + wk[a]);
+    }
+    __syncthreads();
+    if (cell) {
+      au = fma(q.qx, qxx[cq - 1] - xx, fma(q.qy, quv[cq - qx] - uv, fma(q.qz, uwm - uw, au)));
+      av = fma(q.qx, quv[cq - 1] - uv, fma(q.qy, qyy[cq - qx] - yy, fma(q.qz, vwm - vw, av)));
+      aw = fma(q.qx, quw[cq - 1] - uw, fma(q.qy, qvw[cq - qx] - vw, fma(q.qz, zzm - zz, aw)));
+      if (in) {
+        fu[c] = STAGE == 3 ? au : fma(q.f2, au, du);
+        fv[c] = STAGE == 3 ? av : fma(q.f2, av, dv);
+        fw[c] = STAGE == 3 ? aw : fma(q.f2, aw, dw);
+        if (STAGE != 3) {
+          ru[c] = au;
+          rv[c] = av;
+          rw[c] = aw;
+        }
+      }
+      uwm = uw; vwm = vw; zzm = zz;
+      Um = U0; Vm = V0; Wm = W0;
+      U0 = Up; V0 = Vp; W0 = Wp;
+    }
   }
 }
 
@@ -722,26 +892,34 @@ bool encode_field_map(CUtensorMap *m, const Geo &g, const float *f) {
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-// z chunks of a 2.5D predictor launch with nbs resident blocks per SM: the
-// split that keeps the block waves fullest, net of the two halo planes each
-// chunk reads in addition, chunks of at most maxkc planes
-int predict_zchunk(const Geo &g, int nbs, int maxkc) {
+int sm_count() {
   static int nsm = [] {
     int dev = 0, n = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
     return n;
   }();
-  const int tiles = ((g.I + QTX - 1) / QTX) * ((g.J + QTY - 1) / QTY), slots = std::max(1, nsm * nbs);
-  int kc = g.K;
+  return nsm;
+}
+// Planes per z chunk of a kernel that marches `tiles` column tiles along z with
+// `slots` resident blocks: the split that keeps the block waves fullest, net
+// of what a chunk costs in addition (in planes), chunks of at most maxkc planes
+int zchunk(int K, int tiles, int slots, int maxkc, double extra) {
+  slots = std::max(1, slots);
+  const int most = std::min(K, 64);
+  int kc = K;
   double best = -1.;
-  for (int nz = 1; nz <= std::min(g.K, 64); ++nz) {
-    const int kcz = (g.K + nz - 1) / nz, nb = tiles * ((g.K + kcz - 1) / kcz);
-    if (kcz > maxkc && nz < std::min(g.K, 64)) continue;
-    const double waves = (double)nb / slots, eff = waves / std::ceil(waves) * kcz / (kcz + 2.);
+  for (int nz = 1; nz <= most; ++nz) {
+    const int kcz = (K + nz - 1) / nz, nb = tiles * ((K + kcz - 1) / kcz);
+    if (kcz > maxkc && nz < most) continue;
+    const double waves = (double)nb / slots, eff = waves / std::ceil(waves) * kcz / (kcz + extra);
     if (eff > best + 1e-9) { best = eff; kc = kcz; }
   }
   return kc;
+}
+// the FP32 predictors, nbs resident blocks per SM: two halo planes a chunk
+int predict_zchunk(const Geo &g, int nbs, int maxkc) {
+  return zchunk(g.K, ((g.I + QTX - 1) / QTX) * ((g.J + QTY - 1) / QTY), sm_count() * nbs, maxkc, 2.);
 }
 int quad_blocks_per_sm() {
   static int n = [] {
@@ -797,6 +975,44 @@ bool launch_predict_tma(cudaStream_t s, const Geo &g, int stage, const float *u,
   return true;
 }
 
+// Tiles of the FP64 predictor: equal parts of at most 32 x-cells, then as many
+// rows as 256 threads take in equal parts (the kernel's cost is its FP64
+// instructions, so cells beyond the grid count in full; coalescing hardly
+// does).  z chunks by the block-wave model below; a chunk costs the fluxes
+// through its lowest faces and two planes' loads in addition, about 0.4 planes.
+void launch_predict_d(cudaStream_t s, const Geo &g, int stage, const double *u, const double *v, const double *w,
+                      const double *p, double *ru, double *rv, double *rw, double *fu, double *fv, double *fw,
+                      double f1, double f2, double f3, const double *cb, double bcoef) {
+  auto parts = [](int n, int most) {
+    const int m = (n + most - 1) / most;
+    return (n + m - 1) / m;
+  };
+  const int tx = parts(g.I, 32), ty = parts(g.J, 256 / tx), nt = (tx * ty + 31) / 32 * 32;
+  const size_t smem = (size_t)(8 * (tx + 2) * (ty + 2) + 5 * (tx + 1) * (ty + 1)) * sizeof(double);
+  PredCoef q;
+  const double f = stage == 3 ? f2 : 1.;
+  q.qx = f * 0.25 * g.dxi; q.qy = f * 0.25 * g.dyi; q.qz = f * 0.25 * g.dzi;
+  q.vx = f * (g.visc * g.dxi * g.dxi); q.vy = f * (g.visc * g.dyi * g.dyi); q.vz = f * (g.visc * g.dzi * g.dzi);
+  q.vc = -2. * (q.vx + q.vy + q.vz);
+  q.gx = -f1 * g.dxi; q.gy = -f1 * g.dyi; q.gz = -f1 * g.dzi;
+  q.f2 = stage == 1 ? f1 : f2;
+  q.mf3 = -f3;
+  q.bc = f * bcoef;
+  const int tiles = ((g.I + tx - 1) / tx) * ((g.J + ty - 1) / ty);
+  const int kc = zchunk(g.K, tiles, sm_count() * 2, 64, 0.4);
+  dim3 grd((g.I + tx - 1) / tx, (g.J + ty - 1) / ty, (g.K + kc - 1) / kc);
+  auto go = [&](auto kern) { kern<<<grd, nt, smem, s>>>(g, u, v, w, p, ru, rv, rw, fu, fv, fw, q, cb, tx, ty, kc); };
+  if (cb) {
+    if (stage == 1) go(k_predict_d<1, true>);
+    else if (stage == 2) go(k_predict_d<2, true>);
+    else go(k_predict_d<3, true>);
+  } else {
+    if (stage == 1) go(k_predict_d<1, false>);
+    else if (stage == 2) go(k_predict_d<2, false>);
+    else go(k_predict_d<3, false>);
+  }
+}
+
 template <typename TU, typename T>
 void launch_predict(cudaStream_t s, const Geo &g, int stage, const TU *u, const TU *v, const TU *w, const TU *p,
                     T *ru, T *rv, T *rw, T *fu, T *fv, T *fw, double f1, double f2, double f3, const double *cb,
@@ -850,14 +1066,18 @@ void launch_predict(cudaStream_t s, const Geo &g, int stage, const TU *u, const 
     return;
     }
   }
-  dim3 blk(64, 4, 1);
-  dim3 grd((g.I + 63) / 64, (g.J + 3) / 4, g.K);
-  if (stage == 1)
-    k_predict<TU, T, 1><<<grd, blk, 0, s>>>(g, u, v, w, p, ru, rv, rw, fu, fv, fw, (T)f1, (T)f2, (T)f3, cb, bcoef);
-  else if (stage == 2)
-    k_predict<TU, T, 2><<<grd, blk, 0, s>>>(g, u, v, w, p, ru, rv, rw, fu, fv, fw, (T)f1, (T)f2, (T)f3, cb, bcoef);
-  else
-    k_predict<TU, T, 3><<<grd, blk, 0, s>>>(g, u, v, w, p, ru, rv, rw, fu, fv, fw, (T)f1, (T)f2, (T)f3, cb, bcoef);
+  if constexpr (sizeof(T) == 8) {
+    launch_predict_d(s, g, stage, u, v, w, p, ru, rv, rw, fu, fv, fw, f1, f2, f3, cb, bcoef);
+  } else {
+    dim3 blk(64, 4, 1);
+    dim3 grd((g.I + 63) / 64, (g.J + 3) / 4, g.K);
+    if (stage == 1)
+      k_predict<TU, T, 1><<<grd, blk, 0, s>>>(g, u, v, w, p, ru, rv, rw, fu, fv, fw, (T)f1, (T)f2, (T)f3, cb, bcoef);
+    else if (stage == 2)
+      k_predict<TU, T, 2><<<grd, blk, 0, s>>>(g, u, v, w, p, ru, rv, rw, fu, fv, fw, (T)f1, (T)f2, (T)f3, cb, bcoef);
+    else
+      k_predict<TU, T, 3><<<grd, blk, 0, s>>>(g, u, v, w, p, ru, rv, rw, fu, fv, fw, (T)f1, (T)f2, (T)f3, cb, bcoef);
+  }
 }
 template void launch_predict<double, double>(cudaStream_t, const Geo &, int, const double *, const double *,
                                              const double *, const double *, double *, double *, double *,
