@@ -261,7 +261,7 @@ struct DivScale {
 // With phi1 (defect correction, DF): the right-hand side is the divergence
 // residual of the corrected velocity u* - f grad(phi1) (correc's FP32
 // expressions), formed on the fly instead of read from a stored state.
-template <int N1, int N2, bool DF>
+template <int N1, int N2>
 __global__ void __launch_bounds__(128) k_fillps_fftx_r(Geo g, const float *__restrict__ fu,
                                                        const float *__restrict__ fv, float *__restrict__ fw,
                                                        float2 *__restrict__ S, const float2 *__restrict__ twM,
@@ -277,7 +277,6 @@ __global__ void __launch_bounds__(128) k_fillps_fftx_r(Geo g, const float *__res
   const int row0 = blockIdx.x * ROWS;
   const int nrow = g.J * g.K;
   const float fx_hi = ds.xh, fx_lo = ds.xl, fy_hi = ds.yh, fy_lo = ds.yl, fz_hi = ds.zh, fz_lo = ds.zl;
-  const float fxs = ds.xh, fys = ds.yh, fzs = ds.zh;
   const int PL = g.I * g.J;
   // 1. right-hand side, packed z_m = x_{2m} + i x_{2m+1}; four consecutive
   // i per thread with 128-bit loads (I % 4 == 0 on this path)
@@ -302,7 +301,7 @@ __global__ void __launch_bounds__(128) k_fillps_fftx_r(Geo g, const float *__res
       float wk[4] = {w4.x, w4.y, w4.z, w4.w}, wkm[4] = {wm4.x, wm4.y, wm4.z, wm4.w};
       float vv[4] = {v4.x, v4.y, v4.z, v4.w}, vjm[4] = {vm4.x, vm4.y, vm4.z, vm4.w};
       float uu[4] = {u4.x, u4.y, u4.z, u4.w}, uim[4] = {um1, u4.x, u4.y, u4.z};
-      if (DF && phi1) {
+      if (phi1) {
         // u - fi (phi(i+1) - phi(i)) etc. as correc stores them (w = 0 on
         // the walls k = K and 0)
         const float4 p4 = *reinterpret_cast<const float4 *>(phi1 + c);
@@ -328,22 +327,18 @@ __global__ void __launch_bounds__(128) k_fillps_fftx_r(Geo g, const float *__res
       }
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        if constexpr (DF) {
-          // divergence residual in double-float arithmetic: exact differences
-          // of the FP32 velocities, products with the split FP64 factors
-          float dh, dl, th, tl, sh, sl;
-          two_sum(wk[e], -wkm[e], dh, dl);
-          df_mul(dh, dl, fz_hi, fz_lo, sh, sl);
-          two_sum(vv[e], -vjm[e], dh, dl);
-          df_mul(dh, dl, fy_hi, fy_lo, th, tl);
-          df_add(sh, sl, th, tl, sh, sl);
-          two_sum(uu[e], -uim[e], dh, dl);
-          df_mul(dh, dl, fx_hi, fx_lo, th, tl);
-          df_add(sh, sl, th, tl, sh, sl);
-          val[e] = sh + sl;
-        } else {
-          val[e] = (wk[e] - wkm[e]) * fzs + (vv[e] - vjm[e]) * fys + (uu[e] - uim[e]) * fxs;
-        }
+        // divergence residual in double-float arithmetic: exact differences
+        // of the FP32 velocities, products with the split FP64 factors
+        float dh, dl, th, tl, sh, sl;
+        two_sum(wk[e], -wkm[e], dh, dl);
+        df_mul(dh, dl, fz_hi, fz_lo, sh, sl);
+        two_sum(vv[e], -vjm[e], dh, dl);
+        df_mul(dh, dl, fy_hi, fy_lo, th, tl);
+        df_add(sh, sl, th, tl, sh, sl);
+        two_sum(uu[e], -uim[e], dh, dl);
+        df_mul(dh, dl, fx_hi, fx_lo, th, tl);
+        df_add(sh, sl, th, tl, sh, sl);
+        val[e] = sh + sl;
       }
     }
     *reinterpret_cast<float4 *>(reinterpret_cast<float *>(A + r * RS) + i0) = make_float4(val[0], val[1], val[2], val[3]);
@@ -366,80 +361,10 @@ __global__ void __launch_bounds__(128) k_fillps_fftx_r(Geo g, const float *__res
   }
 }
 
-// complex FFT along y; a group of N2 threads per kx-column, 256 threads
-template <int N1, int N2>
-__global__ void __launch_bounds__(256) k_ffty_r(Geo g, float2 *__restrict__ S, const float2 *__restrict__ twJ, int inv) {
-  constexpr int J = N1 * N2, COLS = 256 / N2, LD = J + 1;
-  extern __shared__ __align__(16) unsigned char smr[];
-  float2 *A = reinterpret_cast<float2 *>(smr);  // [COLS][LD]
-  float2 *EX = A + COLS * LD;                   // [COLS][N1*(N2+1)]
-  const int kx0 = blockIdx.x * COLS;
-  float2 *plane = S + (long)blockIdx.y * J * g.MX;
-  // the block's columns straight into shared memory by asynchronous 8-byte
-  // copies (all of a thread's loads in flight together; zero fill beyond MX)
-  for (int q = threadIdx.x; q < J * COLS; q += blockDim.x) {
-    const int jy = q / COLS, cx = q - jy * COLS;
-    const int kx = kx0 + cx;
-    const bool ok = kx < g.MX;
-    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&A[cx * LD + jy]);
-    const float2 *src = ok ? &plane[(long)jy * g.MX + kx] : plane;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(ok ? 8 : 0));
-  }
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-  __syncthreads();
-  const int grp = threadIdx.x / N2, t = threadIdx.x - grp * N2;
-  fft_group<N1, N2>(A + grp * LD, EX + grp * N1 * (N2 + 1), t, twJ, inv, kx0 + grp < g.MX);
-  __syncthreads();
-  for (int q = threadIdx.x; q < J * COLS; q += blockDim.x) {
-    const int jy = q / COLS, cx = q - jy * COLS;
-    const int kx = kx0 + cx;
-    if (kx < g.MX) plane[(long)jy * g.MX + kx] = A[cx * LD + jy];
-  }
-}
-
-// inverse real FFT along x: spectrum row -> phi(i,j,k), k = 1..K
-template <int N1, int N2>
-__global__ void __launch_bounds__(128) k_ifftx_r(Geo g, const float2 *__restrict__ S, float *__restrict__ phi,
-                                                 const float2 *__restrict__ twM, const float2 *__restrict__ twN) {
-  constexpr int M = N1 * N2, ROWS = 128 / N2;
-  constexpr int RS = M + 8, ES = N1 * (N2 + 1) + 8;  // padded group strides
-  __shared__ __align__(16) float2 A[ROWS * RS];
-  __shared__ float2 EX[ROWS * ES];
-  const int row0 = blockIdx.x * ROWS;
-  const int nrow = g.J * g.K;
-  // pack X_k and conj(X_{M-k}) straight from the (L2-resident) spectrum
-  for (int q = threadIdx.x; q < ROWS * M; q += blockDim.x) {
-    const int r = q / M, kx = q - r * M;
-    const int row = row0 + r;
-    float2 Xk = make_float2(0.f, 0.f), Xc = Xk;
-    if (row < nrow) {
-      Xk = S[(long)row * g.MX + kx];
-      Xc = cconj(S[(long)row * g.MX + (M - kx)]);
-    }
-    const float2 E = cscale(cadd(Xk, Xc), 0.5f);
-    const float2 O = cmul(cscale(csub(Xk, Xc), 0.5f), cconj(__ldg(&twN[kx])));
-    A[r * RS + kx] = cadd(E, cmk<float2>(-O.y, O.x));  // E + i O
-  }
-  __syncthreads();
-  const int grp = threadIdx.x / N2, t = threadIdx.x - grp * N2;
-  fft_group<N1, N2>(A + grp * RS, EX + grp * ES, t, twM, 1, true);
-  __syncthreads();
-  constexpr int Q = 2 * M / 4;
-  for (int q = threadIdx.x; q < ROWS * Q; q += blockDim.x) {
-    const int r = q / Q, i0 = (q - r * Q) * 4;
-    const int row = row0 + r;
-    if (row >= nrow) continue;
-    const int j = row % g.J, k = row / g.J + 1;
-    *reinterpret_cast<float4 *>(phi + fidx(g, i0, j, k)) =
-        *reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(A + r * RS) + i0);
-  }
-}
-
-// dispatch of the register FFT kernels for one length pair (M = I/2, J)
+// dispatch of the register FFT of the divergence residual for M = I/2
 template <int M1, int M2>
 bool launch_fftx_r(cudaStream_t s, const Geo &g, const float *fu, const float *fv, float *fw, float2 *S,
-                   const float2 *twM, const float2 *twN, double a, double b, double c, bool df, bool inv, float *phi,
-                   const PoissonResid &rs) {
+                   const float2 *twM, const float2 *twN, double a, double b, double c, const PoissonResid &rs) {
   const int nrow = g.J * g.K;
   constexpr int ROWS = 128 / M2;
   const int grid = (nrow + ROWS - 1) / ROWS;
@@ -449,54 +374,21 @@ bool launch_fftx_r(cudaStream_t s, const Geo &g, const float *fu, const float *f
   ds.xh = (float)a; ds.xl = (float)(a - (double)ds.xh);
   ds.yh = (float)b; ds.yl = (float)(b - (double)ds.yh);
   ds.zh = (float)c; ds.zl = (float)(c - (double)ds.zh);
-  if (inv) k_ifftx_r<M1, M2><<<grid, 128, 0, s>>>(g, S, phi, twM, twN);
-  else if (df)
-    k_fillps_fftx_r<M1, M2, true><<<grid, 128, 0, s>>>(g, fu, fv, fw, S, twM, twN, ds, rs.phi1, rs.fi, rs.fj, rs.fk);
-  else
-    k_fillps_fftx_r<M1, M2, false><<<grid, 128, 0, s>>>(g, fu, fv, fw, S, twM, twN, ds, nullptr, 0.f, 0.f, 0.f);
+  k_fillps_fftx_r<M1, M2><<<grid, 128, 0, s>>>(g, fu, fv, fw, S, twM, twN, ds, rs.phi1, rs.fi, rs.fj, rs.fk);
   return true;
 }
 bool fftx_r(cudaStream_t s, const Geo &g, const float *fu, const float *fv, float *fw, float2 *S, const float2 *twM,
-            const float2 *twN, double a, double b, double c, bool df, bool inv, float *phi, const PoissonResid &rs) {
+            const float2 *twN, double a, double b, double c, const PoissonResid &rs) {
   switch (g.I / 2) {
-    case 16: return launch_fftx_r<4, 4>(s, g, fu, fv, fw, S, twM, twN, a, b, c, df, inv, phi, rs);
-    case 32: return launch_fftx_r<8, 4>(s, g, fu, fv, fw, S, twM, twN, a, b, c, df, inv, phi, rs);
-    case 64: return launch_fftx_r<8, 8>(s, g, fu, fv, fw, S, twM, twN, a, b, c, df, inv, phi, rs);
-    case 128: return launch_fftx_r<16, 8>(s, g, fu, fv, fw, S, twM, twN, a, b, c, df, inv, phi, rs);
-    case 256: return launch_fftx_r<16, 16>(s, g, fu, fv, fw, S, twM, twN, a, b, c, df, inv, phi, rs);
+    case 16: return launch_fftx_r<4, 4>(s, g, fu, fv, fw, S, twM, twN, a, b, c, rs);
+    case 32: return launch_fftx_r<8, 4>(s, g, fu, fv, fw, S, twM, twN, a, b, c, rs);
+    case 64: return launch_fftx_r<8, 8>(s, g, fu, fv, fw, S, twM, twN, a, b, c, rs);
+    case 128: return launch_fftx_r<16, 8>(s, g, fu, fv, fw, S, twM, twN, a, b, c, rs);
+    case 256: return launch_fftx_r<16, 16>(s, g, fu, fv, fw, S, twM, twN, a, b, c, rs);
     default: return false;
   }
 }
 bool poisson_fused_residual_ok(const Geo &g) { return reg_n2(g.I / 2) && reg_n2(g.J) && g.I % 4 == 0; }
-template <int N1, int N2>
-size_t ffty_r_smem() { return (size_t)(256 / N2) * ((N1 * N2 + 1) + N1 * (N2 + 1)) * sizeof(float2); }
-template <int N1, int N2>
-void launch_ffty_r1(cudaStream_t s, const Geo &g, float2 *S, const float2 *twJ, int inv) {
-  constexpr int COLS = 256 / N2;
-  dim3 grid((g.MX + COLS - 1) / COLS, g.K);
-  k_ffty_r<N1, N2><<<grid, 256, ffty_r_smem<N1, N2>(), s>>>(g, S, twJ, inv);
-}
-bool ffty_r(cudaStream_t s, const Geo &g, float2 *S, const float2 *twJ, int inv) {
-  switch (g.J) {
-    case 16: launch_ffty_r1<4, 4>(s, g, S, twJ, inv); return true;
-    case 32: launch_ffty_r1<8, 4>(s, g, S, twJ, inv); return true;
-    case 64: launch_ffty_r1<8, 8>(s, g, S, twJ, inv); return true;
-    case 128: launch_ffty_r1<16, 8>(s, g, S, twJ, inv); return true;
-    case 256: launch_ffty_r1<16, 16>(s, g, S, twJ, inv); return true;
-    default: return false;
-  }
-}
-int ffty_r_set_smem_limits() {
-  cudaError_t e[5] = {
-      cudaFuncSetAttribute(k_ffty_r<4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ffty_r_smem<4, 4>()),
-      cudaFuncSetAttribute(k_ffty_r<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ffty_r_smem<8, 4>()),
-      cudaFuncSetAttribute(k_ffty_r<8, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ffty_r_smem<8, 8>()),
-      cudaFuncSetAttribute(k_ffty_r<16, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ffty_r_smem<16, 8>()),
-      cudaFuncSetAttribute(k_ffty_r<16, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ffty_r_smem<16, 16>())};
-  for (cudaError_t x : e)
-    if (x != cudaSuccess) return -1;
-  return 0;
-}
 
 // ---------------------------------------------------------------------------
 // fillps + forward real FFT along x.  One CTA handles ROWS rows (j,k).
@@ -910,6 +802,23 @@ __global__ void __launch_bounds__(128) k_ifftx(Geo g, FftPlan plx, const typenam
   }
 }
 
+// Thomas sweep along z between the forward and inverse transforms
+template <typename T>
+void launch_thomas(cudaStream_t s, const Geo &g, typename cpx<T>::t *S, const double *zt, const float2 *thomas_df) {
+  const long ncol = (long)g.MX * g.J;
+  const unsigned grid = (unsigned)((ncol + 127) / 128);
+  const double scale = 1.0 / ((double)(g.I / 2) * g.J), a2 = g.dzi * g.dzi;
+  if constexpr (sizeof(T) == 4) {
+    const float a2h = (float)a2, a2l = (float)(a2 - (double)a2h);
+    k_thomas_df<<<grid, 128, 0, s>>>(g, S, thomas_df, thomas_df + (long)g.K * (g.J / 2 + 1) * g.MX, a2h, a2l,
+                                     (float)scale);
+  } else if (g.zper) {
+    k_thomas_cyclic<<<grid, 128, 0, s>>>(g, S, zt, zt + g.MX, a2, scale, const_cast<double *>(zt) + g.MX + g.J);
+  } else {
+    k_thomas<T><<<grid, 128, 0, s>>>(g, S, zt, a2, scale);
+  }
+}
+
 template <typename TIn, typename T>
 void launch_poisson(cudaStream_t s, const Geo &g, const FftPlan &plx, const FftPlan &ply, const TIn *fu,
                     const TIn *fv, TIn *fw, void *spec, T *phi, const void *twM, const void *twN, const void *twJ,
@@ -920,86 +829,65 @@ void launch_poisson(cudaStream_t s, const Geo &g, const FftPlan &plx, const FftP
   const int M = g.I / 2;
   const int rows = g.I <= 256 ? 4 : 2;
   const int nrow = g.J * g.K;
-  size_t smx = (size_t)2 * rows * M * sizeof(C);
-  if constexpr (sizeof(T) == 4 && sizeof(TIn) == 4) {
-    // register four-step FFTs for the supported lengths
-    if (reg_n2(M) && reg_n2(g.J)) {
-      float2 *Sf = reinterpret_cast<float2 *>(spec);
-      const float2 *tM = (const float2 *)twM, *tN = (const float2 *)twN, *tJ = (const float2 *)twJ;
-      hook(0, 1);
-      fftx_r(s, g, (const float *)fu, (const float *)fv, (float *)fw, Sf, tM, tN, dtidxi, dtidyi, dtidzi, res64, false,
-             nullptr, resid);
-      hook(0, 0);
-      hook(1, 1);
-      ffty_r(s, g, Sf, tJ, 0);
-      hook(1, 0);
-      const long ncol = (long)g.MX * g.J;
-      const double scale = 1.0 / ((double)M * g.J);
-      hook(2, 1);
-      const double a2 = g.dzi * g.dzi;
-      const float a2h = (float)a2, a2l = (float)(a2 - (double)a2h);
-      k_thomas_df<<<(unsigned)((ncol + 127) / 128), 128, 0, s>>>(
-          g, Sf, thomas_df, thomas_df + (long)g.K * (g.J / 2 + 1) * g.MX, a2h, a2l, (float)scale);
-      hook(2, 0);
-      hook(3, 1);
-      ffty_r(s, g, Sf, tJ, 1);
-      hook(3, 0);
-      hook(4, 1);
-      fftx_r(s, g, nullptr, nullptr, nullptr, Sf, tM, tN, 0., 0., 0., false, true, (float *)phi, PoissonResid{});
-      hook(4, 0);
-      if (launches) *launches += 5;
-      return;
+  const size_t smx = (size_t)2 * rows * M * sizeof(C);
+  // the radix kernels take every transform they have a plan for; the
+  // divergence residual (res64) keeps its own first transform
+  const bool radix = fft_radix_ok<T>(g);
+  bool done = false;
+  hook(0, 1);
+  if constexpr (sizeof(TIn) == sizeof(T)) {
+    if (radix && !res64) {
+      fft_radix_fillps_x<T>(s, g, fu, fv, fw, spec, twM, twN, dtidxi, dtidyi, dtidzi);
+      done = true;
     }
   }
-  hook(0, 1);
-  if (res64 && sizeof(TIn) == 4)
-    k_fillps_fftx<TIn, T, float, true><<<(nrow + rows - 1) / rows, 128, smx, s>>>(
-        g, plx, fu, fv, fw, S, (const C *)twM, (const C *)twN, dtidxi, dtidyi, dtidzi, rows);
-  else if (res64)
-    k_fillps_fftx<TIn, T, double><<<(nrow + rows - 1) / rows, 128, smx, s>>>(g, plx, fu, fv, fw, S, (const C *)twM,
-                                                                            (const C *)twN, dtidxi, dtidyi, dtidzi,
-                                                                            rows);
-  else
-    k_fillps_fftx<TIn, T, TIn><<<(nrow + rows - 1) / rows, 128, smx, s>>>(g, plx, fu, fv, fw, S, (const C *)twM,
-                                                                         (const C *)twN, dtidxi, dtidyi, dtidzi,
-                                                                         rows);
+  if constexpr (sizeof(T) == 4 && sizeof(TIn) == 4) {
+    if (!done && res64 && poisson_fused_residual_ok(g))
+      done = fftx_r(s, g, fu, fv, fw, (float2 *)spec, (const float2 *)twM, (const float2 *)twN, dtidxi, dtidyi, dtidzi,
+                    resid);
+  }
+  if (!done) {
+    if (res64 && sizeof(TIn) == 4)
+      k_fillps_fftx<TIn, T, float, true><<<(nrow + rows - 1) / rows, 128, smx, s>>>(
+          g, plx, fu, fv, fw, S, (const C *)twM, (const C *)twN, dtidxi, dtidyi, dtidzi, rows);
+    else if (res64)
+      k_fillps_fftx<TIn, T, double><<<(nrow + rows - 1) / rows, 128, smx, s>>>(
+          g, plx, fu, fv, fw, S, (const C *)twM, (const C *)twN, dtidxi, dtidyi, dtidzi, rows);
+    else
+      k_fillps_fftx<TIn, T, TIn><<<(nrow + rows - 1) / rows, 128, smx, s>>>(
+          g, plx, fu, fv, fw, S, (const C *)twM, (const C *)twN, dtidxi, dtidyi, dtidzi, rows);
+  }
   hook(0, 0);
   const int cols = 8;
-  size_t smy = (size_t)2 * (g.J + 1) * cols * sizeof(C);
-  dim3 gy((g.MX + cols - 1) / cols, g.K);
+  const size_t smy = (size_t)2 * (g.J + 1) * cols * sizeof(C);
+  const dim3 gy((g.MX + cols - 1) / cols, g.K);
+  auto ffty = [&](int inv) {
+    if (radix) fft_radix_y<T>(s, g, spec, twJ, inv);
+    else k_ffty<T><<<gy, 256, smy, s>>>(g, ply, S, (const C *)twJ, cols, inv);
+  };
   hook(1, 1);
-  k_ffty<T><<<gy, 256, smy, s>>>(g, ply, S, (const C *)twJ, cols, 0);
+  ffty(0);
   hook(1, 0);
-  const long ncol = (long)g.MX * g.J;
-  const double scale = 1.0 / ((double)M * g.J);
   hook(2, 1);
-  if constexpr (sizeof(T) == 4) {
-    const double a2 = g.dzi * g.dzi;
-    const float a2h = (float)a2, a2l = (float)(a2 - (double)a2h);
-    k_thomas_df<<<(unsigned)((ncol + 127) / 128), 128, 0, s>>>(
-        g, reinterpret_cast<float2 *>(S), thomas_df, thomas_df + (long)g.K * (g.J / 2 + 1) * g.MX, a2h, a2l,
-        (float)scale);
-  } else if (g.zper) {
-    k_thomas_cyclic<<<(unsigned)((ncol + 127) / 128), 128, 0, s>>>(g, reinterpret_cast<double2 *>(S), zt, zt + g.MX,
-                                                                    g.dzi * g.dzi, scale,
-                                                                    const_cast<double *>(zt) + g.MX + g.J);
-  } else {
-    k_thomas<T><<<(unsigned)((ncol + 127) / 128), 128, 0, s>>>(g, S, zt, g.dzi * g.dzi, scale);
-  }
+  launch_thomas<T>(s, g, S, zt, thomas_df);
   hook(2, 0);
   hook(3, 1);
-  k_ffty<T><<<gy, 256, smy, s>>>(g, ply, S, (const C *)twJ, cols, 1);
+  ffty(1);
   hook(3, 0);
-  size_t smi = (size_t)(2 * rows * M + rows * (M + 1)) * sizeof(C);
   hook(4, 1);
-  k_ifftx<T><<<(nrow + rows - 1) / rows, 128, smi, s>>>(g, plx, S, phi, (const C *)twM, (const C *)twN, rows);
+  if (radix) {
+    fft_radix_ix<T>(s, g, spec, phi, twM, twN);
+  } else {
+    const size_t smi = (size_t)(2 * rows * M + rows * (M + 1)) * sizeof(C);
+    k_ifftx<T><<<(nrow + rows - 1) / rows, 128, smi, s>>>(g, plx, S, phi, (const C *)twM, (const C *)twN, rows);
+  }
   hook(4, 0);
   if (launches) *launches += 5;
 }
 
 template <typename T>
 int poisson_set_smem_limits() {
-  if (sizeof(T) == 4 && ffty_r_set_smem_limits() != 0) return -1;
+  if (fft_radix_set_smem_limits<T>() != 0) return -1;
   cudaError_t e[4];
   e[0] = cudaFuncSetAttribute(k_fillps_fftx<T, T, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   if (sizeof(T) == 4)

@@ -73,6 +73,16 @@ void launch_poisson(cudaStream_t s, const Geo &g, const FftPlan &plx, const FftP
                     const float2 *thomas_df = nullptr,  // FP32 spectrum: double-float pivot tables
                     PoissonHook hook = PoissonHook{nullptr, nullptr}, PoissonResid resid = PoissonResid{});
 template <typename T> int poisson_set_smem_limits();
+// fft_radix_kernels.cu: the transforms of grids whose I/2 and J are products
+// of two or three small radices (fft_radix_ok)
+template <typename T> bool fft_radix_ok(const Geo &g);
+template <typename T>
+void fft_radix_fillps_x(cudaStream_t s, const Geo &g, const T *fu, const T *fv, T *fw, void *spec, const void *twM,
+                        const void *twN, double sx, double sy, double sz);
+template <typename T> void fft_radix_y(cudaStream_t s, const Geo &g, void *spec, const void *twJ, int inv);
+template <typename T>
+void fft_radix_ix(cudaStream_t s, const Geo &g, const void *spec, T *phi, const void *twM, const void *twN);
+template <typename T> int fft_radix_set_smem_limits();
 
 // ibm_kernels.cu
 // rows (y, z) of a particle's box with a recorded x extent; boxes with more

@@ -1,0 +1,87 @@
+"""Tiled and transform kernels at the edges of their ranges, against the oracle."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from interparts_mpich_gb300 import IBMSolver
+from interparts_mpich_gb300.cases import Case, boundp
+from oracle.oracle import OracleSolver
+
+from _util import PLAIN_TOL_CALL, interior, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _state(case, seed):
+    """Random interior fields, walls as bounduvw leaves them."""
+    c = Case(name="noise", itot=case.itot, jtot=case.jtot, ktot=case.ktot, lx=case.lx, ly=case.ly, lz=case.lz,
+             visc=case.visc, seed=seed, flow="poi", perturb=0.3, bc_top=case.bc_top, bc_bot=case.bc_bot)
+    f = c.initial_fields()
+    rng = np.random.default_rng(seed)
+    for n in ("p", "durk", "dvrk", "dwrk"):
+        f[n] = np.asfortranarray(rng.uniform(-1, 1, case.shape))
+    boundp(f["p"])
+    return f
+
+
+# one cell beyond, at and below the 32-cell tile width, tiles of unequal
+# sides, the smallest grid, more planes than one z chunk
+@pytest.mark.parametrize("grid", [(4, 4, 4), (6, 32, 9), (32, 8, 5), (36, 9, 70), (64, 27, 4), (54, 16, 33), (108, 12, 6)])
+@pytest.mark.parametrize("buoyancy", [False, True])
+def test_predictor_tiles(gpu_lib, grid, buoyancy):
+    nx, ny, nz = grid
+    case = Case(name="tiles", itot=nx, jtot=ny, ktot=nz, lx=nx / 32, ly=ny / 24, lz=nz / 40, visc=1e-2)
+    fields = _state(case, 5)
+    dt = 1e-3
+    solvers = [IBMSolver(case), OracleSolver(case)]
+    out = []
+    for s in solvers:
+        s.setup(fields=fields)
+        if buoyancy:
+            rng = np.random.default_rng(9)
+            s.set_scalar(np.asfortranarray(rng.uniform(-1, 1, case.shape)), beta=0.3)
+        got = []
+        for r in (1, 2, 3):
+            s.rk(r, dt)
+            got.append({n: interior(a).copy() for n, a in s.get_intermediate().items()})
+        f = s.get_fields()
+        got.append({n: interior(f[n]).copy() for n in ("durk", "dvrk", "dwrk")})
+        out.append(got)
+    for a, b in zip(*out):
+        for n in a:
+            assert rel_l2(a[n], b[n]) < PLAIN_TOL_CALL, n
+
+
+# lengths of two radices (12 x 16 = 192, 9 x 9, 2 x 2, 16 x 16), of three
+# (6 x 8 x 8 = 384, 6 x 9 x 9 = 486), of none (2 and 3, left to the general stages)
+@pytest.mark.parametrize("grid", [(8, 4, 5), (6, 18, 4), (162, 16, 4), (54, 54, 6), (384, 6, 4), (768, 4, 4), (8, 384, 4),
+                                  (16, 486, 4), (512, 12, 4), (4, 6, 8)])
+def test_projection_lengths(gpu_lib, grid):
+    nx, ny, nz = grid
+    case = Case(name="fft", itot=nx, jtot=ny, ktot=nz, lx=nx / 32, ly=ny / 32, lz=nz / 32, visc=1e-2)
+    fields = _state(case, 7)
+    out = []
+    for s in (IBMSolver(case), OracleSolver(case)):
+        s.setup(fields=fields)
+        s.rk(1, 1e-3)
+        s.project(1, 1e-3)
+        out.append({n: interior(a) for n, a in s.get_fields().items() if n in "uvwp"})
+    for n in "uvw":
+        assert rel_l2(out[0][n], out[1][n]) < PLAIN_TOL_CALL, n
+    d = out[0]["p"] - out[1]["p"]  # the zero mode is free: its pin differs with the rounding
+    assert np.linalg.norm(d - d.mean()) < 10 * PLAIN_TOL_CALL * np.linalg.norm(out[1]["p"])
+
+
+# odd lengths in y (the oracle's eigenvalue table, as the reference's, covers
+# even ones only): the projected velocity is free of divergence, to six
+# rounded terms of size 2 x 32 with room for the solve (2^-53 each)
+@pytest.mark.parametrize("grid", [(16, 81, 4), (8, 729, 4), (12, 27, 7)])
+def test_projection_divergence(gpu_lib, grid):
+    nx, ny, nz = grid
+    case = Case(name="odd", itot=nx, jtot=ny, ktot=nz, lx=nx / 32, ly=ny / 32, lz=nz / 32, visc=1e-2)
+    s = IBMSolver(case)
+    s.setup(fields=_state(case, 7))
+    s.rk(1, 1e-3)
+    s.project(1, 1e-3)
+    assert s.chkdiv()[1] < 1e-11
