@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(256) k_ffty(Geo g, FftPlan ply, typename cpx<T
 // Thomas sweep along z for every (kx,ky) (solver.f90:94-134), FP64, with
 // the precomputed pivots zt (pivot reciprocal for k<K, denominator for k=K).
 template <typename T>
-__global__ void __launch_bounds__(128) k_thomas(Geo g, typename cpx<T>::t *__restrict__ S,
+__global__ void __launch_bounds__(64) k_thomas(Geo g, typename cpx<T>::t *__restrict__ S,
                                                 const double *__restrict__ zt, double a2, double scale) {
   typedef typename cpx<T>::t C;
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -581,88 +581,77 @@ __global__ void __launch_bounds__(128) k_thomas(Geo g, typename cpx<T>::t *__res
 }
 
 // Periodic z: the cyclic tridiagonal solve of every (kx, ky) mode in FP64,
-// one thread per column: Sherman-Morrison around the Thomas sweep (diagonal
-// -2 a2 + xy, off-diagonals and corners a2; gamma = -b), the zero mode
-// (xy = 0) pinned at its last plane.  The same operation order as the
-// oracle's cyclic_solve; the two right-hand sides (the spectrum and the
-// Sherman-Morrison vector) are swept together.  xy = xrt(kx) + yrt(ky) from
-// the host tables.
-__global__ void __launch_bounds__(128) k_thomas_cyclic(Geo g, double2 *__restrict__ S, const double *__restrict__ xrt,
-                                                       const double *__restrict__ yrt, double a2, double scale,
-                                                       double *__restrict__ work) {
+// one thread per column: Sherman-Morrison around the Thomas sweep (T: diagonal
+// -2 a2 + xy with its two ends changed, off-diagonals a2; u = (gamma, 0.., 0,
+// a2), gamma = -b), the zero mode pinned at its last plane.  Everything that
+// does not depend on the right-hand side comes from tables over (k, |ky|, kx):
+//   cp[k] = a2 / den_k, iv[k] = 1 / den_k (the pivots), z = T^-1 u,
+//   gi = 1 / (gamma (1 + z_0 + a2 z_(K-1) / gamma)).
+// T is symmetric, so the factor of the correction, f = (y_0 + a2 y_(K-1) /
+// gamma) gamma gi with y = T^-1 r, is (z . r) gi: it is known after the forward
+// sweep, and the back substitution stores y - f z at once.  The dependent
+// chain is one multiply-add a plane in each direction (three divisions before,
+// and two more passes over the column): 64^3, 279 -> 40 us.
+__global__ void __launch_bounds__(64) k_thomas_cyclic(Geo g, double2 *__restrict__ S, const double *__restrict__ tab,
+                                                      double scale) {
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   const long ncol = (long)g.MX * g.J;
   if (t >= ncol) return;
   const int kx = (int)(t % g.MX), ky = (int)(t / g.MX);
-  const long sstride = (long)g.J * g.MX;
-  double2 *s = S + t;
-  double *cp = work + t, *zz = work + ncol * g.K + t;  // [K][ncol] each
-  const double xy = xrt[kx] + yrt[ky];
-  const double b = -2. * a2 + xy;
+  const int kyy = ky <= g.J / 2 ? ky : g.J - ky;
+  const long sstride = ncol, zst = (long)(g.J / 2 + 1) * g.MX, col = (long)kyy * g.MX + kx;
   const int K = g.K;
-  auto rd = [&](int k) { const double2 v = s[k * sstride]; return make_double2(v.x * scale, v.y * scale); };
-  if (xy == 0.) {  // rows 0..K-2 with the last unknown pinned to 0
-    const int n = K - 1;
-    double den = b;
-    cp[0] = a2 / den;
-    double2 r = rd(0);
-    r = make_double2(r.x / den, r.y / den);
-    s[0] = r;
-    for (int k = 1; k < n; ++k) {
-      den = b - a2 * cp[(long)(k - 1) * ncol];
-      cp[(long)k * ncol] = a2 / den;
-      const double2 v = rd(k);
-      r = make_double2((v.x - a2 * r.x) / den, (v.y - a2 * r.y) / den);
-      s[k * sstride] = r;
+  const double *cp = tab + col, *iv = cp + K * zst, *z = iv + K * zst;
+  const double gi = tab[3 * K * zst + col];
+  double2 *s = S + t;
+  constexpr int PF = 16;
+  double2 r = make_double2(0., 0.), f = r;
+  for (int k0 = 0; k0 < K; k0 += PF) {
+    double2 v[PF];
+    double c[PF], d[PF], e[PF];
+#pragma unroll
+    for (int q = 0; q < PF; ++q) {
+      const int k = k0 + q;
+      if (k < K) { v[q] = s[k * sstride]; c[q] = cp[k * zst]; d[q] = iv[k * zst]; e[q] = z[k * zst]; }
     }
-    for (int k = n - 2; k >= 0; --k) {
-      const double2 v = s[k * sstride];
-      const double c = cp[(long)k * ncol];
-      r = make_double2(v.x - c * r.x, v.y - c * r.y);
-      s[k * sstride] = r;
+#pragma unroll
+    for (int q = 0; q < PF; ++q) {
+      const int k = k0 + q;
+      if (k >= K) break;
+      const double2 w = make_double2(v[q].x * scale, v[q].y * scale);
+      f.x = fma(e[q], w.x, f.x);
+      f.y = fma(e[q], w.y, f.y);
+      const double m = k ? -c[q] : 0.;
+      r.x = fma(m, r.x, w.x * d[q]);
+      r.y = fma(m, r.y, w.y * d[q]);
+      v[q] = r;
     }
-    s[(long)(K - 1) * sstride] = make_double2(0., 0.);
-    return;
+#pragma unroll
+    for (int q = 0; q < PF; ++q)
+      if (k0 + q < K) s[(k0 + q) * sstride] = v[q];
   }
-  const double gamma = -b;
-  const double b0 = b - gamma, bn = b - a2 * a2 / gamma;
-  // forward sweep of both right-hand sides: the spectrum r and u = (gamma, 0.., 0, a2)
-  double den = b0;
-  cp[0] = a2 / den;
-  double2 r = rd(0);
-  r = make_double2(r.x / den, r.y / den);
-  s[0] = r;
-  double z = gamma / den;
-  zz[0] = z;
-  for (int k = 1; k < K; ++k) {
-    const double bk = k == K - 1 ? bn : b;
-    den = bk - a2 * cp[(long)(k - 1) * ncol];
-    cp[(long)k * ncol] = a2 / den;
-    const double2 v = rd(k);
-    r = make_double2((v.x - a2 * r.x) / den, (v.y - a2 * r.y) / den);
-    s[k * sstride] = r;
-    const double uk = k == K - 1 ? a2 : 0.;
-    z = (uk - a2 * z) / den;
-    zz[(long)k * ncol] = z;
-  }
-  // back substitution of both
-  for (int k = K - 2; k >= 0; --k) {
-    const double2 v = s[k * sstride];
-    const double c = cp[(long)k * ncol];
-    r = make_double2(v.x - c * r.x, v.y - c * r.y);
-    s[k * sstride] = r;
-    z = zz[(long)k * ncol] - c * z;
-    zz[(long)k * ncol] = z;
-  }
-  // r, z hold row 0; rows K-1 from memory
-  const double2 rl = s[(long)(K - 1) * sstride];
-  const double zl = zz[(long)(K - 1) * ncol];
-  const double fdn = 1. + z + a2 * zl / gamma;
-  const double fx = (r.x + a2 * rl.x / gamma) / fdn, fy = (r.y + a2 * rl.y / gamma) / fdn;
-  for (int k = 0; k < K; ++k) {
-    const double2 v = s[k * sstride];
-    const double zk = zz[(long)k * ncol];
-    s[k * sstride] = make_double2(v.x - fx * zk, v.y - fy * zk);
+  f.x *= -gi;
+  f.y *= -gi;
+  r = make_double2(0., 0.);
+  for (int k1 = K - 1; k1 >= 0; k1 -= PF) {
+    double2 v[PF];
+    double c[PF], e[PF];
+#pragma unroll
+    for (int q = 0; q < PF; ++q) {
+      const int k = k1 - q;
+      if (k >= 0) { v[q] = s[k * sstride]; c[q] = cp[k * zst]; e[q] = z[k * zst]; }
+    }
+#pragma unroll
+    for (int q = 0; q < PF; ++q) {
+      const int k = k1 - q;
+      if (k < 0) break;
+      r.x = fma(-c[q], r.x, v[q].x);
+      r.y = fma(-c[q], r.y, v[q].y);
+      v[q] = make_double2(fma(f.x, e[q], r.x), fma(f.y, e[q], r.y));
+    }
+#pragma unroll
+    for (int q = 0; q < PF; ++q)
+      if (k1 - q >= 0) s[(k1 - q) * sstride] = v[q];
   }
 }
 
@@ -674,7 +663,7 @@ __global__ void __launch_bounds__(128) k_thomas_cyclic(Geo g, double2 *__restric
 // recurrence carries its value in double-float from plane to plane; the
 // forward intermediate between the sweeps is kept in the FP32 spectrum, and
 // the 1/(M*J) FFT scale is applied at the final FP32 store.
-__global__ void __launch_bounds__(128) k_thomas_df(Geo g, float2 *__restrict__ S, const float2 *__restrict__ zt,
+__global__ void __launch_bounds__(64) k_thomas_df(Geo g, float2 *__restrict__ S, const float2 *__restrict__ zt,
                                                    const float2 *__restrict__ azt, float a2h, float a2l,
                                                    float fscale) {
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -806,16 +795,18 @@ __global__ void __launch_bounds__(128) k_ifftx(Geo g, FftPlan plx, const typenam
 template <typename T>
 void launch_thomas(cudaStream_t s, const Geo &g, typename cpx<T>::t *S, const double *zt, const float2 *thomas_df) {
   const long ncol = (long)g.MX * g.J;
-  const unsigned grid = (unsigned)((ncol + 127) / 128);
+  // small blocks: the columns spread over the SMs (FP64: each has its own slow
+  // pipe; 96 x 108 x 75, 5292 columns: 47.6 us with 128 threads, 45.4 with 32)
+  const int bs = ncol < 64 * 1216 ? 32 : 64;
   const double scale = 1.0 / ((double)(g.I / 2) * g.J), a2 = g.dzi * g.dzi;
   if constexpr (sizeof(T) == 4) {
     const float a2h = (float)a2, a2l = (float)(a2 - (double)a2h);
-    k_thomas_df<<<grid, 128, 0, s>>>(g, S, thomas_df, thomas_df + (long)g.K * (g.J / 2 + 1) * g.MX, a2h, a2l,
+    k_thomas_df<<<(unsigned)((ncol + bs - 1) / bs), bs, 0, s>>>(g, S, thomas_df, thomas_df + (long)g.K * (g.J / 2 + 1) * g.MX, a2h, a2l,
                                      (float)scale);
   } else if (g.zper) {
-    k_thomas_cyclic<<<grid, 128, 0, s>>>(g, S, zt, zt + g.MX, a2, scale, const_cast<double *>(zt) + g.MX + g.J);
+    k_thomas_cyclic<<<(unsigned)((ncol + bs - 1) / bs), bs, 0, s>>>(g, S, zt, scale);
   } else {
-    k_thomas<T><<<grid, 128, 0, s>>>(g, S, zt, a2, scale);
+    k_thomas<T><<<(unsigned)((ncol + bs - 1) / bs), bs, 0, s>>>(g, S, zt, a2, scale);
   }
 }
 
