@@ -549,7 +549,8 @@ int alloc_all(ibm_ctx *c) {
       if ((st = dalloc(c, &c->ib.psum, (size_t)9 * np))) return st;
       if ((st = dalloc(c, &c->ib.rsum, (size_t)3 * np))) return st;
     } else {
-      if ((st = dalloc(c, &c->ib.st, npl))) return st;
+      if ((st = dalloc(c, &c->ib.so, npl))) return st;
+      if ((st = dalloc(c, &c->ib.sw, SW_N * npl))) return st;
     }
     if ((st = dalloc(c, &c->ib.nla, np))) return st;
     if ((st = dalloc(c, &c->pb.pf, (size_t)PF_N * np))) return st;
@@ -817,17 +818,21 @@ int forcing_run(ibm_ctx *c, double dt, int nl_iter, int kind) {
     }
     return IBM_OK;
   }
-  PROBED(IBM_PROBE_STENCIL, launch_ibm_stencil<double>(c->stream, g, c->pg, c->ib));
+  PROBED(IBM_PROBE_STENCIL, launch_ibm_stencil(c->stream, g, c->pg, c->ib));
   LAUNCHED(1);
   for (int it = 0; it < nl_iter; ++it) {
     PROBED(IBM_PROBE_INTERP,
-           launch_ibm_interp_force<double>(c->stream, g, c->pg, c->ib, c->fu, c->fv, c->fw, dt, it == 0 ? 1 : 0));
+           launch_ibm_interp_force(c->stream, g, c->pg, c->ib, c->fu, c->fv, c->fw, dt, it == 0 ? 1 : 0));
     LAUNCHED(1);
+    if (it == nl_iter - 1) {
+      launch_ibm_force_torque(c->stream, c->pg, c->ib);
+      LAUNCHED(1);
+    }
     if (it == 0 && !g.zper) {  // dwdtf(:,:,k1) carries only S(F) (interp_spread.f90:267-269)
       launch_zero_plane<double>(c->stream, g, c->fw, g.K + 1);
       LAUNCHED(1);
     }
-    PROBED(IBM_PROBE_SPREAD, launch_ibm_spread<double>(c->stream, g, c->pg, c->ib, c->fu, c->fv, c->fw, dt, it == 0));
+    PROBED(IBM_PROBE_SPREAD, launch_ibm_spread(c->stream, g, c->pg, c->ib, c->fu, c->fv, c->fw, dt));
     LAUNCHED(1);
   }
   return IBM_OK;
@@ -1154,7 +1159,7 @@ int ibm_destroy(ibm_ctx *c) {
   drop_graphs(c);
   void *ptrs[] = {c->u, c->v, c->w, c->p, c->ru, c->rv, c->rw, c->fu, c->fv, c->fw, c->phi, c->spec, c->zt, c->twM,
                   c->twN, c->twJ, c->scratch, c->dout, c->href, c->ib.xfp, c->ib.yfp, c->ib.zfp, c->ib.ul, c->ib.vl,
-                  c->ib.wl, c->ib.dudtl, c->ib.dvdtl, c->ib.dwdtl, c->ib.fxl, c->ib.fyl, c->ib.fzl, c->ib.st,
+                  c->ib.wl, c->ib.dudtl, c->ib.dvdtl, c->ib.dwdtl, c->ib.fxl, c->ib.fyl, c->ib.fzl, c->ib.so, c->ib.sw,
                   c->ib.nla, c->ib.diag, c->pb.pf, c->pb.cf, c->pb.qmax, c->pb.firstc, c->pb.ofirstc, c->pb.nb,
                   c->pb.mslv, c->pb.rkp, c->pb.sincos, c->pb.err, c->pb.red, c->pb.pos4, c->pb.cstart, c->pb.cfill, c->pb.citem, c->pb.ccell, c->ru32, c->rv32, c->rw32, c->fu32,
                   c->fv32, c->fw32, c->phi32, c->phi32b, c->spec32, c->twM32, c->twN32, c->twJ32, c->ib.rec, c->ib.pref, c->ib.pcen, c->ib.fxs, c->ib.fys, c->ib.fzs, c->ib.pvh, c->ib.pvl, c->ib.slip, c->ib.bgeo, c->ib.rowm, c->u32, c->v32,
@@ -1951,7 +1956,7 @@ int ibm_slip_residual(ibm_ctx *c, double *maxres, double *rmsres) {
   // re-interpolate the forced field (valid between ibm_forcing_loop and ibm_project)
   if (c->mixed) c->launches += -1 + launch_ibm_interp_force_f(c->stream, c->g, c->pg, c->ib, c->fu32, c->fv32, c->fw32,
                                                              1., -2);
-  else launch_ibm_interp_force<double>(c->stream, c->g, c->pg, c->ib, c->fu, c->fv, c->fw, 1., -1);
+  else launch_ibm_interp_force(c->stream, c->g, c->pg, c->ib, c->fu, c->fv, c->fw, 1., -1);
   LAUNCHED(1);
   launch_slip_residual(c->stream, c->pg, c->ib, c->dout + 16);
   LAUNCHED(1);

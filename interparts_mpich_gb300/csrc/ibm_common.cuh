@@ -39,13 +39,6 @@ enum CField { CF_DX, CF_DY, CF_DZ, CF_DXT, CF_DYT, CF_DZT, CF_DUT, CF_DVT, CF_DW
 enum RKField { RK_FX, RK_FY, RK_FZ, RK_TX, RK_TY, RK_TZ, RK_TT, RK_CFX, RK_CFY, RK_CFZ,
                RK_CTX, RK_CTY, RK_CTZ, RK_DUDT, RK_DVDT, RK_DWDT, RK_DOMX, RK_DOMY, RK_DOMZ, RK_N };
 
-// Per-point stencil of the 3-point delta (interp_spread.f90:76-130), cached
-// once per substep because the points do not move during the forcing loop.
-struct PointStencil {
-  int ilow, jlow, klow, ilows, jlows, klows;  // reference indices
-  double phix[3], phiy[3], phiz[3], phixh[3], phiyh[3], phizh[3];
-};
-
 // Mixed form: one velocity component of one Lagrangian point: index of tap
 // (0,0,0) of the 3x3x3 block (x, y unwrapped) and the component's FP32 delta
 // weights wx[3], wy[3], wz[3], formed in registers from the point's record

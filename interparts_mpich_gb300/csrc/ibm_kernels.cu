@@ -18,18 +18,49 @@
 
 namespace ibmk {
 
-// stencil of one point (interp_spread.f90:76-130): same arithmetic as the
-// reference, single rank (zstart = 1)
-__global__ void __launch_bounds__(256) k_ibm_stencil(Geo g, PartGeo pg, IbmBuffers b) {
+// The plain form's IBM kernels are bound by FP64 issue (a warp instruction in
+// about 18 cycles per SM).  So the weights are formed once per substep, one
+// square root per axis and offset (6 a point, 18 with one per node), products
+// and sums are fused by hand where the stencil indices and decisions do not
+// hang on them, and a thread takes one component of one point: a single sphere
+// (719 points at D = 16 dx) still spreads over 34 SMs.  Blocks take the three
+// components of the same points in turn, so that their weights come from L2.
+//   1000 spheres of 16 dx: stencil 587 -> 238 us, interpolation 427 -> 171,
+//   spreading 276 -> 252 (63 M FP64 atomic adds), force sums (last pass) 34
+//   one sphere: stencil 35 -> 10 us, interpolation 70 -> 8, spreading 19 -> 6
+
+// delta weights at three consecutive nodes, r1 the signed distance of node 1.
+// |r1| <= 1/2: node 1 takes the inner branch of kernel.f90:7-25, nodes 0 and 2
+// the outer one, and all share s = sqrt(1 - 3 r1^2); any other r1 (an origin
+// clamped at a wall) takes the general form node by node.
+__device__ __forceinline__ void delta3wd(double r1, double *w, long n) {
+  if (fabs(r1) <= 0.5) {
+    const double s = sqrt(fma(-3. * r1, r1, 1.));
+    w[0] = (1. / 6.) * (fma(3., r1, 2.) - s);
+    w[n] = (1. / 3.) * (1. + s);
+    w[2 * n] = (1. / 6.) * (fma(-3., r1, 2.) - s);
+  } else {
+    w[0] = delta3(r1 - 1.);
+    w[n] = delta3(r1);
+    w[2 * n] = delta3(r1 + 1.);
+  }
+}
+// periodic images of a coordinate: floor(t / l) without the division where t
+// lies in the domain (the quotient of t < l rounds below one)
+__device__ __forceinline__ int image(double t, double l) { return t >= 0. && t < l ? 0 : (int)floor(t / l); }
+
+// stencil of one point (interp_spread.f90:76-130), single rank (zstart = 1):
+// origins in so, weights in sw (field-major, SW_*)
+__global__ void __launch_bounds__(64) k_ibm_stencil(Geo g, PartGeo pg, IbmBuffers b) {
   const int n = pg.np * pg.nl;  // < 2^31 points (checked at create)
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const int p = t / pg.nl, l = t - p * pg.nl;
     if (l >= b.nla[p]) continue;
     const double xfp = b.xfp[t], yfp = b.yfp[t], zfp = b.zfp[t];
-    double coorxfp = xfp * g.dxi - (double)((long)floor((xfp - 0.5 * g.dx) / g.lx) * g.I) - (1 - 1);
-    double cooryfp = yfp * g.dyi - (double)((long)floor((yfp - 0.5 * g.dy) / g.ly) * g.J) - (1 - 1);
+    double coorxfp = xfp * g.dxi - (double)((long)image(xfp - 0.5 * g.dx, g.lx) * g.I);
+    double cooryfp = yfp * g.dyi - (double)((long)image(yfp - 0.5 * g.dy, g.ly) * g.J);
     // periodic z: the image rule of x and y along z (no wall clamps below)
-    double coorzfp = g.zper ? zfp * g.dzi - (double)((long)floor((zfp - 0.5 * g.dz) / g.lz) * g.K) : zfp * g.dzi;
+    double coorzfp = g.zper ? zfp * g.dzi - (double)((long)image(zfp - 0.5 * g.dz, g.lz) * g.K) : zfp * g.dzi;
     // Guard: a point outside the grid (or a non-finite position) would index
     // outside the arrays; flag it and park the point at a safe location.
     if (!(coorxfp >= 0. && coorxfp <= g.I + 1.) || !(cooryfp >= 0. && cooryfp <= g.J + 1.) ||
@@ -37,190 +68,183 @@ __global__ void __launch_bounds__(256) k_ibm_stencil(Geo g, PartGeo pg, IbmBuffe
       atomicExch(&b.err[2], 1);
       coorxfp = 1.; cooryfp = 1.; coorzfp = 1.5;
     }
-    PointStencil s;
-    s.ilows = fnint(coorxfp) - 1;
-    s.jlows = fnint(cooryfp) - 1;
-    s.klows = g.zper ? fnint(coorzfp) - 1 : max(fnint(coorzfp) - 1, 1);
-    s.ilow = (int)floor(coorxfp);
-    s.jlow = (int)floor(cooryfp);
-    s.klow = g.zper ? (int)floor(coorzfp) : max(min((int)floor(coorzfp), g.K - 2), 1);
+    const int ilows = fnint(coorxfp) - 1, jlows = fnint(cooryfp) - 1;
+    const int klows = g.zper ? fnint(coorzfp) - 1 : max(fnint(coorzfp) - 1, 1);
+    const int ilow = (int)floor(coorxfp), jlow = (int)floor(cooryfp);
+    const int klow = g.zper ? (int)floor(coorzfp) : max(min((int)floor(coorzfp), g.K - 2), 1);
+    // the staggered origins as offsets from the centred ones (-1..2)
+    b.so[t] = make_int4(ilow, jlow, klow, (ilows - ilow + 8) | (jlows - jlow + 8) << 8 | (klows - klow + 8) << 16);
+    const long nn = n;
+    double *w = b.sw + t;
+    delta3wd(1. * (ilows + 1) - coorxfp, w + SW_X * nn, nn);
+    delta3wd(1. * (jlows + 1) - cooryfp, w + SW_Y * nn, nn);
+    delta3wd(1. * (klows + 1) - coorzfp, w + SW_Z * nn, nn);
+    delta3wd(1. * ilow + .5 - coorxfp, w + SW_XH * nn, nn);
+    delta3wd(1. * jlow + .5 - cooryfp, w + SW_YH * nn, nn);
+    delta3wd(1. * klow + .5 - coorzfp, w + SW_ZH * nn, nn);
+  }
+}
+
+// component C (0 u, 1 v, 2 w) of point t: offsets of its 3 x 3 x 3 taps along
+// each axis (periodic images folded in) and its weights
+template <int C> struct Taps {
+  int ox[3], oy[3];
+  long oz[3];
+  double wx[3], wy[3], wz[3];
+  __device__ __forceinline__ Taps(const Geo &g, const IbmBuffers &b, long n, int t) {
+    const int4 o = b.so[t];
+    const int i0 = o.x + (C == 0 ? (o.w & 255) - 8 : 0), j0 = o.y + (C == 1 ? ((o.w >> 8) & 255) - 8 : 0),
+              k0 = o.z + (C == 2 ? ((o.w >> 16) & 255) - 8 : 0);
+    const double *w = b.sw + t;
+#pragma unroll
     for (int m = 0; m < 3; ++m) {
-      s.phix[m] = delta3(1. * s.ilows + m - coorxfp);
-      s.phiy[m] = delta3(1. * s.jlows + m - cooryfp);
-      s.phiz[m] = delta3(1. * s.klows + m - coorzfp);
-      s.phixh[m] = delta3(1. * s.ilow + m - .5 - coorxfp);
-      s.phiyh[m] = delta3(1. * s.jlow + m - .5 - cooryfp);
-      s.phizh[m] = delta3(1. * s.klow + m - .5 - coorzfp);
+      ox[m] = wrapm(i0 + m - 1, g.I);
+      oy[m] = wrapm(j0 + m - 1, g.J) * g.I;
+      oz[m] = zwrap(g, k0 + m) * g.plane;
+      wx[m] = w[((C == 0 ? SW_X : SW_XH) + m) * n];
+      wy[m] = w[((C == 1 ? SW_Y : SW_YH) + m) * n];
+      wz[m] = w[((C == 2 ? SW_Z : SW_ZH) + m) * n];
     }
-    b.st[t] = s;
   }
+};
+
+// blocks of IB_T points, the three components of a chunk in consecutive blocks
+constexpr int IB_T = 64;
+inline int ibm_blocks(const PartGeo &pg) {
+  const long need = 3L * (((long)pg.np * pg.nl + IB_T - 1) / IB_T);
+  return (int)(need < 3 * 152 * 32 ? need : 3 * 152 * 32);
 }
 
-template <typename T>
-void launch_ibm_stencil(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuffers b) {
-  k_ibm_stencil<<<1216, 256, 0, s>>>(g, pg, b);
-}
-template void launch_ibm_stencil<double>(cudaStream_t, const Geo &, const PartGeo &, IbmBuffers);
-template void launch_ibm_stencil<float>(cudaStream_t, const Geo &, const PartGeo &, IbmBuffers);
-
-
-
-// interpolation of the three staggered components at point t
-// separable form of the 27-tap sums of interp_spread.f90:132-154:
-// sum_k phiz_k sum_j phiy_j sum_i phix_i f_ijk (same terms, fewer FP64 ops)
-template <typename FU, typename FV, typename FW>
-__device__ __forceinline__ void interp_sep(const PointStencil &s, FU U, FV V, FW W, double &ou, double &ov,
-                                           double &ow) {
-  double au = 0., av = 0., aw = 0.;
-  for (int k = 0; k < 3; ++k) {
-    double su = 0., sv = 0., sw = 0.;
-    for (int j = 0; j < 3; ++j) {
-      double ru = 0., rv = 0., rw = 0.;
-      for (int i = 0; i < 3; ++i) {
-        ru += U(i, j, k) * s.phix[i];
-        rv += V(i, j, k) * s.phixh[i];
-        rw += W(i, j, k) * s.phixh[i];
+// eulr2lagr (the separable form of the 27-tap sums of interp_spread.f90:132-154,
+// 39 multiply-adds) and the point force of complagrforces / updtlagrforces
+template <int C>
+__device__ __forceinline__ void interp_points(const Geo &g, const PartGeo &pg, const IbmBuffers &b,
+                                              const double *__restrict__ f, double dti, int first) {
+  const int n = pg.np * pg.nl;
+  const double *U = C == 0 ? b.ul : (C == 1 ? b.vl : b.wl);
+  double *I = C == 0 ? b.dudtl : (C == 1 ? b.dvdtl : b.dwdtl), *F = C == 0 ? b.fxl : (C == 1 ? b.fyl : b.fzl);
+  for (int t = (int)(blockIdx.x / 3) * IB_T + threadIdx.x; t < n; t += (int)(gridDim.x / 3) * IB_T) {
+    const int p = t / pg.nl;
+    if (t - p * pg.nl >= b.nla[p]) continue;
+    const Taps<C> s(g, b, n, t);
+    double acc = 0.;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      double sj = 0.;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const double *r = f + s.oz[k] + s.oy[j];
+        sj = fma(fma(r[s.ox[2]], s.wx[2], fma(r[s.ox[1]], s.wx[1], r[s.ox[0]] * s.wx[0])), s.wy[j], sj);
       }
-      su += ru * s.phiyh[j];
-      sv += rv * s.phiy[j];
-      sw += rw * s.phiyh[j];
+      acc = fma(sj, s.wz[k], acc);
     }
-    au += su * s.phizh[k];
-    av += sv * s.phizh[k];
-    aw += sw * s.phiz[k];
+    I[t] = acc;
+    if (first < 0) continue;  // interpolation only (slip residual)
+    const double d = U[t] - acc;
+    F[t] = first ? d * dti : fma(d, dti, F[t]);
   }
-  ou = au; ov = av; ow = aw;
+}
+__global__ void __launch_bounds__(IB_T) k_ibm_interp_force(Geo g, PartGeo pg, IbmBuffers b,
+                                                           const double *__restrict__ fu,
+                                                           const double *__restrict__ fv,
+                                                           const double *__restrict__ fw, double dti, int first) {
+  const int c = blockIdx.x % 3;
+  if (c == 0) interp_points<0>(g, pg, b, fu, dti, first);
+  else if (c == 1) interp_points<1>(g, pg, b, fv, dti, first);
+  else interp_points<2>(g, pg, b, fw, dti, first);
 }
 
-template <typename T>
-__device__ __forceinline__ void interp_point(const Geo &g, const PointStencil &s, const T *__restrict__ fu,
-                                             const T *__restrict__ fv, const T *__restrict__ fw, double &ou,
-                                             double &ov, double &ow) {
-  int ix[3], ixh[3], jy[3], jyh[3];
-  for (int m = 0; m < 3; ++m) {
-    ix[m] = wrapm(s.ilows + m - 1, g.I);
-    ixh[m] = wrapm(s.ilow + m - 1, g.I);
-    jy[m] = wrapm(s.jlows + m - 1, g.J);
-    jyh[m] = wrapm(s.jlow + m - 1, g.J);
-  }
-  int kz[3], kzs[3];
-  for (int m = 0; m < 3; ++m) {
-    kz[m] = zwrap(g, s.klow + m);
-    kzs[m] = zwrap(g, s.klows + m);
-  }
-  interp_sep(s, [&](int i, int j, int k) { return (double)fu[fidx(g, ix[i], jyh[j], kz[k])]; },
-             [&](int i, int j, int k) { return (double)fv[fidx(g, ixh[i], jy[j], kz[k])]; },
-             [&](int i, int j, int k) { return (double)fw[fidx(g, ixh[i], jyh[j], kzs[k])]; }, ou, ov, ow);
-}
-
-// eulr2lagr + complagrforces/updtlagrforces for one particle per block:
-// interpolation, point force update and the per-particle force/torque sums.
-template <typename T>
-__global__ void __launch_bounds__(256) k_ibm_interp_force(Geo g, PartGeo pg, IbmBuffers b, const T *__restrict__ fu,
-                                                          const T *__restrict__ fv, const T *__restrict__ fw,
-                                                          double dti, int first) {
-  const int p = blockIdx.x;
-  const int nla = b.nla[p];
-  const double *pf = b.pf;
-  const double px = pf[PF_X * pg.np + p], py = pf[PF_Y * pg.np + p], pz = pf[PF_Z * pg.np + p];
-  double sfx = 0, sfy = 0, sfz = 0, stx = 0, sty = 0, stz = 0;
+// force and torque sums of one particle per block (complagrforces), after the
+// last pass only: each pass's totals replace the ones before
+__global__ void __launch_bounds__(128) k_ibm_force_torque(PartGeo pg, IbmBuffers b) {
+  const int p = blockIdx.x, np = pg.np, nla = b.nla[p];
+  const double px = b.pf[PF_X * np + p], py = b.pf[PF_Y * np + p], pz = b.pf[PF_Z * np + p];
+  double s[6] = {0., 0., 0., 0., 0., 0.};
   for (int l = threadIdx.x; l < nla; l += blockDim.x) {
     const long t = (long)p * pg.nl + l;
-    const PointStencil s = b.st[t];
-    double iu, iv, iw;
-    interp_point<T>(g, s, fu, fv, fw, iu, iv, iw);
-    b.dudtl[t] = iu; b.dvdtl[t] = iv; b.dwdtl[t] = iw;
-    if (first < 0) continue;  // interpolation only (slip residual)
-    double fx, fy, fz;
-    if (first) {
-      fx = (b.ul[t] - iu) * dti;
-      fy = (b.vl[t] - iv) * dti;
-      fz = (b.wl[t] - iw) * dti;
-    } else {
-      fx = b.fxl[t] + (b.ul[t] - iu) * dti;
-      fy = b.fyl[t] + (b.vl[t] - iv) * dti;
-      fz = b.fzl[t] + (b.wl[t] - iw) * dti;
-    }
-    b.fxl[t] = fx; b.fyl[t] = fy; b.fzl[t] = fz;
+    const double fx = b.fxl[t], fy = b.fyl[t], fz = b.fzl[t];
     const double rx = b.xfp[t] - px, ry = b.yfp[t] - py, rz = b.zfp[t] - pz;
-    sfx += fx; sfy += fy; sfz += fz;
-    stx = stx + ry * fz - rz * fy;
-    sty = sty + rz * fx - rx * fz;
-    stz = stz + rx * fy - ry * fx;
+    s[0] += fx; s[1] += fy; s[2] += fz;
+    s[3] = fma(-rz, fy, fma(ry, fz, s[3]));
+    s[4] = fma(-rx, fz, fma(rz, fx, s[4]));
+    s[5] = fma(-ry, fx, fma(rx, fy, s[5]));
   }
-  __shared__ double red[6][256];
-  red[0][threadIdx.x] = sfx; red[1][threadIdx.x] = sfy; red[2][threadIdx.x] = sfz;
-  red[3][threadIdx.x] = stx; red[4][threadIdx.x] = sty; red[5][threadIdx.x] = stz;
+  __shared__ double red[6][4];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) s[q] += __shfl_down_sync(0xffffffffu, s[q], d);
+    if ((threadIdx.x & 31) == 0) red[q][threadIdx.x >> 5] = s[q];
+  }
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int q = 0; q < 6; ++q) red[q][threadIdx.x] += red[q][threadIdx.x + o];
-    __syncthreads();
+  if (threadIdx.x < 6) {
+    const int q = threadIdx.x;
+    const double v = ((red[q][0] + red[q][1]) + (red[q][2] + red[q][3])) * p_dvl(pg, p);
+    const int f[6] = {PF_FXLTOT, PF_FYLTOT, PF_FZLTOT, PF_TQX, PF_TQY, PF_TQZ};
+    b.pf[f[q] * np + p] = v;
+    red[q][0] = v;
   }
-  if (threadIdx.x == 0 && first >= 0) {
-    double *pw = b.pf;
-    const double dV = p_dvl(pg, p);
-    const double tx = red[3][0] * dV, ty = red[4][0] * dV, tz = red[5][0] * dV;
-    pw[PF_FXLTOT * pg.np + p] = red[0][0] * dV;
-    pw[PF_FYLTOT * pg.np + p] = red[1][0] * dV;
-    pw[PF_FZLTOT * pg.np + p] = red[2][0] * dV;
-    pw[PF_TQX * pg.np + p] = tx;
-    pw[PF_TQY * pg.np + p] = ty;
-    pw[PF_TQZ * pg.np + p] = tz;
-    const double phi = pw[PF_PHI * pg.np + p];
-    pw[PF_TQTHETA * pg.np + p] = (ty * cos(phi)) - (tx * sin(phi));
+  __syncwarp();
+  if (threadIdx.x == 0) {
+    const double phi = b.pf[PF_PHI * np + p];
+    b.pf[PF_TQTHETA * np + p] = (red[4][0] * cos(phi)) - (red[3][0] * sin(phi));
   }
 }
 
-template <typename T>
-void launch_ibm_interp_force(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuffers b, const T *fu, const T *fv,
-                             const T *fw, double dt, int first) {
-  if (pg.np == 0) return;
-  k_ibm_interp_force<T><<<pg.np, 256, 0, s>>>(g, pg, b, fu, fv, fw, 1. / dt, first);
+void launch_ibm_stencil(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuffers b) {
+  k_ibm_stencil<<<ibm_blocks(pg) / 3, IB_T, 0, s>>>(g, pg, b);
 }
-template void launch_ibm_interp_force<double>(cudaStream_t, const Geo &, const PartGeo &, IbmBuffers, const double *,
-                                              const double *, const double *, double, int);
+
+void launch_ibm_interp_force(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuffers b, const double *fu,
+                             const double *fv, const double *fw, double dt, int first) {
+  k_ibm_interp_force<<<ibm_blocks(pg), IB_T, 0, s>>>(g, pg, b, fu, fv, fw, 1. / dt, first);
+}
+void launch_ibm_force_torque(cudaStream_t s, const PartGeo &pg, IbmBuffers b) {
+  k_ibm_force_torque<<<pg.np, 128, 0, s>>>(pg, b);
+}
 
 // lagr2eulr increment: spread dF = (U_l - u~_l)/dt with the terms of
-// interp_spread.f90:329-355, F*coeff0*phix*phiy*phiz, the (j,k) factor
-// formed once per row of three taps
-template <typename T>
-__global__ void __launch_bounds__(256) k_ibm_spread(Geo g, PartGeo pg, IbmBuffers b, T *__restrict__ fu,
-                                                    T *__restrict__ fv, T *__restrict__ fw, double dti,
-                                                    double coeff0_, double dt) {
-  const int n = pg.np * pg.nl;  // < 2^31 points (checked at create)
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    const int p = t / pg.nl, l = t - p * pg.nl;
-    if (l >= b.nla[p]) continue;
-    const PointStencil s = b.st[t];
+// interp_spread.f90:329-355, F*coeff0*phix*phiy*phiz, the z and y factors
+// taken in before the row of three taps (41 FP64 instructions and 27 atomic
+// adds a component)
+template <int C>
+__device__ __forceinline__ void spread_points(const Geo &g, const PartGeo &pg, const IbmBuffers &b,
+                                              double *__restrict__ f, double dti, double coeff0_, double dt) {
+  const int n = pg.np * pg.nl;
+  const double *U = C == 0 ? b.ul : (C == 1 ? b.vl : b.wl), *I = C == 0 ? b.dudtl : (C == 1 ? b.dvdtl : b.dwdtl);
+  for (int t = (int)(blockIdx.x / 3) * IB_T + threadIdx.x; t < n; t += (int)(gridDim.x / 3) * IB_T) {
+    const int p = t / pg.nl;
+    if (t - p * pg.nl >= b.nla[p]) continue;
+    const Taps<C> s(g, b, n, t);
     // the particle's own Lagrangian volume when polydisperse
     const double coeff0 = pg.poly ? (pg.pdvl[p] / pg.dVeul) * dt : coeff0_;
-    const double dfx = (b.ul[t] - b.dudtl[t]) * dti;
-    const double dfy = (b.vl[t] - b.dvdtl[t]) * dti;
-    const double dfz = (b.wl[t] - b.dwdtl[t]) * dti;
-    int ix[3], ixh[3], jy[3], jyh[3];
-    for (int m = 0; m < 3; ++m) {
-      ix[m] = wrapm(s.ilows + m - 1, g.I);
-      ixh[m] = wrapm(s.ilow + m - 1, g.I);
-      jy[m] = wrapm(s.jlows + m - 1, g.J);
-      jyh[m] = wrapm(s.jlow + m - 1, g.J);
-    }
+    const double d = (U[t] - I[t]) * dti * coeff0;
+#pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const int kz = zwrap(g, s.klow + k), kzs = zwrap(g, s.klows + k);
+      const double dk = d * s.wz[k];
+#pragma unroll
       for (int j = 0; j < 3; ++j) {
-        const double a = dfx * coeff0 * s.phiyh[j] * s.phizh[k];
-        const double bb = dfy * coeff0 * s.phiy[j] * s.phizh[k];
-        const double cc = dfz * coeff0 * s.phiyh[j] * s.phiz[k];
-        for (int i = 0; i < 3; ++i) {
-          atomicAdd(&fu[fidx(g, ix[i], jyh[j], kz)], (T)(a * s.phix[i]));
-          atomicAdd(&fv[fidx(g, ixh[i], jy[j], kz)], (T)(bb * s.phixh[i]));
-          atomicAdd(&fw[fidx(g, ixh[i], jyh[j], kzs)], (T)(cc * s.phixh[i]));
-        }
+        const double dj = dk * s.wy[j];
+        double *r = f + s.oz[k] + s.oy[j];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) atomicAdd(r + s.ox[i], dj * s.wx[i]);
       }
     }
   }
 }
-
+__global__ void __launch_bounds__(IB_T) k_ibm_spread(Geo g, PartGeo pg, IbmBuffers b, double *__restrict__ fu,
+                                                     double *__restrict__ fv, double *__restrict__ fw, double dti,
+                                                     double coeff0, double dt) {
+  const int c = blockIdx.x % 3;
+  if (c == 0) spread_points<0>(g, pg, b, fu, dti, coeff0, dt);
+  else if (c == 1) spread_points<1>(g, pg, b, fv, dti, coeff0, dt);
+  else spread_points<2>(g, pg, b, fw, dti, coeff0, dt);
+}
+void launch_ibm_spread(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuffers b, double *fu, double *fv,
+                       double *fw, double dt) {
+  const double coeff0 = (pg.dVlagr / pg.dVeul) * dt;
+  k_ibm_spread<<<ibm_blocks(pg), IB_T, 0, s>>>(g, pg, b, fu, fv, fw, 1. / dt, coeff0, dt);
+}
 
 template <typename T>
 __global__ void k_zero_plane(Geo g, T *f, int k) {
@@ -262,17 +286,6 @@ __global__ void k_slip_residual(PartGeo pg, IbmBuffers b, double *out) {
 void launch_slip_residual(cudaStream_t s, const PartGeo &pg, IbmBuffers b, double *out) {
   k_slip_residual<<<1, 256, 0, s>>>(pg, b, out);
 }
-
-template <typename T>
-void launch_ibm_spread(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuffers b, T *fu, T *fv, T *fw, double dt,
-                       int first) {
-  (void)first;
-  if (pg.np == 0) return;
-  const double coeff0 = (pg.dVlagr / pg.dVeul) * dt;
-  k_ibm_spread<T><<<1216, 256, 0, s>>>(g, pg, b, fu, fv, fw, 1. / dt, coeff0, dt);
-}
-template void launch_ibm_spread<double>(cudaStream_t, const Geo &, const PartGeo &, IbmBuffers, double *, double *,
-                                        double *, double, int);
 
 // targets of the slots reserved since the last call: (F_final - F0) * dt, the
 // correction the plain passes 1.. added after pass 0

@@ -88,10 +88,14 @@ template <typename T> int fft_radix_set_smem_limits();
 // rows (y, z) of a particle's box with a recorded x extent; boxes with more
 // rows are read whole
 constexpr int IBM_BOX_ROWS = 1024;
+// fields of IbmBuffers::sw: the weights of three nodes along an axis, of the
+// staggered origin (nearest face) and of the centred one (H)
+enum { SW_X = 0, SW_Y = 3, SW_Z = 6, SW_XH = 9, SW_YH = 12, SW_ZH = 15, SW_N = 18 };
 struct IbmBuffers {
   // per-point arrays [np*nl]
   double *xfp, *yfp, *zfp, *ul, *vl, *wl, *dudtl, *dvdtl, *dwdtl, *fxl, *fyl, *fzl;
-  PointStencil *st;
+  int4 *so;     // plain form: [np*nl] stencil origins (centred i, j, k; staggered ones as packed offsets)
+  double *sw;   // plain form: [18][np*nl] delta weights, SW_* + node
   PointRec *rec;     // mixed form: [np*nl] compact point records (make_cs)
   float *fxs, *fys, *fzs;  // mixed forms: [np*nl] point forces F_l (FP32; fxl.. hold FP64 copies at the boundary)
   float4 *pvh, *pvl;       // mixed forms: [np] particle velocity u, v, w as FP32 pairs hi + lo
@@ -107,14 +111,13 @@ struct IbmBuffers {
   double *psum;      // [np*9] mixed form: per-component force and lever-arm sums
   float *rsum;       // [np*3] mixed form: per-component sums of the first-pass slip (U - u~)^2
 };
-template <typename T>
 void launch_ibm_stencil(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuffers b);
-template <typename T>
-void launch_ibm_interp_force(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuffers b, const T *fu,
-                             const T *fv, const T *fw, double dt, int first);
-template <typename T>
-void launch_ibm_spread(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuffers b, T *fu, T *fv, T *fw,
-                       double dt, int first);
+// first 1: the first pass (F = the increment), 0: F accumulates, -1: the interpolation alone
+void launch_ibm_interp_force(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuffers b, const double *fu,
+                             const double *fv, const double *fw, double dt, int first);
+void launch_ibm_force_torque(cudaStream_t s, const PartGeo &pg, IbmBuffers b);
+void launch_ibm_spread(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuffers b, double *fu, double *fv,
+                       double *fw, double dt);
 template <typename T>
 void launch_zero_plane(cudaStream_t s, const Geo &g, T *f, int k);
 void launch_slip_residual(cudaStream_t s, const PartGeo &pg, IbmBuffers b, double *out);
