@@ -564,7 +564,7 @@ int alloc_all(ibm_ctx *c) {
     const int nt = c->pg.ntab;  // entries of each point table (nl, or the sum of the point counts)
     if ((st = dalloc(c, &c->pb.sincos, (size_t)4 * nt))) return st;
     if ((st = dalloc(c, &c->pb.err, 8))) return st;
-    if ((st = dalloc(c, &c->pb.red, (size_t)10 * np))) return st;
+    if ((st = dalloc(c, &c->pb.red, (size_t)(1 + 9 * SI_SLICES) * np))) return st;
     if ((st = dalloc(c, &c->pb.pos4, (size_t)np))) return st;
     const size_t ncell = (size_t)c->pg.ncx * c->pg.ncy * c->pg.ncz;
     if ((st = dalloc(c, &c->pb.cstart, ncell + 1))) return st;
@@ -1142,7 +1142,7 @@ ibm_ctx *ibm_create(const ibm_params *P) {
   int st = alloc_all(c);
   if (st == IBM_OK) st = build_solver_tables(c);
   if (st == IBM_OK && (poisson_set_smem_limits<double>() != 0 || poisson_set_smem_limits<float>() != 0 ||
-                       mlp_set_smem_limits() != 0 || ibm_set_smem_limits(c->pg.box_cap) != 0))
+                       mlp_set_smem_limits() != 0 || sphere_set_smem_limits() != 0 || ibm_set_smem_limits(c->pg.box_cap) != 0))
     st = set_err(c, IBM_E_CUDA, "cudaFuncSetAttribute failed");
   if (st == IBM_OK) st = cuda_err(c, cudaStreamSynchronize(c->stream), "create");
   if (st != IBM_OK) {

@@ -141,6 +141,40 @@ __device__ __forceinline__ float sqrt_apx(float x) {
   asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// FP64 square root and quotient from FP32 seeds by Newton (Heron) steps on the
+// residual.  This GPU issues FP64 at 1/64 of the FP32 rate, so what counts is
+// the number of FP64 instructions: the seed's conversions are done on the bit
+// patterns by the integer pipe, leaving four (sqrt) and five (quotient) FP64
+// instructions, where the CUDA functions take three to five times as many.
+// Two steps take the seed's relative error of 3e-7 to 1e-13 and below 1e-19, so
+// the results are those of the last rounding (at most one ulp off).  Arguments
+// outside the FP32 range take the CUDA operations.
+__device__ __forceinline__ bool fp32_range(double x) {  // positive, normal in FP32, its root and reciprocal too
+  const unsigned h = (unsigned)__double2hiint(x);
+  return h >= 0x38200000u && h < 0x47c00000u;
+}
+__device__ __forceinline__ float d2f_trunc(double x) {
+  return __uint_as_float((((unsigned)__double2hiint(x) - 0x38000000u) << 3) | ((unsigned)__double2loint(x) >> 29));
+}
+__device__ __forceinline__ double f2d_exact(float f) {  // positive normal
+  const unsigned b = __float_as_uint(f);
+  return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+}
+__device__ __forceinline__ double sqrt_newton(double x) {
+  if (!fp32_range(x)) return sqrt(x);
+  const float xf = d2f_trunc(x), yf = rsqrtf(xf);
+  double s = f2d_exact(xf * yf);
+  const double r = f2d_exact(0.5f * yf);
+  s = fma(fma(-s, s, x), r, s);
+  return fma(fma(-s, s, x), r, s);
+}
+__device__ __forceinline__ double div_newton(double n, double d) {  // d > 0
+  if (!fp32_range(d)) return n / d;
+  const double r = f2d_exact(__fdividef(1.f, d2f_trunc(d)));
+  double q = n * r;
+  q = fma(fma(-q, d, n), r, q);
+  return fma(fma(-q, d, n), r, q);
+}
 // FP32 delta weights at three consecutive nodes m = 0, 1, 2 of a point whose
 // signed distance from node 1 is r1 = x_1 - x_point (in cells).  For r1 in
 // (-0.5, 0.5] node 1 takes the inner branch of kernel.f90:7-25 and nodes 0

@@ -25,9 +25,9 @@ namespace ibmk {
 // hang on them, and a thread takes one component of one point: a single sphere
 // (719 points at D = 16 dx) still spreads over 34 SMs.  Blocks take the three
 // components of the same points in turn, so that their weights come from L2.
-//   1000 spheres of 16 dx: stencil 587 -> 238 us, interpolation 427 -> 171,
+//   1000 spheres of 16 dx: stencil 587 -> 202 us, interpolation 427 -> 171,
 //   spreading 276 -> 252 (63 M FP64 atomic adds), force sums (last pass) 34
-//   one sphere: stencil 35 -> 10 us, interpolation 70 -> 8, spreading 19 -> 6
+//   one sphere: stencil 35 -> 9 us, interpolation 70 -> 8, spreading 19 -> 6
 
 // delta weights at three consecutive nodes, r1 the signed distance of node 1.
 // |r1| <= 1/2: node 1 takes the inner branch of kernel.f90:7-25, nodes 0 and 2
@@ -35,7 +35,7 @@ namespace ibmk {
 // clamped at a wall) takes the general form node by node.
 __device__ __forceinline__ void delta3wd(double r1, double *w, long n) {
   if (fabs(r1) <= 0.5) {
-    const double s = sqrt(fma(-3. * r1, r1, 1.));
+    const double s = sqrt_newton(fma(-3. * r1, r1, 1.));
     w[0] = (1. / 6.) * (fma(3., r1, 2.) - s);
     w[n] = (1. / 3.) * (1. + s);
     w[2 * n] = (1. / 6.) * (fma(-3., r1, 2.) - s);

@@ -221,6 +221,8 @@ size_t mlp_norm_scratch();
 int launch_mlp_norm(cudaStream_t s, int n, const float *feat, const float *targ, double *scratch, float *norm);
 
 // particle_kernels.cu
+constexpr int SI_SLICES = 8;  // blocks that share one (particle, component) of the sphere integrals, at most
+int sphere_set_smem_limits();
 struct PartBuffers {
   double *pf;     // [PF_N*np]
   double *cf;     // [CF_N*np*nq]
@@ -232,7 +234,7 @@ struct PartBuffers {
   double *rkp;    // [RK_N*np]
   double *sincos; // [4*nl]: sin(theta), cos(theta), sin(phi), cos(phi)
   int *err;       // [8] error flags ([4]: learned-forcing MMA wait timeout)
-  double *red;    // [10*np]: volume [np], sphere-integral partials [np][3][3]
+  double *red;    // [(1 + 9 SI_SLICES) np]: volume [np], sphere-integral partials [np][slice][3][3]
   float4 *pos4;   // [np] FP32 snapshot positions (w: master flag) for the collision filter
   int *cstart;    // [ncell+1] cell list of the snapshot positions: first item of each cell
   int *cfill;     // [ncell] scatter cursors

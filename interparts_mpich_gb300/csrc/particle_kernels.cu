@@ -8,6 +8,9 @@
 // Compiled without FMA contraction: these are few, sequential-per-particle
 // operations whose roundings are kept equal to the reference so that the
 // integer contact lists (firstc/qmax) come out identical.
+#include <algorithm>
+#include <cmath>
+
 #include "kernels.cuh"
 
 namespace ibmk {
@@ -119,19 +122,14 @@ __device__ __forceinline__ float corner_fraction_f(float radius, float dxm2, flo
 // (p, comp); a thread owns whole i-lines (fixed j, k), so the lever arms ry,
 // rz of the torque are constant along its line and only
 //   S0 = sum f*w,  Sx = sum rx*f*w
-// accumulate per cell (FP64).  w = 1 for cells inside radin or with all
-// corners inside, 0 with all corners outside, else the corner fraction.
-// Classification: FP32 screening of the squared corner distances with a
-// relative margin (1e-5) far above its rounding; in the plain form every
-// cell the screen cannot decide goes to a shared-memory queue that all
-// threads then run through the reference's FP64 tests (full warps for the
-// FP64 work).  The mixed form (GEO32) evaluates the cut cells in FP32.
+// accumulate per cell (double-float).  w = 1 for cells inside radin or with
+// all corners inside, 0 with all corners outside, else the corner fraction,
+// classified and evaluated in FP32 (the mixed forms).
 // Output: b.red[np + (p*3 + comp)*3 + {0,1,2}] = {S0, torque_a, torque_b}
 // without the dVeul factor (k_sphere_final).
-template <typename T, bool GEO32>
-__global__ void __launch_bounds__(256) k_sphere_int(Geo g, PartGeo pg, PartBuffers b, const T *__restrict__ u,
-                                                    const T *__restrict__ v, const T *__restrict__ w) {
-  constexpr int AX = 128, QCAP = 2048;
+__global__ void __launch_bounds__(256) k_sphere_int(Geo g, PartGeo pg, PartBuffers b, const float *__restrict__ u,
+                                                    const float *__restrict__ v, const float *__restrict__ w) {
+  constexpr int AX = 128;
   const int np = pg.np;
   const int p = blockIdx.x, comp = blockIdx.y;
   const int ms = b.mslv[p];
@@ -140,57 +138,39 @@ __global__ void __launch_bounds__(256) k_sphere_int(Geo g, PartGeo pg, PartBuffe
   // is computed by one thread and read from shared memory: FP64 issues at a
   // small fraction of the FP32 rate, and every thread repeating it cost more
   // than the line sums themselves.
-  __shared__ double s_radin2, s_cx, s_cy, s_cz, s_rad, s_rthr;
-  __shared__ float s_thr[7];
+  __shared__ double s_cx, s_cy, s_cz, s_rad;
+  __shared__ float s_thr[3];
   __shared__ int s_box[6];  // ilow, ni, jlow, nj, klow, nk
   if (threadIdx.x == 0) {
     const double rad = p_rad(pg, p), rth = p_rthr(pg, p);  // the particle's own when polydisperse
     const double radin = rad - 2. * g.dx;
-    const double radin2 = radin * radin;
-    s_radin2 = radin2;
     s_rad = rad;
-    s_rthr = rth;
-    // sqrt(d2) >= radius  <=>  d2 >= rthr (rthr: smallest double whose
-    // correctly rounded square root is >= radius)
-    s_thr[0] = (float)(radin2 * (1. - 1e-5));
-    s_thr[1] = (float)(radin2 * (1. + 1e-5));
-    s_thr[2] = (float)(rth * (1. - 1e-5));
-    s_thr[3] = (float)(rth * (1. + 1e-5));
-    s_thr[4] = (float)radin2;
-    s_thr[5] = (float)rth;
-    s_thr[6] = (float)rad;
+    s_thr[0] = (float)(radin * radin);
+    s_thr[1] = (float)rth;
+    s_thr[2] = (float)rad;
   }
   __syncthreads();
   const double radius = s_rad, dx = g.dx, dy = g.dy, dz = g.dz;
-  const double radin2 = s_radin2, rthr = s_rthr;
-  const float radin2_lo = s_thr[0], radin2_hi = s_thr[1], rthr_lo = s_thr[2], rthr_hi = s_thr[3];
-  const float radin2f = s_thr[4], rthrf = s_thr[5], radiusf = s_thr[6];
-  __shared__ double sxm[AX], sxp[AX], srx[AX], sym[AX], syp[AX], sry[AX], szm[AX], szp[AX], srz[AX];
+  const float radin2f = s_thr[0], rthrf = s_thr[1], radiusf = s_thr[2];
   __shared__ float fxm[AX], fxp[AX], fym[AX], fyp[AX], fzm[AX], fzp[AX];
-  // rx, ry, rz as double-float pairs (mixed form)
-  __shared__ float frxh[GEO32 ? AX : 1], frxl[GEO32 ? AX : 1], fryh[GEO32 ? AX : 1], fryl[GEO32 ? AX : 1];
-  __shared__ float frzh[GEO32 ? AX : 1], frzl[GEO32 ? AX : 1];
-  __shared__ int queue[GEO32 ? 1 : QCAP];
-  __shared__ int qn;
+  // rx, ry, rz as double-float pairs
+  __shared__ float frxh[AX], frxl[AX], fryh[AX], fryl[AX], frzh[AX], frzl[AX];
   __shared__ double red[3][256];
-  const T *F = comp == 0 ? u : (comp == 1 ? v : w);
+  const float *F = comp == 0 ? u : (comp == 1 ? v : w);
   const int *nbf = b.nb + (long)p * 9;
-  double a0 = 0., ta = 0., tb = 0.;
-  // mixed form: the same three sums in double-float across the lines
+  // the three sums in double-float across the lines
   float A0h = 0.f, A0l = 0.f, TAh = 0.f, TAl = 0.f, TBh = 0.f, TBl = 0.f;
   // lever arms per component: ta += la * f*w, tb += lb * f*w with
   // comp 0: (rz, -ry), comp 1: (-rz, rx), comp 2: (ry, -rx)
-  // copies nb = 0..8 (x/y images); with periodic z each also at z -+ lz
-  const int nzs = pg.zper ? 3 : 1;
-  for (int nbz = 0; nbz < 9 * nzs; ++nbz) {
-    const int nb = nbz / nzs, zs = nbz - nb * nzs;
+  // copies nb = 0..8 (x/y images)
+  for (int nb = 0; nb < 9; ++nb) {
     if (nb > 0 && nbf[nb] != 1) continue;
     __syncthreads();  // previous copy done with the tables and the box
     if (threadIdx.x == 0) {
       int nbrecv = nb;
       if (nb > 0) { nbrecv = nb + 4; if (nbrecv > 8) nbrecv -= 8; }
       double cx = PF(PF_X), cy = PF(PF_Y);
-      const double cz = PF(PF_Z) + (zs == 1 ? -pg.lz : (zs == 2 ? pg.lz : 0.));
+      const double cz = PF(PF_Z);
       if (nb > 0) copy_shift_sphere(nbrecv, g.lx, g.ly, cx, cy);
       int ilow = fnint((cx - radius) * g.dxi - 2.), ihigh = fnint((cx + radius) * g.dxi + 2.);
       int jlow = fnint((cy - radius) * g.dyi - 2.), jhigh = fnint((cy + radius) * g.dyi + 2.);
@@ -222,180 +202,92 @@ __global__ void __launch_bounds__(256) k_sphere_int(Geo g, PartGeo pg, PartBuffe
         double mn, pl;
         if (comp == 0) { mn = 0. + (i - 0.5) * dx; pl = 0. + (i + 0.5) * dx; }
         else { mn = 0. + (i - 1) * dx; pl = 0. + i * dx; }
-        sxm[t] = (mn - cx) * (mn - cx); sxp[t] = (pl - cx) * (pl - cx);
-        fxm[t] = (float)sxm[t]; fxp[t] = (float)sxp[t];
-        srx[t] = 0. + (i - 0.5) * dx - cx;
-        if constexpr (GEO32) {
-          frxh[t] = (float)srx[t];
-          frxl[t] = (float)(srx[t] - (double)frxh[t]);
-        }
+        fxm[t] = (float)((mn - cx) * (mn - cx));
+        fxp[t] = (float)((pl - cx) * (pl - cx));
+        const double rx = 0. + (i - 0.5) * dx - cx;
+        frxh[t] = (float)rx;
+        frxl[t] = (float)(rx - (double)frxh[t]);
       }
       if (t < nj) {
         const int j = jlow + t;
         double mn, pl;
         if (comp == 1) { mn = 0. + (j - 0.5) * dy; pl = 0. + (j + 0.5) * dy; }
         else { mn = 0. + (j - 1) * dy; pl = 0. + j * dy; }
-        sym[t] = (mn - cy) * (mn - cy); syp[t] = (pl - cy) * (pl - cy);
-        fym[t] = (float)sym[t]; fyp[t] = (float)syp[t];
-        sry[t] = 0. + (j - 0.5) * dy - cy;
-        if constexpr (GEO32) {
-          fryh[t] = (float)sry[t];
-          fryl[t] = (float)(sry[t] - (double)fryh[t]);
-        }
+        fym[t] = (float)((mn - cy) * (mn - cy));
+        fyp[t] = (float)((pl - cy) * (pl - cy));
+        const double ry = 0. + (j - 0.5) * dy - cy;
+        fryh[t] = (float)ry;
+        fryl[t] = (float)(ry - (double)fryh[t]);
       }
       if (t < nk) {
         const int k = klow + t;
         double mn, pl;
         if (comp < 2) { mn = (k - 1) * dz; pl = k * dz; }
         else { mn = (k - 0.5) * dz; pl = (k + 0.5) * dz; }
-        szm[t] = (mn - cz) * (mn - cz); szp[t] = (pl - cz) * (pl - cz);
-        fzm[t] = (float)szm[t]; fzp[t] = (float)szp[t];
-        srz[t] = (k - 0.5) * dz - cz;
-        if constexpr (GEO32) {
-          frzh[t] = (float)srz[t];
-          frzl[t] = (float)(srz[t] - (double)frzh[t]);
-        }
+        fzm[t] = (float)((mn - cz) * (mn - cz));
+        fzp[t] = (float)((pl - cz) * (pl - cz));
+        const double rz = (k - 0.5) * dz - cz;
+        frzh[t] = (float)rz;
+        frzl[t] = (float)(rz - (double)frzh[t]);
       }
     }
-    if (threadIdx.x == 0) qn = 0;
     __syncthreads();
     const int nlines = nj * nk;
     const long row0 = fidx(g, ilow - 1, 0, 0);
-    for (int base = 0; base < nlines; base += blockDim.x) {
-      const int L = base + threadIdx.x;
-      if (L < nlines) {
-        const int tj = L % nj, tk = L / nj;
-        const float yzp = fyp[tj] + fzp[tk];
-        const float ymin = fminf(fym[tj], fyp[tj]) + fminf(fzm[tk], fzp[tk]);
-        const float ymax = fmaxf(fym[tj], fyp[tj]) + fmaxf(fzm[tk], fzp[tk]);
-        const long lo = row0 + fidx(g, 0, jlow + tj - 1, klow + tk);
-        double s0 = 0., sx = 0.;
-        float s0h = 0.f, s0l = 0.f, sxh = 0.f, sxl = 0.f;  // mixed form: double-float line sums
-        for (int ti = 0; ti < ni; ++ti) {
-          const float dxp2f = fxp[ti], dxm2f = fxm[ti];
-          const float dist2f = dxp2f + yzp;
-          const float mind2f = fminf(dxm2f, dxp2f) + ymin;
-          if (GEO32) {
-            if (!(dist2f < radin2f) && mind2f >= rthrf) continue;  // outside
-          } else {
-            if (!(dist2f < radin2_lo) && !(dist2f <= radin2_hi) && mind2f > rthr_hi) continue;
-          }
-          if constexpr (GEO32) {
-            // FP32 velocity times FP32 weight, summed along the line in
-            // double-float (error-free products and sums on the FP32 pipes)
-            const float ff = F ? (float)F[lo + ti] : 1.f;
-            float wgt = 1.f;
-            if (!(dist2f < radin2f)) {
-              const float maxd2f = fmaxf(dxm2f, dxp2f) + ymax;
-              if (!(maxd2f < rthrf))
-                wgt = corner_fraction_f(radiusf, dxm2f, dxp2f, fym[tj], fyp[tj], fzm[tk], fzp[tk]);
-            }
-            float ph = ff, pe = 0.f;
-            if (wgt != 1.f) two_prod(ff, wgt, ph, pe);
-            df_add(s0h, s0l, ph, pe, s0h, s0l);
-            if (comp != 0) {
-              float qh, ql;
-              df_mul(ph, pe, frxh[ti], frxl[ti], qh, ql);
-              df_add(sxh, sxl, qh, ql, sxh, sxl);
-            }
-            continue;
-          }
-          const double f = F ? (double)F[lo + ti] : 1.;
-          double fw;
-          {
-            bool sure = dist2f < radin2_lo;  // surely inside radin
-            if (!sure && dist2f > radin2_hi) {
-              const float maxd2f = fmaxf(dxm2f, dxp2f) + ymax;
-              sure = maxd2f < rthr_lo;  // surely all corners inside
-            }
-            if (!sure) {  // the reference's FP64 test decides
-              const int q = atomicAdd(&qn, 1);
-              if (q < QCAP) {
-                queue[q] = ti | (tj << 8) | (tk << 16);
-                continue;
-              }
-              // queue full: decide here
-              const double dxp2 = sxp[ti], dyp2 = syp[tj], dzp2 = szp[tk];
-              double frac = 1.;
-              if (!(dxp2 + dyp2 + dzp2 < radin2)) {
-                const double dxm2 = sxm[ti], dym2 = sym[tj], dzm2 = szm[tk];
-                const double mind2 = fmin(dxm2, dxp2) + fmin(dym2, dyp2) + fmin(dzm2, dzp2);
-                if (mind2 >= rthr) continue;
-                const double maxd2 = fmax(dxm2, dxp2) + fmax(dym2, dyp2) + fmax(dzm2, dzp2);
-                if (!(maxd2 < rthr)) frac = corner_fraction(radius, dxm2, dxp2, dym2, dyp2, dzm2, dzp2);
-              }
-              fw = f * frac;
-            } else {
-              fw = f;
-            }
-          }
-          s0 += fw;
-          sx = fma(srx[ti], fw, sx);
+    for (int L = blockIdx.z * blockDim.x + threadIdx.x; L < nlines; L += gridDim.z * blockDim.x) {
+      const int tj = L % nj, tk = L / nj;
+      const float yzp = fyp[tj] + fzp[tk];
+      const float ymin = fminf(fym[tj], fyp[tj]) + fminf(fzm[tk], fzp[tk]);
+      const float ymax = fmaxf(fym[tj], fyp[tj]) + fmaxf(fzm[tk], fzp[tk]);
+      const long lo = row0 + fidx(g, 0, jlow + tj - 1, klow + tk);
+      float s0h = 0.f, s0l = 0.f, sxh = 0.f, sxl = 0.f;  // double-float line sums
+      for (int ti = 0; ti < ni; ++ti) {
+        const float dxp2f = fxp[ti], dxm2f = fxm[ti];
+        const float dist2f = dxp2f + yzp;
+        const float mind2f = fminf(dxm2f, dxp2f) + ymin;
+        if (!(dist2f < radin2f) && mind2f >= rthrf) continue;  // outside
+        // FP32 velocity times FP32 weight, summed along the line in
+        // double-float (error-free products and sums on the FP32 pipes)
+        const float ff = F ? (float)F[lo + ti] : 1.f;
+        float wgt = 1.f;
+        if (!(dist2f < radin2f)) {
+          const float maxd2f = fmaxf(dxm2f, dxp2f) + ymax;
+          if (!(maxd2f < rthrf))
+            wgt = corner_fraction_f(radiusf, dxm2f, dxp2f, fym[tj], fyp[tj], fzm[tk], fzp[tk]);
         }
-        if constexpr (GEO32) {
-          // the line sums into the thread's double-float totals (no FP64
-          // per line)
+        float ph = ff, pe = 0.f;
+        if (wgt != 1.f) two_prod(ff, wgt, ph, pe);
+        df_add(s0h, s0l, ph, pe, s0h, s0l);
+        if (comp != 0) {
           float qh, ql;
-          df_add(A0h, A0l, s0h, s0l, A0h, A0l);
-          if (comp == 0) {
-            df_mul(s0h, s0l, frzh[tk], frzl[tk], qh, ql);
-            df_add(TAh, TAl, qh, ql, TAh, TAl);
-            df_mul(s0h, s0l, fryh[tj], fryl[tj], qh, ql);
-            df_add(TBh, TBl, -qh, -ql, TBh, TBl);
-          } else if (comp == 1) {
-            df_mul(s0h, s0l, frzh[tk], frzl[tk], qh, ql);
-            df_add(TAh, TAl, -qh, -ql, TAh, TAl);
-            df_add(TBh, TBl, sxh, sxl, TBh, TBl);
-          } else {
-            df_mul(s0h, s0l, fryh[tj], fryl[tj], qh, ql);
-            df_add(TAh, TAl, qh, ql, TAh, TAl);
-            df_add(TBh, TBl, -sxh, -sxl, TBh, TBl);
-          }
-        } else {
-          const double ry = sry[tj], rz = srz[tk];
-          a0 += s0;
-          if (comp == 0) { ta = fma(rz, s0, ta); tb = fma(-ry, s0, tb); }
-          else if (comp == 1) { ta = fma(-rz, s0, ta); tb += sx; }
-          else { ta = fma(ry, s0, ta); tb -= sx; }
+          df_mul(ph, pe, frxh[ti], frxl[ti], qh, ql);
+          df_add(sxh, sxl, qh, ql, sxh, sxl);
         }
       }
-      if (!GEO32) {
-        __syncthreads();
-        const int nq = min(qn, QCAP);
-        for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-          const int e = queue[q];
-          const int ti = e & 0xff, tj = (e >> 8) & 0xff, tk = e >> 16;
-          const double dxp2 = sxp[ti], dyp2 = syp[tj], dzp2 = szp[tk];
-          double frac = 1.;
-          if (!(dxp2 + dyp2 + dzp2 < radin2)) {
-            const double dxm2 = sxm[ti], dym2 = sym[tj], dzm2 = szm[tk];
-            const double mind2 = fmin(dxm2, dxp2) + fmin(dym2, dyp2) + fmin(dzm2, dzp2);
-            if (mind2 >= rthr) continue;
-            const double maxd2 = fmax(dxm2, dxp2) + fmax(dym2, dyp2) + fmax(dzm2, dzp2);
-            if (!(maxd2 < rthr)) frac = corner_fraction(radius, dxm2, dxp2, dym2, dyp2, dzm2, dzp2);
-          }
-          const double fw = (F ? (double)F[row0 + fidx(g, ti, jlow + tj - 1, klow + tk)] : 1.) * frac;
-          const double rx = srx[ti], ry = sry[tj], rz = srz[tk];
-          a0 += fw;
-          if (comp == 0) { ta = fma(rz, fw, ta); tb = fma(-ry, fw, tb); }
-          else if (comp == 1) { ta = fma(-rz, fw, ta); tb = fma(rx, fw, tb); }
-          else { ta = fma(ry, fw, ta); tb = fma(-rx, fw, tb); }
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) qn = 0;
-        __syncthreads();
+      // the line sums into the thread's double-float totals (no FP64
+      // per line)
+      float qh, ql;
+      df_add(A0h, A0l, s0h, s0l, A0h, A0l);
+      if (comp == 0) {
+        df_mul(s0h, s0l, frzh[tk], frzl[tk], qh, ql);
+        df_add(TAh, TAl, qh, ql, TAh, TAl);
+        df_mul(s0h, s0l, fryh[tj], fryl[tj], qh, ql);
+        df_add(TBh, TBl, -qh, -ql, TBh, TBl);
+      } else if (comp == 1) {
+        df_mul(s0h, s0l, frzh[tk], frzl[tk], qh, ql);
+        df_add(TAh, TAl, -qh, -ql, TAh, TAl);
+        df_add(TBh, TBl, sxh, sxl, TBh, TBl);
+      } else {
+        df_mul(s0h, s0l, fryh[tj], fryl[tj], qh, ql);
+        df_add(TAh, TAl, qh, ql, TAh, TAl);
+        df_add(TBh, TBl, -sxh, -sxl, TBh, TBl);
       }
     }
   }
-  if constexpr (GEO32) {
-    a0 += (double)A0h + (double)A0l;
-    ta += (double)TAh + (double)TAl;
-    tb += (double)TBh + (double)TBl;
-  }
   // block sums: three warps, each over one of the staged partials
-  red[0][threadIdx.x] = a0;
-  red[1][threadIdx.x] = ta;
-  red[2][threadIdx.x] = tb;
+  red[0][threadIdx.x] = (double)A0h + (double)A0l;
+  red[1][threadIdx.x] = (double)TAh + (double)TAl;
+  red[2][threadIdx.x] = (double)TBh + (double)TBl;
   __syncthreads();
   const int wq = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (wq < 3) {
@@ -403,7 +295,246 @@ __global__ void __launch_bounds__(256) k_sphere_int(Geo g, PartGeo pg, PartBuffe
     for (int q = lane; q < (int)blockDim.x; q += 32) x += red[wq][q];
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) x += __shfl_down_sync(0xffffffffu, x, d);
-    if (lane == 0) b.red[np + ((long)p * 3 + comp) * 3 + wq] = x;
+    if (lane == 0) b.red[np + (((long)p * gridDim.z + blockIdx.z) * 3 + comp) * 3 + wq] = x;
+  }
+}
+
+// The plain form of the same sums, FP64.  Bound by FP64 issue, most of it the
+// square roots of the cut cells' corner distances: each corner belongs to up
+// to eight cells, so the signed distances R - |x - c| are formed once per grid
+// node (in the reference's expression, only within a cell diagonal of the
+// surface, compacted into full warps) and a cut cell reads its eight from
+// shared memory.  Classification as in the mixed form, by FP32 screening of
+// the squared corner distances with a relative margin (1e-5) far above its
+// rounding; a cell that the screen leaves open is evaluated, which gives
+// exactly 1 or 0 where all its corners lie on one side.
+// A block takes the planes of slice blockIdx.z of the box, a slab of nodes at a
+// time (ncap doubles of shared memory, small enough for five blocks an SM: the
+// phases of one overlap the others'; a sphere too wide for two node planes
+// forms its corner distances cell by cell).  1000 spheres of 16 dx: 1063 ->
+// 542 us (a warp per row of cells in place of a thread per line: 682); one
+// sphere, 8 slices: 82 -> 35 us.
+constexpr int SI_T = 128, SI_AX = 128, SI_QCAP = 1024, SI_NODES = 16384;
+__global__ void __launch_bounds__(SI_T, 5) k_sphere_int_d(Geo g, PartGeo pg, PartBuffers b, const double *__restrict__ u,
+                                                      const double *__restrict__ v, const double *__restrict__ w,
+                                                      int ncap) {
+  // [ncap] signed distances, then the node queue of ncap / 2 entries
+  extern __shared__ __align__(16) double s_node[];
+  int *nqueue = reinterpret_cast<int *>(s_node + ncap);
+  const int np = pg.np, p = blockIdx.x, comp = blockIdx.y, nsl = gridDim.z;
+  if (b.mslv[p] <= 0) return;
+  __shared__ double s_c[3], s_rad, s_radin2, s_rthr;
+  __shared__ float s_thr[5];
+  __shared__ int s_box[6];  // ilow, ni, jlow, nj, klow, nk
+  __shared__ double sx2[SI_AX + 1], sy2[SI_AX + 1], sz2[SI_AX + 1], srx[SI_AX], sry[SI_AX], srz[SI_AX];
+  __shared__ float fx[SI_AX + 1], fy[SI_AX + 1], fz[SI_AX + 1];
+  __shared__ int queue[SI_QCAP];
+  __shared__ int qn, nn;
+  __shared__ double red[3][SI_T / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    const double rad = p_rad(pg, p), rth = p_rthr(pg, p);  // the particle's own when polydisperse
+    const double radin = rad - 2. * g.dx, diag = 1.001 * sqrt(g.dx * g.dx + g.dy * g.dy + g.dz * g.dz);
+    const double lo = rad > diag ? rad - diag : 0.;
+    s_rad = rad;
+    s_rthr = rth;
+    s_radin2 = radin * radin;
+    s_thr[0] = (float)(s_radin2 * (1. + 1e-5));
+    s_thr[1] = (float)(rth * (1. - 1e-5));
+    s_thr[2] = (float)(rth * (1. + 1e-5));
+    s_thr[3] = (float)(lo * lo * (1. - 1e-5));
+    s_thr[4] = (float)((rad + diag) * (rad + diag) * (1. + 1e-5));
+  }
+  __syncthreads();
+  const double radius = s_rad, radin2 = s_radin2, rthr = s_rthr, dx = g.dx, dy = g.dy, dz = g.dz;
+  const float radin2_hi = s_thr[0], rthr_lo = s_thr[1], rthr_hi = s_thr[2], band_lo = s_thr[3], band_hi = s_thr[4];
+  // below the margin of radin^2 (a radius under two cells: radin2 is of the
+  // wrong side, but so it is in the reference's test)
+  const float radin2_lo = (float)(radin2 * (1. - 1e-5));
+  const double *F = comp == 0 ? u : (comp == 1 ? v : w);
+  const int *nbf = b.nb + (long)p * 9;
+  // ta += la f w, tb += lb f w with comp 0: (rz, -ry), 1: (-rz, rx), 2: (ry, -rx)
+  double a0 = 0., ta = 0., tb = 0.;
+  const int nzs = pg.zper ? 3 : 1;  // periodic z: each copy also at z -+ lz
+  for (int nbz = 0; nbz < 9 * nzs; ++nbz) {
+    const int nb = nbz / nzs, zs = nbz - nb * nzs;
+    if (nb > 0 && nbf[nb] != 1) continue;
+    __syncthreads();  // previous copy done with the tables and the box
+    if (threadIdx.x == 0) {
+      int nbrecv = nb;
+      if (nb > 0) { nbrecv = nb + 4; if (nbrecv > 8) nbrecv -= 8; }
+      double cx = PF(PF_X), cy = PF(PF_Y);
+      const double cz = PF(PF_Z) + (zs == 1 ? -pg.lz : (zs == 2 ? pg.lz : 0.));
+      if (nb > 0) copy_shift_sphere(nbrecv, g.lx, g.ly, cx, cy);
+      const int ilow = max(fnint((cx - radius) * g.dxi - 2.), 1), ihigh = min(fnint((cx + radius) * g.dxi + 2.), g.I);
+      const int jlow = max(fnint((cy - radius) * g.dyi - 2.), 1), jhigh = min(fnint((cy + radius) * g.dyi + 2.), g.J);
+      const int klow = max(fnint((cz - radius) * g.dzi - 2.), 1), khigh = min(fnint((cz + radius) * g.dzi + 2.), g.K);
+      s_c[0] = cx; s_c[1] = cy; s_c[2] = cz;
+      s_box[0] = ilow; s_box[1] = ihigh - ilow + 1;
+      s_box[2] = jlow; s_box[3] = jhigh - jlow + 1;
+      s_box[4] = klow; s_box[5] = khigh - klow + 1;
+    }
+    __syncthreads();
+    const double cx = s_c[0], cy = s_c[1], cz = s_c[2];
+    const int ilow = s_box[0], ni = s_box[1], jlow = s_box[2], nj = s_box[3], klow = s_box[4], nk = s_box[5];
+    if (ni <= 0 || nj <= 0 || nk <= 0) continue;
+    if (ni > SI_AX || nj > SI_AX || nk > SI_AX) {  // sphere wider than the axis tables: flag, skip
+      if (threadIdx.x == 0) atomicExch(&b.err[3], 1);
+      continue;
+    }
+    // squared distances of the node planes and cell-centre offsets, in the
+    // reference's expressions (intgr_over_sphere.f90:335-508); a cell's upper
+    // face and the next one's lower face have the same expression's value
+    for (int t = threadIdx.x; t <= SI_AX; t += blockDim.x) {
+      if (t <= ni) {
+        const int i = ilow + t;
+        const double q = (comp == 0 ? 0. + (i - 0.5) * dx : 0. + (i - 1) * dx) - cx;
+        sx2[t] = q * q;
+        fx[t] = (float)sx2[t];
+        if (t < ni) srx[t] = 0. + (i - 0.5) * dx - cx;
+      }
+      if (t <= nj) {
+        const int j = jlow + t;
+        const double q = (comp == 1 ? 0. + (j - 0.5) * dy : 0. + (j - 1) * dy) - cy;
+        sy2[t] = q * q;
+        fy[t] = (float)sy2[t];
+        if (t < nj) sry[t] = 0. + (j - 0.5) * dy - cy;
+      }
+      if (t <= nk) {
+        const int k = klow + t;
+        const double q = (comp < 2 ? (k - 1) * dz : (k - 0.5) * dz) - cz;
+        sz2[t] = q * q;
+        fz[t] = (float)sz2[t];
+        if (t < nk) srz[t] = (k - 0.5) * dz - cz;
+      }
+    }
+    const int per = (nk + nsl - 1) / nsl, z0 = blockIdx.z * per, z1 = min(nk, z0 + per);
+    const int ex = ni + 1, ep = ex * (nj + 1);  // nodes of a row, of a plane
+    const int ring = ncap / ep;                 // node planes held, in turn
+    const bool nodes = ring >= 2;
+    const int slab = nodes ? ring - 1 : nk;
+    const long row0 = fidx(g, ilow - 1, 0, 0);
+    auto direct = [&](int ti, int tj, int tk) {  // corner fraction without the node table
+      if (sx2[ti + 1] + sy2[tj + 1] + sz2[tk + 1] < radin2) return 1.;
+      const double mind2 = fmin(sx2[ti], sx2[ti + 1]) + fmin(sy2[tj], sy2[tj + 1]) + fmin(sz2[tk], sz2[tk + 1]);
+      if (mind2 >= rthr) return 0.;
+      return corner_fraction(radius, sx2[ti], sx2[ti + 1], sy2[tj], sy2[tj + 1], sz2[tk], sz2[tk + 1]);
+    };
+    int slot0 = 0;  // slot of plane zb (a slab is a plane short of the ring)
+    for (int zb = z0; zb < z1; zb += slab, slot0 = slot0 ? slot0 - 1 : ring - 1) {
+      const int ze = min(z1, zb + slab);  // cell planes zb..ze-1, node planes zb..ze
+      auto node = [&](int ti, int tj, int tk) -> double & {
+        int q = slot0 + tk - zb;
+        if (q >= ring) q -= ring;
+        return s_node[q * ep + tj * ex + ti];
+      };
+      if (threadIdx.x == 0) { qn = 0; nn = 0; }
+      __syncthreads();
+      if (nodes) {
+        // the nodes within a diagonal of the surface, a warp a row (plane zb
+        // is the last slab's uppermost)
+        for (int t0 = 0; t0 < ex; t0 += 32) {
+          const int ti = t0 + lane;
+          const float xf = ti < ex ? fx[ti] : 4.f * band_hi;
+          for (int tk = zb == z0 ? zb : zb + 1; tk <= ze; ++tk) {
+            const float zf = fz[tk];
+            for (int tj = wid; tj <= nj; tj += SI_T / 32) {
+              const float d2 = fy[tj] + zf + xf;
+              const bool near = d2 >= band_lo && d2 <= band_hi;
+              const unsigned m = __ballot_sync(0xffffffffu, near);
+              if (!m) continue;
+              int at = 0;
+              if (lane == 0) at = atomicAdd(&nn, __popc(m));
+              at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+              if (near) {
+                if (at < ncap / 2) nqueue[at] = ti | (tj << 8) | (tk << 16);
+                else node(ti, tj, tk) = radius - sqrt_newton(sx2[ti] + sy2[tj] + sz2[tk]);
+              }
+            }
+          }
+        }
+      }
+      // cells surely inside, a thread a line (fixed j, k: opposite lever arms
+      // rx cancel within its sum, the others come in once); the open ones go
+      // to the queue
+      const int nlines = nj * (ze - zb);
+      for (int L = threadIdx.x; L < nlines; L += SI_T) {
+        const int lk = L / nj, tj = L - lk * nj, tk = zb + lk;
+        const float ymin = fminf(fy[tj], fy[tj + 1]) + fminf(fz[tk], fz[tk + 1]);
+        const float ymax = fmaxf(fy[tj], fy[tj + 1]) + fmaxf(fz[tk], fz[tk + 1]);
+        const float yzp = fy[tj + 1] + fz[tk + 1];
+        const double *f = F ? F + row0 + fidx(g, 0, jlow + tj - 1, klow + tk) : nullptr;
+        double s0 = 0., sx = 0.;
+        float xm, xp = fx[0];
+        for (int ti = 0; ti < ni; ++ti) {
+          xm = xp;
+          xp = fx[ti + 1];
+          const float d2 = xp + yzp;
+          if (!(d2 <= radin2_hi) && fminf(xm, xp) + ymin > rthr_hi) continue;  // outside
+          double fv;
+          if (d2 < radin2_lo || fmaxf(xm, xp) + ymax < rthr_lo) {
+            fv = f ? f[ti] : 1.;
+          } else {
+            const int q = atomicAdd(&qn, 1);
+            if (q < SI_QCAP) {
+              queue[q] = ti | (tj << 8) | (tk << 16) | (d2 <= radin2_hi ? 1 << 24 : 0);
+              continue;
+            }
+            fv = (f ? f[ti] : 1.) * direct(ti, tj, tk);  // queue full
+          }
+          s0 += fv;
+          if (comp != 0) sx = fma(srx[ti], fv, sx);
+        }
+        a0 += s0;
+        if (comp == 0) { ta = fma(srz[tk], s0, ta); tb = fma(-sry[tj], s0, tb); }
+        else if (comp == 1) { ta = fma(-srz[tk], s0, ta); tb += sx; }
+        else { ta = fma(sry[tj], s0, ta); tb -= sx; }
+      }
+      __syncthreads();
+      const int nnode = min(nn, ncap / 2);
+      for (int q = threadIdx.x; q < nnode; q += SI_T) {
+        const int e = nqueue[q], ti = e & 0xff, tj = (e >> 8) & 0xff, tk = e >> 16;
+        node(ti, tj, tk) = radius - sqrt_newton(sx2[ti] + sy2[tj] + sz2[tk]);
+      }
+      __syncthreads();
+      const int nq = min(qn, SI_QCAP);
+      for (int q = threadIdx.x; q < nq; q += SI_T) {
+        const int e = queue[q], ti = e & 0xff, tj = (e >> 8) & 0xff, tk = (e >> 16) & 0xff;
+        const double fv = F ? F[row0 + fidx(g, ti, jlow + tj - 1, klow + tk)] : 1.;
+        double frac;
+        if (!nodes || (e >> 24)) {  // (or within the margin of radin^2)
+          frac = direct(ti, tj, tk);
+        } else {
+          // positive part over magnitude, (S + A) / 2A: S = A inside, -A outside
+          const double *n0 = &node(ti, tj, tk), *n1 = &node(ti, tj, tk + 1);
+          const double c0 = n0[0], c1 = n0[1], c2 = n0[ex], c3 = n0[ex + 1], c4 = n1[0], c5 = n1[1], c6 = n1[ex],
+                       c7 = n1[ex + 1];
+          const double S = ((c0 + c1) + (c2 + c3)) + ((c4 + c5) + (c6 + c7));
+          const double A = ((fabs(c0) + fabs(c1)) + (fabs(c2) + fabs(c3))) + ((fabs(c4) + fabs(c5)) + (fabs(c6) + fabs(c7)));
+          frac = div_newton(0.5 * (S + A), A);
+        }
+        const double fw = fv * frac;
+        const double rx = srx[ti], ry = sry[tj], rz = srz[tk];
+        a0 += fw;
+        if (comp == 0) { ta = fma(rz, fw, ta); tb = fma(-ry, fw, tb); }
+        else if (comp == 1) { ta = fma(-rz, fw, ta); tb = fma(rx, fw, tb); }
+        else { ta = fma(ry, fw, ta); tb = fma(-rx, fw, tb); }
+      }
+      __syncthreads();
+    }
+  }
+  double s3[3] = {a0, ta, tb};
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) s3[q] += __shfl_down_sync(0xffffffffu, s3[q], d);
+    if (lane == 0) red[q][wid] = s3[q];
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    double x = 0.;
+    for (int q = 0; q < SI_T / 32; ++q) x += red[threadIdx.x][q];
+    b.red[np + (((long)p * nsl + blockIdx.z) * 3 + comp) * 3 + threadIdx.x] = x;
   }
 }
 
@@ -411,8 +542,8 @@ __global__ void __launch_bounds__(256) k_sphere_int(Geo g, PartGeo pg, PartBuffe
 __device__ __forceinline__ void snapshot_particle(const PartGeo &pg, PartBuffers &b, int p);
 // snap: also take the collision iteration's snapshot of this particle (the
 // positions and velocities the integrals leave unchanged), saving its launch
-template <typename T>
-__global__ void k_sphere_final(PartGeo pg, PartBuffers b, int type, int snap) {
+// nsl: slices per (particle, component), summed in order
+__global__ void k_sphere_final(PartGeo pg, PartBuffers b, int type, int snap, int nsl) {
   const int np = pg.np;
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= np) return;
@@ -422,7 +553,11 @@ __global__ void k_sphere_final(PartGeo pg, PartBuffers b, int type, int snap) {
   const double dV = pg.dVeul;
   double A[3] = {0, 0, 0}, tq[3] = {0, 0, 0};
   if (ms > 0) {
-    const double *s = b.red + np + (long)p * 9;  // [comp][S0, ta, tb]
+    double s[9];  // [comp][S0, ta, tb]
+    const double *part = b.red + np + (long)p * 9 * nsl;
+    for (int q = 0; q < 9; ++q) s[q] = part[q];
+    for (int z = 1; z < nsl; ++z)
+      for (int q = 0; q < 9; ++q) s[q] += part[9 * z + q];
     for (int c = 0; c < 3; ++c) A[c] = s[3 * c] * dV;
     tq[0] = (s[3 * 1 + 1] + s[3 * 2 + 1]) * dV;
     tq[1] = (s[3 * 0 + 1] + s[3 * 2 + 2]) * dV;
@@ -437,13 +572,25 @@ template <typename T>
 void launch_sphere_integrals(cudaStream_t s, const Geo &g, const PartGeo &pg, PartBuffers b, const T *u, const T *v,
                              const T *w, int type, bool snapshot) {
   if (pg.np == 0) return;
-  const dim3 grid(pg.np, 3);
   const bool unit = type == 1;  // volume: integrate w = 1 (F == nullptr)
-  if constexpr (sizeof(T) == 4)
-    k_sphere_int<T, true><<<grid, 256, 0, s>>>(g, pg, b, unit ? nullptr : u, unit ? nullptr : v, unit ? nullptr : w);
-  else
-    k_sphere_int<T, false><<<grid, 256, 0, s>>>(g, pg, b, unit ? nullptr : u, unit ? nullptr : v, unit ? nullptr : w);
-  k_sphere_final<T><<<(pg.np + 127) / 128, 128, 0, s>>>(pg, b, type, snapshot ? 1 : 0);
+  u = unit ? nullptr : u; v = unit ? nullptr : v; w = unit ? nullptr : w;
+  // few particles: several blocks share a (particle, component)
+  const int nsl = std::max(1, std::min(SI_SLICES, 304 / (3 * pg.np)));
+  const dim3 grid(pg.np, 3, nsl);
+  if constexpr (sizeof(T) == 4) {
+    k_sphere_int<<<grid, 256, 0, s>>>(g, pg, b, u, v, w);
+  } else {
+    // nodes of the largest sphere's box: a slab of up to 24 KB (five blocks an
+    // SM), two planes at least (up to 128 KB)
+    const long ep = (long)(std::ceil(2. * pg.rmax * g.dxi) + 7.) * (long)(std::ceil(2. * pg.rmax * g.dyi) + 7.);
+    const int ncap = (int)(2 * ep <= 3072 ? 3072 : (2 * ep <= SI_NODES ? 2 * ep : 0));
+    k_sphere_int_d<<<grid, SI_T, (size_t)ncap * (sizeof(double) + 2), s>>>(g, pg, b, u, v, w, ncap);
+  }
+  k_sphere_final<<<(pg.np + 127) / 128, 128, 0, s>>>(pg, b, type, snapshot ? 1 : 0, nsl);
+}
+int sphere_set_smem_limits() {
+  return cudaFuncSetAttribute(k_sphere_int_d, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              SI_NODES * (int)(sizeof(double) + 2)) == cudaSuccess ? 0 : -1;
 }
 template void launch_sphere_integrals<double>(cudaStream_t, const Geo &, const PartGeo &, PartBuffers,
                                               const double *, const double *, const double *, int, bool);

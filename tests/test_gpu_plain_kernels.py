@@ -85,3 +85,31 @@ def test_projection_divergence(gpu_lib, grid):
     s.rk(1, 1e-3)
     s.project(1, 1e-3)
     assert s.chkdiv()[1] < 1e-11
+
+
+# radius in cells, particles, grid: below two cells (the reference's inner
+# test reaches past the surface), one sphere shared by several blocks, a box
+# of one slab, of several, of node planes too large for shared memory, and
+# cells of unequal sides
+@pytest.mark.parametrize("r,n,grid,aspect", [(0.8, 3, (24, 24, 12), 1.0), (1.6, 5, (24, 24, 24), 1.0),
+                                             (8.0, 1, (32, 32, 32), 1.0), (8.0, 40, (96, 96, 96), 1.0),
+                                             (14.0, 4, (72, 72, 48), 1.0), (24.0, 2, (108, 54, 64), 1.0),
+                                             (47.0, 1, (128, 108, 104), 1.0), (6.0, 7, (48, 64, 32), 1.7)])
+def test_sphere_integrals(gpu_lib, r, n, grid, aspect):
+    nx, ny, nz = grid
+    h = 1.0 / 64
+    lx, ly, lz = nx * h, ny * h * aspect, nz * h / aspect
+    rng = np.random.default_rng(3)
+    rad = r * h
+    # anywhere in x and y (periodic images), clear of the walls in z
+    c = np.stack([rng.uniform(0, lx, n), rng.uniform(0, ly, n), rng.uniform(rad, lz - rad, n)], 1)
+    case = Case(name="spheres", itot=nx, jtot=ny, ktot=nz, lx=lx, ly=ly, lz=lz, visc=1e-2, radius=rad, np=n, centres=c)
+    fields = _state(case, 11)
+    got = []
+    for s in (IBMSolver(case), OracleSolver(case)):
+        vol = s.setup(fields=fields)
+        p = s.get_particles(lagrangian=False)
+        got.append((vol, np.stack([p.intu, p.intv, p.intw]), np.stack([p.intomx, p.intomy, p.intomz])))
+    assert abs(got[0][0] - got[1][0]) < PLAIN_TOL_CALL * got[1][0]
+    for q in (1, 2):
+        assert rel_l2(got[0][q], got[1][q]) < PLAIN_TOL_CALL
