@@ -562,10 +562,10 @@ int alloc_all(ibm_ctx *c) {
     if ((st = dalloc(c, &c->pb.mslv, np))) return st;
     if ((st = dalloc(c, &c->pb.rkp, (size_t)RK_N * np))) return st;
     const int nt = c->pg.ntab;  // entries of each point table (nl, or the sum of the point counts)
-    if ((st = dalloc(c, &c->pb.sincos, (size_t)4 * nt))) return st;
+    if ((st = dalloc(c, &c->pb.off, (size_t)3 * nt))) return st;
     if ((st = dalloc(c, &c->pb.err, 8))) return st;
     if ((st = dalloc(c, &c->pb.red, (size_t)(1 + 9 * SI_SLICES) * np))) return st;
-    if ((st = dalloc(c, &c->pb.pos4, (size_t)np))) return st;
+    if ((st = dalloc(c, &c->pb.pos4, (size_t)2 * np))) return st;
     const size_t ncell = (size_t)c->pg.ncx * c->pg.ncy * c->pg.ncz;
     if ((st = dalloc(c, &c->pb.cstart, ncell + 1))) return st;
     if ((st = dalloc(c, &c->pb.cfill, ncell))) return st;
@@ -574,14 +574,21 @@ int alloc_all(ibm_ctx *c) {
     if ((st = dalloc(c, &c->ib.diag, 8))) return st;
     c->ib.pf = c->pb.pf;
     c->ib.err = c->pb.err;
-    std::vector<double> sc((size_t)4 * nt);
-    for (int l = 0; l < nt; ++l) {
-      sc[l] = std::sin(c->thetarc[l]);
-      sc[nt + l] = std::cos(c->thetarc[l]);
-      sc[2 * nt + l] = std::sin(c->phirc[l]);
-      sc[3 * nt + l] = std::cos(c->phirc[l]);
+    // offsets radfp*st*cp, radfp*st*sp, radfp*ct of the force points (products
+    // rounded one by one, as coordsfp.f90:44-79 forms them)
+    std::vector<double> off((size_t)3 * nt);
+    for (int p = 0, l = 0; l < nt; ++p) {
+      const int n = c->pg.poly ? c->pnl_h[p] : nt;
+      const double radfp = c->pg.poly ? c->pradfp_h[p] : c->pg.radfp;
+      for (int e = 0; e < n; ++e, ++l) {
+        const double rst = radfp * std::sin(c->thetarc[l]);
+        off[l] = rst * std::cos(c->phirc[l]);
+        off[nt + l] = rst * std::sin(c->phirc[l]);
+        off[2 * (size_t)nt + l] = radfp * std::cos(c->thetarc[l]);
+      }
     }
-    CK(cudaMemcpyAsync(c->pb.sincos, sc.data(), sc.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->pb.off, off.data(), off.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
     if (c->pg.poly) {  // per-sphere sizes on the device
       if ((st = dalloc(c, &c->psize, (size_t)6 * np))) return st;
       if ((st = dalloc(c, &c->pcount, (size_t)2 * np))) return st;
@@ -927,17 +934,15 @@ int project(ibm_ctx *c, int rkiter, double dt) {
 
 int newton_euler(ibm_ctx *c, int rkiter, double dt) {
   if (c->pg.np == 0) return IBM_OK;
-  launch_save_old(c->stream, c->pg, c->pb);
-  LAUNCHED(1);
   probe_mark(c, IBM_PROBE_SPHERE);
-  // the sphere integrals' final kernel also takes the first collision
-  // iteration's snapshot
+  // the sphere integrals' final kernel also saves the last substep's state and
+  // takes the first collision iteration's snapshot
   if (c->mixed) launch_sphere_integrals<float>(c->stream, c->g, c->pg, c->pb, c->u32, c->v32, c->w32, 23, true);
   else launch_sphere_integrals<double>(c->stream, c->g, c->pg, c->pb, c->u, c->v, c->w, 23, true);
   probe_mark(c, IBM_PROBE_SPHERE);
   LAUNCHED(1);
   for (int iter = 0; iter <= 1; ++iter) {
-    c->launches += launch_collide_update(c->stream, c->pg, c->pb, iter, rkiter, dt, iter > 0);
+    c->launches += launch_collide_update(c->stream, c->pg, c->pb, iter, rkiter, dt);
     LAUNCHED(0);
   }
   launch_ne_finalize(c->stream, c->pg, c->pb, c->ib, 0);
@@ -1161,7 +1166,7 @@ int ibm_destroy(ibm_ctx *c) {
                   c->twN, c->twJ, c->scratch, c->dout, c->href, c->ib.xfp, c->ib.yfp, c->ib.zfp, c->ib.ul, c->ib.vl,
                   c->ib.wl, c->ib.dudtl, c->ib.dvdtl, c->ib.dwdtl, c->ib.fxl, c->ib.fyl, c->ib.fzl, c->ib.so, c->ib.sw,
                   c->ib.nla, c->ib.diag, c->pb.pf, c->pb.cf, c->pb.qmax, c->pb.firstc, c->pb.ofirstc, c->pb.nb,
-                  c->pb.mslv, c->pb.rkp, c->pb.sincos, c->pb.err, c->pb.red, c->pb.pos4, c->pb.cstart, c->pb.cfill, c->pb.citem, c->pb.ccell, c->ru32, c->rv32, c->rw32, c->fu32,
+                  c->pb.mslv, c->pb.rkp, c->pb.off, c->pb.err, c->pb.red, c->pb.pos4, c->pb.cstart, c->pb.cfill, c->pb.citem, c->pb.ccell, c->ru32, c->rv32, c->rw32, c->fu32,
                   c->fv32, c->fw32, c->phi32, c->phi32b, c->spec32, c->twM32, c->twN32, c->twJ32, c->ib.rec, c->ib.pref, c->ib.pcen, c->ib.fxs, c->ib.fys, c->ib.fzs, c->ib.pvh, c->ib.pvl, c->ib.slip, c->ib.bgeo, c->ib.rowm, c->u32, c->v32,
                   c->w32, c->p32, c->plo32, c->thomas_df, c->ib.psum, c->ib.rsum, c->noise_y, c->noise_par, c->ph.G, c->ph.W0, c->ph.W1, c->stat_part,
                   c->cfield, c->cnext, c->crk, c->ferr, c->psize, c->pcount};

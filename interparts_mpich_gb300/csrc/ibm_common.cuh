@@ -28,8 +28,9 @@ enum PField {
   PF_OX, PF_OY, PF_OZ, PF_OTHETA, PF_OPHI, PF_OU, PF_OV, PF_OW, PF_OOMX, PF_OOMY, PF_OOMZ, PF_OOMTHETA,
   PF_OINTU, PF_OINTV, PF_OINTW, PF_OINTOMX, PF_OINTOMY, PF_OINTOMZ,
   PF_OCOLFX, PF_OCOLFY, PF_OCOLFZ, PF_OCOLTX, PF_OCOLTY, PF_OCOLTZ,
-  // snapshot of the collision pass (anb(:,0)): x,y,z,u,v,w,omx,omy,omz
-  PF_SX, PF_SY, PF_SZ, PF_SU, PF_SV, PF_SW, PF_SOMX, PF_SOMY, PF_SOMZ,
+  // snapshots of the collision pass (anb(:,0)), x,y,z,u,v,w,omx,omy,omz, of
+  // both iterations in turn
+  PF_SX, PF_S_LAST = PF_SX + 2 * 9 - 1,
   PF_N
 };
 // contact arrays: current and old
@@ -101,7 +102,6 @@ struct PartGeo {
 
 // per-sphere sizes: the particle's own when polydisperse, else the scalars
 __device__ __forceinline__ double p_rad(const PartGeo &pg, int p) { return pg.poly ? pg.prad[p] : pg.radius; }
-__device__ __forceinline__ double p_radfp(const PartGeo &pg, int p) { return pg.poly ? pg.pradfp[p] : pg.radfp; }
 __device__ __forceinline__ double p_dvl(const PartGeo &pg, int p) { return pg.poly ? pg.pdvl[p] : pg.dVlagr; }
 __device__ __forceinline__ double p_vol(const PartGeo &pg, int p) { return pg.poly ? pg.pvol[p] : pg.volp; }
 __device__ __forceinline__ double p_mi(const PartGeo &pg, int p) { return pg.poly ? pg.pmi[p] : pg.mominert; }

@@ -232,24 +232,22 @@ struct PartBuffers {
   int *nb;        // [np*9]
   int *mslv;      // [np]
   double *rkp;    // [RK_N*np]
-  double *sincos; // [4*nl]: sin(theta), cos(theta), sin(phi), cos(phi)
+  double *off;    // [3*ntab]: force-point offsets from the centre, x, y, z
   int *err;       // [8] error flags ([4]: learned-forcing MMA wait timeout)
   double *red;    // [(1 + 9 SI_SLICES) np]: volume [np], sphere-integral partials [np][slice][3][3]
-  float4 *pos4;   // [np] FP32 snapshot positions (w: master flag) for the collision filter
+  float4 *pos4;   // [2][np] FP32 positions (w: master flag) of both iterations' snapshots, for the collision filter
   int *cstart;    // [ncell+1] cell list of the snapshot positions: first item of each cell
   int *cfill;     // [ncell] scatter cursors
   int *citem;     // [np] particle indices by cell, ascending within a cell
   int *ccell;     // [np] cell of each particle
 };
+// substep: also save the last substep's state and take the first collision
+// iteration's snapshot
 template <typename T>
 void launch_sphere_integrals(cudaStream_t s, const Geo &g, const PartGeo &pg, PartBuffers b, const T *u, const T *v,
-                             const T *w, int type, bool snapshot = false);
-void launch_save_old(cudaStream_t s, const PartGeo &pg, PartBuffers b);
-// snapshot: take the iteration's snapshot first (false when the sphere
-// integrals' final kernel took it)
+                             const T *w, int type, bool substep = false);
 // returns the number of kernels launched
-int launch_collide_update(cudaStream_t s, const PartGeo &pg, PartBuffers b, int iter, int rkiter, double dt,
-                          bool snapshot = true);
+int launch_collide_update(cudaStream_t s, const PartGeo &pg, PartBuffers b, int iter, int rkiter, double dt);
 void launch_ne_finalize(cudaStream_t s, const PartGeo &pg, PartBuffers b, IbmBuffers ib, int init_flags);
 
 

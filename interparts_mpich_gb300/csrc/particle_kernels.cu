@@ -19,33 +19,6 @@ namespace ibmk {
 #define CFA(f, q) b.cf[((long)(f) * np + p) * nq + (q)]
 
 // ---------------------------------------------------------------------------
-// new -> old (intgr_nwtn_eulr.f90:77-118)
-// ---------------------------------------------------------------------------
-__global__ void k_save_old(PartGeo pg, PartBuffers b) {
-  // one element per thread: the scalar fields x..coltz and the contact
-  // fields dx..dwt of every master particle into their "old" copies
-  const int np = pg.np, nq = pg.nq;
-  const long nps = (long)(PF_COLTZ - PF_X + 1) * np;
-  const long ncf = (long)(CF_DWT - CF_DX + 1) * np * nq;
-  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < nps + ncf; e += (long)gridDim.x * blockDim.x) {
-    if (e < nps) {
-      const int f = PF_X + (int)(e / np), p = (int)(e % np);
-      if (b.mslv[p] > 0) b.pf[(long)(f + (PF_OX - PF_X)) * np + p] = b.pf[(long)f * np + p];
-    } else {
-      const long r = e - nps;
-      const int f = CF_DX + (int)(r / ((long)np * nq));
-      const long pq = r % ((long)np * nq);
-      const int p = (int)(pq / nq);
-      if (b.mslv[p] > 0) b.cf[(long)(f + (CF_ODX - CF_DX)) * np * nq + pq] = b.cf[(long)f * np * nq + pq];
-    }
-  }
-}
-void launch_save_old(cudaStream_t s, const PartGeo &pg, PartBuffers b) {
-  if (pg.np == 0) return;
-  k_save_old<<<304, 256, 0, s>>>(pg, b);
-}
-
-// ---------------------------------------------------------------------------
 // intgr_over_sphere.  One block per particle; the self-neighbour copies of a
 // particle near the periodic edges integrate the wrapped part of the box
 // (intgr_over_sphere.f90:84-112 and :298-313).  type 1 = volume, type 2 =
@@ -538,39 +511,52 @@ __global__ void __launch_bounds__(SI_T, 5) k_sphere_int_d(Geo g, PartGeo pg, Par
   }
 }
 
-// unit field for the volume sums (type 1)
-__device__ __forceinline__ void snapshot_particle(const PartGeo &pg, PartBuffers &b, int p);
-// snap: also take the collision iteration's snapshot of this particle (the
-// positions and velocities the integrals leave unchanged), saving its launch
-// nsl: slices per (particle, component), summed in order
-__global__ void k_sphere_final(PartGeo pg, PartBuffers b, int type, int snap, int nsl) {
-  const int np = pg.np;
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+// Totals of the sphere integrals, a warp per particle; nsl: slices per
+// (particle, component), summed in order.  With substep set it is the step
+// into Newton-Euler as well: the state of the last substep is saved (new ->
+// old, intgr_nwtn_eulr.f90:77-118; the integrals are the only part of it that
+// changes before the collision pass) and the first collision iteration's
+// snapshot taken, two launches fewer.
+__device__ __forceinline__ void snapshot_particle(const PartGeo &pg, PartBuffers &b, int p, int iter, int lane);
+__global__ void __launch_bounds__(128) k_sphere_final(PartGeo pg, PartBuffers b, int type, int substep, int nsl) {
+  const int np = pg.np, nq = pg.nq;
+  const int p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (p >= np) return;
-  if (snap) snapshot_particle(pg, b, p);
   const int ms = b.mslv[p];
+  if (substep) {
+    if (ms > 0) {
+      for (int f = PF_X + lane; f <= PF_COLTZ; f += 32) PF(f + (PF_OX - PF_X)) = PF(f);
+      for (int e = lane; e < (CF_DWT - CF_DX + 1) * nq; e += 32) {
+        const int f = CF_DX + e / nq, q = e % nq;
+        CFA(f + (CF_ODX - CF_DX), q) = CFA(f, q);
+      }
+    }
+    snapshot_particle(pg, b, p, 0, lane);
+    __syncwarp();
+  }
   if (ms == 0) return;
   const double dV = pg.dVeul;
-  double A[3] = {0, 0, 0}, tq[3] = {0, 0, 0};
-  if (ms > 0) {
-    double s[9];  // [comp][S0, ta, tb]
-    const double *part = b.red + np + (long)p * 9 * nsl;
-    for (int q = 0; q < 9; ++q) s[q] = part[q];
-    for (int z = 1; z < nsl; ++z)
-      for (int q = 0; q < 9; ++q) s[q] += part[9 * z + q];
-    for (int c = 0; c < 3; ++c) A[c] = s[3 * c] * dV;
-    tq[0] = (s[3 * 1 + 1] + s[3 * 2 + 1]) * dV;
-    tq[1] = (s[3 * 0 + 1] + s[3 * 2 + 2]) * dV;
-    tq[2] = (s[3 * 0 + 2] + s[3 * 1 + 2]) * dV;
+  double s = 0.;  // lane 3 c + q: quantity q = S0, ta, tb of component c
+  if (ms > 0 && lane < 9) {
+    const double *part = b.red + np + (long)p * 9 * nsl + lane;
+    s = part[0];
+    for (int z = 1; z < nsl; ++z) s += part[9 * z];
   }
-  if (type == 1) b.red[p] = A[0];  // volume of the u-cells (intgr_over_sphere.f90:607-622)
-  if (type == 1 || type == 2 || type == 23) { PF(PF_INTU) = A[0]; PF(PF_INTV) = A[1]; PF(PF_INTW) = A[2]; }
-  if (type == 3 || type == 23) { PF(PF_INTOMX) = tq[0]; PF(PF_INTOMY) = tq[1]; PF(PF_INTOMZ) = tq[2]; }
+  // lanes 0..2: the linear integral of component c and the torque component c
+  const int c = lane < 3 ? lane : 0;
+  const double A = __shfl_sync(0xffffffffu, s, 3 * c);
+  // torques: (1, ta) + (2, ta), (0, ta) + (2, tb), (0, tb) + (1, tb)
+  const double ta = __shfl_sync(0xffffffffu, s, c == 0 ? 4 : (c == 1 ? 1 : 2));
+  const double tb = __shfl_sync(0xffffffffu, s, c == 0 ? 7 : (c == 1 ? 8 : 5));
+  if (lane >= 3) return;
+  if (type == 1 && lane == 0) b.red[p] = A * dV;  // volume of the u-cells (intgr_over_sphere.f90:607-622)
+  if (type == 1 || type == 2 || type == 23) PF(PF_INTU + c) = A * dV;
+  if (type == 3 || type == 23) PF(PF_INTOMX + c) = (ta + tb) * dV;
 }
 
 template <typename T>
 void launch_sphere_integrals(cudaStream_t s, const Geo &g, const PartGeo &pg, PartBuffers b, const T *u, const T *v,
-                             const T *w, int type, bool snapshot) {
+                             const T *w, int type, bool substep) {
   if (pg.np == 0) return;
   const bool unit = type == 1;  // volume: integrate w = 1 (F == nullptr)
   u = unit ? nullptr : u; v = unit ? nullptr : v; w = unit ? nullptr : w;
@@ -586,7 +572,7 @@ void launch_sphere_integrals(cudaStream_t s, const Geo &g, const PartGeo &pg, Pa
     const int ncap = (int)(2 * ep <= 3072 ? 3072 : (2 * ep <= SI_NODES ? 2 * ep : 0));
     k_sphere_int_d<<<grid, SI_T, (size_t)ncap * (sizeof(double) + 2), s>>>(g, pg, b, u, v, w, ncap);
   }
-  k_sphere_final<<<(pg.np + 127) / 128, 128, 0, s>>>(pg, b, type, snapshot ? 1 : 0, nsl);
+  k_sphere_final<<<(pg.np + 3) / 4, 128, 0, s>>>(pg, b, type, substep ? 1 : 0, nsl);
 }
 int sphere_set_smem_limits() {
   return cudaFuncSetAttribute(k_sphere_int_d, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -603,7 +589,7 @@ template void launch_sphere_integrals<float>(cudaStream_t, const Geo &, const Pa
 // 430-432); the tangential history is still evolved and stored.
 // ---------------------------------------------------------------------------
 // the scalar normal lubrication force f1 of lubrication (collisions.f90:222-438)
-__device__ double d_lub_f1(const PartGeo &pg, double pu, double pv, double pw, int idq, double nx, double ny,
+__device__ __noinline__ double d_lub_f1(const PartGeo &pg, double pu, double pv, double pw, int idq, double nx, double ny,
                            double nz, double eps, double u_nb, double v_nb, double w_nb, double coeff_f) {
   const double u1a = pu * nx + pv * ny + pw * nz;
   const double u1b = u_nb * nx + v_nb * ny + w_nb * nz;
@@ -659,7 +645,7 @@ struct PState {  // the particle's own state held in registers by the collision 
   double u, v, w, omx, omy, omz, colfx, colfy, colfz;
 };
 
-__device__ void d_collisions(const PartGeo &pg, PartBuffers &b, int p, PState &S, int qq, int idq, double dist,
+__device__ __noinline__ void d_collisions(const PartGeo &pg, PartBuffers &b, int p, PState &S, int qq, int idq, double dist,
                              double deltax, double deltay, double deltaz, double u_nb, double v_nb, double w_nb,
                              double omx_nb, double omy_nb, double omz_nb, double dtsub, double rkab) {
   const int np = pg.np, nq = pg.nq;
@@ -737,7 +723,7 @@ __device__ void d_collisions(const PartGeo &pg, PartBuffers &b, int p, PState &S
   CFA(CF_DUT, q) = dut; CFA(CF_DVT, q) = dvt; CFA(CF_DWT, q) = dwt;
 }
 
-__device__ void d_remove_contact(const PartGeo &pg, PartBuffers &b, int p, int i, int &qlast) {
+__device__ __noinline__ void d_remove_contact(const PartGeo &pg, PartBuffers &b, int p, int i, int &qlast) {
   const int np = pg.np, nq = pg.nq;
   const int a = i - 1, l = qlast - 1;
   int *fc = b.firstc + (long)p * nq, *ofc = b.ofirstc + (long)p * nq;
@@ -786,19 +772,21 @@ __device__ __forceinline__ double minimg(double a0, double a1, double a2) {
 #define COLL_WARPS 4
 #define COLL_CAP 64
 
-// snapshot of the collision iteration (anb(:,0), intgr_nwtn_eulr.f90:153-206)
-__device__ __forceinline__ void snapshot_particle(const PartGeo &pg, PartBuffers &b, int p) {
+// snapshot of collision iteration iter (anb(:,0), intgr_nwtn_eulr.f90:153-206),
+// a warp per particle.  Each iteration has its own, so that one iteration's
+// update can take the next one's while others still read.
+__device__ __forceinline__ void snapshot_particle(const PartGeo &pg, PartBuffers &b, int p, int iter, int lane) {
   const int np = pg.np;
   const bool m = b.mslv[p] > 0;
-  PF(PF_SX) = m ? PF(PF_X) : 0.; PF(PF_SY) = m ? PF(PF_Y) : 0.; PF(PF_SZ) = m ? PF(PF_Z) : 0.;
-  PF(PF_SU) = m ? PF(PF_U) : 0.; PF(PF_SV) = m ? PF(PF_V) : 0.; PF(PF_SW) = m ? PF(PF_W) : 0.;
-  PF(PF_SOMX) = m ? PF(PF_OMX) : 0.; PF(PF_SOMY) = m ? PF(PF_OMY) : 0.; PF(PF_SOMZ) = m ? PF(PF_OMZ) : 0.;
-  // FP32 copy of the snapshot positions for the candidate filter (w: master flag)
-  b.pos4[p] = make_float4((float)PF(PF_SX), (float)PF(PF_SY), (float)PF(PF_SZ), m ? 1.f : 0.f);
-}
-__global__ void k_snapshot(PartGeo pg, PartBuffers b) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < pg.np) snapshot_particle(pg, b, p);
+  double v = 0.;
+  if (lane < 9) {
+    const int f = lane < 3 ? PF_X + lane : (lane < 6 ? PF_U + lane - 3 : PF_OMX + lane - 6);
+    v = m ? PF(f) : 0.;
+    PF(PF_SX + 9 * iter + lane) = v;
+  }
+  // FP32 copy of the positions for the candidate filter (w: master flag)
+  const float x = (float)v, y = __shfl_sync(0xffffffffu, x, 1), z = __shfl_sync(0xffffffffu, x, 2);
+  if (lane == 0) b.pos4[(long)iter * np + p] = make_float4(x, y, z, m ? 1.f : 0.f);
 }
 
 // Uniform cell list of the snapshot positions (one block): cell of every
@@ -813,7 +801,8 @@ __device__ __forceinline__ int coll_cell(const PartGeo &pg, float4 x) {
   cz = min(max(cz, 0), pg.ncz - 1);
   return (cz * pg.ncy + cy) * pg.ncx + cx;
 }
-__global__ void __launch_bounds__(1024) k_cell_build(PartGeo pg, PartBuffers b) {
+__global__ void __launch_bounds__(1024) k_cell_build(PartGeo pg, PartBuffers b, int iter) {
+  b.pos4 += (long)iter * pg.np;
   const int np = pg.np, ncell = pg.ncx * pg.ncy * pg.ncz, tid = threadIdx.x;
   __shared__ int part[1024];
   for (int q = tid; q < ncell; q += 1024) b.cfill[q] = 0;
@@ -867,35 +856,51 @@ __device__ __forceinline__ bool coll_near(float4 q, float pxf, float pyf, float 
   return dxf * dxf + dyf * dyf + dzf * dzf < thr2;
 }
 
-// One warp per particle: a coarse FP32 periodic-distance filter selects the
+// One warp per particle.  A coarse FP32 periodic-distance filter selects the
 // partners that can interact (lubrication range, contact, or listed in
-// firstc), from the 27 cells of the cell list around the particle (or from
-// all particles when the grid is narrower than three cells), in ascending
-// particle order; lane 0 then walks them in the reference (nb, q) order,
-// handles the walls, integrates Newton-Euler and accumulates sumrk3.
+// firstc), in ascending particle order, from the 27 cells of the cell list
+// around the particle or from all particles (few of them, or a grid narrower
+// than three cells).  The lanes evaluate 32 (copy, candidate) pairs at a time;
+// lane 0 then walks those that have an effect in the reference's (nb, q)
+// order for the force sums and the contact bookkeeping, and handles the walls.
+// Newton-Euler and sumrk3 run with a lane per component and accumulator: the
+// kernel's cost is its FP64 instructions (a warp's in about 16 cycles of its
+// SM), and those of one lane cost as much as a warp's.  Each quantity keeps
+// the sequential pass's arithmetic.
+// 1000 spheres: 44.5 -> 20.5 us an iteration, and the cell list (9 us) and
+// snapshot (7 us) kernels beside it gone; one sphere: 26 -> 14.
 __global__ void __launch_bounds__(32 * COLL_WARPS) k_collide_update(PartGeo pg, PartBuffers b, int iter, int rkiter,
-                                                                   double dt) {
+                                                                   double dt, int scan, double3 gterm) {
   __shared__ int cand[COLL_WARPS][COLL_CAP];
-  __shared__ int ncand[COLL_WARPS];
+  __shared__ int ncand[COLL_WARPS], nfar[COLL_WARPS];
   __shared__ int fcs[COLL_WARPS][16];  // the particle's first contact partners (nq <= 15 here)
   const int np = pg.np, nq = pg.nq;
   const int wid = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int p = blockIdx.x * COLL_WARPS + wid;
   if (p >= np) return;
-  if (lane == 0) ncand[wid] = 0;
+  const float4 *pos4 = b.pos4 + (long)iter * np;
+  const int SX = PF_SX + 9 * iter, SU = SX + 3, SOM = SX + 6;  // this iteration's snapshot
+  if (lane == 0) { ncand[wid] = 0; nfar[wid] = 0; }
   const double radius = p_rad(pg, p);
   const int qmax0 = b.qmax[p];
   const int *fc = b.firstc + (long)p * nq;
   if (lane < qmax0 && lane < 16) fcs[wid][lane] = fc[lane];
   __syncwarp();
-  // FP32 filter distance: 2.1 R (polydisperse: 1.05 (R + Rmax), a superset
-  // of every pair's 1.05 (Rp + Rq))
-  const float thr = pg.poly ? 1.05f * (float)(radius + pg.rmax) : 2.1f * (float)radius;
-  const float thr2 = thr * thr;
+  // FP32 filter: a pair interacts below eps = 0.025, within 1.0125 of the sum
+  // of the radii (the equivalent radius is at most half of it); 1.02 leaves
+  // room for the FP32 positions (polydisperse: with Rmax, a superset).  The
+  // list's capacity is held to the wider 1.05.
+  const float rsumf = pg.poly ? (float)(radius + pg.rmax) : 2.f * (float)radius;
+  const float thr2 = (1.02f * rsumf) * (1.02f * rsumf), far2 = (1.05f * rsumf) * (1.05f * rsumf);
   const float lxf = (float)pg.lx, lyf = (float)pg.ly;
-  const float4 pp = b.pos4[p];
+  const float4 pp = pos4[p];
   const float pxf = pp.x, pyf = pp.y, pzf = pp.z;
-  if (pg.ncx >= 3 && pg.ncy >= 3) {
+  auto listed = [&](int id) {
+    for (int i = 0; i < qmax0; ++i)
+      if ((i < 16 ? fcs[wid][i] : fc[i]) == id) return true;
+    return false;
+  };
+  if (!scan) {
     // cell list: lane t < 27 scans neighbouring cell t; partners in firstc
     // beyond the filter distance are added by the lane of their slot; then
     // the list is sorted ascending (as the full scan produces it)
@@ -908,10 +913,13 @@ __global__ void __launch_bounds__(32 * COLL_WARPS) k_collide_update(PartGeo pg, 
         const int c = (z * pg.ncy + y) * pg.ncx + x;
         for (int t = b.cstart[c]; t < b.cstart[c + 1]; ++t) {
           const int q = b.citem[t];
-          const float4 qp = b.pos4[q];
-          if (q != p && qp.w != 0.f && coll_near(qp, pxf, pyf, pzf, lxf, lyf, thr2)) {
+          const float4 qp = pos4[q];
+          if (q == p || qp.w == 0.f || !coll_near(qp, pxf, pyf, pzf, lxf, lyf, far2)) continue;
+          if (coll_near(qp, pxf, pyf, pzf, lxf, lyf, thr2)) {
             const int pos = atomicAdd(&ncand[wid], 1);
             if (pos < COLL_CAP) cand[wid][pos] = q;
+          } else if (!listed(b.mslv[q])) {
+            atomicAdd(&nfar[wid], 1);
           }
         }
       }
@@ -920,7 +928,7 @@ __global__ void __launch_bounds__(32 * COLL_WARPS) k_collide_update(PartGeo pg, 
       const int id = fc[lane];
       if (id >= 1 && id <= np) {
         const int q = id - 1;
-        const float4 qp = b.pos4[q];
+        const float4 qp = pos4[q];
         if (q != p && qp.w != 0.f && b.mslv[q] == id && !coll_near(qp, pxf, pyf, pzf, lxf, lyf, thr2)) {
           const int pos = atomicAdd(&ncand[wid], 1);
           if (pos < COLL_CAP) cand[wid][pos] = q;
@@ -941,40 +949,41 @@ __global__ void __launch_bounds__(32 * COLL_WARPS) k_collide_update(PartGeo pg, 
     if (lane + 32 < n) cand[wid][r1] = v1;
     __syncwarp();
   } else {
-  // candidates in ascending q: within the collision distance or already in
-  // contact; four slices of 32 per round, loads issued together
-  constexpr int SL = 4;
-  for (int base = 0; base < np; base += 32 * SL) {
-    float4 qp[SL];
-    int qms[SL];
+    // candidates in ascending q: within the collision distance or already in
+    // contact; eight slices of 32 per round, loads issued together
+    constexpr int SL = 8;
+    for (int base = 0; base < np; base += 32 * SL) {
+      float4 qp[SL];
 #pragma unroll
-    for (int u = 0; u < SL; ++u) {
-      const int q = base + 32 * u + lane;
-      qp[u] = q < np ? b.pos4[q] : make_float4(0.f, 0.f, 0.f, 0.f);  // w: 1 for masters
-      qms[u] = q < np ? b.mslv[q] : 0;
-    }
+      for (int u = 0; u < SL; ++u) {
+        const int q = base + 32 * u + lane;
+        qp[u] = q < np ? pos4[q] : make_float4(0.f, 0.f, 0.f, 0.f);  // w: 1 for masters
+      }
 #pragma unroll
-    for (int u = 0; u < SL; ++u) {
-      const int q = base + 32 * u + lane;
-      bool c = false;
-      if (q < np && q != p && qp[u].w != 0.f) {
-        c = coll_near(qp[u], pxf, pyf, pzf, lxf, lyf, thr2);
-        for (int i = 0; i < qmax0 && !c; ++i) c = ((i < 16 ? fcs[wid][i] : fc[i]) == qms[u]);
+      for (int u = 0; u < SL; ++u) {
+        const int q = base + 32 * u + lane;
+        const bool ok = q < np && q != p && qp[u].w != 0.f;
+        bool c = ok && coll_near(qp[u], pxf, pyf, pzf, lxf, lyf, thr2);
+        if (qmax0 > 0 && ok && !c) c = listed(b.mslv[q]);
+        const bool f = ok && !c && coll_near(qp[u], pxf, pyf, pzf, lxf, lyf, far2);
+        const unsigned m = __ballot_sync(0xffffffffu, c), mf = __ballot_sync(0xffffffffu, f);
+        if (!(m | mf)) continue;
+        if (c) {
+          const int pos = ncand[wid] + __popc(m & ((1u << lane) - 1u));
+          if (pos < COLL_CAP) cand[wid][pos] = q;
+        }
+        __syncwarp();
+        if (lane == 0) { ncand[wid] += __popc(m); nfar[wid] += __popc(mf); }
+        __syncwarp();
       }
-      const unsigned m = __ballot_sync(0xffffffffu, c);
-      if (c) {
-        const int pos = ncand[wid] + __popc(m & ((1u << lane) - 1u));
-        if (pos < COLL_CAP) cand[wid][pos] = q;
-      }
-      __syncwarp();
-      if (lane == 0) ncand[wid] += __popc(m);
-      __syncwarp();
     }
-  }
   }
   int nc = ncand[wid];
-  if (nc > COLL_CAP) { if (lane == 0) atomicExch(&b.err[0], 1); nc = COLL_CAP; }
-  if (b.mslv[p] <= 0) return;
+  if (nc + nfar[wid] > COLL_CAP) { if (lane == 0) atomicExch(&b.err[0], 1); nc = min(nc, COLL_CAP); }
+  if (b.mslv[p] <= 0) {
+    if (iter == 0) snapshot_particle(pg, b, p, 1, lane);
+    return;
+  }
   const int idp = b.mslv[p];
   const double rkab = pg.rkab[rkiter - 1];
   const int itermax = 1;
@@ -982,51 +991,53 @@ __global__ void __launch_bounds__(32 * COLL_WARPS) k_collide_update(PartGeo pg, 
   S.u = PF(PF_U); S.v = PF(PF_V); S.w = PF(PF_W); S.omx = PF(PF_OMX); S.omy = PF(PF_OMY); S.omz = PF(PF_OMZ);
   S.colfx = 0.; S.colfy = 0.; S.colfz = 0.;
   const double px = PF(PF_X), py = PF(PF_Y), pz = PF(PF_Z);
-  int qlast = b.qmax[p];
+  int qlast = qmax0;
   int *fcw = b.firstc + (long)p * nq, *ofcw = b.ofirstc + (long)p * nq;
-  // (i) other particles, nb-outer / q-inner as in the reference.  The 32
-  // lanes evaluate the geometry and the lubrication force f1 of 32 (copy,
-  // candidate) pairs at a time; lane 0 then takes them in the reference's
-  // order for the force sums, the contact bookkeeping and the collision
-  // forces, with the same arithmetic as a sequential pass.
+  // (i) other particles, nb-outer / q-inner as in the reference.  Pairs out of
+  // lubrication and contact range (with room for the copies' roundings) and
+  // not listed have no effect and are passed over.
   const int npair = pg.nb_copies * nc;
   for (int base = 0; base < npair; base += 32) {
     const int k = base + lane;
-    int q = 0, idq = 0, use = 0, lub = 0;
+    int q = 0, idq = 0, lub = 0;
+    bool act = false;
     double dist = 0., deltax = 0., deltay = 0., deltaz = 0., nx = 0., ny = 0., nz = 0., f1 = 0.;
     double qu = 0., qv = 0., qw = 0.;
     if (k < npair) {
       const int nb = k / nc, ci = k - nb * nc;
       q = cand[wid][ci];
-      use = idp != b.mslv[q] && b.mslv[q] > 0;
-      if (use) {
-        idq = b.mslv[q];
-        double qx = b.pf[(long)PF_SX * np + q], qy = b.pf[(long)PF_SY * np + q];
-        const double qz = b.pf[(long)PF_SZ * np + q];
+      idq = b.mslv[q];
+      if (idp != idq && idq > 0) {
+        double qx = b.pf[(long)SX * np + q], qy = b.pf[(long)(SX + 1) * np + q];
+        const double qz = b.pf[(long)(SX + 2) * np + q];
         copy_shift_coll(nb, pg.lx, pg.ly, qx, qy);
         deltaz = qz - pz;
         deltax = minimg(qx - px, qx - pg.lx - px, qx + pg.lx - px);
         deltay = minimg(qy - py, qy - pg.ly - py, qy + pg.ly - py);
         dist = sqrt(deltax * deltax + deltay * deltay + deltaz * deltaz);
-        nx = deltax / dist; ny = deltay / dist; nz = deltaz / dist;
         // polydisperse: contact at the sum of the radii, eps and the
         // lubrication prefactor with the equivalent radius (pair_consts)
         const double rqq = p_rad(pg, q);
         const double rsum = pg.poly ? radius + rqq : 2. * radius;
-        const double re = pg.poly ? 2. * radius * rqq / (radius + rqq) : radius;
-        const double eps = (dist - rsum) / re;
-        qu = b.pf[(long)PF_SU * np + q]; qv = b.pf[(long)PF_SV * np + q]; qw = b.pf[(long)PF_SW * np + q];
-        if ((eps < 0.025) && (eps > 0.)) {
-          lub = 1;
-          f1 = d_lub_f1(pg, S.u, S.v, S.w, idq, nx, ny, nz, eps, qu, qv, qw,
-                        pg.poly ? 6. * IBM_PI * pg.visc * re : pg.coeff_f);
+        // (the shifted copies' minimum image can miss the nearest one, so all
+        // copies of a partner that may touch count: they can end its contact)
+        const float tf = 1.01f * (float)rsum;
+        act = dist < 1.02 * rsum || coll_near(pos4[q], pxf, pyf, pzf, lxf, lyf, tf * tf) || listed(idq);
+        if (act) {
+          nx = deltax / dist; ny = deltay / dist; nz = deltaz / dist;
+          const double re = pg.poly ? 2. * radius * rqq / (radius + rqq) : radius;
+          const double eps = (dist - rsum) / re;
+          qu = b.pf[(long)SU * np + q]; qv = b.pf[(long)(SU + 1) * np + q]; qw = b.pf[(long)(SU + 2) * np + q];
+          if ((eps < 0.025) && (eps > 0.)) {
+            lub = 1;
+            f1 = d_lub_f1(pg, S.u, S.v, S.w, idq, nx, ny, nz, eps, qu, qv, qw,
+                          pg.poly ? 6. * IBM_PI * pg.visc * re : pg.coeff_f);
+          }
         }
       }
     }
-    const int cnt = min(32, npair - base);
-    for (int j = 0; j < cnt; ++j) {
-      const int juse = __shfl_sync(0xffffffffu, use, j);
-      if (!juse) continue;  // uniform across the warp
+    for (unsigned todo = __ballot_sync(0xffffffffu, act); todo; todo &= todo - 1) {
+      const int j = __ffs(todo) - 1;
       const int jq = __shfl_sync(0xffffffffu, q, j), jidq = __shfl_sync(0xffffffffu, idq, j);
       const int jlub = __shfl_sync(0xffffffffu, lub, j);
       const double jdist = __shfl_sync(0xffffffffu, dist, j);
@@ -1050,9 +1061,8 @@ __global__ void __launch_bounds__(32 * COLL_WARPS) k_collide_update(PartGeo pg, 
         if (jidq == fcw[i - 1]) {
           if (jdist < jrsum) {
             qq = i;
-            d_collisions(pg, b, p, S, qq, jidq, jdist, jdx, jdy, jdz, jqu, jqv, jqw,
-                         b.pf[(long)PF_SOMX * np + jq], b.pf[(long)PF_SOMY * np + jq], b.pf[(long)PF_SOMZ * np + jq],
-                         dt, rkab);
+            d_collisions(pg, b, p, S, qq, jidq, jdist, jdx, jdy, jdz, jqu, jqv, jqw, b.pf[(long)SOM * np + jq],
+                         b.pf[(long)(SOM + 1) * np + jq], b.pf[(long)(SOM + 2) * np + jq], dt, rkab);
           } else if (iter == itermax) {
             d_remove_contact(pg, b, p, i, qlast);
           }
@@ -1067,117 +1077,128 @@ __global__ void __launch_bounds__(32 * COLL_WARPS) k_collide_update(PartGeo pg, 
         }
         qq = qlast;
         d_new_contact(pg, b, p, qq);
-        d_collisions(pg, b, p, S, qq, jidq, jdist, jdx, jdy, jdz, jqu, jqv, jqw,
-                     b.pf[(long)PF_SOMX * np + jq], b.pf[(long)PF_SOMY * np + jq], b.pf[(long)PF_SOMZ * np + jq],
-                     dt, rkab);
+        d_collisions(pg, b, p, S, qq, jidq, jdist, jdx, jdy, jdz, jqu, jqv, jqw, b.pf[(long)SOM * np + jq],
+                     b.pf[(long)(SOM + 1) * np + jq], b.pf[(long)(SOM + 2) * np + jq], dt, rkab);
         fcw[qlast - 1] = jidq;
         ofcw[qlast - 1] = jidq;
       }
       b.qmax[p] = qlast;
     }
   }
-  if (lane != 0) return;
-  // (ii) walls (intgr_nwtn_eulr.f90:503-603)
+  // (ii) walls (intgr_nwtn_eulr.f90:503-603), where one lies within the
+  // lubrication range 1.075 R (FP32 screen) or is listed
   const int botw = np + 1, topw = np + 2;
-  const int qm_w = b.qmax[p];
-  for (int qw_ = botw; qw_ <= topw; ++qw_) {
-    const int idq = qw_;
-    if (pg.zper) break;  // periodic z: no walls
-    const double deltax = 0., deltay = 0., deltaz = (qw_ - botw) * pg.lz - pz;
-    const double dist = sqrt(deltax * deltax + deltay * deltay + deltaz * deltaz);
-    const double deltan = radius - dist;
-    const double nx = deltax / dist, ny = deltay / dist, nz = deltaz / dist;
-    int qq = 0;
-    const double eps = -deltan / radius;
-    if ((eps < 0.075) && (eps > 0.))
-      d_lubrication(pg, S.u, S.v, S.w, idq, nx, ny, nz, eps, 0., 0., 0.,
-                    pg.poly ? 6. * IBM_PI * pg.visc * radius : pg.coeff_f, S.colfx, S.colfy, S.colfz);
-    for (int i = 1; i <= qm_w; ++i) {
-      if (idq == fcw[i - 1]) {
-        qq = i;
-        if (dist < radius) {
-          d_collisions(pg, b, p, S, qq, idq, dist, deltax, deltay, deltaz, 0., 0., 0., 0., 0., 0., dt, rkab);
-        } else if (iter == itermax) {
-          d_remove_contact(pg, b, p, i, qlast);
+  const float wallf = 1.08f * (float)radius;
+  if (!pg.zper && (pzf < wallf || (float)pg.lz - pzf < wallf || !isfinite(pzf) || listed(botw) || listed(topw)) &&
+      lane == 0) {
+    const int qm_w = b.qmax[p];
+    for (int qw_ = botw; qw_ <= topw; ++qw_) {
+      const int idq = qw_;
+      const double deltax = 0., deltay = 0., deltaz = (qw_ - botw) * pg.lz - pz;
+      const double dist = sqrt(deltax * deltax + deltay * deltay + deltaz * deltaz);
+      const double deltan = radius - dist;
+      const double nx = deltax / dist, ny = deltay / dist, nz = deltaz / dist;
+      int qq = 0;
+      const double eps = -deltan / radius;
+      if ((eps < 0.075) && (eps > 0.))
+        d_lubrication(pg, S.u, S.v, S.w, idq, nx, ny, nz, eps, 0., 0., 0.,
+                      pg.poly ? 6. * IBM_PI * pg.visc * radius : pg.coeff_f, S.colfx, S.colfy, S.colfz);
+      for (int i = 1; i <= qm_w; ++i) {
+        if (idq == fcw[i - 1]) {
+          qq = i;
+          if (dist < radius) {
+            d_collisions(pg, b, p, S, qq, idq, dist, deltax, deltay, deltaz, 0., 0., 0., 0., 0., 0., dt, rkab);
+          } else if (iter == itermax) {
+            d_remove_contact(pg, b, p, i, qlast);
+          }
         }
       }
-    }
-    if ((qq == 0) && (dist < radius)) {
-      qlast = qlast + 1;
-      if (qlast > nq) { atomicExch(&b.err[1], 1); qlast = nq; continue; }
-      qq = qlast;
-      d_new_contact(pg, b, p, qq);
-      d_collisions(pg, b, p, S, qq, idq, dist, deltax, deltay, deltaz, 0., 0., 0., 0., 0., 0., dt, rkab);
-      fcw[qlast - 1] = idq;
-      ofcw[qlast - 1] = idq;
+      if ((qq == 0) && (dist < radius)) {
+        qlast = qlast + 1;
+        if (qlast > nq) { atomicExch(&b.err[1], 1); qlast = nq; continue; }
+        qq = qlast;
+        d_new_contact(pg, b, p, qq);
+        d_collisions(pg, b, p, S, qq, idq, dist, deltax, deltay, deltaz, 0., 0., 0., 0., 0., 0., dt, rkab);
+        fcw[qlast - 1] = idq;
+        ofcw[qlast - 1] = idq;
+      }
     }
   }
-  b.qmax[p] = qlast;
-  // Newton-Euler (intgr_nwtn_eulr.f90:611-667); colflg is reset to 0 first
-  const double colflgx = 0., colflgy = 0., colflgz = 0.;
+  if (lane == 0) b.qmax[p] = qlast;
+  // Newton-Euler (intgr_nwtn_eulr.f90:611-667): lane c < 3 takes component c
+  // of the translation and of the rotation; colflg is reset to 0 first
+  const int c = lane < 3 ? lane : 0;
+  const double colx = __shfl_sync(0xffffffffu, S.colfx, 0), coly = __shfl_sync(0xffffffffu, S.colfy, 0),
+               colz = __shfl_sync(0xffffffffu, S.colfz, 0);
+  const double colf = c == 0 ? colx : (c == 1 ? coly : colz);
   const double vol = p_vol(pg, p), rr = pg.ratiorho;  // ap%vol, ap%ratiorho (coordsfp.f90:96-102)
   const double vr = vol * rr;
-  const double ou = PF(PF_OU), ov = PF(PF_OV), ow = PF(PF_OW);
-  double nu = ou + (1 - colflgx) * ((-1.) * dt * (PF(PF_FXLTOT)) / vr + (PF(PF_INTU) - PF(PF_OINTU)) / vr) +
-              rkab * dt * pg.gacc[0] * (1. - (1. / rr)) + rkab * 0.5 * dt * (S.colfx + PF(PF_OCOLFX)) / vr;
-  PF(PF_X) = PF(PF_OX) + rkab * 0.5 * dt * (nu + ou);
-  double nv = ov + (1 - colflgy) * ((-1.) * dt * (PF(PF_FYLTOT)) / vr + (PF(PF_INTV) - PF(PF_OINTV)) / vr) +
-              rkab * dt * pg.gacc[1] * (1. - (1. / rr)) + rkab * 0.5 * dt * (S.colfy + PF(PF_OCOLFY)) / vr;
-  PF(PF_Y) = PF(PF_OY) + rkab * 0.5 * dt * (nv + ov);
-  double nw = ow + (1 - colflgz) * ((-1.) * dt * (PF(PF_FZLTOT)) / vr + (PF(PF_INTW) - PF(PF_OINTW)) / vr) +
-              rkab * dt * pg.gacc[2] * (1. - (1. / rr)) + rkab * 0.5 * dt * (S.colfz + PF(PF_OCOLFZ)) / vr;
-  PF(PF_Z) = PF(PF_OZ) + rkab * 0.5 * dt * (nw + ow);
-  PF(PF_U) = nu; PF(PF_V) = nv; PF(PF_W) = nw;
-  PF(PF_COLFX) = S.colfx; PF(PF_COLFY) = S.colfy; PF(PF_COLFZ) = S.colfz;
-  PF(PF_COLTX) = 0.; PF(PF_COLTY) = 0.; PF(PF_COLTZ) = 0.;
-  double omx, omy, omz;
+  const double ou = PF(PF_OU + c);
+  // gterm: rkab dt gacc (1 - 1/ratiorho), formed once on the host
+  const double nu = ou + ((-1.) * dt * (PF(PF_FXLTOT + c)) / vr + (PF(PF_INTU + c) - PF(PF_OINTU + c)) / vr) +
+                    (c == 0 ? gterm.x : (c == 1 ? gterm.y : gterm.z)) + rkab * 0.5 * dt * (colf + PF(PF_OCOLFX + c)) / vr;
+  const double nx = PF(PF_OX + c) + rkab * 0.5 * dt * (nu + ou);
+  double om = 0.;
   if (pg.rotation) {
     const double mr = p_mi(pg, p) * rr;
-    omx = PF(PF_OOMX) + (-1.) * dt * PF(PF_TQX) / mr + (PF(PF_INTOMX) - PF(PF_OINTOMX)) / mr +
-          rkab * 0.5 * dt * (PF(PF_COLTX) + PF(PF_OCOLTX)) / mr;
-    omy = PF(PF_OOMY) + (-1.) * dt * PF(PF_TQY) / mr + (PF(PF_INTOMY) - PF(PF_OINTOMY)) / mr +
-          rkab * 0.5 * dt * (PF(PF_COLTY) + PF(PF_OCOLTY)) / mr;
-    omz = PF(PF_OOMZ) + (-1.) * dt * PF(PF_TQZ) / mr + (PF(PF_INTOMZ) - PF(PF_OINTOMZ)) / mr +
-          rkab * 0.5 * dt * (PF(PF_COLTZ) + PF(PF_OCOLTZ)) / mr;
-  } else {
-    omx = 0.0; omy = 0.0; omz = 0.0;
+    om = PF(PF_OOMX + c) + (-1.) * dt * PF(PF_TQX + c) / mr + (PF(PF_INTOMX + c) - PF(PF_OINTOMX + c)) / mr +
+         rkab * 0.5 * dt * (0. + PF(PF_OCOLTX + c)) / mr;
   }
-  PF(PF_OMX) = omx; PF(PF_OMY) = omy; PF(PF_OMZ) = omz;
-  const double phi = PF(PF_OPHI) + 0.5 * rkab * dt * (omz + PF(PF_OOMZ));
-  PF(PF_PHI) = phi;
-  const double omtheta = (omy * cos(phi)) - (omx * sin(phi));
-  PF(PF_OMTHETA) = omtheta;
-  PF(PF_THETA) = PF(PF_OTHETA) + rkab * 0.5 * dt * (omtheta + PF(PF_OOMTHETA));
-  // sumrk3 (intgr_nwtn_eulr.f90:1586-1669)
-  double *r = b.rkp + (long)p * RK_N;
-  if (rkiter == 1)
-    for (int t = 0; t < RK_N; ++t) r[t] = 0.;
-  const double dpdy_new = 0.;
-  r[RK_FX] = r[RK_FX] + (-1.) * PF(PF_FXLTOT) + (PF(PF_INTU) - PF(PF_OINTU)) / dt;
-  r[RK_FY] = r[RK_FY] + (-1.) * PF(PF_FYLTOT) + (PF(PF_INTV) - PF(PF_OINTV)) / dt;
-  r[RK_FZ] = r[RK_FZ] + (-1.) * PF(PF_FZLTOT) + (PF(PF_INTW) - PF(PF_OINTW)) / dt;
-  r[RK_TX] = r[RK_TX] + (-1.) * PF(PF_TQX) + (PF(PF_INTOMX) - PF(PF_OINTOMX)) / dt;
-  r[RK_TY] = r[RK_TY] + (-1.) * PF(PF_TQY) + (PF(PF_INTOMY) - PF(PF_OINTOMY)) / dt;
-  r[RK_TZ] = r[RK_TZ] + (-1.) * PF(PF_TQZ) + (PF(PF_INTOMZ) - PF(PF_OINTOMZ)) / dt;
-  r[RK_TT] = r[RK_TT] + (-1.) * (-dpdy_new * p_dvl(pg, p));
-  r[RK_CFX] = r[RK_CFX] + 0.5 * rkab * (S.colfx + PF(PF_OCOLFX));
-  r[RK_CFY] = r[RK_CFY] + 0.5 * rkab * (S.colfy + PF(PF_OCOLFY));
-  r[RK_CFZ] = r[RK_CFZ] + 0.5 * rkab * (S.colfz + PF(PF_OCOLFZ));
-  r[RK_CTX] = r[RK_CTX] + 0.5 * rkab * (PF(PF_COLTX) + PF(PF_OCOLTX));
-  r[RK_CTY] = r[RK_CTY] + 0.5 * rkab * (PF(PF_COLTY) + PF(PF_OCOLTY));
-  r[RK_CTZ] = r[RK_CTZ] + 0.5 * rkab * (PF(PF_COLTZ) + PF(PF_OCOLTZ));
-  r[RK_DUDT] = r[RK_DUDT] + (nu - ou) / dt;
-  r[RK_DVDT] = r[RK_DVDT] + (nv - ov) / dt;
-  r[RK_DWDT] = r[RK_DWDT] + (nw - ow) / dt;
+  const double omx = __shfl_sync(0xffffffffu, om, 0), omy = __shfl_sync(0xffffffffu, om, 1),
+               omz = __shfl_sync(0xffffffffu, om, 2);
+  // sumrk3 (intgr_nwtn_eulr.f90:1586-1669): lane t owns accumulator t.
+  // 0..5: -F + (I - Iold)/dt of the forces and torques; 6: nothing (dpdy = 0);
+  // 7..12: the collision terms; 13..15: the accelerations; 16..18: unused
+  {
+    const int t = lane;
+    const double nuc = __shfl_sync(0xffffffffu, nu, t >= 13 && t <= 15 ? t - 13 : 0);
+    if (t < RK_N) {
+      double *r = b.rkp + (long)p * RK_N + t;
+      double a = rkiter == 1 ? 0. : *r;
+      if (t < 6 || (t >= 13 && t <= 15)) {
+        const double num = t < 6 ? PF(PF_INTU + t) - PF(PF_OINTU + t) : nuc - PF(PF_OU + t - 13);
+        if (t < 6) a = a + (-1.) * PF(PF_FXLTOT + t);
+        a = a + num / dt;
+      } else if (t >= 7 && t <= 12) {
+        const double col = t == 7 ? colx : (t == 8 ? coly : (t == 9 ? colz : 0.));
+        a = a + 0.5 * rkab * (col + PF(PF_OCOLFX + t - 7));
+      }
+      *r = a;
+    }
+  }
+  __syncwarp();
+  if (lane < 3) {
+    PF(PF_X + c) = nx;
+    PF(PF_U + c) = nu;
+    PF(PF_OMX + c) = om;
+    PF(PF_COLFX + c) = colf;
+    PF(PF_COLTX + c) = 0.;
+  }
+  if (lane == 0) {
+    const double phi = PF(PF_OPHI) + 0.5 * rkab * dt * (omz + PF(PF_OOMZ));
+    PF(PF_PHI) = phi;
+    // without rotation about x and y the product with the angle's functions
+    // is zero for any finite angle
+    const double omtheta = (omx == 0. && omy == 0. && isfinite(phi)) ? 0. : (omy * cos(phi)) - (omx * sin(phi));
+    PF(PF_OMTHETA) = omtheta;
+    PF(PF_THETA) = PF(PF_OTHETA) + rkab * 0.5 * dt * (omtheta + PF(PF_OOMTHETA));
+  }
+  if (iter == 0) {
+    __syncwarp();
+    snapshot_particle(pg, b, p, 1, lane);
+  }
 }
 
-int launch_collide_update(cudaStream_t s, const PartGeo &pg, PartBuffers b, int iter, int rkiter, double dt,
-                          bool snapshot) {
+int launch_collide_update(cudaStream_t s, const PartGeo &pg, PartBuffers b, int iter, int rkiter, double dt) {
   if (pg.np == 0) return 0;
   int n = 1;
-  if (snapshot) { k_snapshot<<<(pg.np + 127) / 128, 128, 0, s>>>(pg, b); ++n; }
-  if (pg.ncx >= 3 && pg.ncy >= 3) { k_cell_build<<<1, 1024, 0, s>>>(pg, b); ++n; }
-  k_collide_update<<<(pg.np + COLL_WARPS - 1) / COLL_WARPS, 32 * COLL_WARPS, 0, s>>>(pg, b, iter, rkiter, dt);
+  // the search over all particles costs np^2 / 32 FP32 tests in place of the
+  // cell list's one-block kernel (9 us at 1000 particles): even at about 4000
+  const int scan = pg.np <= 2048 || pg.ncx < 3 || pg.ncy < 3;
+  if (!scan) { k_cell_build<<<1, 1024, 0, s>>>(pg, b, iter); ++n; }
+  const double rkab = pg.rkab[rkiter - 1], f = 1. - (1. / pg.ratiorho);
+  const double3 gt = make_double3(rkab * dt * pg.gacc[0] * f, rkab * dt * pg.gacc[1] * f, rkab * dt * pg.gacc[2] * f);
+  k_collide_update<<<(pg.np + COLL_WARPS - 1) / COLL_WARPS, 32 * COLL_WARPS, 0, s>>>(pg, b, iter, rkiter, dt, scan, gt);
   return n;
 }
 
@@ -1186,6 +1207,8 @@ int launch_collide_update(cudaStream_t s, const PartGeo &pg, PartBuffers b, int 
 // new Lagrangian points with their rigid-body velocity (:1438-1485).
 // One block per particle; the compaction of points flagged `isout` keeps the
 // reference order.
+// FP64 per point: three additions onto the tabulated offsets (twelve operations
+// more when the sphere spins); 1000 spheres of 16 dx: 44 -> 24 us.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_ne_finalize(PartGeo pg, PartBuffers b, IbmBuffers ib, int init) {
   const int np = pg.np;
@@ -1240,33 +1263,31 @@ __global__ void __launch_bounds__(256) k_ne_finalize(PartGeo pg, PartBuffers b, 
   }
   __syncthreads();
   // nl: the per-particle capacity of the Lagrangian arrays; the sphere's
-  // own point count, table offset and shell radius when polydisperse
+  // own point count and table offset when polydisperse
   const int nl = pg.nl, nlp = p_nl(pg, p), nt = pg.ntab;
-  const double radfp = p_radfp(pg, p);
-  const double *sct = b.sincos + p_toff(pg, p);
+  const double *off3 = b.off + p_toff(pg, p);
   const int wid = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const float lxf = (float)pg.lx, lyf = (float)pg.ly;
+  // isout (periodic image outside 1..I, 1..J) is impossible for points within
+  // half a domain of it: a screen of the whole sphere decides that, else the
+  // reference's FP64 test point by point
+  const double rs = 1.01 * p_rad(pg, p);
+  const bool inside = sx - rs > -0.4 * pg.lx && sx + rs < 1.4 * pg.lx && sy - rs > -0.4 * pg.ly && sy + rs < 1.4 * pg.ly;
+  const bool spin = !(somx == 0. && somy == 0. && somz == 0.);
   for (int l0 = 0; l0 < nlp; l0 += blockDim.x) {
     const int l = l0 + threadIdx.x;
     bool keep = false;
     double xfploc = 0, yfploc = 0, zfploc = 0, rx = 0, ry = 0, rz = 0;
     if (l < nlp && b.mslv[p] != 0) {
-      const double st = sct[l], ct = sct[nt + l], sp = sct[2 * nt + l], cp = sct[3 * nt + l];
-      // offsets from the centre, radfp*st*cp etc. with the reference's
-      // rounding; they also serve as (xfp - xc) in the point velocities
-      const double rst = radfp * st;
-      rx = rst * cp;
-      ry = rst * sp;
-      rz = radfp * ct;
+      // offsets from the centre, radfp*st*cp etc. (table, the reference's
+      // rounding); they also serve as (xfp - xc) in the point velocities
+      rx = off3[l];
+      ry = off3[nt + l];
+      rz = off3[2 * nt + l];
       xfploc = sx + rx;
       yfploc = sy + ry;
       zfploc = sz + rz;
-      // isout (periodic image outside 1..I, 1..J) is impossible for points
-      // within half a domain of it: an FP32 screen decides those, the
-      // reference's FP64 test the rest
-      const float xf = (float)xfploc, yf = (float)yfploc;
       bool isout = false;
-      if (!(xf > -0.4f * lxf && xf < 1.4f * lxf && yf > -0.4f * lyf && yf < 1.4f * lyf)) {
+      if (!inside) {
         double isperiodx = 0., isperiody = 0.;
         if (xfploc < 0. + 0.5 * pg.dx) isperiodx = 1.;
         if (xfploc >= pg.lx + 0.5 * pg.dx) isperiodx = -1.;
@@ -1288,9 +1309,9 @@ __global__ void __launch_bounds__(256) k_ne_finalize(PartGeo pg, PartBuffers b, 
     if (keep) {
       const long t = (long)p * nl + off;
       ib.xfp[t] = xfploc; ib.yfp[t] = yfploc; ib.zfp[t] = zfploc;
-      ib.ul[t] = su + somy * rz - somz * ry;
-      ib.vl[t] = sv + somz * rx - somx * rz;
-      ib.wl[t] = sw + somx * ry - somy * rx;
+      ib.ul[t] = spin ? su + somy * rz - somz * ry : su;
+      ib.vl[t] = spin ? sv + somz * rx - somx * rz : sv;
+      ib.wl[t] = spin ? sw + somx * ry - somy * rx : sw;
     }
     __syncthreads();
     if (threadIdx.x == 0) for (int q = 0; q < (int)(blockDim.x / 32); ++q) base += wcount[q];
