@@ -340,7 +340,6 @@ void derived(ibm_ctx *c) {
   pg.poly = 0;
   pg.ntab = P.nl;
   pg.rmax = P.radius;
-  pg.box_cap = 8192;
   if (!c->prad_h.empty()) {
     // polydisperse: per-sphere point counts, shells, Lagrangian volumes
     // (coordsfp.f90:84-90), volumes and moments of inertia (coordsfp.f90:
@@ -369,10 +368,6 @@ void derived(ibm_ctx *c) {
     }
     pg.ntab = off;
     pg.rmax = rmax;
-    // the largest (particle, component) box of the mixed form: the shell's
-    // extent plus the 3-point stencils, per axis
-    const int ext = (int)std::ceil(2. * (rmax - retrac) * g.dxi + 6.);
-    pg.box_cap = std::min(40960, std::max(8192, ext * ext * ext));
     // collision cell list: cells >= 1.01 x 2.1 Rmax wide
     const double w = 1.01 * 2.1 * rmax;
     pg.ncx = std::max(1, (int)std::floor(P.lx / w));
@@ -382,6 +377,12 @@ void derived(ibm_ctx *c) {
     pg.ciy = (float)(pg.ncy / P.ly);
     pg.ciz = (float)(pg.ncz / P.lz);
   }
+  // the largest (particle, component) box of the mixed form, per axis the
+  // shell's extent and the 3-point stencils, its rows padded to the aligned
+  // quads that cover them; at most 160 KB of shared memory
+  auto ext = [&](double di) { return (long)std::floor(2. * (pg.rmax - 0.3 / g.dxi) * di) + 5; };
+  const long row = P.np > 0 ? (ext(g.dxi) + 3 + 3) / 4 * 4 : 0;
+  pg.box_cap = P.np > 0 ? (int)std::min(40960L, std::max(8192L, row * ext(g.dyi) * ext(g.dzi))) : 8192;
 }
 
 // twiddles and the Thomas pivots (initsolver.f90:10-66)
@@ -546,6 +547,8 @@ int alloc_all(ibm_ctx *c) {
       if ((st = dalloc(c, &c->ib.slip, 3 * npl))) return st;
       if ((st = dalloc(c, &c->ib.bgeo, (size_t)24 * np))) return st;
       if ((st = dalloc(c, &c->ib.rowm, (size_t)3 * IBM_BOX_ROWS * np))) return st;
+      if ((st = dalloc(c, &c->ib.bst, (size_t)3 * IBM_BST * np))) return st;
+      if ((st = dalloc(c, &c->ib.order, 3 * npl))) return st;
       if ((st = dalloc(c, &c->ib.psum, (size_t)9 * np))) return st;
       if ((st = dalloc(c, &c->ib.rsum, (size_t)3 * np))) return st;
     } else {
@@ -735,7 +738,8 @@ int forcing_learned(ibm_ctx *c, double dt, int nl_iter) {
   // (their own probe class: they return at once unless the gate fell back)
   for (int it = 1; it < nl_iter; ++it) {
     PROBED(IBM_PROBE_GATED, c->launches += -1 + launch_ibm_interp_force_f(c->stream, g, c->pg, c->ib, c->fu32,
-                                                                          c->fv32, c->fw32, dt, 0, c->gate));
+                                                                          c->fv32, c->fw32, dt, 0, c->gate,
+                                                                          it == nl_iter - 1));
     PROBED(IBM_PROBE_GATED,
            launch_ibm_spread_f(c->stream, g, c->pg, c->ib, c->fu32, c->fv32, c->fw32, dt, LearnedForce{}, c->gate));
     LAUNCHED(2);
@@ -793,7 +797,8 @@ int forcing_run(ibm_ctx *c, double dt, int nl_iter, int kind) {
     LAUNCHED(3);  // reference floors, point records, boxes
     for (int it = 0; it < npass; ++it) {
       PROBED(IBM_PROBE_INTERP, c->launches += -1 + launch_ibm_interp_force_f(c->stream, g, c->pg, c->ib, c->fu32,
-                                                                             c->fv32, c->fw32, dt, it == 0 ? 1 : 0));
+                                                                             c->fv32, c->fw32, dt, it == 0 ? 1 : 0,
+                                                                             nullptr, it == npass - 1));
       LAUNCHED(1);
       if (c->harvesting && it == 0) {
         // features from the field the first pass interpolated (before any
@@ -1147,7 +1152,7 @@ ibm_ctx *ibm_create(const ibm_params *P) {
   int st = alloc_all(c);
   if (st == IBM_OK) st = build_solver_tables(c);
   if (st == IBM_OK && (poisson_set_smem_limits<double>() != 0 || poisson_set_smem_limits<float>() != 0 ||
-                       mlp_set_smem_limits() != 0 || sphere_set_smem_limits() != 0 || ibm_set_smem_limits(c->pg.box_cap) != 0))
+                       mlp_set_smem_limits() != 0 || sphere_set_smem_limits() != 0 || ibm_set_smem_limits(c->pg) != 0))
     st = set_err(c, IBM_E_CUDA, "cudaFuncSetAttribute failed");
   if (st == IBM_OK) st = cuda_err(c, cudaStreamSynchronize(c->stream), "create");
   if (st != IBM_OK) {
@@ -1167,7 +1172,7 @@ int ibm_destroy(ibm_ctx *c) {
                   c->ib.wl, c->ib.dudtl, c->ib.dvdtl, c->ib.dwdtl, c->ib.fxl, c->ib.fyl, c->ib.fzl, c->ib.so, c->ib.sw,
                   c->ib.nla, c->ib.diag, c->pb.pf, c->pb.cf, c->pb.qmax, c->pb.firstc, c->pb.ofirstc, c->pb.nb,
                   c->pb.mslv, c->pb.rkp, c->pb.off, c->pb.err, c->pb.red, c->pb.pos4, c->pb.cstart, c->pb.cfill, c->pb.citem, c->pb.ccell, c->ru32, c->rv32, c->rw32, c->fu32,
-                  c->fv32, c->fw32, c->phi32, c->phi32b, c->spec32, c->twM32, c->twN32, c->twJ32, c->ib.rec, c->ib.pref, c->ib.pcen, c->ib.fxs, c->ib.fys, c->ib.fzs, c->ib.pvh, c->ib.pvl, c->ib.slip, c->ib.bgeo, c->ib.rowm, c->u32, c->v32,
+                  c->fv32, c->fw32, c->phi32, c->phi32b, c->spec32, c->twM32, c->twN32, c->twJ32, c->ib.rec, c->ib.pref, c->ib.pcen, c->ib.fxs, c->ib.fys, c->ib.fzs, c->ib.pvh, c->ib.pvl, c->ib.slip, c->ib.bgeo, c->ib.rowm, c->ib.bst, c->ib.order, c->u32, c->v32,
                   c->w32, c->p32, c->plo32, c->thomas_df, c->ib.psum, c->ib.rsum, c->noise_y, c->noise_par, c->ph.G, c->ph.W0, c->ph.W1, c->stat_part,
                   c->cfield, c->cnext, c->crk, c->ferr, c->psize, c->pcount};
   for (void *q : ptrs)

@@ -1,18 +1,30 @@
 // ibm_mixed_kernels.cu -- the multidirect IBM loop of the mixed form
 // (interp_spread.f90, forcing.f90 restated for FP32 fields).
 //
-// Per Lagrangian point and velocity component a 48-byte stencil record
-// (origin of the 3x3x3 tap block and the component's 9 delta weights) is
-// built once per substep; the per-particle, per-component box of cells the
-// stencils touch is computed once as well.  Interpolation and spreading then
-// run one block per (particle, component) on a shared-memory copy of that
-// box: interpolation reads it with coalesced rows, spreading accumulates into
-// it and flushes each touched cell to HBM once.
+// Once per substep: a 16-byte record per Lagrangian point, the box of cells the
+// stencils touch per particle and component, and the order in which the points
+// are taken.  Interpolation and spreading then run one block per (particle,
+// component) on a shared-memory copy of that box: interpolation reads it by
+// asynchronous 16-byte copies, spreading accumulates into it and flushes each
+// touched quad of cells to HBM once.
+//
+// What bounds the two is the box's 27 accesses a point: at random places 32
+// lanes meet 3 to 4 times in some bank (the shared-memory pipe was 70 % busy in
+// the spreading).  The offsets of the 27 taps from a point's first one are the
+// same for every point, so points whose first taps lie in 32 different banks
+// never conflict: lane q takes the points whose first tap is in bank q (a
+// counting sort in k_ibm_box_geom, once for the five or six passes that use
+// it).  Beyond that it is latency, phase by phase: the loads of a phase are
+// issued together, ahead of their use.  1000 spheres of 16 dx / 1400 of 12 to
+// 24: spreading 94 -> 67 / 321 -> 146 us, interpolation 81 -> 75 / 277 -> 160
+// (its force sums in the last pass only), box geometry 22 -> 26 / 36 -> 47.
 //
 // Origins come from the FP64 point coordinates exactly as the FP64 form
 // computes them; delta weights, interpolation sums and spreading are FP32;
 // point forces F_l and the per-particle force/torque sums stay FP64.
 #include <cuda_bf16.h>
+
+#include <type_traits>
 
 #include "kernels.cuh"
 
@@ -91,13 +103,50 @@ __global__ void __launch_bounds__(256) k_ibm_points(Geo g, PartGeo pg, IbmBuffer
 // cz*nby + cy] = the cells the stencils touch in that row (bit cx): a
 // sphere's shell touches about 40 % of its box, and a row through the
 // sphere only its two ends.
-__global__ void __launch_bounds__(256) k_ibm_box_geom(PartGeo pg, IbmBuffers b, int K) {
-  const int p = blockIdx.x, c = blockIdx.y;
+// Its copy in shared memory: with I a multiple of 4 the rows hold the aligned
+// quads of x-cells that cover them (a quad never straddles the periodic wrap),
+// so that whole quads move; else the rows alone.
+struct BoxLay {
+  int x0, y0, z0, nbx, nby, nbz;  // first cell (x, y not wrapped) and extents
+  int sh, pitch, cells;           // cells before x0 in a row, row length, size
+  __device__ __forceinline__ BoxLay(const int *bg, int I) {
+    x0 = bg[0] + bg[2]; y0 = bg[1] + bg[3]; z0 = bg[4];
+    nbx = bg[5]; nby = bg[6]; nbz = bg[7];
+    const bool quads = (I & 3) == 0;
+    sh = quads ? x0 & 3 : 0;
+    pitch = quads ? (sh + nbx + 3) & ~3 : nbx;
+    cells = pitch * nby * nbz;
+  }
+  // usable: fits cap and narrower than half the periodic domain (so relative
+  // indices are unambiguous)
+  __device__ __forceinline__ bool ok(long cap, int I, int J) const {
+    return nbx > 0 && (long)pitch * nby * nbz <= cap && nbx < I / 2 && nby < J / 2;
+  }
+  // offset of tap (0,0,0) of a point (make_cs origin, relative in x and y)
+  __device__ __forceinline__ int off(const CompStencil &s, const int *bg) const {
+    return ((s.b[2] - bg[4]) * nby + (s.b[1] - bg[3])) * pitch + (s.b[0] - bg[2]) + sh;
+  }
+};
+// q / d for q < 2^16 and 1 <= d < 2^16 as one multiplication
+struct FastDiv {
+  unsigned m;
+  __device__ __forceinline__ explicit FastDiv(int d) : m(0xffffffffu / (unsigned)d + 1u) {}
+  __device__ __forceinline__ int operator()(int q, int d) const { return d == 1 ? q : (int)__umulhi((unsigned)q, m); }
+};
+// Points of particle p, component c by the bank of their first tap:
+// order[(p*3 + c)*nl + bst[q] ..bst[q+1]) = those of bank q, bst[33] = the most
+// of any bank (bst: IBM_BST entries per (p, c)); -1 there where the points are
+// not ordered (box not usable, or more than SPREAD_PRE of them).
+constexpr int SPREAD_PRE = 2048;
+__global__ void __launch_bounds__(256) k_ibm_box_geom(Geo g, PartGeo pg, IbmBuffers b) {
+  const int p = blockIdx.x, c = blockIdx.y, K = g.K;
   const int nla = b.nla[p];
   const PointRec *rp = b.rec + (long)p * pg.nl;
-  __shared__ int mn[3], mx[3];
+  __shared__ int mn[3], mx[3], cnt[32], cur[32];
   __shared__ unsigned rm[IBM_BOX_ROWS];
+  __shared__ unsigned char bank[SPREAD_PRE];
   if (threadIdx.x < 3) { mn[threadIdx.x] = 0x7fffffff; mx[threadIdx.x] = -0x7fffffff; }
+  if (threadIdx.x < 32) cnt[threadIdx.x] = 0;
   for (int q = threadIdx.x; q < IBM_BOX_ROWS; q += blockDim.x) rm[q] = 0u;
   __syncthreads();
   const int4 ref = b.pref[p];
@@ -111,84 +160,144 @@ __global__ void __launch_bounds__(256) k_ibm_box_geom(PartGeo pg, IbmBuffers b, 
     if ((threadIdx.x & 31) == 0) { atomicMin(&mn[d], wl); atomicMax(&mx[d], wh); }
   }
   __syncthreads();
-  const int nbx = mx[0] - mn[0] + 3, nby = mx[1] - mn[1] + 3, nbz = mx[2] - mn[2] + 3;
-  if (nla > 0 && nby * nbz <= IBM_BOX_ROWS && nbx <= 32) {
+  int bg[8] = {ref.x, ref.y, 0, 0, 0, 0, 0, 0};
+  if (nla > 0)
+    for (int d = 0; d < 3; ++d) { bg[2 + d] = mn[d]; bg[5 + d] = mx[d] - mn[d] + 3; }
+  const int nbx = bg[5], nby = bg[6], nbz = bg[7];
+  const BoxLay box(bg, g.I);
+  const bool masks = nla > 0 && nby * nbz <= IBM_BOX_ROWS && nbx <= 32;
+  const bool sorted = nla > 0 && nla <= SPREAD_PRE && box.ok(pg.box_cap, g.I, g.J);
+  if (masks || sorted)
     for (int l = threadIdx.x; l < nla; l += blockDim.x) {
       const CompStencil s = make_cs(rp[l], c, ref.z, K);
-      const int x0 = s.b[0] - mn[0], y0 = s.b[1] - mn[1], z0 = s.b[2] - mn[2];
-      const unsigned bits = 7u << x0;  // cells x0 .. x0 + 2 (x0 + 2 < nbx <= 32)
+      if (sorted) {
+        const int q = box.off(s, bg) & 31;
+        bank[l] = (unsigned char)q;
+        atomicAdd(&cnt[q], 1);
+      }
+      if (masks) {
+        const int x0 = s.b[0] - mn[0], y0 = s.b[1] - mn[1], z0 = s.b[2] - mn[2];
+        const unsigned bits = 7u << x0;  // cells x0 .. x0 + 2 (x0 + 2 < nbx <= 32)
 #pragma unroll
-      for (int k = 0; k < 3; ++k)
+        for (int k = 0; k < 3; ++k)
 #pragma unroll
-        for (int j = 0; j < 3; ++j) atomicOr(&rm[(z0 + k) * nby + y0 + j], bits);
+          for (int j = 0; j < 3; ++j) atomicOr(&rm[(z0 + k) * nby + y0 + j], bits);
+      }
     }
-    __syncthreads();
+  __syncthreads();
+  short *bst = b.bst + ((long)p * 3 + c) * IBM_BST;
+  if (threadIdx.x < 32) {
+    const int q = threadIdx.x, n = cnt[q];
+    int sum = n;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, sum, d);
+      if (q >= d) sum += o;
+    }
+    const int most = __reduce_max_sync(0xffffffffu, n);
+    cur[q] = sum - n;
+    bst[q] = (short)(sum - n);
+    if (q == 31) {
+      bst[32] = (short)sum;
+      bst[33] = sorted ? (short)most : (short)-1;
+    }
+  }
+  if (masks) {
     unsigned *rx = b.rowm + ((long)p * 3 + c) * IBM_BOX_ROWS;
     for (int q = threadIdx.x; q < nby * nbz; q += blockDim.x) rx[q] = rm[q];
   }
-  if (threadIdx.x == 0) {
-    int *o = b.bgeo + ((long)p * 3 + c) * 8;
-    o[0] = ref.x; o[1] = ref.y;
-    if (nla > 0) {
-      o[2] = mn[0]; o[3] = mn[1]; o[4] = mn[2];
-      o[5] = mx[0] - mn[0] + 3; o[6] = nby; o[7] = nbz;
-    } else {
-      o[2] = o[3] = o[4] = o[5] = o[6] = o[7] = 0;
-    }
+  if (threadIdx.x < 8) {
+    int v = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v = threadIdx.x == q ? bg[q] : v;
+    b.bgeo[((long)p * 3 + c) * 8 + threadIdx.x] = v;
   }
+  if (!sorted) return;
+  __syncthreads();
+  unsigned short *ord = b.order + ((long)p * 3 + c) * pg.nl;
+  for (int l = threadIdx.x; l < nla; l += blockDim.x) ord[atomicAdd(&cur[bank[l]], 1)] = (unsigned short)l;
 }
 
 void launch_ibm_stencil_f(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuffers b) {
   if (pg.np == 0) return;
   k_ibm_pref<<<(pg.np + 127) / 128, 128, 0, s>>>(g, pg, b);
   k_ibm_points<<<1216, 256, 0, s>>>(g, pg, b);
-  k_ibm_box_geom<<<dim3(pg.np, 3), 256, 0, s>>>(pg, b, g.K);
+  k_ibm_box_geom<<<dim3(pg.np, 3), 256, 0, s>>>(g, pg, b);
 }
 
-// box usable in shared memory: fits cap and narrower than half the periodic
-// domain (so relative indices are unambiguous)
-__device__ __forceinline__ bool box_ok(const int *bg, int cap, int I, int J) {
-  return bg[5] > 0 && (long)bg[5] * bg[6] * bg[7] <= cap && bg[5] < I / 2 && bg[6] < J / 2;
-}
-// offset of tap (0,0,0) of a point (make_cs origin, relative in x and y) in
-// its particle's box
-__device__ __forceinline__ int box_off(const CompStencil &s, const int *bg) {
-  return ((s.b[2] - bg[4]) * bg[6] + (s.b[1] - bg[3])) * bg[5] + (s.b[0] - bg[2]);
-}
-__device__ __forceinline__ void load_box(const Geo &g, const float *__restrict__ F, const int *bg, float *box,
-                                         const unsigned *__restrict__ rowm) {
-  const int nbx = bg[5], nby = bg[6], nxy = nbx * nby, nbox = nxy * bg[7];
-  const int x0 = bg[0] + bg[2], y0 = bg[1] + bg[3], z0 = bg[4];
-  if ((g.I & 3) == 0) {
-    // rows read as 16-byte quads of x-cells (aligned: I is a multiple of 4,
-    // so a quad never straddles the periodic wrap); cells outside the row
-    // are dropped, and so are quads holding none of the cells the stencils
-    // read (the row masks of k_ibm_box_geom, for boxes up to 32 cells wide)
-    const int a0 = x0 - (((x0 % 4) + 4) % 4);
-    const int nq = (x0 + nbx - a0 + 3) >> 2, nrow = nby * bg[7];
-    const bool masked = nrow <= IBM_BOX_ROWS && nbx <= 32;
-    for (int e = threadIdx.x; e < nrow * nq; e += blockDim.x) {
-      const int row = e / nq, t = e - row * nq;
-      const int cz = row / nby, cy = row - cz * nby, gx = a0 + 4 * t;
-      if (masked) {
-        const unsigned m = rowm[row];
-        const int sh = gx - x0;  // first cell of the quad, -3 .. nbx - 1
-        if (((sh >= 0 ? m >> sh : m << -sh) & 0xFu) == 0u) continue;
-      }
-      const float4 v =
-          __ldg(reinterpret_cast<const float4 *>(&F[fidx(g, wrapm(gx, g.I), wrapm(y0 + cy, g.J), z0 + cz)]));
-      const float vv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int d = 0; d < 4; ++d) {
-        const int cx = gx + d - x0;
-        if (cx >= 0 && cx < nbx) box[row * nbx + cx] = vv[d];
-      }
+// f(e, row, t, gx, gy, gz) for every aligned quad t of every row of a box (e its
+// number): up to eight quads a row (boxes 29 cells wide) a thread keeps its
+// column, so that the loop over rows has no division
+template <typename F>
+__device__ __forceinline__ void box_quads(const Geo &g, const BoxLay &B, F f) {
+  const int nrow = B.nby * B.nbz, a0 = B.x0 - B.sh, nq = B.pitch >> 2;
+  if (nq <= 8) {
+    const int t = threadIdx.x & 7, step = blockDim.x >> 3;
+    if (t >= nq) return;
+    const int gx = wrapm(a0 + 4 * t, g.I);
+    int row = threadIdx.x >> 3, cz = 0, cy = row;
+#pragma unroll 2
+    for (; row < nrow; row += step, cy += step) {
+      while (cy >= B.nby) { cy -= B.nby; ++cz; }
+      f(row * nq + t, row, t, gx, wrapm(B.y0 + cy, g.J), B.z0 + cz);
     }
     return;
   }
-  for (int q = threadIdx.x; q < nbox; q += blockDim.x) {
-    const int cz = q / nxy, r = q - cz * nxy, cy = r / nbx, cx = r - cy * nbx;
-    box[q] = __ldg(&F[fidx(g, wrapm(x0 + cx, g.I), wrapm(y0 + cy, g.J), z0 + cz)]);
+  const FastDiv dq(nq), dy(B.nby);
+  for (int e = threadIdx.x; e < nrow * nq; e += blockDim.x) {
+    const int row = dq(e, nq), t = e - row * nq, cz = dy(row, B.nby), cy = row - cz * B.nby;
+    f(e, row, t, wrapm(a0 + 4 * t, g.I), wrapm(B.y0 + cy, g.J), B.z0 + cz);
+  }
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+// the block's copy of a box; complete after cp_async_wait and a barrier
+__device__ __forceinline__ void load_box(const Geo &g, const float *__restrict__ F, const BoxLay &B, float *box,
+                                         const unsigned *rowm) {
+  if ((g.I & 3) == 0) {
+    // whole quads by asynchronous copies, all of a thread's in flight
+    // together; those holding none of the cells the stencils read (the row
+    // masks of k_ibm_box_geom, for boxes up to 32 cells wide) are left out
+    const bool masked = B.nby * B.nbz <= IBM_BOX_ROWS && B.nbx <= 32;
+    const uint32_t sm = (uint32_t)__cvta_generic_to_shared(box);
+    box_quads(g, B, [&](int e, int row, int t, int gx, int gy, int gz) {
+      bool take = true;
+      if (masked) {
+        const unsigned m = rowm[row];
+        const int sh = 4 * t - B.sh;  // first cell of the quad, -3 .. nbx - 1
+        take = ((sh >= 0 ? m >> sh : m << -sh) & 0xFu) != 0u;
+      }
+      if (take) cp_async16(sm + 16u * (unsigned)e, &F[fidx(g, gx, gy, gz)]);
+    });
+    return;
+  }
+  const int nxy = B.nbx * B.nby;
+  for (int q = threadIdx.x; q < B.cells; q += blockDim.x) {
+    const int cz = q / nxy, r = q - cz * nxy, cy = r / B.nbx, cx = r - cy * B.nbx;
+    box[q] = __ldg(&F[fidx(g, wrapm(B.x0 + cx, g.I), wrapm(B.y0 + cy, g.J), B.z0 + cz)]);
+  }
+}
+// Runs f(l, record) over the points of a (particle, component) in bank order:
+// lane q of each warp the points of bank q, warps in turn; while f runs, the
+// next point's record and the index after it are on their way.
+template <typename F>
+__device__ __forceinline__ void by_bank(const short *bst, const unsigned short *ord, const PointRec *rp, F f) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, e1 = bst[lane + 1];
+  int e = bst[lane] + (threadIdx.x >> 5);
+  int l = e < e1 ? (int)ord[e] : -1;
+  e += nw;
+  int l2 = e < e1 ? (int)ord[e] : -1;
+  PointRec r = rp[max(l, 0)];
+  while (__any_sync(0xffffffffu, l >= 0)) {
+    e += nw;
+    const int l3 = e < e1 ? (int)ord[e] : -1;
+    const PointRec r2 = rp[max(l2, 0)];
+    if (l >= 0) f(l, r);
+    l = l2;
+    l2 = l3;
+    r = r2;
   }
 }
 // Lever arms of the torque terms of component c (c=0: (rz, ry), c=1:
@@ -206,34 +315,35 @@ __device__ __forceinline__ double point_u(const PartGeo &pg, const double *Ua, d
   return pg.rotation ? Ua[t] : Up;
 }
 
-// 27-tap interpolation of one component, k outer, j, i inner, each term
-// f * (wx_i * (wy_j * wz_k))
+// 27-tap interpolation of one component, row by row: sum over k, j of
+// (wy_j wz_k) (sum over i of wx_i f_ijk)
 template <typename TAP>
 __device__ __forceinline__ float interp27(const CompStencil &s, TAP tap) {
   float acc = 0.f;
 #pragma unroll
   for (int k = 0; k < 3; ++k)
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const float wyz = s.w[3 + j] * s.w[6 + k];
-#pragma unroll
-      for (int i = 0; i < 3; ++i) acc += tap(i, j, k) * (s.w[i] * wyz);
-    }
+    for (int j = 0; j < 3; ++j)
+      acc = fmaf(s.w[3 + j] * s.w[6 + k],
+                 fmaf(tap(2, j, k), s.w[2], fmaf(tap(1, j, k), s.w[1], tap(0, j, k) * s.w[0])), acc);
   return acc;
 }
 
 // ---------------------------------------------------------------------------
 // eulr2lagr + complagrforces/updtlagrforces: block (particle, component).
-// Interpolated component to dudtl/dvdtl/dwdtl; with first >= 0 the FP64
-// point-force update of the component and its partial sums (sum F_c and the
-// two lever-arm moments of F_c in the torque) to psum; k_ibm_force_sums
-// combines the components.  first == -1: the residual sum of (U - u~)^2 only
+// With first >= 0 the slip and the point-force update of the component, and in
+// a loop's last pass (LAST: each pass's sums replace the ones before) its
+// partial sums (sum F_c and the two lever-arm moments of F_c in the torque) to
+// psum; k_ibm_force_sums combines the components.  first == -1: the residual sum of (U - u~)^2 only
 // (FP32: it feeds the learned loop's gate), dudtl left as it was; first ==
 // -2: the interpolation to dudtl only (the slip-residual diagnostic).
 // ---------------------------------------------------------------------------
-// box capacity: pg.box_cap cells (8192 = 32 KB for spheres up to about
-// D = 16 dx; polydisperse runs size it for the largest sphere)
+// box capacity: pg.box_cap cells, sized for the largest sphere (9600 = 38 KB
+// at D = 16 dx)
 constexpr int INTERP_THREADS = 256;
+// interpolation: the box and the values of up to SPREAD_PRE points
+inline int interp_pts(const PartGeo &pg) { return pg.nl < SPREAD_PRE ? pg.nl : SPREAD_PRE; }
+inline size_t interp_smem(const PartGeo &pg) { return (size_t)(pg.box_cap + interp_pts(pg)) * sizeof(float); }
 
 // FP32 sum over the block (blockDim a multiple of 32, at most 1024), to every thread
 __device__ __forceinline__ float block_sum_all(float a) {
@@ -252,11 +362,11 @@ __device__ __forceinline__ float block_sum_all(float a) {
 // template parameters: FP64 instructions of an if-converted branch issue
 // under a false predicate and still occupy the FP64 pipe, which this GPU
 // runs at 1/64 of the FP32 rate.
-template <int FIRST, bool ROT>
-__global__ void __launch_bounds__(INTERP_THREADS, 4) k_ibm_interp_comp_f(Geo g, PartGeo pg, IbmBuffers b,
+template <int FIRST, bool ROT, bool LAST>
+__global__ void __launch_bounds__(INTERP_THREADS, 3) k_ibm_interp_comp_f(Geo g, PartGeo pg, IbmBuffers b,
                                                            const float *__restrict__ fu, const float *__restrict__ fv,
                                                            const float *__restrict__ fw, double dti,
-                                                           const int *__restrict__ gate) {
+                                                           const int *__restrict__ gate, int npt) {
   constexpr int first = FIRST;
   if (gate && *gate == 0) return;  // learned form: plain pass not needed
   const int p = blockIdx.x, c = blockIdx.y;
@@ -265,49 +375,81 @@ __global__ void __launch_bounds__(INTERP_THREADS, 4) k_ibm_interp_comp_f(Geo g, 
   const float *F = c == 0 ? fu : (c == 1 ? fv : fw);
   extern __shared__ __align__(16) unsigned char ibox_sm[];
   float *box = reinterpret_cast<float *>(ibox_sm);
+  float *sacc = box + pg.box_cap;  // [npt] the row masks while the box loads, then the interpolated values
   __shared__ int bg[8];
+  __shared__ short sbst[IBM_BST];
   __shared__ float kc[4];  // FP32 1/dt and grid spacings, converted once per block
+  // everything the block needs to know of its box, in one round of loads
+  const unsigned *rowm = b.rowm + ((long)p * 3 + c) * IBM_BOX_ROWS;
+  const int nmask = min(npt, IBM_BOX_ROWS);
+#pragma unroll 4
+  for (int q = threadIdx.x; q < nmask; q += INTERP_THREADS) reinterpret_cast<unsigned *>(sacc)[q] = __ldg(&rowm[q]);
   if (threadIdx.x < 8) bg[threadIdx.x] = b.bgeo[((long)p * 3 + c) * 8 + threadIdx.x];
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + IBM_BST)
+    sbst[threadIdx.x - 64] = b.bst[((long)p * 3 + c) * IBM_BST + threadIdx.x - 64];
   if (threadIdx.x == 32) {
     kc[0] = (float)dti;
     kc[1] = (float)g.dx;
     kc[2] = (float)g.dy;
     kc[3] = (float)g.dz;
   }
+  const float4 vh = b.pvh[p], vl = b.pvl[p];
+  const int4 ref = b.pref[p];
+  const float4 cf = b.pcen[p];
   __syncthreads();
-  const bool boxed = box_ok(bg, pg.box_cap, g.I, g.J);
+  const BoxLay B(bg, g.I);
+  const bool boxed = B.ok(pg.box_cap, g.I, g.J);
+  const bool sorted = sbst[33] >= 0;   // (then boxed as well)
+  const PointRec *rp = b.rec + t0;
   if (boxed) {
-    load_box(g, F, bg, box, b.rowm + ((long)p * 3 + c) * IBM_BOX_ROWS);
+    load_box(g, F, B, box, B.nby * B.nbz <= nmask ? reinterpret_cast<const unsigned *>(sacc) : rowm);
+    cp_async_wait();
     __syncthreads();
   }
   double *dud = c == 0 ? b.dudtl : (c == 1 ? b.dvdtl : b.dwdtl);
   const double *Ua = c == 0 ? b.ul : (c == 1 ? b.vl : b.wl);
-  float *Fl = c == 0 ? b.fxs : (c == 1 ? b.fys : b.fzs);
-  float *slip = b.slip + c * npl;
-  const float4 vh = b.pvh[p], vl = b.pvl[p];
+  float *__restrict__ Fl = c == 0 ? b.fxs : (c == 1 ? b.fys : b.fzs);
+  float *__restrict__ slip = b.slip + c * npl;
   const float2 Us = c == 0 ? make_float2(vh.x, vl.x) : (c == 1 ? make_float2(vh.y, vl.y) : make_float2(vh.z, vl.z));
-  const int4 ref = b.pref[p];
-  const float4 cf = b.pcen[p];
   const float hx = kc[1], hy = kc[2], hz = kc[3];
   const float dtif = kc[0];
-  const PointRec *rp = b.rec + t0;
-  const int ys = bg[5], zs = bg[5] * bg[6];
+  const int ys = B.pitch, zs = B.pitch * B.nby;
+  auto tapbox = [&](const CompStencil &s) {
+    const float *q = box + B.off(s, bg);
+    return interp27(s, [&](int i, int j, int k) { return q[i + j * ys + k * zs]; });
+  };
+  // the forces of the earlier passes of this thread's first points, ahead of
+  // the interpolation
+  constexpr int FP = 4;
+  float fl[FP];
+  if constexpr (FIRST == 0) {
+#pragma unroll
+    for (int q = 0; q < FP; ++q) {
+      const int l = threadIdx.x + q * INTERP_THREADS;
+      fl[q] = l < nla ? Fl[t0 + l] : 0.f;
+    }
+  }
+  if (sorted) {
+    by_bank(sbst, b.order + ((long)p * 3 + c) * pg.nl, rp, [&](int l, const PointRec &r) { sacc[l] = tapbox(make_cs(r, c, ref.z, g.K)); });
+    __syncthreads();
+  }
   // per-thread force and lever-arm sums in FP32 (a few points per thread),
   // the block's sums in FP64
   float sF = 0.f, sa = 0.f, sb = 0.f;
   float r2 = 0.f, r0 = 0.f;
-  for (int l = threadIdx.x; l < nla; l += blockDim.x) {
+  int pass = 0;
+  for (int l = threadIdx.x; l < nla; l += INTERP_THREADS, ++pass) {
     const long t = t0 + l;
-    const PointRec rr = rp[l];
-    const CompStencil s = make_cs(rr, c, ref.z, g.K);
     float acc;
-    if (boxed) {
-      const float *B = box + box_off(s, bg);
-      acc = interp27(s, [&](int i, int j, int k) { return B[i + j * ys + k * zs]; });
+    if (sorted) {
+      acc = sacc[l];
     } else {
-      acc = interp27(s, [&](int i, int j, int k) {
-        return __ldg(&F[fidx(g, wrapm(ref.x + s.b[0] + i, g.I), wrapm(ref.y + s.b[1] + j, g.J), s.b[2] + k)]);
-      });
+      const CompStencil s = make_cs(rp[l], c, ref.z, g.K);
+      if (boxed) acc = tapbox(s);
+      else
+        acc = interp27(s, [&](int i, int j, int k) {
+          return __ldg(&F[fidx(g, wrapm(ref.x + s.b[0] + i, g.I), wrapm(ref.y + s.b[1] + j, g.J), s.b[2] + k)]);
+        });
     }
     float2 U = Us;
     if constexpr (ROT) U = split_u(Ua[t]);
@@ -324,13 +466,15 @@ __global__ void __launch_bounds__(INTERP_THREADS, 4) k_ibm_interp_comp_f(Geo g, 
     if constexpr (FIRST == 1) r0 = fmaf(sd, sd, r0);  // first-pass slip, for the learned loop's gate reference
     float ff;  // the point force, FP32 (its sums below, FP64 across the block)
     if constexpr (FIRST == 1) ff = sd * dtif;
-    else ff = fmaf(sd, dtif, Fl[t]);
+    else ff = fmaf(sd, dtif, pass == 0 ? fl[0] : (pass == 1 ? fl[1] : (pass == 2 ? fl[2] : (pass == 3 ? fl[3] : Fl[t]))));
     Fl[t] = ff;
-    float la, lb;
-    lever_arms(rr, cf, c, hx, hy, hz, la, lb);
-    sF += ff;
-    sa = fmaf(la, ff, sa);
-    sb = fmaf(lb, ff, sb);
+    if constexpr (LAST) {
+      float la, lb;
+      lever_arms(rp[l], cf, c, hx, hy, hz, la, lb);
+      sF += ff;
+      sa = fmaf(la, ff, sa);
+      sb = fmaf(lb, ff, sb);
+    }
   }
   // psum[p][c]: force and lever-arm sums, or (first < 0) the residual sum in
   // slot 0 for k_ibm_res_gate
@@ -344,11 +488,24 @@ __global__ void __launch_bounds__(INTERP_THREADS, 4) k_ibm_interp_comp_f(Geo g, 
     const float tot = block_sum_all(r0);
     if (threadIdx.x == 0) b.rsum[(long)p * 3 + c] = tot;
   }
-  __syncthreads();  // the box is dead: its first words hold the partial sums
-  float *st = reinterpret_cast<float *>(ibox_sm);
-  __shared__ double res[3];
-  block_sum3_df(sF, sa, sb, st, res);
-  if (threadIdx.x < 3) b.psum[((long)p * 3 + c) * 3 + threadIdx.x] = res[threadIdx.x];
+  if constexpr (!LAST) return;
+  __syncthreads();  // the box is dead: its first words hold the threads' sums
+  float *st = box;
+  st[threadIdx.x] = sF;
+  st[INTERP_THREADS + threadIdx.x] = sa;
+  st[2 * INTERP_THREADS + threadIdx.x] = sb;
+  __syncthreads();
+  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (q >= 3) return;
+  float h = 0.f, lo = 0.f;  // a warp a sum, in double-float
+#pragma unroll
+  for (int d = 0; d < INTERP_THREADS; d += 32) df_add(h, lo, st[q * INTERP_THREADS + d + lane], 0.f, h, lo);
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    const float oh = __shfl_xor_sync(0xffffffffu, h, d), ol = __shfl_xor_sync(0xffffffffu, lo, d);
+    df_add(h, lo, oh, ol, h, lo);
+  }
+  if (lane == 0) b.psum[((long)p * 3 + c) * 3 + q] = (double)h + (double)lo;
 }
 // per-particle force and torque of updtlagrforces from the component sums
 __global__ void k_ibm_force_sums(PartGeo pg, IbmBuffers b, const int *__restrict__ gate) {
@@ -369,17 +526,22 @@ __global__ void k_ibm_force_sums(PartGeo pg, IbmBuffers b, const int *__restrict
   pw[PF_TQTHETA * pg.np + p] = (ty * cos(phi)) - (tx * sin(phi));
 }
 int launch_ibm_interp_force_f(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuffers b, const float *fu,
-                              const float *fv, const float *fw, double dt, int first, const int *gate) {
+                              const float *fv, const float *fw, double dt, int first, const int *gate, bool last) {
   if (pg.np == 0) return 0;
   const dim3 grd(pg.np, 3);
-  const size_t sm = pg.box_cap * sizeof(float);
-  auto go = [&](auto kern) { kern<<<grd, INTERP_THREADS, sm, s>>>(g, pg, b, fu, fv, fw, 1. / dt, gate); };
-  const bool rot = pg.rotation != 0;
-  if (first == 1) rot ? go(k_ibm_interp_comp_f<1, true>) : go(k_ibm_interp_comp_f<1, false>);
-  else if (first == 0) rot ? go(k_ibm_interp_comp_f<0, true>) : go(k_ibm_interp_comp_f<0, false>);
-  else if (first == -1) rot ? go(k_ibm_interp_comp_f<-1, true>) : go(k_ibm_interp_comp_f<-1, false>);
-  else rot ? go(k_ibm_interp_comp_f<-2, true>) : go(k_ibm_interp_comp_f<-2, false>);
-  if (first < 0) return 1;
+  const size_t sm = interp_smem(pg);
+  const int npt = interp_pts(pg);
+  auto go = [&](auto kern) { kern<<<grd, INTERP_THREADS, sm, s>>>(g, pg, b, fu, fv, fw, 1. / dt, gate, npt); };
+  auto pick = [&](auto rot) {
+    constexpr bool R = decltype(rot)::value;
+    if (first == 1) last ? go(k_ibm_interp_comp_f<1, R, true>) : go(k_ibm_interp_comp_f<1, R, false>);
+    else if (first == 0) last ? go(k_ibm_interp_comp_f<0, R, true>) : go(k_ibm_interp_comp_f<0, R, false>);
+    else if (first == -1) go(k_ibm_interp_comp_f<-1, R, false>);
+    else go(k_ibm_interp_comp_f<-2, R, false>);
+  };
+  if (pg.rotation) pick(std::true_type{});
+  else pick(std::false_type{});
+  if (first < 0 || !last) return 1;
   k_ibm_force_sums<<<(pg.np + 127) / 128, 128, 0, s>>>(pg, b, gate);
   return 2;
 }
@@ -402,7 +564,6 @@ int launch_ibm_interp_force_f(cudaStream_t s, const Geo &g, const PartGeo &pg, I
 // FP32 values into the box instead; boxes beyond pg.box_cap cells add per
 // tap to the field.
 // ---------------------------------------------------------------------------
-constexpr int SPREAD_PRE = 2048;
 constexpr int SPREAD_THREADS = 384;
 
 // the 27 taps of one point into the box: FP32 adds, or fixed-point adds of
@@ -451,7 +612,10 @@ __global__ void __launch_bounds__(SPREAD_THREADS, 3) k_ibm_spread_f(Geo g, PartG
   // coeff0 (coeff0 with the particle's own Lagrangian volume when
   // polydisperse), 1/dt and dt of the learned force
   __shared__ float kc[7];
+  __shared__ short sbst[IBM_BST];
   if (threadIdx.x < 8) bg[threadIdx.x] = b.bgeo[((long)p * 3 + c) * 8 + threadIdx.x];
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + IBM_BST)
+    sbst[threadIdx.x - 64] = b.bst[((long)p * 3 + c) * IBM_BST + threadIdx.x - 64];
   if (threadIdx.x == 32) {
     const double coeff0 = pg.poly ? (pg.pdvl[p] / pg.dVeul) * dt : coeff0_;
     kc[0] = (float)coeff0;
@@ -463,15 +627,17 @@ __global__ void __launch_bounds__(SPREAD_THREADS, 3) k_ibm_spread_f(Geo g, PartG
     kc[6] = (float)g.dz;
   }
   __syncthreads();
-  const bool boxed = box_ok(bg, pg.box_cap, g.I, g.J);
-  const bool staged = boxed && nla <= SPREAD_PRE;
-  const int nbx = bg[5], nby = bg[6], nbox = nbx * nby * bg[7];
+  const BoxLay B(bg, g.I);
+  const bool boxed = B.ok(pg.box_cap, g.I, g.J);
+  const bool staged = boxed && nla <= SPREAD_PRE;  // the points are ordered by bank then
+  const int nby = B.nby, nbox = B.cells;
   if (boxed) {
-    for (int q = threadIdx.x; q < nbox; q += blockDim.x) box[q] = 0.f;
+    for (int q = 4 * threadIdx.x; q < nbox; q += 4 * blockDim.x)
+      *reinterpret_cast<float4 *>(box + q) = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
   }
-  const float *slip = b.slip + c * npl;
-  float *Fl = c == 0 ? b.fxs : (c == 1 ? b.fys : b.fzs);
+  const float *__restrict__ slip = b.slip + c * npl;
+  float *__restrict__ Fl = c == 0 ? b.fxs : (c == 1 ? b.fys : b.fzs);
   const int4 ref = b.pref[p];
   const PointRec *rp = b.rec + t0;
   // per-thread force and lever-arm sums in FP32, the block's sums in FP64
@@ -485,14 +651,28 @@ __global__ void __launch_bounds__(SPREAD_THREADS, 3) k_ibm_spread_f(Geo g, PartG
     dtif = kc[2]; dtf = kc[3];
   }
   const float pcoef = kc[0], ucoef = kc[1];
-  // Taps into the box: points in transposed order, the 32 lanes of a warp
-  // taking points nq apart in the particle's list (neighbouring points have
-  // overlapping stencils, and shared-memory adds to one address in one
-  // instruction serialise).  Prefactors of staged points: natural order
-  // (coalesced loads of the point arrays).
+  // Prefactors of staged points in natural order (coalesced loads of the point
+  // arrays), their taps in bank order below.  Points too many to stage: in
+  // transposed order, the 32 lanes of a warp taking points nq apart in the
+  // particle's list (neighbouring points have overlapping stencils, and
+  // shared-memory adds to one address in one instruction serialise).
   const int nq = (nla + 31) >> 5;
   float asum = 0.f, r0 = 0.f;
-  for (int m = threadIdx.x; m < 32 * nq; m += blockDim.x) {
+  if (!LY && staged) {  // the plain passes: the slips of up to six points, loaded together
+    float sv[(SPREAD_PRE + SPREAD_THREADS - 1) / SPREAD_THREADS];
+#pragma unroll
+    for (int q = 0; q < (SPREAD_PRE + SPREAD_THREADS - 1) / SPREAD_THREADS; ++q) {
+      const int l = threadIdx.x + q * SPREAD_THREADS;
+      sv[q] = l < nla ? slip[t0 + l] * ucoef : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < (SPREAD_PRE + SPREAD_THREADS - 1) / SPREAD_THREADS; ++q) {
+      const int l = threadIdx.x + q * SPREAD_THREADS;
+      if (l < nla) spre[l] = sv[q];
+      asum += fabsf(sv[q]);
+    }
+  }
+  for (int m = threadIdx.x; m < ((!LY && staged) ? 0 : 32 * nq); m += blockDim.x) {
     const int l = staged ? m : (m & 31) * nq + (m >> 5);
     if (l >= nla) continue;
     const long t = t0 + l;
@@ -522,7 +702,7 @@ __global__ void __launch_bounds__(SPREAD_THREADS, 3) k_ibm_spread_f(Geo g, PartG
     }
     const CompStencil s = make_cs(rp[l], c, ref.z, g.K);
     if (boxed) {
-      spread27_box<false>(box, s, box_off(s, bg), nbx, nby, pre);
+      spread27_box<false>(box, s, B.off(s, bg), B.pitch, nby, pre);
     } else {
       for (int k = 0; k < 3; ++k)
         for (int j = 0; j < 3; ++j) {
@@ -554,46 +734,37 @@ __global__ void __launch_bounds__(SPREAD_THREADS, 3) k_ibm_spread_f(Geo g, PartG
       frexpf(bound, &e);
       scale = ldexpf(1.f, min(29 - e, 126));
     }
-    for (int m = threadIdx.x; m < 32 * nq; m += blockDim.x) {
-      const int l = (m & 31) * nq + (m >> 5);
-      if (l >= nla) continue;
-      const CompStencil s = make_cs(rp[l], c, ref.z, g.K);
-      const int o = box_off(s, bg);
-      if (scale > 0.f) spread27_box<true>(box, s, o, nbx, nby, spre[l] * scale);
-      else spread27_box<false>(box, s, o, nbx, nby, spre[l]);
-    }
+    by_bank(sbst, b.order + ((long)p * 3 + c) * pg.nl, rp, [&](int l, const PointRec &r) {
+      const CompStencil s = make_cs(r, c, ref.z, g.K);
+      const int o = B.off(s, bg);
+      if (scale > 0.f) spread27_box<true>(box, s, o, B.pitch, nby, spre[l] * scale);
+      else spread27_box<false>(box, s, o, B.pitch, nby, spre[l]);
+    });
   }
   __syncthreads();
   const bool fixed = scale > 0.f;
   const float iscale = fixed ? 1.f / scale : 0.f;  // a power of two: exact
-  auto cell = [&](int q) { return fixed ? (float)ibox[q] * iscale : box[q]; };
-  const int nxy = nbx * nby, x0 = bg[0] + bg[2], y0 = bg[1] + bg[3], z0 = bg[4];
   if ((g.I & 3) == 0) {
-    // flush by 16-byte quads of x-cells (rows padded with zeros to the
-    // aligned quads that cover them; with I a multiple of 4 a quad never
-    // straddles the periodic wrap): one vector atomic per nonzero quad
-    const int a0 = x0 - (((x0 % 4) + 4) % 4);
-    const int nqd = (x0 + nbx - a0 + 3) >> 2, nrow = nby * bg[7];
-    for (int e = threadIdx.x; e < nrow * nqd; e += blockDim.x) {
-      const int row = e / nqd, t = e - row * nqd;
-      const int cz = row / nby, cy = row - cz * nby, gx = a0 + 4 * t;
-      float v[4];
-#pragma unroll
-      for (int d = 0; d < 4; ++d) {
-        const int cx = gx + d - x0;
-        v[d] = (cx >= 0 && cx < nbx) ? cell(row * nbx + cx) : 0.f;
-      }
-      if (v[0] == 0.f && v[1] == 0.f && v[2] == 0.f && v[3] == 0.f) continue;
-      float4 *dst = reinterpret_cast<float4 *>(&F[fidx(g, wrapm(gx, g.I), wrapm(y0 + cy, g.J), z0 + cz)]);
-      atomicAdd(dst, make_float4(v[0], v[1], v[2], v[3]));
-    }
+    // flush by the aligned 16-byte quads of x-cells the rows are made of: one
+    // vector atomic per nonzero quad
+    box_quads(g, B, [&](int e, int, int, int gx, int gy, int gz) {
+      const int4 iv = reinterpret_cast<const int4 *>(ibox)[e];
+      if ((iv.x | iv.y | iv.z | iv.w) == 0) return;
+      float4 v;
+      if (fixed)
+        v = make_float4((float)iv.x * iscale, (float)iv.y * iscale, (float)iv.z * iscale, (float)iv.w * iscale);
+      else
+        v = make_float4(__int_as_float(iv.x), __int_as_float(iv.y), __int_as_float(iv.z), __int_as_float(iv.w));
+      atomicAdd(reinterpret_cast<float4 *>(&F[fidx(g, gx, gy, gz)]), v);
+    });
     return;
   }
+  const int nxy = B.nbx * nby;
   for (int q = threadIdx.x; q < nbox; q += blockDim.x) {
-    const float v = cell(q);
+    const float v = fixed ? (float)ibox[q] * iscale : box[q];
     if (v != 0.f) {
-      const int cz = q / nxy, r = q - cz * nxy, cy = r / nbx, cx = r - cy * nbx;
-      atomicAdd(&F[fidx(g, wrapm(x0 + cx, g.I), wrapm(y0 + cy, g.J), z0 + cz)], v);
+      const int cz = q / nxy, r = q - cz * nxy, cy = r / B.nbx, cx = r - cy * B.nbx;
+      atomicAdd(&F[fidx(g, wrapm(B.x0 + cx, g.I), wrapm(B.y0 + cy, g.J), B.z0 + cz)], v);
     }
   }
 }
@@ -750,23 +921,26 @@ void launch_ibm_features_f(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmB
 }
 
 // the box kernels' dynamic shared memory, raised (never lowered: other
-// contexts may use larger boxes) to box_cap cells
-int ibm_set_smem_limits(int box_cap) {
+// contexts may use larger boxes) to a context's boxes
+int ibm_set_smem_limits(const PartGeo &pg) {
   static int cur = 0;
-  if (box_cap <= cur) return 0;
-  cudaError_t e1 = cudaFuncSetAttribute(k_ibm_spread_f<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        box_cap * (int)sizeof(float));
-  if (e1 == cudaSuccess)
-    e1 = cudaFuncSetAttribute(k_ibm_spread_f<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              box_cap * (int)sizeof(float));
-  cudaError_t e2 = cudaSuccess;
-  for (auto k : {k_ibm_interp_comp_f<1, false>, k_ibm_interp_comp_f<0, false>, k_ibm_interp_comp_f<-1, false>,
-                 k_ibm_interp_comp_f<-2, false>, k_ibm_interp_comp_f<1, true>, k_ibm_interp_comp_f<0, true>,
-                 k_ibm_interp_comp_f<-1, true>, k_ibm_interp_comp_f<-2, true>})
-    if (e2 == cudaSuccess)
-      e2 = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, box_cap * (int)sizeof(float));
-  if (e1 != cudaSuccess || e2 != cudaSuccess) return -1;
-  cur = box_cap;
+  const int need = (int)interp_smem(pg);
+  if (need <= cur) return 0;
+  cudaError_t e = cudaSuccess;
+  auto set = [&](auto k) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+  };
+  set(k_ibm_spread_f<false>);
+  set(k_ibm_spread_f<true>);
+  for (auto k : {k_ibm_interp_comp_f<1, false, false>, k_ibm_interp_comp_f<0, false, false>,
+                 k_ibm_interp_comp_f<1, false, true>, k_ibm_interp_comp_f<0, false, true>,
+                 k_ibm_interp_comp_f<1, true, false>, k_ibm_interp_comp_f<0, true, false>,
+                 k_ibm_interp_comp_f<1, true, true>, k_ibm_interp_comp_f<0, true, true>,
+                 k_ibm_interp_comp_f<-1, false, false>, k_ibm_interp_comp_f<-1, true, false>,
+                 k_ibm_interp_comp_f<-2, false, false>, k_ibm_interp_comp_f<-2, true, false>})
+    set(k);
+  if (e != cudaSuccess) return -1;
+  cur = need;
   return 0;
 }
 

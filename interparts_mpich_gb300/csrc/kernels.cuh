@@ -88,6 +88,7 @@ template <typename T> int fft_radix_set_smem_limits();
 // rows (y, z) of a particle's box with a recorded x extent; boxes with more
 // rows are read whole
 constexpr int IBM_BOX_ROWS = 1024;
+constexpr int IBM_BST = 36;  // entries of IbmBuffers::bst per (particle, component)
 // fields of IbmBuffers::sw: the weights of three nodes along an axis, of the
 // staggered origin (nearest face) and of the centred one (H)
 enum { SW_X = 0, SW_Y = 3, SW_Z = 6, SW_XH = 9, SW_YH = 12, SW_ZH = 15, SW_N = 18 };
@@ -104,6 +105,8 @@ struct IbmBuffers {
   float *slip;       // mixed form: [3][np*nl] slip U - u~ of the last pass (FP32)
   int *bgeo;         // mixed form: [np][3][8] per-particle stencil boxes
   unsigned *rowm;    // mixed form: [np][3][IBM_BOX_ROWS] the cells of every box row the stencils touch (bit cx)
+  short *bst;        // mixed form: [np][3][IBM_BST] first points of the banks in order (k_ibm_box_geom)
+  unsigned short *order;  // mixed form: [np][3][nl] points by the bank of their first tap
   int *nla;          // [np]
   double *pf;        // particle scalar fields [PF_N*np]
   double *diag;      // [8] force totals etc.
@@ -125,7 +128,8 @@ void launch_slip_residual(cudaStream_t s, const PartGeo &pg, IbmBuffers b, doubl
 // forces and per-particle sums
 void launch_ibm_stencil_f(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuffers b);
 int launch_ibm_interp_force_f(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuffers b, const float *fu,
-                              const float *fv, const float *fw, double dt, int first, const int *gate = nullptr);
+                              const float *fv, const float *fw, double dt, int first, const int *gate = nullptr,
+                              bool last = true);  // last: the loop's last pass, which forms the force sums
 // learned form: the network's output Y, its target de-standardisation
 // (mean, sigma) and 1/dt; Y == nullptr: the plain pass
 // Point-force increment spread by k_ibm_spread_f: per point and component
@@ -175,7 +179,7 @@ struct MlpTrainBuffers {
 };
 int mlp_nparam();
 size_t mlp_part_floats(int nb);
-int ibm_set_smem_limits(int box_cap);
+int ibm_set_smem_limits(const PartGeo &pg);
 int mlp_set_smem_limits();
 void launch_mlp_refresh(cudaStream_t s, const float *params, __nv_bfloat16 *w1b, __nv_bfloat16 *w2b);
 void launch_mlp_infer(cudaStream_t s, const __nv_bfloat16 *x, int n, const __nv_bfloat16 *w1b,
