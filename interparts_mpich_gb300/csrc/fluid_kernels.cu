@@ -1477,162 +1477,258 @@ template void launch_dev_to_ref<double>(cudaStream_t, const Geo &, const double 
 template void launch_dev_to_ref<float>(cudaStream_t, const Geo &, const float *, double *);
 
 // ---------------------------------------------------------------------------
-// chkdiv (chkdiv.f90:7-61): block partials of sum(div) and (max|div|, first
-// linear index), combined in a fixed order by a single block.
+// Reductions over the grid: chkdiv, chkdt and the wall shear.  One launch each:
+// the blocks leave partials in the context's scratch and the last one to
+// finish combines them in a fixed order, a partial per lane.  (One thread that
+// walked 608 partials took 98 us for chkdiv, 53 us for chkdt and 6 us for the
+// shear's 64, longer than the sweeps over a 64^3 grid.)  The counter behind
+// the last block's choice wraps back to zero by itself.
 // ---------------------------------------------------------------------------
+constexpr int RED_BLOCKS = 1216;                // partials of one kind
+constexpr int RED_COUNT = 4088;                 // scratch entry of the counters
+__device__ __forceinline__ bool red_last(double *scratch, int which) {
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    unsigned *cnt = reinterpret_cast<unsigned *>(scratch + RED_COUNT) + which;
+    last = atomicInc(cnt, gridDim.x - 1) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  return last;
+}
+__device__ __forceinline__ double warp_sum(double s) {
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(~0u, s, o);
+  return s;
+}
+__device__ __forceinline__ double warp_min(double m) {
+  for (int o = 16; o > 0; o >>= 1) m = fmin(m, __shfl_down_sync(~0u, m, o));
+  return m;
+}
+// Value over 256 threads, valid in thread 0.
+template <typename F>
+__device__ __forceinline__ double block_red(double v, F warp) {
+  __shared__ double sm[8];
+  v = warp(v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int q = 1; q < 8; ++q) {
+      if constexpr (F::sum) v += sm[q];
+      else v = fmin(v, sm[q]);
+    }
+  return v;
+}
+struct RedSum {
+  static constexpr bool sum = true;
+  __device__ double operator()(double v) const { return warp_sum(v); }
+};
+struct RedMin {
+  static constexpr bool sum = false;
+  __device__ double operator()(double v) const { return warp_min(v); }
+};
+// Larger value first, then the smaller index.  Values are kept as the bits of
+// a double >= 0 (or of -1: nothing seen), which order like the integers.
+__device__ __forceinline__ void max_loc(long long &m, long long &l, long long m2, long long l2) {
+  if (m2 > m || (m2 == m && l2 >= 0 && (l < 0 || l2 < l))) { m = m2; l = l2; }
+}
+__device__ __forceinline__ void block_max_loc(long long &m, long long &l) {
+  __shared__ long long sm[8], sl[8];
+  for (int o = 16; o > 0; o >>= 1) {
+    const long long m2 = __shfl_down_sync(~0u, m, o), l2 = __shfl_down_sync(~0u, l, o);
+    max_loc(m, l, m2, l2);
+  }
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) { sm[threadIdx.x >> 5] = m; sl[threadIdx.x >> 5] = l; }
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int q = 1; q < 8; ++q) max_loc(m, l, sm[q], sl[q]);
+}
+// Chunks of 256 cells of one plane, dealt to the blocks in turn: one uniform
+// division a chunk and one 32-bit division a cell.
+__host__ __device__ __forceinline__ int red_chunks(const Geo &g) { return (int)((g.plane + 255) / 256); }
+static int red_blocks(const Geo &g) {
+  const long n = (long)red_chunks(g) * g.K;
+  return (int)(n < RED_BLOCKS ? n : RED_BLOCKS);
+}
+
+// chkdiv (chkdiv.f90:7-61): sum(div) and (max|div|, first linear index).
 template <typename T>
-__global__ void __launch_bounds__(256) k_div_partial(Geo g, const T *__restrict__ u,
-                                                     const T *__restrict__ v, const T *__restrict__ w,
-                                                     double *__restrict__ psum, double *__restrict__ pmax,
-                                                     long long *__restrict__ ploc) {
-  const long n = (long)g.I * g.J * g.K;
-  double s = 0., m = -1.;
-  long long loc = -1;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % g.I), j = (int)((t / g.I) % g.J), k = (int)(t / g.plane) + 1;
-    const long c = fidx(g, i, j, k);
+__global__ void __launch_bounds__(256) k_chkdiv(Geo g, const T *__restrict__ u, const T *__restrict__ v,
+                                                const T *__restrict__ w, double *scratch, double *out) {
+  const int ncp = red_chunks(g);
+  const long nq = (long)ncp * g.K;
+  double s = 0.;
+  long long m = __double_as_longlong(-1.), loc = -1;
+  for (long q = blockIdx.x; q < nq; q += gridDim.x) {
+    const int kk = (int)(q / ncp), k = kk + 1;
+    const int t = (int)(q - (long)kk * ncp) * 256 + (int)threadIdx.x;
+    if (t >= g.plane) continue;
+    const int j = (int)((unsigned)t / (unsigned)g.I), i = t - j * g.I;
+    const long c = (long)k * g.plane + t;
     const double div = ((double)w[c] - (double)w[c - g.plane]) * g.dzi +
                        ((double)v[c] - (double)v[fidx(g, i, wrapm(j - 1, g.J), k)]) * g.dyi +
                        ((double)u[c] - (double)u[fidx(g, wrapm(i - 1, g.I), j, k)]) * g.dxi;
     s += div;
-    const double a = fabs(div);
-    if (a > m) { m = a; loc = t; }
+    const long long a = __double_as_longlong(fabs(div));
+    if (a > m && a <= 0x7ff0000000000000ll) { m = a; loc = c - g.plane; }  // not a NaN
   }
-  __shared__ double ss[256], sm[256];
-  __shared__ long long sl[256];
-  ss[threadIdx.x] = s; sm[threadIdx.x] = m; sl[threadIdx.x] = loc;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      ss[threadIdx.x] += ss[threadIdx.x + o];
-      const double m2 = sm[threadIdx.x + o];
-      const long long l2 = sl[threadIdx.x + o];
-      if (m2 > sm[threadIdx.x] || (m2 == sm[threadIdx.x] && l2 >= 0 && (sl[threadIdx.x] < 0 || l2 < sl[threadIdx.x]))) {
-        sm[threadIdx.x] = m2; sl[threadIdx.x] = l2;
-      }
-    }
-    __syncthreads();
+  double *psum = scratch;
+  long long *pmax = reinterpret_cast<long long *>(scratch + RED_BLOCKS), *ploc = pmax + RED_BLOCKS;
+  s = block_red(s, RedSum());
+  block_max_loc(m, loc);
+  if (threadIdx.x == 0) { psum[blockIdx.x] = s; pmax[blockIdx.x] = m; ploc[blockIdx.x] = loc; }
+  if (!red_last(scratch, 0)) return;
+  s = 0.;
+  m = __double_as_longlong(-1.);
+  loc = -1;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += 256) {
+    s += __ldcg(psum + b);
+    max_loc(m, loc, __ldcg(pmax + b), __ldcg(ploc + b));
   }
-  if (threadIdx.x == 0) { psum[blockIdx.x] = ss[0]; pmax[blockIdx.x] = sm[0]; ploc[blockIdx.x] = sl[0]; }
-}
-__global__ void k_div_final(int nb, const double *psum, const double *pmax, const long long *ploc, double *out) {
-  if (threadIdx.x != 0) return;
-  double s = 0., m = -1.;
-  long long l = -1;
-  for (int b = 0; b < nb; ++b) {
-    s += psum[b];
-    if (pmax[b] > m || (pmax[b] == m && ploc[b] >= 0 && (l < 0 || ploc[b] < l))) { m = pmax[b]; l = ploc[b]; }
-  }
-  out[0] = s; out[1] = m; out[2] = (double)l;
+  s = block_red(s, RedSum());
+  block_max_loc(m, loc);
+  if (threadIdx.x == 0) { out[0] = s; out[1] = __longlong_as_double(m); out[2] = (double)loc; }
 }
 template <typename T>
 void launch_chkdiv(cudaStream_t s, const Geo &g, const T *u, const T *v, const T *w, double *scratch, double *out) {
-  const int nb = 608;
-  double *psum = scratch, *pmax = scratch + nb;
-  long long *ploc = (long long *)(scratch + 2 * nb);
-  k_div_partial<T><<<nb, 256, 0, s>>>(g, u, v, w, psum, pmax, ploc);
-  k_div_final<<<1, 32, 0, s>>>(nb, psum, pmax, ploc, out);
+  k_chkdiv<T><<<red_blocks(g), 256, 0, s>>>(g, u, v, w, scratch, out);
 }
 template void launch_chkdiv<double>(cudaStream_t, const Geo &, const double *, const double *, const double *,
                                     double *, double *);
 template void launch_chkdiv<float>(cudaStream_t, const Geo &, const float *, const float *, const float *, double *,
                                    double *);
 
-// chkdt (chkdt.f90:6-273): min over the three staggered components.
+// chkdt (chkdt.f90:6-273): min over the three staggered components of
+// sqrt(3) / S with S = |u|/dx + |v|/dy + |w|/dz.  Only the largest S counts,
+// so every cell is bounded in FP32 first and the FP64 formula runs where the
+// upper bound reaches the largest lower bound seen, or where the speed may be
+// under the 1e-12 below which a cell gives 99999 instead: a warp or two of a
+// block.  In FP64 throughout the kernel was bound by its eight square roots,
+// the division and 18 conversions a component: 119 us at 64^3.
 template <typename T>
-__global__ void __launch_bounds__(256) k_dt_partial(Geo g, const T *__restrict__ u,
-                                                    const T *__restrict__ v, const T *__restrict__ w,
-                                                    double *__restrict__ pmin) {
-  const long n = (long)g.I * g.J * g.K;
-  double m = 899999.;
+__global__ void __launch_bounds__(256) k_chkdt(Geo g, const T *__restrict__ u, const T *__restrict__ v,
+                                               const T *__restrict__ w, float still, double *scratch, double *out) {
+  const int ncp = red_chunks(g);
+  const long nq = (long)ncp * g.K;
   const double dxi = g.dxi, dyi = g.dyi, dzi = g.dzi;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % g.I), j = (int)((t / g.I) % g.J), k = (int)(t / g.plane) + 1;
-    const int ip = wrapm(i + 1, g.I), im = wrapm(i - 1, g.I), jp = wrapm(j + 1, g.J), jm = wrapm(j - 1, g.J);
-    auto U = [&](int a, int b, int c) { return (double)u[fidx(g, a, b, c)]; };
-    auto V = [&](int a, int b, int c) { return (double)v[fidx(g, a, b, c)]; };
-    auto W = [&](int a, int b, int c) { return (double)w[fidx(g, a, b, c)]; };
-    const double dxi2 = dxi * dxi + dyi * dyi + dzi * dzi;
-    const double dt1 = 1.65 / (4. * g.visc * dxi2);
-    for (int comp = 0; comp < 3; ++comp) {
-      double u2, v2, w2, tt;
-      if (comp == 0) {
-        u2 = U(i, j, k) * U(i, j, k);
-        tt = 0.25 * (V(i, j, k) + V(i, jm, k) + V(ip, j, k) + V(ip, jm, k)); v2 = tt * tt;
-        tt = 0.25 * (W(i, j, k) + W(i, j, k - 1) + W(ip, j, k) + W(ip, j, k - 1)); w2 = tt * tt;
-      } else if (comp == 1) {
-        tt = 0.25 * (U(i, j, k) + U(i, jp, k) + U(im, jp, k) + U(im, j, k)); u2 = tt * tt;
-        v2 = V(i, j, k) * V(i, j, k);
-        tt = 0.25 * (W(i, j, k) + W(i, jp, k) + W(i, jp, k - 1) + W(i, j, k - 1)); w2 = tt * tt;
-      } else {
-        tt = 0.25 * (U(i, j, k) + U(im, j, k) + U(im, j, k + 1) + U(i, j, k + 1)); u2 = tt * tt;
-        tt = 0.25 * (V(i, j, k) + V(i, jm, k) + V(i, jm, k + 1) + V(i, j, k + 1)); v2 = tt * tt;
-        w2 = W(i, j, k) * W(i, j, k);
+  const float dx4 = (float)dxi * 0.25f, dy4 = (float)dyi * 0.25f, dz4 = (float)dzi * 0.25f;
+  double m = 899999.;
+  __shared__ unsigned lmax;  // largest lower bound of S in the block (bits of a float >= 0)
+  if (threadIdx.x == 0) lmax = 0u;
+  __syncthreads();
+  bool first = true;
+  for (long q = blockIdx.x; q < nq; q += gridDim.x) {
+    const int kk = (int)(q / ncp), k = kk + 1;
+    const int t = (int)(q - (long)kk * ncp) * 256 + (int)threadIdx.x;
+    const bool in = t < g.plane;
+    const int j = (int)((unsigned)t / (unsigned)g.I), i = t - j * g.I;
+    float ub = 0.f, lb = 0.f;
+    bool slow = false;  // a component that may be at rest
+    if (in) {
+      const int ip = wrapm(i + 1, g.I), im = wrapm(i - 1, g.I), jp = wrapm(j + 1, g.J), jm = wrapm(j - 1, g.J);
+      auto U = [&](int a, int b, int c) { return (float)u[fidx(g, a, b, c)]; };
+      auto V = [&](int a, int b, int c) { return (float)v[fidx(g, a, b, c)]; };
+      auto W = [&](int a, int b, int c) { return (float)w[fidx(g, a, b, c)]; };
+      const float u0 = U(i, j, k), um = U(im, j, k), v0 = V(i, j, k), vm = V(i, jm, k), w0 = W(i, j, k),
+                  wm = W(i, j, k - 1);
+      // 1e-6 of the terms' magnitudes covers the sums' eight FP32 roundings
+      auto bound = [&](float s, float mag) {
+        const float e = 1.e-6f * mag;
+        lb = fmaxf(lb, s - e);
+        if (!(s + e <= ub)) ub = s + e;  // a NaN stays
+        slow |= !(s - e > still);
+      };
+      const float dx = 4.f * dx4, dy = 4.f * dy4, dz = 4.f * dz4;
+      const float v1 = V(ip, j, k), v2 = V(ip, jm, k), w1 = W(ip, j, k), w2 = W(ip, j, k - 1);
+      bound(fabsf(u0) * dx + fabsf(v0 + vm + v1 + v2) * dy4 + fabsf(w0 + wm + w1 + w2) * dz4,
+            fabsf(u0) * dx + (fabsf(v0) + fabsf(vm) + fabsf(v1) + fabsf(v2)) * dy4 +
+                (fabsf(w0) + fabsf(wm) + fabsf(w1) + fabsf(w2)) * dz4);
+      const float u1 = U(i, jp, k), u2 = U(im, jp, k), w3 = W(i, jp, k), w4 = W(i, jp, k - 1);
+      bound(fabsf(u0 + u1 + u2 + um) * dx4 + fabsf(v0) * dy + fabsf(w0 + w3 + w4 + wm) * dz4,
+            (fabsf(u0) + fabsf(u1) + fabsf(u2) + fabsf(um)) * dx4 + fabsf(v0) * dy +
+                (fabsf(w0) + fabsf(w3) + fabsf(w4) + fabsf(wm)) * dz4);
+      const float u3 = U(im, j, k + 1), u4 = U(i, j, k + 1), v3 = V(i, jm, k + 1), v4 = V(i, j, k + 1);
+      bound(fabsf(u0 + um + u3 + u4) * dx4 + fabsf(v0 + vm + v3 + v4) * dy4 + fabsf(w0) * dz,
+            (fabsf(u0) + fabsf(um) + fabsf(u3) + fabsf(u4)) * dx4 +
+                (fabsf(v0) + fabsf(vm) + fabsf(v3) + fabsf(v4)) * dy4 + fabsf(w0) * dz);
+    }
+    const unsigned wl = __reduce_max_sync(~0u, __float_as_uint(lb));
+    if ((threadIdx.x & 31) == 0) atomicMax(&lmax, wl);
+    if (first) __syncthreads();  // later chunks make do with what is there
+    first = false;
+    const float most = __uint_as_float(max(wl, *(volatile unsigned *)&lmax));
+    if (in && (slow || !(ub < most))) {
+      const int ip = wrapm(i + 1, g.I), im = wrapm(i - 1, g.I), jp = wrapm(j + 1, g.J), jm = wrapm(j - 1, g.J);
+      auto U = [&](int a, int b, int c) { return (double)u[fidx(g, a, b, c)]; };
+      auto V = [&](int a, int b, int c) { return (double)v[fidx(g, a, b, c)]; };
+      auto W = [&](int a, int b, int c) { return (double)w[fidx(g, a, b, c)]; };
+      for (int comp = 0; comp < 3; ++comp) {
+        double u2, v2, w2, tt;
+        if (comp == 0) {
+          u2 = U(i, j, k) * U(i, j, k);
+          tt = 0.25 * (V(i, j, k) + V(i, jm, k) + V(ip, j, k) + V(ip, jm, k)); v2 = tt * tt;
+          tt = 0.25 * (W(i, j, k) + W(i, j, k - 1) + W(ip, j, k) + W(ip, j, k - 1)); w2 = tt * tt;
+        } else if (comp == 1) {
+          tt = 0.25 * (U(i, j, k) + U(i, jp, k) + U(im, jp, k) + U(im, j, k)); u2 = tt * tt;
+          v2 = V(i, j, k) * V(i, j, k);
+          tt = 0.25 * (W(i, j, k) + W(i, jp, k) + W(i, jp, k - 1) + W(i, j, k - 1)); w2 = tt * tt;
+        } else {
+          tt = 0.25 * (U(i, j, k) + U(im, j, k) + U(im, j, k + 1) + U(i, j, k + 1)); u2 = tt * tt;
+          tt = 0.25 * (V(i, j, k) + V(i, jm, k) + V(i, jm, k + 1) + V(i, j, k + 1)); v2 = tt * tt;
+          w2 = W(i, j, k) * W(i, j, k);
+        }
+        const double velo = sqrt(u2 + v2 + w2);
+        double dt2;
+        if (fabs(velo) > 1.e-12) dt2 = sqrt(3.) / (sqrt(u2) * dxi + sqrt(v2) * dyi + sqrt(w2) * dzi);
+        else dt2 = 99999.;
+        m = fmin(m, dt2);
       }
-      const double velo = sqrt(u2 + v2 + w2);
-      double dt2;
-      if (fabs(velo) > 1.e-12) dt2 = sqrt(3.) / (sqrt(u2) * dxi + sqrt(v2) * dyi + sqrt(w2) * dzi);
-      else dt2 = 99999.;
-      m = fmin(m, fmin(dt1, dt2));
     }
   }
-  __shared__ double sm[256];
-  sm[threadIdx.x] = m;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sm[threadIdx.x] = fmin(sm[threadIdx.x], sm[threadIdx.x + o]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) pmin[blockIdx.x] = sm[0];
-}
-__global__ void k_min_final(int nb, const double *p, double *out) {
-  if (threadIdx.x != 0) return;
-  double m = 899999.;
-  for (int b = 0; b < nb; ++b) m = fmin(m, p[b]);
-  out[0] = m;
+  m = fmin(m, 1.65 / (4. * g.visc * (dxi * dxi + dyi * dyi + dzi * dzi)));
+  m = block_red(m, RedMin());
+  if (threadIdx.x == 0) scratch[blockIdx.x] = m;
+  if (!red_last(scratch, 1)) return;
+  m = 899999.;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += 256) m = fmin(m, __ldcg(scratch + b));
+  m = block_red(m, RedMin());
+  if (threadIdx.x == 0) out[0] = m;
 }
 template <typename T>
 void launch_chkdt(cudaStream_t s, const Geo &g, const T *u, const T *v, const T *w, double *scratch, double *out) {
-  const int nb = 608;
-  k_dt_partial<T><<<nb, 256, 0, s>>>(g, u, v, w, scratch);
-  k_min_final<<<1, 32, 0, s>>>(nb, scratch, out);
+  // above this S the speed is certainly over 1e-12
+  const float still = (float)(1.01e-12 * std::sqrt(g.dxi * g.dxi + g.dyi * g.dyi + g.dzi * g.dzi));
+  k_chkdt<T><<<red_blocks(g), 256, 0, s>>>(g, u, v, w, still, scratch, out);
 }
 template void launch_chkdt<double>(cudaStream_t, const Geo &, const double *, const double *, const double *,
                                    double *, double *);
 template void launch_chkdt<float>(cudaStream_t, const Geo &, const float *, const float *, const float *, double *,
                                   double *);
 
-// wall shear of rk1/rk2/rk3 (rk3.f90:80-103): sum over the wall planes,
-// block partials combined in a fixed order.
+// wall shear of rk1/rk2/rk3 (rk3.f90:80-103): sum over the wall planes.
 template <typename T>
-__global__ void __launch_bounds__(256) k_wallshear_partial(Geo g, const T *__restrict__ v, double *__restrict__ part) {
-  __shared__ double sm[256];
+__global__ void __launch_bounds__(256) k_wallshear(Geo g, const T *__restrict__ v, double *scratch, double *out) {
   double s = 0.;
   const long PL = g.plane;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < PL; t += (long)gridDim.x * blockDim.x) {
     const long top = (long)g.K * PL + t, bot = PL + t;
-    s = s + g.visc * ((double)v[top + PL] - (double)v[top]) * g.dzi * (1. / g.dxi) * (1. / g.dyi) -
-        g.visc * ((double)v[bot] - (double)v[bot - PL]) * g.dzi * (1. / g.dxi) * (1. / g.dyi);
+    s += ((double)v[top + PL] - (double)v[top]) - ((double)v[bot] - (double)v[bot - PL]);
   }
-  sm[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = sm[0];
-}
-__global__ void k_sum_final(int nb, const double *__restrict__ part, double *out) {
-  if (threadIdx.x != 0) return;
-  double s = 0.;
-  for (int b = 0; b < nb; ++b) s += part[b];
-  out[0] = s;
+  s = block_red(s, RedSum());
+  if (threadIdx.x == 0) scratch[blockIdx.x] = s;
+  if (!red_last(scratch, 2)) return;
+  s = 0.;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += 256) s += __ldcg(scratch + b);
+  s = block_red(s, RedSum());
+  if (threadIdx.x == 0) out[0] = s * (g.visc * g.dzi * (1. / g.dxi) * (1. / g.dyi));
 }
 template <typename T>
 void launch_wallshear(cudaStream_t s, const Geo &g, const T *v, double *scratch, double *out) {
-  const int nb = 64;
-  k_wallshear_partial<T><<<nb, 256, 0, s>>>(g, v, scratch);
-  k_sum_final<<<1, 32, 0, s>>>(nb, scratch, out);
+  const int n = red_chunks(g);
+  k_wallshear<T><<<n < 256 ? n : 256, 256, 0, s>>>(g, v, scratch, out);
 }
 template void launch_wallshear<double>(cudaStream_t, const Geo &, const double *, double *, double *);
 template void launch_wallshear<float>(cudaStream_t, const Geo &, const float *, double *, double *);

@@ -656,7 +656,7 @@ int predict(ibm_ctx *c, int rkiter, double dt) {
   c->stage = rkiter - 1;
   if (c->mixed) launch_wallshear<float>(c->stream, g, c->v32, c->scratch, c->dout + 8 + (rkiter - 1));
   else launch_wallshear<double>(c->stream, g, c->v, c->scratch, c->dout + 8 + (rkiter - 1));
-  LAUNCHED(2);
+  LAUNCHED(1);
   double f1, f2 = 0, f3 = 0;
   if (rkiter == 1) f1 = dt * (32. / 60.);
   else if (rkiter == 2) { f1 = dt * (8. / 60.); f2 = dt * (25. / 60.); f3 = dt * (17. / 60.); }
@@ -1595,7 +1595,7 @@ int ibm_chkdiv(ibm_ctx *c, double *divtot, double *divmax, int ijk[3]) {
   if (!c) return IBM_E_INVALID;
   if (c->mixed) launch_chkdiv<float>(c->stream, c->g, c->u32, c->v32, c->w32, c->scratch, c->dout);
   else launch_chkdiv<double>(c->stream, c->g, c->u, c->v, c->w, c->scratch, c->dout);
-  LAUNCHED(2);
+  LAUNCHED(1);
   CK(cudaMemcpyAsync(c->hpin, c->dout, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   const double tot = c->hpin[0], mx = c->hpin[1];
@@ -1619,7 +1619,7 @@ int ibm_chkdt(ibm_ctx *c, double *dtmax) {
   if (!c || !dtmax) return IBM_E_INVALID;
   if (c->mixed) launch_chkdt<float>(c->stream, c->g, c->u32, c->v32, c->w32, c->scratch, c->dout);
   else launch_chkdt<double>(c->stream, c->g, c->u, c->v, c->w, c->scratch, c->dout);
-  LAUNCHED(2);
+  LAUNCHED(1);
   CK(cudaMemcpyAsync(c->hpin, c->dout, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   *dtmax = c->hpin[0];

@@ -4,7 +4,7 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
-from interparts_mpich_gb300 import IBMSolver
+from interparts_mpich_gb300 import IBMSolver, _abi
 from interparts_mpich_gb300.cases import Case, boundp
 from oracle.oracle import OracleSolver
 
@@ -113,3 +113,36 @@ def test_sphere_integrals(gpu_lib, r, n, grid, aspect):
     assert abs(got[0][0] - got[1][0]) < PLAIN_TOL_CALL * got[1][0]
     for q in (1, 2):
         assert rel_l2(got[0][q], got[1][q]) < PLAIN_TOL_CALL
+
+
+# planes below, at and beyond a chunk of 256 cells, more chunks than blocks;
+# noise, all at rest (with a viscosity that leaves the limit to the rest
+# value), one moving cell in the last chunk, speeds about the rest limit
+@pytest.mark.parametrize("grid", [(4, 4, 4), (16, 16, 9), (54, 27, 5), (64, 81, 70)])
+@pytest.mark.parametrize("flow", ["noise", "rest", "one", "tiny"])
+@pytest.mark.parametrize("mode", [_abi.IBM_MODE_PLAIN_FP64, _abi.IBM_MODE_MIXED])
+def test_time_step_control(gpu_lib, grid, flow, mode):
+    nx, ny, nz = grid
+    case = Case(name="control", itot=nx, jtot=ny, ktot=nz, lx=nx / 32, ly=ny / 24, lz=nz / 40,
+                visc=1e-4 if flow == "noise" else 1e-14)
+    f = _state(case, 3)
+    if flow != "noise":
+        for n in "uvw":
+            f[n][:] = 0
+    if flow == "one":
+        f["v"][nx - 1, ny - 1, nz - 1] = 0.7
+    if flow == "tiny":
+        f["u"][2, 2, 1:nz:2] = 5e-12
+        f["w"][3, 1:4, 2] = 0.9e-12
+    for n in "uvw":  # what the mixed form holds
+        f[n] = np.asfortranarray(f[n].astype(np.float32).astype(np.float64))
+    g, o = IBMSolver(case, mode=mode), OracleSolver(case)
+    for s in (g, o):
+        s.setup(fields=f)
+    assert abs(g.chkdt() - o.chkdt()) <= 1e-14 * o.chkdt()
+    # a divergence of six terms of size 40 x 2, a sum of n of them: 2^-53 each
+    a, b = g.chkdiv(), o.chkdiv()
+    assert abs(a[1] - b[1]) <= 1e-13
+    # no divergence anywhere: the library names the first cell, the oracle none
+    assert tuple(a[2]) == (tuple(b[2]) if b[1] > 0 else (1, 1, 1))
+    assert abs(a[0] - b[0]) <= 1e-12 * nx * ny * nz
