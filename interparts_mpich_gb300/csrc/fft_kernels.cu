@@ -655,6 +655,44 @@ __global__ void __launch_bounds__(64) k_thomas_cyclic(Geo g, double2 *__restrict
   }
 }
 
+// The tables of k_thomas_cyclic, one thread per (kx, |ky|).  The zero mode is
+// pinned at its last plane: rows 0..K-2 alone, z = 0 (cp = iv = 0 in row K-1).
+// Products are rounded one by one, as on a host.  Formed here rather than there
+// and copied (3 K entries a column): a
+// context of 64^3 cells is ready 0.6 ms earlier.
+__global__ void __launch_bounds__(64) k_cyclic_tables(Geo g, const double *__restrict__ xrt,
+                                                      const double *__restrict__ yrt, double *__restrict__ tab) {
+  const long nz = (long)(g.J / 2 + 1) * g.MX, col = blockIdx.x * 64l + threadIdx.x;
+  if (col >= nz) return;
+  const int K = g.K;
+  const double a2 = g.dzi * g.dzi, xy = xrt[col % g.MX] + yrt[col / g.MX], bb = -2. * a2 + xy, gamma = -bb;
+  const bool zero = xy == 0.;
+  double *cp = tab + col, *iv = cp + K * nz, *z = iv + K * nz;
+  double c = 0., zz = 0.;
+  for (int k = 0; k < K; ++k) {
+    const bool last = k == K - 1;
+    double den = zero ? bb : (k == 0 ? bb - gamma : (last ? bb - a2 * a2 / gamma : bb));
+    den -= __dmul_rn(a2, c);
+    const double v = zero && last ? 0. : 1. / den;
+    c = a2 * v;
+    // forward sweep of T z = u, u = (gamma, 0.., 0, a2)
+    zz = zero ? 0. : ((k == 0 ? gamma : (last ? a2 : 0.)) - __dmul_rn(a2, zz)) * v;
+    cp[k * nz] = c;
+    iv[k * nz] = v;
+    z[k * nz] = zz;
+  }
+  const double zl = zz;
+  for (int k = K - 2; k >= 0; --k) {
+    zz = z[k * nz] - __dmul_rn(cp[k * nz], zz);
+    z[k * nz] = zz;
+  }
+  tab[3 * K * nz + col] = zero ? 0. : 1. / (gamma * (1. + zz + a2 * zl / gamma));
+}
+void launch_cyclic_tables(cudaStream_t s, const Geo &g, const double *xrt, const double *yrt, double *tab) {
+  const long nz = (long)(g.J / 2 + 1) * g.MX;
+  k_cyclic_tables<<<(unsigned)((nz + 63) / 64), 64, 0, s>>>(g, xrt, yrt, tab);
+}
+
 // Thomas sweep of the mixed form in double-float arithmetic (pairs of FP32
 // with error-free products and sums, ~48 significant bits) on the FP32
 // pipes; GB300 issues FP64 at 1/64 of the FP32 rate.  Tables (built on the

@@ -432,40 +432,15 @@ int build_solver_tables(ibm_ctx *c) {
   }
   if (J % 2 == 0) yrt[J / 2] = -4. * g.dyi * g.dyi;
   if (g.zper) {
-    // periodic z (k_thomas_cyclic): pivots cp[k], 1/den_k, the Sherman-Morrison
-    // vector z[k] and its factor for every (kx, |ky|).  The zero mode is pinned
-    // at its last plane: rows 0..K-2 alone, z = 0.
-    const double a2 = g.dzi * g.dzi;
-    const size_t nz = (size_t)(J / 2 + 1) * MX, kz = (size_t)K * nz;
-    std::vector<double> tb(3 * kz + nz, 0.);
-    for (int ky = 0; ky <= J / 2; ++ky)
-      for (int kx = 0; kx < MX; ++kx) {
-        double *cp = &tb[(size_t)ky * MX + kx], *iv = cp + kz, *z = iv + kz, *gi = cp + 3 * kz;
-        const double xy = xrt[kx] + yrt[ky], bb = -2. * a2 + xy;
-        const bool zero = xy == 0.;
-        const double gamma = -bb;
-        for (int k = 0; k < K; ++k) {
-          if (zero && k == K - 1) break;  // cp = iv = 0: the last plane comes out as 0
-          double den = zero ? bb : (k == 0 ? bb - gamma : (k == K - 1 ? bb - a2 * a2 / gamma : bb));
-          if (k) den -= a2 * cp[(size_t)(k - 1) * nz];
-          iv[(size_t)k * nz] = 1. / den;
-          cp[(size_t)k * nz] = a2 * iv[(size_t)k * nz];
-        }
-        if (zero) continue;
-        double zz = gamma * iv[0];
-        z[0] = zz;
-        for (int k = 1; k < K; ++k) {
-          zz = ((k == K - 1 ? a2 : 0.) - a2 * zz) * iv[(size_t)k * nz];
-          z[(size_t)k * nz] = zz;
-        }
-        for (int k = K - 2; k >= 0; --k) {
-          zz = z[(size_t)k * nz] - cp[(size_t)k * nz] * zz;
-          z[(size_t)k * nz] = zz;
-        }
-        *gi = 1. / (gamma * (1. + z[0] + a2 * z[(size_t)(K - 1) * nz] / gamma));
-      }
-    if ((st = dalloc(c, &c->zt, tb.size()))) return st;
-    CK(cudaMemcpyAsync(c->zt, tb.data(), tb.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    // periodic z: the cyclic sweep's tables over (k, |ky|, kx), with the
+    // eigenvalues they are formed from behind them
+    const size_t nz = (size_t)(J / 2 + 1) * MX, n = (size_t)3 * K * nz + nz;
+    if ((st = dalloc(c, &c->zt, n + xrt.size() + yrt.size()))) return st;
+    double *dx = c->zt + n, *dy = dx + xrt.size();
+    CK(cudaMemcpyAsync(dx, xrt.data(), xrt.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(dy, yrt.data(), yrt.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    launch_cyclic_tables(c->stream, g, dx, dy, c->zt);
+    CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->stream));
     return IBM_OK;
   }

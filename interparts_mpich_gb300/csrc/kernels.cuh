@@ -73,6 +73,8 @@ void launch_poisson(cudaStream_t s, const Geo &g, const FftPlan &plx, const FftP
                     const float2 *thomas_df = nullptr,  // FP32 spectrum: double-float pivot tables
                     PoissonHook hook = PoissonHook{nullptr, nullptr}, PoissonResid resid = PoissonResid{});
 template <typename T> int poisson_set_smem_limits();
+// tables of the cyclic sweep (periodic z) from the eigenvalues xrt[MX], yrt[J/2+1]
+void launch_cyclic_tables(cudaStream_t s, const Geo &g, const double *xrt, const double *yrt, double *tab);
 // fft_radix_kernels.cu: the transforms of grids whose I/2 and J are products
 // of two or three small radices (fft_radix_ok)
 template <typename T> bool fft_radix_ok(const Geo &g);
