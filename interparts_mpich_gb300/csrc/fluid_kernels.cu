@@ -1498,37 +1498,36 @@ __device__ __forceinline__ bool red_last(double *scratch, int which) {
   __syncthreads();
   return last;
 }
-__device__ __forceinline__ double warp_sum(double s) {
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(~0u, s, o);
-  return s;
-}
-__device__ __forceinline__ double warp_min(double m) {
-  for (int o = 16; o > 0; o >>= 1) m = fmin(m, __shfl_down_sync(~0u, m, o));
-  return m;
-}
-// Value over 256 threads, valid in thread 0.
-template <typename F>
-__device__ __forceinline__ double block_red(double v, F warp) {
+// Sum over 256 threads, valid in thread 0.
+__device__ __forceinline__ double block_sum(double s) {
   __shared__ double sm[8];
-  v = warp(v);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(~0u, s, o);
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
   __syncthreads();
   if (threadIdx.x == 0)
-    for (int q = 1; q < 8; ++q) {
-      if constexpr (F::sum) v += sm[q];
-      else v = fmin(v, sm[q]);
-    }
-  return v;
+    for (int q = 1; q < 8; ++q) s += sm[q];
+  return s;
 }
-struct RedSum {
-  static constexpr bool sum = true;
-  __device__ double operator()(double v) const { return warp_sum(v); }
-};
-struct RedMin {
-  static constexpr bool sum = false;
-  __device__ double operator()(double v) const { return warp_min(v); }
-};
+// Smallest and largest of doubles >= 0 over 256 threads, valid in thread 0.
+// Their bits order like the integers, which keeps the FP64 pipe out of it.
+__device__ __forceinline__ void block_min_max(double &mn, double &mx) {
+  __shared__ long long sn[8], sx[8];
+  long long n = __double_as_longlong(mn), x = __double_as_longlong(mx);
+  for (int o = 16; o > 0; o >>= 1) {
+    n = min(n, __shfl_down_sync(~0u, n, o));
+    x = max(x, __shfl_down_sync(~0u, x, o));
+  }
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) { sn[threadIdx.x >> 5] = n; sx[threadIdx.x >> 5] = x; }
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int q = 1; q < 8; ++q) { n = min(n, sn[q]); x = max(x, sx[q]); }
+  mn = __longlong_as_double(n);
+  mx = __longlong_as_double(x);
+}
+__device__ __forceinline__ double wide(float f) { return f2d_rn(f); }
+__device__ __forceinline__ double wide(double f) { return f; }
 // Larger value first, then the smaller index.  Values are kept as the bits of
 // a double >= 0 (or of -1: nothing seen), which order like the integers.
 __device__ __forceinline__ void max_loc(long long &m, long long &l, long long m2, long long l2) {
@@ -1568,16 +1567,16 @@ __global__ void __launch_bounds__(256) k_chkdiv(Geo g, const T *__restrict__ u, 
     if (t >= g.plane) continue;
     const int j = (int)((unsigned)t / (unsigned)g.I), i = t - j * g.I;
     const long c = (long)k * g.plane + t;
-    const double div = ((double)w[c] - (double)w[c - g.plane]) * g.dzi +
-                       ((double)v[c] - (double)v[fidx(g, i, wrapm(j - 1, g.J), k)]) * g.dyi +
-                       ((double)u[c] - (double)u[fidx(g, wrapm(i - 1, g.I), j, k)]) * g.dxi;
+    const double div = (wide(w[c]) - wide(w[c - g.plane])) * g.dzi +
+                       (wide(v[c]) - wide(v[fidx(g, i, wrapm(j - 1, g.J), k)])) * g.dyi +
+                       (wide(u[c]) - wide(u[fidx(g, wrapm(i - 1, g.I), j, k)])) * g.dxi;
     s += div;
     const long long a = __double_as_longlong(fabs(div));
     if (a > m && a <= 0x7ff0000000000000ll) { m = a; loc = c - g.plane; }  // not a NaN
   }
   double *psum = scratch;
   long long *pmax = reinterpret_cast<long long *>(scratch + RED_BLOCKS), *ploc = pmax + RED_BLOCKS;
-  s = block_red(s, RedSum());
+  s = block_sum(s);
   block_max_loc(m, loc);
   if (threadIdx.x == 0) { psum[blockIdx.x] = s; pmax[blockIdx.x] = m; ploc[blockIdx.x] = loc; }
   if (!red_last(scratch, 0)) return;
@@ -1588,7 +1587,7 @@ __global__ void __launch_bounds__(256) k_chkdiv(Geo g, const T *__restrict__ u, 
     s += __ldcg(psum + b);
     max_loc(m, loc, __ldcg(pmax + b), __ldcg(ploc + b));
   }
-  s = block_red(s, RedSum());
+  s = block_sum(s);
   block_max_loc(m, loc);
   if (threadIdx.x == 0) { out[0] = s; out[1] = __longlong_as_double(m); out[2] = (double)loc; }
 }
@@ -1602,21 +1601,23 @@ template void launch_chkdiv<float>(cudaStream_t, const Geo &, const float *, con
                                    double *);
 
 // chkdt (chkdt.f90:6-273): min over the three staggered components of
-// sqrt(3) / S with S = |u|/dx + |v|/dy + |w|/dz.  Only the largest S counts,
-// so every cell is bounded in FP32 first and the FP64 formula runs where the
-// upper bound reaches the largest lower bound seen, or where the speed may be
-// under the 1e-12 below which a cell gives 99999 instead: a warp or two of a
-// block.  In FP64 throughout the kernel was bound by its eight square roots,
-// the division and 18 conversions a component: 119 us at 64^3.
+// sqrt(3) / S with S = |u|/dx + |v|/dy + |w|/dz.  Only the largest S counts, so
+// every component is bounded in FP32 first, and S is formed in FP64 where the
+// upper bound reaches the largest lower bound seen: a warp or two of a block.
+// (|t| for the sqrt(t^2) of the reference: the same number unless t^2 leaves
+// the range.)  Cells whose speed may be under the 1e-12 below which the
+// reference takes 99999, and those with an infinity or a NaN, go through its
+// formula as it stands.  In FP64 throughout, the kernel was bound by three
+// square roots and a division a component: 119 us at 64^3, now 26.
 template <typename T>
 __global__ void __launch_bounds__(256) k_chkdt(Geo g, const T *__restrict__ u, const T *__restrict__ v,
                                                const T *__restrict__ w, float still, double *scratch, double *out) {
   const int ncp = red_chunks(g);
   const long nq = (long)ncp * g.K;
   const double dxi = g.dxi, dyi = g.dyi, dzi = g.dzi;
-  const float dx4 = (float)dxi * 0.25f, dy4 = (float)dyi * 0.25f, dz4 = (float)dzi * 0.25f;
-  double m = 899999.;
-  __shared__ unsigned lmax;  // largest lower bound of S in the block (bits of a float >= 0)
+  const float dx = (float)dxi, dy = (float)dyi, dz = (float)dzi;
+  double m = 899999., most_s = 0.;
+  __shared__ unsigned lmax;     // largest lower bound of S in the block (bits of a float >= 0)
   if (threadIdx.x == 0) lmax = 0u;
   __syncthreads();
   bool first = true;
@@ -1625,77 +1626,74 @@ __global__ void __launch_bounds__(256) k_chkdt(Geo g, const T *__restrict__ u, c
     const int t = (int)(q - (long)kk * ncp) * 256 + (int)threadIdx.x;
     const bool in = t < g.plane;
     const int j = (int)((unsigned)t / (unsigned)g.I), i = t - j * g.I;
-    float ub = 0.f, lb = 0.f;
-    bool slow = false;  // a component that may be at rest
+    float ub[3] = {-1.f, -1.f, -1.f}, lb = 0.f;
+    bool slow = false;
+    T u0, um, v0, vm, w0, wm, v1, v2, w1, w2, u1, u2, w3, w4, u3, u4, v3, v4;
     if (in) {
-      const int ip = wrapm(i + 1, g.I), im = wrapm(i - 1, g.I), jp = wrapm(j + 1, g.J), jm = wrapm(j - 1, g.J);
-      auto U = [&](int a, int b, int c) { return (float)u[fidx(g, a, b, c)]; };
-      auto V = [&](int a, int b, int c) { return (float)v[fidx(g, a, b, c)]; };
-      auto W = [&](int a, int b, int c) { return (float)w[fidx(g, a, b, c)]; };
-      const float u0 = U(i, j, k), um = U(im, j, k), v0 = V(i, j, k), vm = V(i, jm, k), w0 = W(i, j, k),
-                  wm = W(i, j, k - 1);
-      // 1e-6 of the terms' magnitudes covers the sums' eight FP32 roundings
-      auto bound = [&](float s, float mag) {
-        const float e = 1.e-6f * mag;
-        lb = fmaxf(lb, s - e);
-        if (!(s + e <= ub)) ub = s + e;  // a NaN stays
-        slow |= !(s - e > still);
+      const long ip = i + 1 < g.I ? 1 : 1 - g.I, im = i ? -1 : g.I - 1;
+      const long jp = j + 1 < g.J ? g.I : g.I - g.plane, jm = j ? -g.I : g.plane - g.I, kp = g.plane;
+      const long c = (long)k * g.plane + t;
+      const T *pu = u + c, *pv = v + c, *pw = w + c;
+      u0 = pu[0]; um = pu[im]; v0 = pv[0]; vm = pv[jm]; w0 = pw[0]; wm = pw[-kp];
+      v1 = pv[ip]; v2 = pv[ip + jm]; w1 = pw[ip]; w2 = pw[ip - kp];
+      u1 = pu[jp]; u2 = pu[im + jp]; w3 = pw[jp]; w4 = pw[jp - kp];
+      u3 = pu[im + kp]; u4 = pu[kp]; v3 = pv[jm + kp]; v4 = pv[kp];
+      // a: the component's own velocity, b and c: four neighbours of the others'
+      auto bound = [&](int e, T a, float da, T b0, T b1, T b2, T b3, float db, T c0, T c1, T c2, T c3, float dc) {
+        const float fa = fabsf((float)a) * da;
+        const float x0 = (float)b0, x1 = (float)b1, x2 = (float)b2, x3 = (float)b3;
+        const float y0 = (float)c0, y1 = (float)c1, y2 = (float)c2, y3 = (float)c3;
+        const float s = fa + 0.25f * (fabsf(x0 + x1 + x2 + x3) * db + fabsf(y0 + y1 + y2 + y3) * dc);
+        const float mag = fa + 0.25f * ((fabsf(x0) + fabsf(x1) + fabsf(x2) + fabsf(x3)) * db +
+                                        (fabsf(y0) + fabsf(y1) + fabsf(y2) + fabsf(y3)) * dc);
+        const float er = 1.e-6f * mag;  // ten FP32 roundings of 2^-24
+        ub[e] = s + er;
+        lb = fmaxf(lb, s - er);
+        slow |= !(s - er > still);
       };
-      const float dx = 4.f * dx4, dy = 4.f * dy4, dz = 4.f * dz4;
-      const float v1 = V(ip, j, k), v2 = V(ip, jm, k), w1 = W(ip, j, k), w2 = W(ip, j, k - 1);
-      bound(fabsf(u0) * dx + fabsf(v0 + vm + v1 + v2) * dy4 + fabsf(w0 + wm + w1 + w2) * dz4,
-            fabsf(u0) * dx + (fabsf(v0) + fabsf(vm) + fabsf(v1) + fabsf(v2)) * dy4 +
-                (fabsf(w0) + fabsf(wm) + fabsf(w1) + fabsf(w2)) * dz4);
-      const float u1 = U(i, jp, k), u2 = U(im, jp, k), w3 = W(i, jp, k), w4 = W(i, jp, k - 1);
-      bound(fabsf(u0 + u1 + u2 + um) * dx4 + fabsf(v0) * dy + fabsf(w0 + w3 + w4 + wm) * dz4,
-            (fabsf(u0) + fabsf(u1) + fabsf(u2) + fabsf(um)) * dx4 + fabsf(v0) * dy +
-                (fabsf(w0) + fabsf(w3) + fabsf(w4) + fabsf(wm)) * dz4);
-      const float u3 = U(im, j, k + 1), u4 = U(i, j, k + 1), v3 = V(i, jm, k + 1), v4 = V(i, j, k + 1);
-      bound(fabsf(u0 + um + u3 + u4) * dx4 + fabsf(v0 + vm + v3 + v4) * dy4 + fabsf(w0) * dz,
-            (fabsf(u0) + fabsf(um) + fabsf(u3) + fabsf(u4)) * dx4 +
-                (fabsf(v0) + fabsf(vm) + fabsf(v3) + fabsf(v4)) * dy4 + fabsf(w0) * dz);
+      bound(0, u0, dx, v0, vm, v1, v2, dy, w0, wm, w1, w2, dz);
+      bound(1, v0, dy, u0, u1, u2, um, dx, w0, w3, w4, wm, dz);
+      bound(2, w0, dz, u0, um, u3, u4, dx, v0, vm, v3, v4, dy);
     }
     const unsigned wl = __reduce_max_sync(~0u, __float_as_uint(lb));
     if ((threadIdx.x & 31) == 0) atomicMax(&lmax, wl);
     if (first) __syncthreads();  // later chunks make do with what is there
     first = false;
     const float most = __uint_as_float(max(wl, *(volatile unsigned *)&lmax));
-    if (in && (slow || !(ub < most))) {
-      const int ip = wrapm(i + 1, g.I), im = wrapm(i - 1, g.I), jp = wrapm(j + 1, g.J), jm = wrapm(j - 1, g.J);
-      auto U = [&](int a, int b, int c) { return (double)u[fidx(g, a, b, c)]; };
-      auto V = [&](int a, int b, int c) { return (double)v[fidx(g, a, b, c)]; };
-      auto W = [&](int a, int b, int c) { return (double)w[fidx(g, a, b, c)]; };
-      for (int comp = 0; comp < 3; ++comp) {
-        double u2, v2, w2, tt;
-        if (comp == 0) {
-          u2 = U(i, j, k) * U(i, j, k);
-          tt = 0.25 * (V(i, j, k) + V(i, jm, k) + V(ip, j, k) + V(ip, jm, k)); v2 = tt * tt;
-          tt = 0.25 * (W(i, j, k) + W(i, j, k - 1) + W(ip, j, k) + W(ip, j, k - 1)); w2 = tt * tt;
-        } else if (comp == 1) {
-          tt = 0.25 * (U(i, j, k) + U(i, jp, k) + U(im, jp, k) + U(im, j, k)); u2 = tt * tt;
-          v2 = V(i, j, k) * V(i, j, k);
-          tt = 0.25 * (W(i, j, k) + W(i, jp, k) + W(i, jp, k - 1) + W(i, j, k - 1)); w2 = tt * tt;
-        } else {
-          tt = 0.25 * (U(i, j, k) + U(im, j, k) + U(im, j, k + 1) + U(i, j, k + 1)); u2 = tt * tt;
-          tt = 0.25 * (V(i, j, k) + V(i, jm, k) + V(i, jm, k + 1) + V(i, j, k + 1)); v2 = tt * tt;
-          w2 = W(i, j, k) * W(i, j, k);
+    if (in && (slow || fmaxf(fmaxf(ub[0], ub[1]), ub[2]) >= most)) {
+      auto comp = [&](int e, T a, double da, T b0, T b1, T b2, T b3, double db, T c0, T c1, T c2, T c3, double dc) {
+        if (!slow && ub[e] < most) return;
+        const double t0 = wide(a), t1 = 0.25 * (wide(b0) + wide(b1) + wide(b2) + wide(b3)),
+                     t2 = 0.25 * (wide(c0) + wide(c1) + wide(c2) + wide(c3));
+        if (!slow) {
+          most_s = fmax(most_s, fabs(t0) * da + fabs(t1) * db + fabs(t2) * dc);
+          return;
         }
-        const double velo = sqrt(u2 + v2 + w2);
-        double dt2;
-        if (fabs(velo) > 1.e-12) dt2 = sqrt(3.) / (sqrt(u2) * dxi + sqrt(v2) * dyi + sqrt(w2) * dzi);
-        else dt2 = 99999.;
-        m = fmin(m, dt2);
-      }
+        const double s0 = t0 * t0, s1 = t1 * t1, s2 = t2 * t2, velo = sqrt(s0 + s1 + s2);
+        m = fmin(m, fabs(velo) > 1.e-12 ? sqrt(3.) / (sqrt(s0) * da + sqrt(s1) * db + sqrt(s2) * dc) : 99999.);
+      };
+      comp(0, u0, dxi, v0, vm, v1, v2, dyi, w0, wm, w1, w2, dzi);
+      comp(1, v0, dyi, u0, u1, u2, um, dxi, w0, w3, w4, wm, dzi);
+      comp(2, w0, dzi, u0, um, u3, u4, dxi, v0, vm, v3, v4, dyi);
     }
   }
-  m = fmin(m, 1.65 / (4. * g.visc * (dxi * dxi + dyi * dyi + dzi * dzi)));
-  m = block_red(m, RedMin());
-  if (threadIdx.x == 0) scratch[blockIdx.x] = m;
+  block_min_max(m, most_s);
+  if (threadIdx.x == 0) { scratch[blockIdx.x] = m; scratch[RED_BLOCKS + blockIdx.x] = most_s; }
   if (!red_last(scratch, 1)) return;
   m = 899999.;
-  for (int b = threadIdx.x; b < (int)gridDim.x; b += 256) m = fmin(m, __ldcg(scratch + b));
-  m = block_red(m, RedMin());
-  if (threadIdx.x == 0) out[0] = m;
+  most_s = 0.;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += 256) {
+    long long n = __double_as_longlong(m), x = __double_as_longlong(most_s);
+    n = min(n, __double_as_longlong(__ldcg(scratch + b)));
+    x = max(x, __double_as_longlong(__ldcg(scratch + RED_BLOCKS + b)));
+    m = __longlong_as_double(n);
+    most_s = __longlong_as_double(x);
+  }
+  block_min_max(m, most_s);
+  if (threadIdx.x == 0) {
+    m = fmin(m, 1.65 / (4. * g.visc * (dxi * dxi + dyi * dyi + dzi * dzi)));
+    out[0] = most_s > 0. ? fmin(m, sqrt(3.) / most_s) : m;
+  }
 }
 template <typename T>
 void launch_chkdt(cudaStream_t s, const Geo &g, const T *u, const T *v, const T *w, double *scratch, double *out) {
@@ -1717,12 +1715,12 @@ __global__ void __launch_bounds__(256) k_wallshear(Geo g, const T *__restrict__ 
     const long top = (long)g.K * PL + t, bot = PL + t;
     s += ((double)v[top + PL] - (double)v[top]) - ((double)v[bot] - (double)v[bot - PL]);
   }
-  s = block_red(s, RedSum());
+  s = block_sum(s);
   if (threadIdx.x == 0) scratch[blockIdx.x] = s;
   if (!red_last(scratch, 2)) return;
   s = 0.;
   for (int b = threadIdx.x; b < (int)gridDim.x; b += 256) s += __ldcg(scratch + b);
-  s = block_red(s, RedSum());
+  s = block_sum(s);
   if (threadIdx.x == 0) out[0] = s * (g.visc * g.dzi * (1. / g.dxi) * (1. / g.dyi));
 }
 template <typename T>
