@@ -1417,59 +1417,112 @@ void launch_correc_mixed(cudaStream_t s, const Geo &g, const float *fu, const fl
   k_correc_mixed<<<grd, blk, 0, s>>>(g, fu, fv, fw, phi, u, v, w, ph, pl, (float)fi, (float)fj, (float)fk);
 }
 
-// double-float pair <-> FP64 array
-__global__ void k_df_to_d(long n, const float *__restrict__ h, const float *__restrict__ l, double *__restrict__ d) {
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x)
-    d[t] = (double)h[t] + (double)l[t];
-}
-__global__ void k_d_to_df(long n, const double *__restrict__ d, float *__restrict__ h, float *__restrict__ l) {
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    const float hh = (float)d[t];
-    h[t] = hh;
-    l[t] = (float)(d[t] - (double)hh);
-  }
-}
-void launch_df_to_d(cudaStream_t s, long n, const float *h, const float *l, double *d) {
-  k_df_to_d<<<1216, 256, 0, s>>>(n, h, l, d);
-}
-void launch_d_to_df(cudaStream_t s, long n, const double *d, float *h, float *l) {
-  k_d_to_df<<<1216, 256, 0, s>>>(n, d, h, l);
-}
-
 // ---------------------------------------------------------------------------
 // Layout conversion between the reference host layout (0:i1,0:j1,0:k1) and
 // the device layout.  to_dev: dev(i,j,k) = ref(i+1,j+1,k).  to_ref fills the
-// x/y ghosts with the periodic values, as bounduvw/boundp leave them.
+// x/y ghosts with the periodic values, as bounduvw/boundp leave them.  LO: the
+// device field is an FP32 pair dev + lo (the mixed form's pressure).
+//
+// Bound by memory: a warp walks rows with four loads of a lane in flight, the
+// row's offset is formed once, and FP32 values are converted on the integer
+// pipe (the conversion instructions issue at the rate of FP64).  A cell per
+// thread with three 64-bit divisions and the conversions, and the pressure
+// through an FP64 array and a second pass, 512 x 512 x 256: FP32 to_dev 273 us,
+// to_ref 385 us, pressure 760 and 757 us; now 116, 132, 168 and 170 (the copy rate: 118
+// and 158).  A conversion instruction that is only predicated off for the normal
+// values still cost its issue: 143 and 146 us, pressure 378 and 414.
 // ---------------------------------------------------------------------------
-template <typename T>
-__global__ void k_ref_to_dev(Geo g, const double *__restrict__ ref, T *__restrict__ dev) {
-  const long n = g.nfield;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % g.I);
-    const int j = (int)((t / g.I) % g.J);
-    const int k = (int)(t / g.plane);
-    const long r = (long)(i + 1) + (long)(g.I + 2) * ((j + 1) + (long)(g.J + 2) * k);
-    dev[t] = (T)ref[r];
+__device__ __forceinline__ double wide(float f) { return f2d_rn(f); }
+__device__ __forceinline__ double wide(double f) { return f; }
+template <typename T, bool LO>
+__global__ void __launch_bounds__(256) k_ref_to_dev(Geo g, const double *__restrict__ ref, T *__restrict__ dev,
+                                                    float *__restrict__ lo) {
+  const int lane = threadIdx.x & 31, nrow = g.J * (g.K + 2), I = g.I;
+  for (int q = (blockIdx.x * 256 + threadIdx.x) >> 5; q < nrow; q += gridDim.x * 8) {
+    const int k = (int)((unsigned)q / (unsigned)g.J), j = q - k * g.J;
+    const double *r = ref + 1 + (long)(I + 2) * (j + 1 + (long)(g.J + 2) * k);
+    T *d = dev + (long)q * I;
+    for (int i0 = lane; i0 < I; i0 += 128) {
+      double x[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (i0 + 32 * e < I) x[e] = r[i0 + 32 * e];
+      bool ok = true;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = i0 + 32 * e;
+        if (i >= I) break;
+        if constexpr (LO) {
+          float h, l;
+          ok &= d2df_int(x[e], h, l);
+          d[i] = h;
+          lo[(long)q * I + i] = l;
+        } else if constexpr (sizeof(T) == 4) {
+          float h;
+          int rem;
+          ok &= d2f_int(x[e], h, rem);
+          d[i] = h;
+        } else {
+          d[i] = x[e];
+        }
+      }
+      if (sizeof(T) == 4 && !ok) {  // a value out of FP32's normal range: the conversion instructions
+#pragma unroll 1
+        for (int i = i0; i < I && i < i0 + 128; i += 32) {
+          const double y = r[i];
+          const float h = (float)y;
+          d[i] = h;
+          if constexpr (LO) lo[(long)q * I + i] = (float)(y - (double)h);
+        }
+      }
+    }
   }
 }
-template <typename T>
-__global__ void k_dev_to_ref(Geo g, const T *__restrict__ dev, double *__restrict__ ref) {
-  const long n = (long)(g.I + 2) * (g.J + 2) * (g.K + 2);
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % (g.I + 2));
-    const int j = (int)((t / (g.I + 2)) % (g.J + 2));
-    const int k = (int)(t / ((long)(g.I + 2) * (g.J + 2)));
-    const int id = wrapm(i - 1, g.I), jd = wrapm(j - 1, g.J);
-    ref[t] = (double)dev[fidx(g, id, jd, k)];
+template <typename T, bool LO>
+__global__ void __launch_bounds__(256) k_dev_to_ref(Geo g, const T *__restrict__ dev, const float *__restrict__ lo,
+                                                    double *__restrict__ ref) {
+  const int lane = threadIdx.x & 31, nrow = (g.J + 2) * (g.K + 2), I = g.I;
+  for (int q = (blockIdx.x * 256 + threadIdx.x) >> 5; q < nrow; q += gridDim.x * 8) {
+    const int k = (int)((unsigned)q / (unsigned)(g.J + 2)), j = wrapm(q - k * (g.J + 2) - 1, g.J);
+    const long row = fidx(g, 0, j, k);
+    const T *d = dev + row;
+    double *r = ref + (long)q * (I + 2);
+    for (int i0 = lane; i0 < I + 2; i0 += 128) {
+      T x[4];
+      float y[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = i0 + 32 * e;
+        if (i < I + 2) {
+          const int id = wrapm(i - 1, I);
+          x[e] = d[id];
+          if constexpr (LO) y[e] = lo[row + id];
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = i0 + 32 * e;
+        if (i >= I + 2) break;
+        if constexpr (LO) r[i] = wide(x[e]) + wide(y[e]);
+        else r[i] = wide(x[e]);
+      }
+    }
   }
 }
+static int row_blocks(int nrow) { return std::min((nrow + 7) / 8, 8 * sm_count()); }
 template <typename T>
 void launch_ref_to_dev(cudaStream_t s, const Geo &g, const double *ref, T *dev) {
-  k_ref_to_dev<T><<<1216, 256, 0, s>>>(g, ref, dev);
+  k_ref_to_dev<T, false><<<row_blocks(g.J * (g.K + 2)), 256, 0, s>>>(g, ref, dev, nullptr);
 }
 template <typename T>
 void launch_dev_to_ref(cudaStream_t s, const Geo &g, const T *dev, double *ref) {
-  k_dev_to_ref<T><<<1216, 256, 0, s>>>(g, dev, ref);
+  k_dev_to_ref<T, false><<<row_blocks((g.J + 2) * (g.K + 2)), 256, 0, s>>>(g, dev, nullptr, ref);
+}
+void launch_ref_to_dev_df(cudaStream_t s, const Geo &g, const double *ref, float *h, float *l) {
+  k_ref_to_dev<float, true><<<row_blocks(g.J * (g.K + 2)), 256, 0, s>>>(g, ref, h, l);
+}
+void launch_dev_to_ref_df(cudaStream_t s, const Geo &g, const float *h, const float *l, double *ref) {
+  k_dev_to_ref<float, true><<<row_blocks((g.J + 2) * (g.K + 2)), 256, 0, s>>>(g, h, l, ref);
 }
 template void launch_ref_to_dev<double>(cudaStream_t, const Geo &, const double *, double *);
 template void launch_ref_to_dev<float>(cudaStream_t, const Geo &, const double *, float *);
@@ -1526,8 +1579,6 @@ __device__ __forceinline__ void block_min_max(double &mn, double &mx) {
   mn = __longlong_as_double(n);
   mx = __longlong_as_double(x);
 }
-__device__ __forceinline__ double wide(float f) { return f2d_rn(f); }
-__device__ __forceinline__ double wide(double f) { return f; }
 // Larger value first, then the smaller index.  Values are kept as the bits of
 // a double >= 0 (or of -1: nothing seen), which order like the integers.
 __device__ __forceinline__ void max_loc(long long &m, long long &l, long long m2, long long l2) {

@@ -488,9 +488,8 @@ int alloc_all(ibm_ctx *c) {
   const Geo &g = c->g;
   const size_t nf = (size_t)g.nfield;
   int st;
-  if ((st = dalloc(c, &c->p, nf))) return st;
   if (!c->mixed) {
-    for (double **f : {&c->u, &c->v, &c->w})
+    for (double **f : {&c->u, &c->v, &c->w, &c->p})
       if ((st = dalloc(c, f, nf))) return st;
     for (double **f : {&c->ru, &c->rv, &c->rw, &c->fu, &c->fv, &c->fw, &c->phi})
       if ((st = dalloc(c, f, nf))) return st;
@@ -1206,41 +1205,50 @@ static const void *device_view(const void *h) {
   return nullptr;
 }
 
-static int upload_field(ibm_ctx *c, const double *h, double *d) {
+// device field <- reference layout (zero without one); lo: an FP32 pair d + lo
+extern "C++" {
+template <typename T>
+static int upload_any(ibm_ctx *c, const double *h, T *d, float *lo = nullptr) {
   const size_t n = (size_t)(c->g.I + 2) * (c->g.J + 2) * (c->g.K + 2);
   if (!h) {
-    CK(cudaMemsetAsync(d, 0, (size_t)c->g.nfield * sizeof(double), c->stream));
+    CK(cudaMemsetAsync(d, 0, (size_t)c->g.nfield * sizeof(T), c->stream));
     return IBM_OK;
   }
-  if (const double *dv = static_cast<const double *>(device_view(h))) {
-    launch_ref_to_dev<double>(c->stream, c->g, dv, d);
-    LAUNCHED(1);
-    return IBM_OK;
+  const double *src = static_cast<const double *>(device_view(h));
+  if (!src) {
+    CK(cudaMemcpyAsync(c->href, h, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    src = c->href;
   }
-  CK(cudaMemcpyAsync(c->href, h, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  launch_ref_to_dev<double>(c->stream, c->g, c->href, d);
+  if constexpr (sizeof(T) == 4) {
+    if (lo) launch_ref_to_dev_df(c->stream, c->g, src, d, lo);
+    else launch_ref_to_dev<T>(c->stream, c->g, src, d);
+  } else {
+    launch_ref_to_dev<T>(c->stream, c->g, src, d);
+  }
   LAUNCHED(1);
   return IBM_OK;
 }
 // the reference-layout copy of one device field into h (synchronised by the
 // caller)
-extern "C++" {
 template <typename T>
-static int download_any(ibm_ctx *c, const T *d, double *h) {
+static int download_any(ibm_ctx *c, const T *d, double *h, const float *lo = nullptr) {
   if (!h) return IBM_OK;
   const size_t n = (size_t)(c->g.I + 2) * (c->g.J + 2) * (c->g.K + 2);
-  if (double *dv = static_cast<double *>(const_cast<void *>(device_view(h)))) {
-    launch_dev_to_ref<T>(c->stream, c->g, d, dv);
-    LAUNCHED(1);
-    return IBM_OK;
+  double *view = static_cast<double *>(const_cast<void *>(device_view(h))), *dst = view ? view : c->href;
+  if constexpr (sizeof(T) == 4) {
+    if (lo) launch_dev_to_ref_df(c->stream, c->g, d, lo, dst);
+    else launch_dev_to_ref<T>(c->stream, c->g, d, dst);
+  } else {
+    launch_dev_to_ref<T>(c->stream, c->g, d, dst);
   }
-  launch_dev_to_ref<T>(c->stream, c->g, d, c->href);
   LAUNCHED(1);
+  if (view) return IBM_OK;
   CK(cudaMemcpyAsync(h, c->href, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));  // href is reused by the next field
   return IBM_OK;
 }
 }  // extern "C++"
+static int upload_field(ibm_ctx *c, const double *h, double *d) { return upload_any<double>(c, h, d); }
 static int download_field(ibm_ctx *c, const double *d, double *h) { return download_any<double>(c, d, h); }
 static int download_field32(ibm_ctx *c, const float *d, double *h) { return download_any<float>(c, d, h); }
 
@@ -1256,27 +1264,13 @@ int ibm_set_fields(ibm_ctx *c, const double *u, const double *v, const double *w
     for (int f = 0; f < 7; ++f)
       if ((st = upload_field(c, hs[f], ds[f]))) return st;
   } else {
-    if ((st = upload_field(c, p, c->p))) return st;
-    launch_d_to_df(c->stream, c->g.nfield, c->p, c->p32, c->plo32);
-    LAUNCHED(1);
-  }
-  if (c->mixed) {
+    if ((st = upload_any<float>(c, p, c->p32, c->plo32))) return st;
     float *d32[6] = {c->u32, c->v32, c->w32, c->ru32, c->rv32, c->rw32};
     const double *h32[6] = {u, v, w, durk, dvrk, dwrk};
-    for (int f = 0; f < 6; ++f) {
-      if (h32[f]) {
-        const size_t n = (size_t)(c->g.I + 2) * (c->g.J + 2) * (c->g.K + 2);
-        const double *src = static_cast<const double *>(device_view(h32[f]));
-        if (!src) {
-          CK(cudaMemcpyAsync(c->href, h32[f], n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-          src = c->href;
-        }
-        launch_ref_to_dev<float>(c->stream, c->g, src, d32[f]);
-        LAUNCHED(1);
-      } else {
-        CK(cudaMemsetAsync(d32[f], 0, (size_t)c->g.nfield * sizeof(float), c->stream));
-      }
-    }
+    for (int f = 0; f < 6; ++f)
+      if ((st = upload_any<float>(c, h32[f], d32[f]))) return st;
+  }
+  if (c->mixed) {
     for (float *f : {c->fu32, c->fv32, c->fw32}) CK(cudaMemsetAsync(f, 0, (size_t)c->g.nfield * sizeof(float), c->stream));
   } else {
     // dudtf starts from zero (module storage), in particular its k1 plane
@@ -1299,11 +1293,7 @@ int ibm_get_fields(ibm_ctx *c, double *u, double *v, double *w, double *p, doubl
     CK(cudaStreamSynchronize(c->stream));
     return IBM_OK;
   }
-  if (p) {
-    launch_df_to_d(c->stream, c->g.nfield, c->p32, c->plo32, c->p);
-    LAUNCHED(1);
-  }
-  if ((st = download_field(c, c->p, p))) return st;
+  if ((st = download_any<float>(c, c->p32, p, c->plo32))) return st;
   const float *d32[6] = {c->u32, c->v32, c->w32, c->ru32, c->rv32, c->rw32};
   double *h32[6] = {u, v, w, durk, dvrk, dwrk};
   for (int f = 0; f < 6; ++f)

@@ -160,44 +160,38 @@ __device__ __forceinline__ double f2d_exact(float f) {  // positive normal
   const unsigned b = __float_as_uint(f);
   return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
 }
-// Conversions with the results of (double)f and (float)d (round to nearest
-// even), on the integer pipe: the conversion instructions issue at the rate of
-// FP64.  Values that are not normal in FP32 take the conversions.
+// (double)f on the integer pipe: the conversion instructions issue at the rate
+// of FP64, predicated off or not, so every kind of value is covered.
 __device__ __forceinline__ double f2d_rn(float f) {
-  const unsigned b = __float_as_uint(f), a = b & 0x7fffffffu, sg = b & 0x80000000u;
-  if (a == 0u || a - 0x00800000u < 0x7f000000u)
-    return __hiloint2double((int)((a ? (a >> 3) + 0x38000000u : 0u) | sg), (int)(b << 29));
-  return (double)f;
+  const bool sub = (__float_as_uint(f) & 0x7f800000u) == 0u;
+  const unsigned b = __float_as_uint(sub ? f * 1.8446744073709552e19f : f), a = b & 0x7fffffffu;  // 2^64
+  unsigned off = sub ? 0x34000000u : 0x38000000u;
+  if (a >= 0x7f800000u) off = 0x70000000u;  // infinity, NaN
+  if (a == 0u) off = 0u;
+  return __hiloint2double((int)(((a >> 3) + off) | (b & 0x80000000u)), (int)(b << 29));
 }
-// rem: d - f in units of d's last place, |rem| <= 2^28 (in the integer path)
+// (float)d, to nearest even, on the integer pipe; false: not a value of FP32's
+// normal range, f is not valid.  rem: d - f in units of d's last place,
+// |rem| <= 2^28.
 __device__ __forceinline__ bool d2f_int(double d, float &f, int &rem) {
   const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d), a = hi & 0x7fffffffu;
   const unsigned r = lo & 0x1fffffffu;
   unsigned b = __funnelshift_l(lo, a - 0x38000000u, 3);
   const bool up = r + (b & 1u) > 0x10000000u;
   b += up;
-  f = __uint_as_float(b | (hi & 0x80000000u));
+  const bool zero = (a | lo) == 0u;
+  f = __uint_as_float((zero ? 0u : b) | (hi & 0x80000000u));
   rem = (int)r - (up ? 0x20000000 : 0);
-  return a - 0x38100000u < 0x47d00000u - 0x38100000u;  // 2^-126 <= |d| < 2^126
+  return zero || a - 0x38100000u < 0x47d00000u - 0x38100000u;  // 2^-126 <= |d| < 2^126
 }
-__device__ __forceinline__ float d2f_rn(double d) {
-  float f;
+// d as an FP32 pair: h = (float)d, l = (float)(d - h); false: not valid
+__device__ __forceinline__ bool d2df_int(double d, float &h, float &l) {
   int rem;
-  if (d2f_int(d, f, rem)) return f;
-  return (float)d;
-}
-// d as an FP32 pair: h = (float)d, l = (float)(d - h)
-__device__ __forceinline__ void d2df(double d, float &h, float &l) {
-  int rem;
-  if (d2f_int(d, h, rem)) {
-    const unsigned hi = (unsigned)__double2hiint(d), e = (hi & 0x7fffffffu) >> 20;  // 2^(e - 1023) <= |d|
-    if (e >= 949u) {  // the last place 2^(e - 1075) is normal in FP32
-      l = (float)((int)hi < 0 ? -rem : rem) * __uint_as_float((e - 948u) << 23);
-      return;
-    }
-  }
-  h = (float)d;
-  l = (float)(d - (double)h);
+  const bool ok = d2f_int(d, h, rem);
+  const unsigned hi = (unsigned)__double2hiint(d), e = (hi & 0x7fffffffu) >> 20;  // 2^(e - 1023) <= |d|
+  // the last place, 2^(e - 1075), is normal in FP32 from e = 949 on
+  l = rem == 0 ? 0.f : (float)((int)hi < 0 ? -rem : rem) * __uint_as_float((e - 948u) << 23);
+  return ok && (e >= 949u || rem == 0);
 }
 __device__ __forceinline__ double sqrt_newton(double x) {
   if (!fp32_range(x)) return sqrt(x);

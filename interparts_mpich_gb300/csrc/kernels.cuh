@@ -31,10 +31,11 @@ void launch_correc_mixed2(cudaStream_t s, const Geo &g, const float *fu, const f
 void launch_correc_mixed(cudaStream_t s, const Geo &g, const float *fu, const float *fv, const float *fw,
                          const float *phi, float *u, float *v, float *w, float *ph, float *pl, double fi, double fj,
                          double fk);
-void launch_df_to_d(cudaStream_t s, long n, const float *h, const float *l, double *d);
-void launch_d_to_df(cudaStream_t s, long n, const double *d, float *h, float *l);
 template <typename T> void launch_ref_to_dev(cudaStream_t s, const Geo &g, const double *ref, T *dev);
 template <typename T> void launch_dev_to_ref(cudaStream_t s, const Geo &g, const T *dev, double *ref);
+// the same for a field held as an FP32 pair h + l
+void launch_ref_to_dev_df(cudaStream_t s, const Geo &g, const double *ref, float *h, float *l);
+void launch_dev_to_ref_df(cudaStream_t s, const Geo &g, const float *h, const float *l, double *ref);
 template <typename T>
 void launch_chkdiv(cudaStream_t s, const Geo &g, const T *u, const T *v, const T *w, double *scratch, double *out);
 template <typename T>

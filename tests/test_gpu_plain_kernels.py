@@ -146,3 +146,36 @@ def test_time_step_control(gpu_lib, grid, flow, mode):
     # no divergence anywhere: the library names the first cell, the oracle none
     assert tuple(a[2]) == (tuple(b[2]) if b[1] > 0 else (1, 1, 1))
     assert abs(a[0] - b[0]) <= 1e-12 * nx * ny * nz
+
+
+# rows below, at and beyond a warp's 32 x 4 cells; values of every kind that
+# rounds: ties, the largest and smallest of FP32, subnormal, zero of both signs
+@pytest.mark.parametrize("grid", [(4, 9, 4), (36, 27, 4), (128, 4, 5), (144, 9, 6), (256, 12, 4)])
+@pytest.mark.parametrize("mode", [_abi.IBM_MODE_PLAIN_FP64, _abi.IBM_MODE_MIXED])
+def test_field_conversions(gpu_lib, grid, mode):
+    nx, ny, nz = grid
+    case = Case(name="layout", itot=nx, jtot=ny, ktot=nz, lx=nx / 32, ly=ny / 32, lz=nz / 32, visc=1e-2)
+    rng = np.random.default_rng(1)
+
+    def field():
+        f = rng.uniform(-1, 1, case.shape) * 10.0 ** rng.integers(-44, 37, case.shape)
+        odd = np.array([0.0, -0.0, 1 + 2.0 ** -24, 1 + 3 * 2.0 ** -24, -1 + 2.0 ** -25, 3.4028234e38, 1.1754944e-38,
+                        1.17549429e-38, 2.0 ** -149, 2.0 ** -150, 2.0 ** 126, 2 - 2.0 ** -30, -(2.0 ** -74), 2.0 ** -75])
+        pick = rng.random(case.shape) < 0.2
+        f[pick] = rng.choice(odd, pick.sum())
+        return np.asfortranarray(f)
+
+    f = {n: field() for n in ("u", "v", "w", "p", "durk", "dvrk", "dwrk")}
+    s = IBMSolver(case, mode=mode)
+    s.set_fields(**f)
+    got = s.get_fields()
+    for n, a in f.items():
+        want = a.copy()
+        if mode == _abi.IBM_MODE_MIXED:
+            hi = a.astype(np.float32)
+            want = hi.astype(np.float64)
+            if n == "p":
+                want += (a - want).astype(np.float32)
+        want[0], want[-1] = want[-2], want[1]
+        want[:, 0], want[:, -1] = want[:, -2], want[:, 1]
+        assert np.array_equal(got[n], want), n
