@@ -112,6 +112,12 @@ __device__ __forceinline__ int p_toff(const PartGeo &pg, int p) { return pg.poly
 __host__ __device__ inline long fidx(const Geo &g, int i, int j, int k) {
   return ((long)k * g.J + j) * g.I + i;
 }
+// q / d for q < 2^16 and 1 <= d < 2^16 as one multiplication
+struct FastDiv {
+  unsigned m;
+  __device__ __forceinline__ explicit FastDiv(int d) : m(0xffffffffu / (unsigned)d + 1u) {}
+  __device__ __forceinline__ int operator()(int q, int d) const { return d == 1 ? q : (int)__umulhi((unsigned)q, m); }
+};
 __device__ __forceinline__ int wrapm(int i, int n) {  // i in [-n, 2n)
   return i < 0 ? i + n : (i >= n ? i - n : i);
 }

@@ -127,12 +127,6 @@ struct BoxLay {
     return ((s.b[2] - bg[4]) * nby + (s.b[1] - bg[3])) * pitch + (s.b[0] - bg[2]) + sh;
   }
 };
-// q / d for q < 2^16 and 1 <= d < 2^16 as one multiplication
-struct FastDiv {
-  unsigned m;
-  __device__ __forceinline__ explicit FastDiv(int d) : m(0xffffffffu / (unsigned)d + 1u) {}
-  __device__ __forceinline__ int operator()(int q, int d) const { return d == 1 ? q : (int)__umulhi((unsigned)q, m); }
-};
 // Points of particle p, component c by the bank of their first tap:
 // order[(p*3 + c)*nl + bst[q] ..bst[q+1]) = those of bank q, bst[33] = the most
 // of any bank (bst: IBM_BST entries per (p, c)); -1 there where the points are
