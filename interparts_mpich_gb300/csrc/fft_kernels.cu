@@ -498,167 +498,96 @@ __global__ void __launch_bounds__(256) k_ffty(Geo g, FftPlan ply, typename cpx<T
   }
 }
 
-// Thomas sweep along z for every (kx,ky) (solver.f90:94-134), FP64, with
-// the precomputed pivots zt (pivot reciprocal for k<K, denominator for k=K).
-template <typename T>
-__global__ void __launch_bounds__(64) k_thomas(Geo g, typename cpx<T>::t *__restrict__ S,
-                                                const double *__restrict__ zt, double a2, double scale) {
-  typedef typename cpx<T>::t C;
-  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const long ncol = (long)g.MX * g.J;
-  if (t >= ncol) return;
-  const int kx = (int)(t % g.MX), ky = (int)(t / g.MX);
+// Thomas sweep along z for every (kx,ky) (solver.f90:94-134), FP64.  With
+// R = dzi^2 r, r the forward value, both sweeps need one factor per (k, |ky|,
+// kx), c_k = dzi^2 / den_k (den_k the pivots; 0 in the last plane of the zero
+// mode, which is pinned there):
+//   R_k = c_k (d_k - R_(k-1)),   X_k = R_k - c_k X_(k+1),   x = X oscale,
+// oscale the transforms' scale over dzi^2.
+//
+// Periodic z (CYC): Sherman-Morrison around the sweep (T: diagonal -2 a2 + xy
+// with its two ends changed, off-diagonals a2 = dzi^2; u = (gamma, 0.., 0, a2),
+// gamma = -b), the zero mode pinned at its last plane.  Tables behind the c_k:
+// z = T^-1 u and gi = 1 / (gamma (1 + z_0 + a2 z_(K-1) / gamma)).  T is
+// symmetric, so the factor of the correction, f = (y_0 + a2 y_(K-1) / gamma)
+// gamma gi with y = T^-1 r, is (z . r) gi: known after the forward sweep, and
+// the back substitution stores y - f z at once.
+//
+// Bound by the instructions of each thread's chain where columns are few, by
+// memory where they are many.  Real and imaginary parts do not meet, so each
+// has a thread; the next planes are loaded while the current ones are worked
+// on.  64^3 cyclic: 40 -> 22 us, 96 x 108 x 75: 45 -> 19, 384 x 192 x 128:
+// 104 -> 78 (a thread per complex column, pivots and dzi^2 apart).
+template <bool CYC>
+__global__ void __launch_bounds__(64) k_thomas(Geo g, double *__restrict__ S, const double *__restrict__ tab,
+                                               double oscale) {
+  const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const int ncol = g.MX * g.J;
+  if (e >= 2l * ncol) return;
+  const int t = (int)(e >> 1), ky = t / g.MX, kx = t - ky * g.MX;
   const int kyy = ky <= g.J / 2 ? ky : g.J - ky;
-  const long zstride = (long)(g.J / 2 + 1) * g.MX;
-  const double *z = zt + (long)kyy * g.MX + kx;
-  const long sstride = (long)g.J * g.MX;
-  C *s = S + t;
-  // The recurrence is a dependent chain over k; loads of the next planes
-  // are issued in groups of PF so that several are in flight at once.
+  const int sst = 2 * ncol, zst = (g.J / 2 + 1) * g.MX, K = g.K;
+  const double *cp = tab + kyy * g.MX + kx, *zp = cp + (long)K * zst;
+  double *s = S + e;
   constexpr int PF = 8;
-  auto ld = [&](int k) -> double2 {
-    const C v = s[k * sstride];
-    return make_double2((double)v.x * scale, (double)v.y * scale);
+  double v[2][PF], c[2][PF], z[2][CYC ? PF : 1];
+  double r = 0., f = 0.;
+  // plane k0 + q (forward), k0 - q (backward)
+  auto load = [&](int slot, int k0, int dir) {
+    const double *sk = s + (long)k0 * sst, *ck = cp + (long)k0 * zst, *zk = zp + (long)k0 * zst;
+    const int n = dir > 0 ? K - k0 : k0 + 1;
+#pragma unroll
+    for (int q = 0; q < PF; ++q)
+      if (q < n) {
+        v[slot][q] = sk[(long)(dir * q) * sst];
+        c[slot][q] = ck[(long)(dir * q) * zst];
+        if constexpr (CYC) z[slot][q] = zk[(long)(dir * q) * zst];
+      }
   };
-  auto st = [&](int k, double2 v) { C o; o.x = (decltype(o.x))v.x; o.y = (decltype(o.y))v.y; s[k * sstride] = o; };
-  const int K = g.K;
-  double2 prev = make_double2(0., 0.);
-  for (int k0 = 0; k0 < K; k0 += PF) {
-    double2 buf[PF];
-    double zb[PF];
+  auto fwd = [&](int slot, int k0) {
+    double *sk = s + (long)k0 * sst;
 #pragma unroll
     for (int q = 0; q < PF; ++q) {
-      const int k = k0 + q;
-      if (k < K) { buf[q] = ld(k); zb[q] = z[(long)k * zstride]; }
+      if (k0 + q >= K) break;
+      if constexpr (CYC) f = fma(z[slot][q], v[slot][q], f);
+      r = fma(-c[slot][q], r, c[slot][q] * v[slot][q]);
+      sk[(long)q * sst] = r;
     }
+  };
+  auto bwd = [&](int slot, int k0) {
+    double *sk = s + (long)k0 * sst;
 #pragma unroll
     for (int q = 0; q < PF; ++q) {
-      const int k = k0 + q;
-      if (k >= K) break;
-      double2 cur = buf[q];
-      if (k == 0) {
-        cur = make_double2(cur.x * zb[q], cur.y * zb[q]);
-      } else if (k < K - 1) {
-        cur = make_double2((cur.x - a2 * prev.x) * zb[q], (cur.y - a2 * prev.y) * zb[q]);
-      } else {
-        const double den = zb[q];
-        if (den != 0.) cur = make_double2((cur.x - a2 * prev.x) / den, (cur.y - a2 * prev.y) / den);
-        else cur = make_double2(0., 0.);
-      }
-      buf[q] = cur;
-      prev = cur;
+      if (k0 - q < 0) break;
+      r = fma(-c[slot][q], r, v[slot][q]);
+      sk[-(long)q * sst] = CYC ? fma(f, z[slot][q], r * oscale) : r * oscale;
     }
-#pragma unroll
-    for (int q = 0; q < PF; ++q)
-      if (k0 + q < K) st(k0 + q, buf[q]);
+  };
+  load(0, 0, 1);
+  for (int k0 = 0; k0 < K; k0 += 2 * PF) {
+    if (k0 + PF < K) load(1, k0 + PF, 1);
+    fwd(0, k0);
+    if (k0 + PF >= K) break;
+    if (k0 + 2 * PF < K) load(0, k0 + 2 * PF, 1);
+    fwd(1, k0 + PF);
   }
-  // back substitution, d(k) = c(k)*z(k) with c(k) = dzi^2 for k < kmax
-  for (int k1 = K - 2; k1 >= 0; k1 -= PF) {
-    double2 buf[PF];
-    double zb[PF];
-#pragma unroll
-    for (int q = 0; q < PF; ++q) {
-      const int k = k1 - q;
-      if (k >= 0) {
-        const C v = s[k * sstride];
-        buf[q] = make_double2((double)v.x, (double)v.y);
-        zb[q] = z[(long)k * zstride];
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < PF; ++q) {
-      const int k = k1 - q;
-      if (k < 0) break;
-      const double d = a2 * zb[q];
-      const double2 cur = make_double2(buf[q].x - d * prev.x, buf[q].y - d * prev.y);
-      buf[q] = cur;
-      prev = cur;
-    }
-#pragma unroll
-    for (int q = 0; q < PF; ++q)
-      if (k1 - q >= 0) st(k1 - q, buf[q]);
+  // z . r is in units of the right-hand side, z of the solution's
+  if constexpr (CYC) f *= -zp[(long)K * zst] * (g.dzi * g.dzi) * oscale;
+  r = 0.;
+  load(0, K - 1, -1);
+  for (int k0 = K - 1; k0 >= 0; k0 -= 2 * PF) {
+    if (k0 - PF >= 0) load(1, k0 - PF, -1);
+    bwd(0, k0);
+    if (k0 - PF < 0) break;
+    if (k0 - 2 * PF >= 0) load(0, k0 - 2 * PF, -1);
+    bwd(1, k0 - PF);
   }
 }
 
-// Periodic z: the cyclic tridiagonal solve of every (kx, ky) mode in FP64,
-// one thread per column: Sherman-Morrison around the Thomas sweep (T: diagonal
-// -2 a2 + xy with its two ends changed, off-diagonals a2; u = (gamma, 0.., 0,
-// a2), gamma = -b), the zero mode pinned at its last plane.  Everything that
-// does not depend on the right-hand side comes from tables over (k, |ky|, kx):
-//   cp[k] = a2 / den_k, iv[k] = 1 / den_k (the pivots), z = T^-1 u,
-//   gi = 1 / (gamma (1 + z_0 + a2 z_(K-1) / gamma)).
-// T is symmetric, so the factor of the correction, f = (y_0 + a2 y_(K-1) /
-// gamma) gamma gi with y = T^-1 r, is (z . r) gi: it is known after the forward
-// sweep, and the back substitution stores y - f z at once.  The dependent
-// chain is one multiply-add a plane in each direction (three divisions before,
-// and two more passes over the column): 64^3, 279 -> 40 us.
-__global__ void __launch_bounds__(64) k_thomas_cyclic(Geo g, double2 *__restrict__ S, const double *__restrict__ tab,
-                                                      double scale) {
-  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const long ncol = (long)g.MX * g.J;
-  if (t >= ncol) return;
-  const int kx = (int)(t % g.MX), ky = (int)(t / g.MX);
-  const int kyy = ky <= g.J / 2 ? ky : g.J - ky;
-  const long sstride = ncol, zst = (long)(g.J / 2 + 1) * g.MX, col = (long)kyy * g.MX + kx;
-  const int K = g.K;
-  const double *cp = tab + col, *iv = cp + K * zst, *z = iv + K * zst;
-  const double gi = tab[3 * K * zst + col];
-  double2 *s = S + t;
-  constexpr int PF = 16;
-  double2 r = make_double2(0., 0.), f = r;
-  for (int k0 = 0; k0 < K; k0 += PF) {
-    double2 v[PF];
-    double c[PF], d[PF], e[PF];
-#pragma unroll
-    for (int q = 0; q < PF; ++q) {
-      const int k = k0 + q;
-      if (k < K) { v[q] = s[k * sstride]; c[q] = cp[k * zst]; d[q] = iv[k * zst]; e[q] = z[k * zst]; }
-    }
-#pragma unroll
-    for (int q = 0; q < PF; ++q) {
-      const int k = k0 + q;
-      if (k >= K) break;
-      const double2 w = make_double2(v[q].x * scale, v[q].y * scale);
-      f.x = fma(e[q], w.x, f.x);
-      f.y = fma(e[q], w.y, f.y);
-      const double m = k ? -c[q] : 0.;
-      r.x = fma(m, r.x, w.x * d[q]);
-      r.y = fma(m, r.y, w.y * d[q]);
-      v[q] = r;
-    }
-#pragma unroll
-    for (int q = 0; q < PF; ++q)
-      if (k0 + q < K) s[(k0 + q) * sstride] = v[q];
-  }
-  f.x *= -gi;
-  f.y *= -gi;
-  r = make_double2(0., 0.);
-  for (int k1 = K - 1; k1 >= 0; k1 -= PF) {
-    double2 v[PF];
-    double c[PF], e[PF];
-#pragma unroll
-    for (int q = 0; q < PF; ++q) {
-      const int k = k1 - q;
-      if (k >= 0) { v[q] = s[k * sstride]; c[q] = cp[k * zst]; e[q] = z[k * zst]; }
-    }
-#pragma unroll
-    for (int q = 0; q < PF; ++q) {
-      const int k = k1 - q;
-      if (k < 0) break;
-      r.x = fma(-c[q], r.x, v[q].x);
-      r.y = fma(-c[q], r.y, v[q].y);
-      v[q] = make_double2(fma(f.x, e[q], r.x), fma(f.y, e[q], r.y));
-    }
-#pragma unroll
-    for (int q = 0; q < PF; ++q)
-      if (k1 - q >= 0) s[(k1 - q) * sstride] = v[q];
-  }
-}
-
-// The tables of k_thomas_cyclic, one thread per (kx, |ky|).  The zero mode is
+// The tables of k_thomas<true>, one thread per (kx, |ky|).  The zero mode is
 // pinned at its last plane: rows 0..K-2 alone, z = 0 (cp = iv = 0 in row K-1).
 // Products are rounded one by one, as on a host.  Formed here rather than there
-// and copied (3 K entries a column): a
+// and copied (2 K entries a column): a
 // context of 64^3 cells is ready 0.6 ms earlier.
 __global__ void __launch_bounds__(64) k_cyclic_tables(Geo g, const double *__restrict__ xrt,
                                                       const double *__restrict__ yrt, double *__restrict__ tab) {
@@ -667,7 +596,7 @@ __global__ void __launch_bounds__(64) k_cyclic_tables(Geo g, const double *__res
   const int K = g.K;
   const double a2 = g.dzi * g.dzi, xy = xrt[col % g.MX] + yrt[col / g.MX], bb = -2. * a2 + xy, gamma = -bb;
   const bool zero = xy == 0.;
-  double *cp = tab + col, *iv = cp + K * nz, *z = iv + K * nz;
+  double *cp = tab + col, *z = cp + K * nz;
   double c = 0., zz = 0.;
   for (int k = 0; k < K; ++k) {
     const bool last = k == K - 1;
@@ -678,7 +607,6 @@ __global__ void __launch_bounds__(64) k_cyclic_tables(Geo g, const double *__res
     // forward sweep of T z = u, u = (gamma, 0.., 0, a2)
     zz = zero ? 0. : ((k == 0 ? gamma : (last ? a2 : 0.)) - __dmul_rn(a2, zz)) * v;
     cp[k * nz] = c;
-    iv[k * nz] = v;
     z[k * nz] = zz;
   }
   const double zl = zz;
@@ -686,107 +614,84 @@ __global__ void __launch_bounds__(64) k_cyclic_tables(Geo g, const double *__res
     zz = z[k * nz] - __dmul_rn(cp[k * nz], zz);
     z[k * nz] = zz;
   }
-  tab[3 * K * nz + col] = zero ? 0. : 1. / (gamma * (1. + zz + a2 * zl / gamma));
+  tab[2 * K * nz + col] = zero ? 0. : 1. / (gamma * (1. + zz + a2 * zl / gamma));
 }
 void launch_cyclic_tables(cudaStream_t s, const Geo &g, const double *xrt, const double *yrt, double *tab) {
   const long nz = (long)(g.J / 2 + 1) * g.MX;
   k_cyclic_tables<<<(unsigned)((nz + 63) / 64), 64, 0, s>>>(g, xrt, yrt, tab);
 }
 
-// Thomas sweep of the mixed form in double-float arithmetic (pairs of FP32
-// with error-free products and sums, ~48 significant bits) on the FP32
-// pipes; GB300 issues FP64 at 1/64 of the FP32 rate.  Tables (built on the
-// host in FP64, split hi + lo): zt[k] for k < K-1 and 1/den for k = K-1 (0
-// for the zero mode), azt[k] = dzi^2 * zt[k] for the back substitution.  The
-// recurrence carries its value in double-float from plane to plane; the
-// forward intermediate between the sweeps is kept in the FP32 spectrum, and
-// the 1/(M*J) FFT scale is applied at the final FP32 store.
-__global__ void __launch_bounds__(64) k_thomas_df(Geo g, float2 *__restrict__ S, const float2 *__restrict__ zt,
-                                                   const float2 *__restrict__ azt, float a2h, float a2l,
-                                                   float fscale) {
-  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const long ncol = (long)g.MX * g.J;
-  if (t >= ncol) return;
-  const int kx = (int)(t % g.MX), ky = (int)(t / g.MX);
+// The same sweep for the mixed form in double-float arithmetic (pairs of FP32
+// with error-free products and sums, ~48 significant bits) on the FP32 pipes;
+// GB300 issues FP64 at 1/64 of the FP32 rate.  Table: c_k, formed in FP64 and
+// split hi + lo.  The recurrence carries its value in double-float from plane
+// to plane; the forward intermediate between the sweeps is kept in the FP32
+// spectrum, and oscale (a pair) is applied at the final FP32 store.  256^3:
+// 70 -> 64 us, 512 x 512 x 256: 271 -> 229.
+__global__ void __launch_bounds__(64) k_thomas_df(Geo g, float *__restrict__ S, const float2 *__restrict__ tab,
+                                                  float osh, float osl) {
+  const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const int ncol = g.MX * g.J;
+  if (e >= 2l * ncol) return;
+  const int t = (int)(e >> 1), ky = t / g.MX, kx = t - ky * g.MX;
   const int kyy = ky <= g.J / 2 ? ky : g.J - ky;
-  const long zstride = (long)(g.J / 2 + 1) * g.MX;
-  const float2 *z = zt + (long)kyy * g.MX + kx;
-  const float2 *az = azt + (long)kyy * g.MX + kx;
-  const long sstride = (long)g.J * g.MX;
-  float2 *s = S + t;
-  const int K = g.K;
+  const int sst = 2 * ncol, zst = (g.J / 2 + 1) * g.MX, K = g.K;
+  const float2 *cp = tab + kyy * g.MX + kx;
+  float *s = S + e;
   constexpr int PF = 16;
-  // previous plane's value, real and imaginary parts, double-float
-  float prh = 0.f, prl = 0.f, pih = 0.f, pil = 0.f;
-  // Both sweeps run over chunks of PF planes with the next chunk's loads
-  // issued before the current chunk is computed (two buffers), so that the
-  // HBM latency of a chunk overlaps the dependent double-float chain of the
-  // previous one.
-  float2 buf[2][PF], cb[2][PF];
-  auto load_fwd = [&](int slot, int k0) {
+  float v[2][PF];
+  float2 c[2][PF];
+  float rh = 0.f, rl = 0.f;
+  auto load = [&](int slot, int k0, int dir) {
+    const float *sk = s + (long)k0 * sst;
+    const float2 *ck = cp + (long)k0 * zst;
+    const int n = dir > 0 ? K - k0 : k0 + 1;
 #pragma unroll
-    for (int q = 0; q < PF; ++q) {
-      const int k = k0 + q;
-      if (k < K) { buf[slot][q] = s[k * sstride]; cb[slot][q] = z[(long)k * zstride]; }
-    }
+    for (int q = 0; q < PF; ++q)
+      if (q < n) {
+        v[slot][q] = sk[(long)(dir * q) * sst];
+        c[slot][q] = ck[(long)(dir * q) * zst];
+      }
   };
   auto fwd = [&](int slot, int k0) {
+    float *sk = s + (long)k0 * sst;
 #pragma unroll
     for (int q = 0; q < PF; ++q) {
-      const int k = k0 + q;
-      if (k >= K) break;
-      float rh = buf[slot][q].x, rl = 0.f, ih = buf[slot][q].y, il = 0.f;
-      if (k > 0) {  // d - dzi^2 * prev
-        float qh, ql;
-        df_mul(a2h, a2l, prh, prl, qh, ql);
-        df_add(rh, rl, -qh, -ql, rh, rl);
-        df_mul(a2h, a2l, pih, pil, qh, ql);
-        df_add(ih, il, -qh, -ql, ih, il);
-      }
-      // times the pivot reciprocal (k < K-1) or 1/den (k = K-1)
-      df_mul(rh, rl, cb[slot][q].x, cb[slot][q].y, prh, prl);
-      df_mul(ih, il, cb[slot][q].x, cb[slot][q].y, pih, pil);
-      const float2 o = make_float2(__fadd_rn(prh, prl), __fadd_rn(pih, pil));
-      if (k < K - 1) s[k * sstride] = o;
-      else s[k * sstride] = make_float2(o.x * fscale, o.y * fscale);
+      if (k0 + q >= K) break;
+      float h, l;
+      df_add(v[slot][q], 0.f, -rh, -rl, h, l);
+      df_mul(h, l, c[slot][q].x, c[slot][q].y, rh, rl);
+      sk[(long)q * sst] = rh;
     }
   };
-  load_fwd(0, 0);
+  auto bwd = [&](int slot, int k0) {
+    float *sk = s + (long)k0 * sst;
+#pragma unroll
+    for (int q = 0; q < PF; ++q) {
+      if (k0 - q < 0) break;
+      float h, l;
+      df_mul(c[slot][q].x, c[slot][q].y, rh, rl, h, l);
+      df_add(v[slot][q], 0.f, -h, -l, rh, rl);
+      sk[-(long)q * sst] = fmaf(rh, osh, fmaf(rh, osl, rl * osh));
+    }
+  };
+  load(0, 0, 1);
   for (int k0 = 0; k0 < K; k0 += 2 * PF) {
-    if (k0 + PF < K) load_fwd(1, k0 + PF);
+    if (k0 + PF < K) load(1, k0 + PF, 1);
     fwd(0, k0);
     if (k0 + PF >= K) break;
-    if (k0 + 2 * PF < K) load_fwd(0, k0 + 2 * PF);
+    if (k0 + 2 * PF < K) load(0, k0 + 2 * PF, 1);
     fwd(1, k0 + PF);
   }
-  // back substitution x_k = x'_k - dzi^2 z_k x_{k+1}
-  auto load_bwd = [&](int slot, int k1) {
-#pragma unroll
-    for (int q = 0; q < PF; ++q) {
-      const int k = k1 - q;
-      if (k >= 0) { buf[slot][q] = s[k * sstride]; cb[slot][q] = az[(long)k * zstride]; }
-    }
-  };
-  auto bwd = [&](int slot, int k1) {
-#pragma unroll
-    for (int q = 0; q < PF; ++q) {
-      const int k = k1 - q;
-      if (k < 0) break;
-      float qh, ql;
-      df_mul(cb[slot][q].x, cb[slot][q].y, prh, prl, qh, ql);
-      df_add(buf[slot][q].x, 0.f, -qh, -ql, prh, prl);
-      df_mul(cb[slot][q].x, cb[slot][q].y, pih, pil, qh, ql);
-      df_add(buf[slot][q].y, 0.f, -qh, -ql, pih, pil);
-      s[k * sstride] = make_float2(__fadd_rn(prh, prl) * fscale, __fadd_rn(pih, pil) * fscale);
-    }
-  };
-  if (K >= 2) load_bwd(0, K - 2);
-  for (int k1 = K - 2; k1 >= 0; k1 -= 2 * PF) {
-    if (k1 - PF >= 0) load_bwd(1, k1 - PF);
-    bwd(0, k1);
-    if (k1 - PF < 0) break;
-    if (k1 - 2 * PF >= 0) load_bwd(0, k1 - 2 * PF);
-    bwd(1, k1 - PF);
+  // the last plane is final, and goes on unrounded
+  s[(long)(K - 1) * sst] = fmaf(rh, osh, fmaf(rh, osl, rl * osh));
+  load(0, K - 2, -1);
+  for (int k0 = K - 2; k0 >= 0; k0 -= 2 * PF) {
+    if (k0 - PF >= 0) load(1, k0 - PF, -1);
+    bwd(0, k0);
+    if (k0 - PF < 0) break;
+    if (k0 - 2 * PF >= 0) load(0, k0 - 2 * PF, -1);
+    bwd(1, k0 - PF);
   }
 }
 
@@ -832,19 +737,19 @@ __global__ void __launch_bounds__(128) k_ifftx(Geo g, FftPlan plx, const typenam
 // Thomas sweep along z between the forward and inverse transforms
 template <typename T>
 void launch_thomas(cudaStream_t s, const Geo &g, typename cpx<T>::t *S, const double *zt, const float2 *thomas_df) {
-  const long ncol = (long)g.MX * g.J;
+  const long n = 2l * g.MX * g.J;
   // small blocks: the columns spread over the SMs (FP64: each has its own slow
-  // pipe; 96 x 108 x 75, 5292 columns: 47.6 us with 128 threads, 45.4 with 32)
-  const int bs = ncol < 64 * 1216 ? 32 : 64;
-  const double scale = 1.0 / ((double)(g.I / 2) * g.J), a2 = g.dzi * g.dzi;
+  // pipe)
+  const int bs = n < 64 * 1216 ? 32 : 64;
+  const unsigned nb = (unsigned)((n + bs - 1) / bs);
+  const double oscale = 1.0 / ((double)(g.I / 2) * g.J) / (g.dzi * g.dzi);
   if constexpr (sizeof(T) == 4) {
-    const float a2h = (float)a2, a2l = (float)(a2 - (double)a2h);
-    k_thomas_df<<<(unsigned)((ncol + bs - 1) / bs), bs, 0, s>>>(g, S, thomas_df, thomas_df + (long)g.K * (g.J / 2 + 1) * g.MX, a2h, a2l,
-                                     (float)scale);
+    const float osh = (float)oscale;
+    k_thomas_df<<<nb, bs, 0, s>>>(g, (float *)S, thomas_df, osh, (float)(oscale - (double)osh));
   } else if (g.zper) {
-    k_thomas_cyclic<<<(unsigned)((ncol + bs - 1) / bs), bs, 0, s>>>(g, S, zt, scale);
+    k_thomas<true><<<nb, bs, 0, s>>>(g, (double *)S, zt, oscale);
   } else {
-    k_thomas<T><<<(unsigned)((ncol + bs - 1) / bs), bs, 0, s>>>(g, S, zt, a2, scale);
+    k_thomas<false><<<nb, bs, 0, s>>>(g, (double *)S, zt, oscale);
   }
 }
 

@@ -434,7 +434,7 @@ int build_solver_tables(ibm_ctx *c) {
   if (g.zper) {
     // periodic z: the cyclic sweep's tables over (k, |ky|, kx), with the
     // eigenvalues they are formed from behind them
-    const size_t nz = (size_t)(J / 2 + 1) * MX, n = (size_t)3 * K * nz + nz;
+    const size_t nz = (size_t)(J / 2 + 1) * MX, n = (size_t)2 * K * nz + nz;
     if ((st = dalloc(c, &c->zt, n + xrt.size() + yrt.size()))) return st;
     double *dx = c->zt + n, *dy = dx + xrt.size();
     CK(cudaMemcpyAsync(dx, xrt.data(), xrt.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
@@ -444,42 +444,36 @@ int build_solver_tables(ibm_ctx *c) {
     CK(cudaStreamSynchronize(c->stream));
     return IBM_OK;
   }
+  // the sweeps' factors dzi^2 / den, 0 in the last plane of the zero mode
   const long zst = (long)(J / 2 + 1) * MX;
+  const double a2 = g.dzi * g.dzi;
   std::vector<double> z((size_t)zst * K);
   for (int ky = 0; ky <= J / 2; ++ky)
     for (int kx = 0; kx < MX; ++kx) {
       const double xy = xrt[kx] + yrt[ky];
-      double zz = 1. / (b[1] + xy);
-      double d = cc[1] * zz;
-      z[(size_t)ky * MX + kx] = zz;
+      double d = cc[1] * (1. / (b[1] + xy));
+      z[(size_t)ky * MX + kx] = d;
       for (int k = 2; k <= K - 1; ++k) {
         const double bb = b[k] + xy;
-        zz = 1. / (bb - a[k] * d);
-        d = cc[k] * zz;
-        z[(size_t)(k - 1) * zst + (size_t)ky * MX + kx] = zz;
+        d = cc[k] * (1. / (bb - a[k] * d));
+        z[(size_t)(k - 1) * zst + (size_t)ky * MX + kx] = d;
       }
-      const double bb = b[K] + xy;
-      z[(size_t)(K - 1) * zst + (size_t)ky * MX + kx] = bb - a[K] * d;
+      const double den = b[K] + xy - a[K] * d;
+      z[(size_t)(K - 1) * zst + (size_t)ky * MX + kx] = den != 0. ? a2 / den : 0.;
     }
-  if ((st = dalloc(c, &c->zt, z.size()))) return st;
-  CK(cudaMemcpyAsync(c->zt, z.data(), z.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  if (c->mixed) {
-    // double-float tables of the mixed form: pivots with 1/den in the last
-    // plane (0 for the zero mode, den == 0), and dzi^2 * pivot
-    std::vector<float2> t(2 * z.size());
-    const double a2 = g.dzi * g.dzi;
-    auto split = [](double v) {
-      const float h = (float)v;
-      return make_float2(h, (float)(v - (double)h));
-    };
+  if (c->mixed) {  // as FP32 pairs
+    std::vector<float2> t(z.size());
     for (size_t q = 0; q < z.size(); ++q) {
-      const bool last = q >= (size_t)(K - 1) * zst;
-      t[q] = split(last ? (z[q] != 0. ? 1. / z[q] : 0.) : z[q]);
-      t[z.size() + q] = split(a2 * z[q]);
+      const float h = (float)z[q];
+      t[q] = make_float2(h, (float)(z[q] - (double)h));
     }
     if ((st = dalloc(c, &c->thomas_df, t.size()))) return st;
     CK(cudaMemcpyAsync(c->thomas_df, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    return IBM_OK;
   }
+  if ((st = dalloc(c, &c->zt, z.size()))) return st;
+  CK(cudaMemcpyAsync(c->zt, z.data(), z.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   return IBM_OK;
 }
