@@ -2292,12 +2292,19 @@ int ibm_mlp_fit(ibm_ctx *c, const float *params_in, const float *x, const float 
   if (!c || !params_in || !x || !t || nb < 1 || nsteps < 0 || !(lr > 0)) return IBM_E_INVALID;
   MlpTrainBuffers B{};
   int st = mlp_scratch(c, params_in, x, t, nb, B);
+  // the losses stay on the device until the last step: a copy to pageable
+  // memory after each one held the host back for 10 us
+  float *dl = nullptr;
+  if (st == IBM_OK && losses && nsteps > 0) st = dalloc(c, &dl, (size_t)nsteps);
   cudaError_t e = cudaSuccess;
+  MlpTrainBuffers Bq = B;
   for (int q = 0; st == IBM_OK && e == cudaSuccess && q < nsteps; ++q) {
-    c->launches += launch_mlp_train_step(c->stream, B, B.x, B.t, nb, nb, 0u, 0, q + 1, (float)lr, 1, nullptr);
+    if (dl) Bq.loss = dl + q;
+    c->launches += launch_mlp_train_step(c->stream, Bq, B.x, B.t, nb, nb, 0u, 0, q + 1, (float)lr, 1, nullptr);
     e = cudaGetLastError();
-    if (e == cudaSuccess && losses) e = cudaMemcpyAsync(losses + q, B.loss, sizeof(float), cudaMemcpyDeviceToHost, c->stream);
   }
+  if (st == IBM_OK && e == cudaSuccess && dl)
+    e = cudaMemcpyAsync(losses, dl, (size_t)nsteps * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
   if (st == IBM_OK && e == cudaSuccess && params_out)
     e = cudaMemcpyAsync(params_out, B.params, mlp_nparam() * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
   int herr = 0;
@@ -2307,6 +2314,7 @@ int ibm_mlp_fit(ibm_ctx *c, const float *params_in, const float *x, const float 
   if (st == IBM_OK && herr) st = set_err(c, IBM_E_NOT_CONVERGED, "tensor-core MMA wait timed out");
   cudaStreamSynchronize(c->stream);
   free_mlp_batch(B);
+  cudaFree(dl);
   free_mlp_model(B);
   return st;
 }

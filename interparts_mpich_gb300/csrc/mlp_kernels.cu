@@ -674,7 +674,11 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, int amn, int bmn
 // byte offset)
 __device__ __forceinline__ uint64_t mn_desc(uint32_t saddr, uint32_t kstride) { return umma_desc(saddr, kstride, 128); }
 
-constexpr int TT_THREADS = 256;
+// Four threads a row, a quarter of the hidden columns each: the element-wise
+// parts between the products are what bounds the kernel (one CTA an SM, a
+// chain of six products), 27 -> 21.5 us a launch of 64 tiles against two
+// threads a row and gradients stored row by row.
+constexpr int TT_THREADS = 512;
 constexpr int TT_XK = NIN + 16;   // X, a column of ones, zeros
 constexpr int TT_HK = NH + 16;    // H1, a column of ones, zeros
 constexpr int TT_DYN = 16;        // dY hi (columns 0..2), lo (3..5), zeros
@@ -723,10 +727,6 @@ __device__ __forceinline__ uint32_t bf2_bits(float a, float b) {
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t *>(&v);
 }
-__device__ __forceinline__ void st4f(float *p, const float *v) {
-  *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
-}
-
 __global__ void __launch_bounds__(TT_THREADS, 1) k_mlp_train_tc(const MlpTrainArgs A) {
   extern __shared__ __align__(16) unsigned char tt_sm[];
   unsigned char *W1s = tt_sm + TT_OW1, *W2s = tt_sm + TT_OW2, *Xs = tt_sm + TT_OX, *H1s = tt_sm + TT_OH1,
@@ -778,7 +778,8 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_mlp_train_tc(const MlpTrainAr
   __syncthreads();
   tc_fence_after();
   const uint32_t T0 = *tslot;
-  const int q4 = warp & 3, hf = warp >> 2;  // TMEM lane quarter, column half
+  const int q4 = warp & 3, qt = warp >> 2;  // TMEM lane quarter, column quarter
+  const int col = qt * 32;
   const int r = q4 * 32 + lane;              // this thread's row of the tile (its TMEM lane)
   const uint32_t lb = (uint32_t)(q4 * 32) << 16;
   const bool valid = row0 + r < A.nb;
@@ -814,23 +815,19 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_mlp_train_tc(const MlpTrainAr
   bool ok = mma_wait();
   // H1 = bf16(gelu(Z1 + b1)), and the ones column
   if (ok) {
-#pragma unroll 1
-    for (int cc = 0; cc < 2; ++cc) {
-      const int col = hf * 64 + cc * 32;
-      float v[32];
-      tmem_ld32(T0 + lb + col, v);
+    float v[32];
+    tmem_ld32(T0 + lb + col, v);
 #pragma unroll
-      for (int c8 = 0; c8 < 32; c8 += 8) {
-        uint32_t pk[4];
+    for (int c8 = 0; c8 < 32; c8 += 8) {
+      uint32_t pk[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int c = col + c8 + 2 * e;
-          pk[e] = bf2_bits(gelu_f(v[c8 + 2 * e] + fs[TF_B1 + c]), gelu_f(v[c8 + 2 * e + 1] + fs[TF_B1 + c + 1]));
-        }
-        *reinterpret_cast<uint4 *>(H1s + cm_off(r, col + c8, TT_SB_H1)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+      for (int e = 0; e < 4; ++e) {
+        const int c = col + c8 + 2 * e;
+        pk[e] = bf2_bits(gelu_f(v[c8 + 2 * e] + fs[TF_B1 + c]), gelu_f(v[c8 + 2 * e + 1] + fs[TF_B1 + c + 1]));
       }
+      *reinterpret_cast<uint4 *>(H1s + cm_off(r, col + c8, TT_SB_H1)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
     }
-    if (hf == 1) {
+    if (qt == 3) {
       *reinterpret_cast<uint4 *>(H1s + cm_off(r, NH, TT_SB_H1)) = make_uint4(valid ? 0x3F80u : 0u, 0u, 0u, 0u);
       *reinterpret_cast<uint4 *>(H1s + cm_off(r, NH + 8, TT_SB_H1)) = make_uint4(0u, 0u, 0u, 0u);
     }
@@ -846,33 +843,41 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_mlp_train_tc(const MlpTrainAr
     umma_commit(bar);
   }
   if (ok) ok = mma_wait();
-  // H2 = bf16(gelu(Z2 + b2)); layer 3 on the FP32 pipes (each column half
-  // a partial dot product)
+  // H2 = bf16(gelu(Z2 + b2))
   if (ok) {
-    float yp[NOUT] = {0.f, 0.f, 0.f};
-#pragma unroll 1
-    for (int cc = 0; cc < 2; ++cc) {
-      const int col = hf * 64 + cc * 32;
-      float v[32];
-      tmem_ld32(T0 + 128 + lb + col, v);
+    float v[32];
+    tmem_ld32(T0 + 128 + lb + col, v);
 #pragma unroll
-      for (int c8 = 0; c8 < 32; c8 += 8) {
-        uint32_t pk[4];
+    for (int c8 = 0; c8 < 32; c8 += 8) {
+      uint32_t pk[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int c = col + c8 + 2 * e;
-          const __nv_bfloat162 hb =
-              __floats2bfloat162_rn(gelu_f(v[c8 + 2 * e] + fs[TF_B2 + c]), gelu_f(v[c8 + 2 * e + 1] + fs[TF_B2 + c + 1]));
-          const float ha = __low2float(hb), hc = __high2float(hb);
+      for (int e = 0; e < 4; ++e) {
+        const int c = col + c8 + 2 * e;
+        pk[e] = bf2_bits(gelu_f(v[c8 + 2 * e] + fs[TF_B2 + c]), gelu_f(v[c8 + 2 * e + 1] + fs[TF_B2 + c + 1]));
+      }
+      *reinterpret_cast<uint4 *>(H2s + cm_off(r, col + c8, TT_SB_H)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+    }
+  }
+  __syncthreads();
+  // layer 3 on the FP32 pipes: each column half a partial dot product, outputs
+  // 0 and 1 by one thread of the row, output 2 by another
+  if (ok) {
+    const int hf = qt >> 1, o0 = qt & 1 ? 2 : 0, o1 = qt & 1 ? 2 : 1;
+    float y0 = 0.f, y1 = 0.f;
 #pragma unroll
-          for (int o = 0; o < NOUT; ++o) yp[o] += ha * fs[TF_W3 + o * NH + c] + hc * fs[TF_W3 + o * NH + c + 1];
-          pk[e] = *reinterpret_cast<const uint32_t *>(&hb);
-        }
-        *reinterpret_cast<uint4 *>(H2s + cm_off(r, col + c8, TT_SB_H)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+    for (int c8 = 0; c8 < 64; c8 += 8) {
+      const uint4 hv = *reinterpret_cast<const uint4 *>(H2s + cm_off(r, hf * 64 + c8, TT_SB_H));
+      const uint32_t hw[4] = {hv.x, hv.y, hv.z, hv.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int c = hf * 64 + c8 + 2 * e;
+        const float ha = __uint_as_float(hw[e] << 16), hc = __uint_as_float(hw[e] & 0xffff0000u);
+        y0 += ha * fs[TF_W3 + o0 * NH + c] + hc * fs[TF_W3 + o0 * NH + c + 1];
+        y1 += ha * fs[TF_W3 + o1 * NH + c] + hc * fs[TF_W3 + o1 * NH + c + 1];
       }
     }
-#pragma unroll
-    for (int o = 0; o < NOUT; ++o) fs[TF_YP + (hf * 128 + r) * 4 + o] = yp[o];
+    fs[TF_YP + (hf * 128 + r) * 4 + o0] = y0;
+    if (o1 != o0) fs[TF_YP + (hf * 128 + r) * 4 + o1] = y1;
   }
   __syncthreads();
   if (ok) {
@@ -884,9 +889,9 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_mlp_train_tc(const MlpTrainAr
       const float yv = (fs[TF_YP + r * 4 + o] + fs[TF_YP + (128 + r) * 4 + o]) + fs[TF_B3 + o];
       e[o] = valid ? yv - A.T[src * NOUT + o] : 0.f;
       dy[o] = (2.f / (float)A.nb) * e[o];
-      if (hf == 0 && valid && A.y) A.y[(long)(row0 + r) * NOUT + o] = yv;
+      if (qt == 0 && valid && A.y) A.y[(long)(row0 + r) * NOUT + o] = yv;
     }
-    if (hf == 0) {
+    if (qt == 0) {
       float hi[NOUT], lo[NOUT];
 #pragma unroll
       for (int o = 0; o < NOUT; ++o) {
@@ -905,27 +910,23 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_mlp_train_tc(const MlpTrainAr
         for (int k = 0; k < 4; ++k) fs[TF_RED + q4 * 4 + k] = s[k];
     }
     // dZ2 = bf16((dY W3) gelu'(Z2 + b2)), Z2 read again
-#pragma unroll 1
-    for (int cc = 0; cc < 2; ++cc) {
-      const int col = hf * 64 + cc * 32;
-      float v[32];
-      tmem_ld32(T0 + 128 + lb + col, v);
+    float v[32];
+    tmem_ld32(T0 + 128 + lb + col, v);
 #pragma unroll
-      for (int c8 = 0; c8 < 32; c8 += 8) {
-        uint32_t pk[4];
+    for (int c8 = 0; c8 < 32; c8 += 8) {
+      uint32_t pk[4];
 #pragma unroll
-        for (int ee = 0; ee < 4; ++ee) {
-          float d[2];
+      for (int ee = 0; ee < 4; ++ee) {
+        float d[2];
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int c = col + c8 + 2 * ee + u;
-            const float dh = dy[0] * fs[TF_W3 + c] + dy[1] * fs[TF_W3 + NH + c] + dy[2] * fs[TF_W3 + 2 * NH + c];
-            d[u] = dh * gelu_grad_f(v[c8 + 2 * ee + u] + fs[TF_B2 + c]);
-          }
-          pk[ee] = bf2_bits(d[0], d[1]);
+        for (int u = 0; u < 2; ++u) {
+          const int c = col + c8 + 2 * ee + u;
+          const float dh = dy[0] * fs[TF_W3 + c] + dy[1] * fs[TF_W3 + NH + c] + dy[2] * fs[TF_W3 + 2 * NH + c];
+          d[u] = dh * gelu_grad_f(v[c8 + 2 * ee + u] + fs[TF_B2 + c]);
         }
-        *reinterpret_cast<uint4 *>(D2s + cm_off(r, col + c8, TT_SB_H)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        pk[ee] = bf2_bits(d[0], d[1]);
       }
+      *reinterpret_cast<uint4 *>(D2s + cm_off(r, col + c8, TT_SB_H)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
     }
   }
   issued();
@@ -950,22 +951,18 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_mlp_train_tc(const MlpTrainAr
   if (ok) ok = mma_wait();
   // dZ1 = bf16(dH1 gelu'(Z1 + b1)) into H2's tile (read by the completed MMAs)
   if (ok) {
-#pragma unroll 1
-    for (int cc = 0; cc < 2; ++cc) {
-      const int col = hf * 64 + cc * 32;
-      float dh[32], z[32];
-      tmem_ld32(T0 + 128 + lb + col, dh);
-      tmem_ld32(T0 + lb + col, z);
+    float dh[32], z[32];
+    tmem_ld32(T0 + 128 + lb + col, dh);
+    tmem_ld32(T0 + lb + col, z);
 #pragma unroll
-      for (int c8 = 0; c8 < 32; c8 += 8) {
-        uint32_t pk[4];
+    for (int c8 = 0; c8 < 32; c8 += 8) {
+      uint32_t pk[4];
 #pragma unroll
-        for (int ee = 0; ee < 4; ++ee) {
-          const int c = col + c8 + 2 * ee, j = c8 + 2 * ee;
-          pk[ee] = bf2_bits(dh[j] * gelu_grad_f(z[j] + fs[TF_B1 + c]), dh[j + 1] * gelu_grad_f(z[j + 1] + fs[TF_B1 + c + 1]));
-        }
-        *reinterpret_cast<uint4 *>(H2s + cm_off(r, col + c8, TT_SB_H)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+      for (int ee = 0; ee < 4; ++ee) {
+        const int c = col + c8 + 2 * ee, j = c8 + 2 * ee;
+        pk[ee] = bf2_bits(dh[j] * gelu_grad_f(z[j] + fs[TF_B1 + c]), dh[j + 1] * gelu_grad_f(z[j + 1] + fs[TF_B1 + c + 1]));
       }
+      *reinterpret_cast<uint4 *>(H2s + cm_off(r, col + c8, TT_SB_H)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
     }
   }
   issued();
@@ -978,42 +975,28 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_mlp_train_tc(const MlpTrainAr
     umma_commit(bar);
   }
   if (ok) ok = mma_wait();
-  // the tile's gradient (TMEM lane = output neuron) and loss
+  // the tile's gradient (TMEM lane = output neuron) and loss; W1 and W2 with
+  // the neurons inside, so that a warp stores whole lines (part_index)
   if (ok) {
     float *P = A.part + (long)blockIdx.x * TT_PSTRIDE;
     const int o = r;
-    float v[32];
-    if (hf == 0) {
-#pragma unroll 1
-      for (int cc = 0; cc < 2; ++cc) {
-        tmem_ld32(T0 + lb + cc * 32, v);
+    float v[32], v8[8];
+    if (qt < NIN / 32) {
+      tmem_ld32(T0 + lb + col, v);
 #pragma unroll
-        for (int k = 0; k < 32; k += 4) st4f(P + o * NIN + cc * 32 + k, v + k);
-      }
+      for (int k = 0; k < 32; ++k) P[(col + k) * NH + o] = v[k];
     } else {
-      tmem_ld32(T0 + lb + 64, v);
-#pragma unroll
-      for (int k = 0; k < 32; k += 4) st4f(P + o * NIN + 64 + k, v + k);
-      float v8[8];
       tmem_ld8(T0 + lb + NIN, v8);
       P[OFF_B1 + o] = v8[0];
-    }
-#pragma unroll 1
-    for (int cc = 0; cc < 2; ++cc) {
-      const int col = hf * 64 + cc * 32;
-      tmem_ld32(T0 + 256 + lb + col, v);
-#pragma unroll
-      for (int k = 0; k < 32; k += 4) st4f(P + OFF_W2 + o * NH + col + k, v + k);
-    }
-    float v8[8];
-    if (hf == 1) {
       tmem_ld8(T0 + 256 + NH + lb, v8);
       P[OFF_B2 + o] = v8[0];
-    } else {
       tmem_ld8(T0 + 400 + lb, v8);
 #pragma unroll
       for (int k = 0; k < NOUT; ++k) P[OFF_W3 + k * NH + o] = v8[k] + v8[NOUT + k];
     }
+    tmem_ld32(T0 + 256 + lb + col, v);
+#pragma unroll
+    for (int k = 0; k < 32; ++k) P[OFF_W2 + (col + k) * NH + o] = v[k];
     if (tid == 0)
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -1030,31 +1013,51 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_mlp_train_tc(const MlpTrainAr
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(T0));
 }
 
+// parameter of entry t of a tile's gradient (W1 and W2 lie transposed there)
+__device__ __forceinline__ int part_index(int t) {
+  if (t < NH * NIN) return (t % NH) * NIN + t / NH;
+  if (t >= OFF_W2 && t < OFF_W2 + NH * NH) return OFF_W2 + (t - OFF_W2) % NH * NH + (t - OFF_W2) / NH;
+  return t;
+}
 // the tiles' gradients summed in tile order (deterministic) into grad and
 // the loss; with adam: one Adam step of the FP32 masters and their BF16
-// copies
-__global__ void __launch_bounds__(256) k_mlp_reduce_adam(const float *__restrict__ part, int nparts,
+// copies.  Bound by the latency of the partials' reads, so 32 are in flight and
+// the blocks small enough to reach every SM: 64 tiles, 8.8 -> 5.8 us.
+constexpr int RA_THREADS = 64;
+__global__ void __launch_bounds__(RA_THREADS) k_mlp_reduce_adam(const float *__restrict__ part, int nparts,
                                                          float *__restrict__ grad, float *__restrict__ loss,
                                                          float *__restrict__ p, float *__restrict__ m,
                                                          float *__restrict__ v, bf16 *__restrict__ w1b,
                                                          bf16 *__restrict__ w2b, int adam, float lr, float b1, float b2,
                                                          float eps, float c1, float c2) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t > NPARAM) return;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e > NPARAM) return;
+  const int t = part_index(e);
+  float m0 = 0.f, v0 = 0.f, p0 = 0.f;
+  if (adam && e < NPARAM) { m0 = m[t]; v0 = v[t]; p0 = p[t]; }
   float s = 0.f;
-#pragma unroll 8
-  for (int c = 0; c < nparts; ++c) s += part[(long)c * TT_PSTRIDE + t];
-  if (t == NPARAM) {
+  for (int c0 = 0; c0 < nparts; c0 += 32) {
+    float x[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q)
+      if (c0 + q < nparts) x[q] = part[(long)(c0 + q) * TT_PSTRIDE + e];
+#pragma unroll
+    for (int q = 0; q < 32; ++q)
+      if (c0 + q < nparts) s += x[q];
+  }
+  if (e == NPARAM) {
     *loss = s;
     return;
   }
   grad[t] = s;
   if (!adam) return;
-  const float mm = b1 * m[t] + (1.f - b1) * s;
-  const float vv = b2 * v[t] + (1.f - b2) * s * s;
+  // fused by hand: a training run is sensitive to the last bit, which is not to
+  // depend on what the compiler fuses
+  const float mm = fmaf(1.f - b1, s, b1 * m0);
+  const float vv = fmaf((1.f - b2) * s, s, b2 * v0);
   m[t] = mm;
   v[t] = vv;
-  const float pn = p[t] - lr * (mm / c1) / (sqrtf(vv / c2) + eps);
+  const float pn = p0 - lr * (mm / c1) / (sqrtf(vv / c2) + eps);
   p[t] = pn;
   if (t < NH * NIN) w1b[t] = __float2bfloat16(pn);
   else if (t >= OFF_W2 && t < OFF_W2 + NH * NH) w2b[t - OFF_W2] = __float2bfloat16(pn);
@@ -1082,7 +1085,7 @@ int launch_mlp_train_step(cudaStream_t s, const MlpTrainBuffers &B, const bf16 *
   k_mlp_train_tc<<<ntile, TT_THREADS, TT_SMEM, s>>>(A);
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = adam ? 1.f - powf(b1, (float)step) : 1.f, c2 = adam ? 1.f - powf(b2, (float)step) : 1.f;
-  k_mlp_reduce_adam<<<(NPARAM + 1 + 255) / 256, 256, 0, s>>>(B.part, ntile, B.grad, B.loss, B.params, B.m, B.v, B.w1b,
+  k_mlp_reduce_adam<<<(NPARAM + RA_THREADS) / RA_THREADS, RA_THREADS, 0, s>>>(B.part, ntile, B.grad, B.loss, B.params, B.m, B.v, B.w1b,
                                                              B.w2b, adam, lr, b1, b2, 1e-8f, c1, c2);
   return 2;
 }
