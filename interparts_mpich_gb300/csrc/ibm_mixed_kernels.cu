@@ -334,7 +334,17 @@ __device__ __forceinline__ float interp27(const CompStencil &s, TAP tap) {
 // ---------------------------------------------------------------------------
 // box capacity: pg.box_cap cells, sized for the largest sphere (9600 = 38 KB
 // at D = 16 dx)
-constexpr int INTERP_THREADS = 256;
+// Threads NT of a block and the blocks MB an SM is to hold (which sets the
+// registers), for interpolation and spreading.  A block waits for its box, its
+// points and its flush, so the SM needs other blocks to work on: four of 256
+// threads where their shared memory fits, else (boxes of more than 50 KB, two
+// blocks an SM and fewer) blocks of 512.  1000 spheres of 16 dx (38 KB):
+// interpolation 80 us with three blocks of 256 and 80 registers, 72 with four
+// (320 or 192 threads: 79 and more); spreading 69 with three of 384, 61.5.  1400
+// spheres of up to 24 dx (100 KB): 163 -> 161 and 148 -> 143 (four of 256: 177
+// and 154).
+constexpr int NT_MANY = 256, MB_MANY = 4, NT_FEW = 512, MB_FEW = 2;
+inline bool many_blocks(size_t smem) { return MB_MANY * (smem + 1024) <= 227 * 1024; }
 // interpolation: the box and the values of up to SPREAD_PRE points
 inline int interp_pts(const PartGeo &pg) { return pg.nl < SPREAD_PRE ? pg.nl : SPREAD_PRE; }
 inline size_t interp_smem(const PartGeo &pg) { return (size_t)(pg.box_cap + interp_pts(pg)) * sizeof(float); }
@@ -356,8 +366,8 @@ __device__ __forceinline__ float block_sum_all(float a) {
 // template parameters: FP64 instructions of an if-converted branch issue
 // under a false predicate and still occupy the FP64 pipe, which this GPU
 // runs at 1/64 of the FP32 rate.
-template <int FIRST, bool ROT, bool LAST>
-__global__ void __launch_bounds__(INTERP_THREADS, 3) k_ibm_interp_comp_f(Geo g, PartGeo pg, IbmBuffers b,
+template <int FIRST, bool ROT, bool LAST, int NT, int MB>
+__global__ void __launch_bounds__(NT, MB) k_ibm_interp_comp_f(Geo g, PartGeo pg, IbmBuffers b,
                                                            const float *__restrict__ fu, const float *__restrict__ fv,
                                                            const float *__restrict__ fw, double dti,
                                                            const int *__restrict__ gate, int npt) {
@@ -377,7 +387,7 @@ __global__ void __launch_bounds__(INTERP_THREADS, 3) k_ibm_interp_comp_f(Geo g, 
   const unsigned *rowm = b.rowm + ((long)p * 3 + c) * IBM_BOX_ROWS;
   const int nmask = min(npt, IBM_BOX_ROWS);
 #pragma unroll 4
-  for (int q = threadIdx.x; q < nmask; q += INTERP_THREADS) reinterpret_cast<unsigned *>(sacc)[q] = __ldg(&rowm[q]);
+  for (int q = threadIdx.x; q < nmask; q += NT) reinterpret_cast<unsigned *>(sacc)[q] = __ldg(&rowm[q]);
   if (threadIdx.x < 8) bg[threadIdx.x] = b.bgeo[((long)p * 3 + c) * 8 + threadIdx.x];
   if (threadIdx.x >= 64 && threadIdx.x < 64 + IBM_BST)
     sbst[threadIdx.x - 64] = b.bst[((long)p * 3 + c) * IBM_BST + threadIdx.x - 64];
@@ -419,7 +429,7 @@ __global__ void __launch_bounds__(INTERP_THREADS, 3) k_ibm_interp_comp_f(Geo g, 
   if constexpr (FIRST == 0) {
 #pragma unroll
     for (int q = 0; q < FP; ++q) {
-      const int l = threadIdx.x + q * INTERP_THREADS;
+      const int l = threadIdx.x + q * NT;
       fl[q] = l < nla ? Fl[t0 + l] : 0.f;
     }
   }
@@ -432,7 +442,7 @@ __global__ void __launch_bounds__(INTERP_THREADS, 3) k_ibm_interp_comp_f(Geo g, 
   float sF = 0.f, sa = 0.f, sb = 0.f;
   float r2 = 0.f, r0 = 0.f;
   int pass = 0;
-  for (int l = threadIdx.x; l < nla; l += INTERP_THREADS, ++pass) {
+  for (int l = threadIdx.x; l < nla; l += NT, ++pass) {
     const long t = t0 + l;
     float acc;
     if (sorted) {
@@ -486,14 +496,14 @@ __global__ void __launch_bounds__(INTERP_THREADS, 3) k_ibm_interp_comp_f(Geo g, 
   __syncthreads();  // the box is dead: its first words hold the threads' sums
   float *st = box;
   st[threadIdx.x] = sF;
-  st[INTERP_THREADS + threadIdx.x] = sa;
-  st[2 * INTERP_THREADS + threadIdx.x] = sb;
+  st[NT + threadIdx.x] = sa;
+  st[2 * NT + threadIdx.x] = sb;
   __syncthreads();
   const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (q >= 3) return;
   float h = 0.f, lo = 0.f;  // a warp a sum, in double-float
 #pragma unroll
-  for (int d = 0; d < INTERP_THREADS; d += 32) df_add(h, lo, st[q * INTERP_THREADS + d + lane], 0.f, h, lo);
+  for (int d = 0; d < NT; d += 32) df_add(h, lo, st[q * NT + d + lane], 0.f, h, lo);
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) {
     const float oh = __shfl_xor_sync(0xffffffffu, h, d), ol = __shfl_xor_sync(0xffffffffu, lo, d);
@@ -525,16 +535,17 @@ int launch_ibm_interp_force_f(cudaStream_t s, const Geo &g, const PartGeo &pg, I
   const dim3 grd(pg.np, 3);
   const size_t sm = interp_smem(pg);
   const int npt = interp_pts(pg);
-  auto go = [&](auto kern) { kern<<<grd, INTERP_THREADS, sm, s>>>(g, pg, b, fu, fv, fw, 1. / dt, gate, npt); };
-  auto pick = [&](auto rot) {
+  auto pick = [&](auto rot, auto many) {
     constexpr bool R = decltype(rot)::value;
-    if (first == 1) last ? go(k_ibm_interp_comp_f<1, R, true>) : go(k_ibm_interp_comp_f<1, R, false>);
-    else if (first == 0) last ? go(k_ibm_interp_comp_f<0, R, true>) : go(k_ibm_interp_comp_f<0, R, false>);
-    else if (first == -1) go(k_ibm_interp_comp_f<-1, R, false>);
-    else go(k_ibm_interp_comp_f<-2, R, false>);
+    constexpr int NT = decltype(many)::value ? NT_MANY : NT_FEW, MB = decltype(many)::value ? MB_MANY : MB_FEW;
+    auto go = [&](auto kern) { kern<<<grd, NT, sm, s>>>(g, pg, b, fu, fv, fw, 1. / dt, gate, npt); };
+    if (first == 1) last ? go(k_ibm_interp_comp_f<1, R, true, NT, MB>) : go(k_ibm_interp_comp_f<1, R, false, NT, MB>);
+    else if (first == 0) last ? go(k_ibm_interp_comp_f<0, R, true, NT, MB>) : go(k_ibm_interp_comp_f<0, R, false, NT, MB>);
+    else if (first == -1) go(k_ibm_interp_comp_f<-1, R, false, NT, MB>);
+    else go(k_ibm_interp_comp_f<-2, R, false, NT, MB>);
   };
-  if (pg.rotation) pick(std::true_type{});
-  else pick(std::false_type{});
+  auto rot = [&](auto many) { pg.rotation ? pick(std::true_type{}, many) : pick(std::false_type{}, many); };
+  many_blocks(sm) ? rot(std::true_type{}) : rot(std::false_type{});
   if (first < 0 || !last) return 1;
   k_ibm_force_sums<<<(pg.np + 127) / 128, 128, 0, s>>>(pg, b, gate);
   return 2;
@@ -558,8 +569,6 @@ int launch_ibm_interp_force_f(cudaStream_t s, const Geo &g, const PartGeo &pg, I
 // FP32 values into the box instead; boxes beyond pg.box_cap cells add per
 // tap to the field.
 // ---------------------------------------------------------------------------
-constexpr int SPREAD_THREADS = 384;
-
 // the 27 taps of one point into the box: FP32 adds, or fixed-point adds of
 // rint(pre * w) (pre already scaled)
 template <bool FIXED>
@@ -580,8 +589,8 @@ __device__ __forceinline__ void spread27_box(float *box, const CompStencil &s, i
 
 // LY: a learned (or perturbation) force is given (lf.Y), as a template
 // parameter so that the plain passes issue none of its FP64 work
-template <bool LY>
-__global__ void __launch_bounds__(SPREAD_THREADS, 3) k_ibm_spread_f(Geo g, PartGeo pg, IbmBuffers b, float *__restrict__ fu,
+template <bool LY, int NT, int MB>
+__global__ void __launch_bounds__(NT, MB) k_ibm_spread_f(Geo g, PartGeo pg, IbmBuffers b, float *__restrict__ fu,
                                                       float *__restrict__ fv, float *__restrict__ fw, double dti,
                                                       double coeff0_, LearnedForce lf,
                                                       const int *__restrict__ gate, double dt) {
@@ -653,15 +662,15 @@ __global__ void __launch_bounds__(SPREAD_THREADS, 3) k_ibm_spread_f(Geo g, PartG
   const int nq = (nla + 31) >> 5;
   float asum = 0.f, r0 = 0.f;
   if (!LY && staged) {  // the plain passes: the slips of up to six points, loaded together
-    float sv[(SPREAD_PRE + SPREAD_THREADS - 1) / SPREAD_THREADS];
+    float sv[(SPREAD_PRE + NT - 1) / NT];
 #pragma unroll
-    for (int q = 0; q < (SPREAD_PRE + SPREAD_THREADS - 1) / SPREAD_THREADS; ++q) {
-      const int l = threadIdx.x + q * SPREAD_THREADS;
+    for (int q = 0; q < (SPREAD_PRE + NT - 1) / NT; ++q) {
+      const int l = threadIdx.x + q * NT;
       sv[q] = l < nla ? slip[t0 + l] * ucoef : 0.f;
     }
 #pragma unroll
-    for (int q = 0; q < (SPREAD_PRE + SPREAD_THREADS - 1) / SPREAD_THREADS; ++q) {
-      const int l = threadIdx.x + q * SPREAD_THREADS;
+    for (int q = 0; q < (SPREAD_PRE + NT - 1) / NT; ++q) {
+      const int l = threadIdx.x + q * NT;
       if (l < nla) spre[l] = sv[q];
       asum += fabsf(sv[q]);
     }
@@ -766,12 +775,14 @@ void launch_ibm_spread_f(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmBuf
                          float *fw, double dt, const LearnedForce &lf, const int *gate) {
   if (pg.np == 0) return;
   const double coeff0 = (pg.dVlagr / pg.dVeul) * dt;
-  auto go = [&](auto kern) {
-    kern<<<dim3(pg.np, 3), SPREAD_THREADS, pg.box_cap * sizeof(float), s>>>(g, pg, b, fu, fv, fw, 1. / dt, coeff0, lf,
-                                                                          gate, dt);
+  const size_t sm = pg.box_cap * sizeof(float);
+  auto pick = [&](auto many) {
+    constexpr int NT = decltype(many)::value ? NT_MANY : NT_FEW, MB = decltype(many)::value ? MB_MANY : MB_FEW;
+    auto go = [&](auto kern) { kern<<<dim3(pg.np, 3), NT, sm, s>>>(g, pg, b, fu, fv, fw, 1. / dt, coeff0, lf, gate, dt); };
+    lf.Y ? go(k_ibm_spread_f<true, NT, MB>) : go(k_ibm_spread_f<false, NT, MB>);
   };
-  if (lf.Y) go(k_ibm_spread_f<true>);
-  else go(k_ibm_spread_f<false>);
+  // its prefactors besides the box
+  many_blocks(sm + SPREAD_PRE * sizeof(float)) ? pick(std::true_type{}) : pick(std::false_type{});
 }
 void launch_ibm_force_sums(cudaStream_t s, const PartGeo &pg, IbmBuffers b) {
   if (pg.np == 0) return;
@@ -924,15 +935,20 @@ int ibm_set_smem_limits(const PartGeo &pg) {
   auto set = [&](auto k) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
   };
-  set(k_ibm_spread_f<false>);
-  set(k_ibm_spread_f<true>);
-  for (auto k : {k_ibm_interp_comp_f<1, false, false>, k_ibm_interp_comp_f<0, false, false>,
-                 k_ibm_interp_comp_f<1, false, true>, k_ibm_interp_comp_f<0, false, true>,
-                 k_ibm_interp_comp_f<1, true, false>, k_ibm_interp_comp_f<0, true, false>,
-                 k_ibm_interp_comp_f<1, true, true>, k_ibm_interp_comp_f<0, true, true>,
-                 k_ibm_interp_comp_f<-1, false, false>, k_ibm_interp_comp_f<-1, true, false>,
-                 k_ibm_interp_comp_f<-2, false, false>, k_ibm_interp_comp_f<-2, true, false>})
-    set(k);
+  auto all = [&](auto many) {
+    constexpr int NT = decltype(many)::value ? NT_MANY : NT_FEW, MB = decltype(many)::value ? MB_MANY : MB_FEW;
+    set(k_ibm_spread_f<false, NT, MB>);
+    set(k_ibm_spread_f<true, NT, MB>);
+    for (auto k : {k_ibm_interp_comp_f<1, false, false, NT, MB>, k_ibm_interp_comp_f<0, false, false, NT, MB>,
+                   k_ibm_interp_comp_f<1, false, true, NT, MB>, k_ibm_interp_comp_f<0, false, true, NT, MB>,
+                   k_ibm_interp_comp_f<1, true, false, NT, MB>, k_ibm_interp_comp_f<0, true, false, NT, MB>,
+                   k_ibm_interp_comp_f<1, true, true, NT, MB>, k_ibm_interp_comp_f<0, true, true, NT, MB>,
+                   k_ibm_interp_comp_f<-1, false, false, NT, MB>, k_ibm_interp_comp_f<-1, true, false, NT, MB>,
+                   k_ibm_interp_comp_f<-2, false, false, NT, MB>, k_ibm_interp_comp_f<-2, true, false, NT, MB>})
+      set(k);
+  };
+  all(std::true_type{});
+  all(std::false_type{});
   if (e != cudaSuccess) return -1;
   cur = need;
   return 0;
