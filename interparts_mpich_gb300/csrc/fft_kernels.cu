@@ -626,10 +626,11 @@ void launch_cyclic_tables(cudaStream_t s, const Geo &g, const double *xrt, const
 // GB300 issues FP64 at 1/64 of the FP32 rate.  Table: c_k, formed in FP64 and
 // split hi + lo.  The recurrence carries its value in double-float from plane
 // to plane; the forward intermediate between the sweeps is kept in the FP32
-// spectrum, and oscale (a pair) is applied at the final FP32 store.  256^3:
-// 70 -> 64 us, 512 x 512 x 256: 271 -> 229.
+// spectrum; 1 / dzi^2 (a pair) and the transforms' scale are applied at the
+// final FP32 store.  256^3:
+// 70 -> 65 us, 512 x 512 x 256: 271 -> 231.
 __global__ void __launch_bounds__(64) k_thomas_df(Geo g, float *__restrict__ S, const float2 *__restrict__ tab,
-                                                  float osh, float osl) {
+                                                  float iah, float ial, float fscale) {
   const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
   const int ncol = g.MX * g.J;
   if (e >= 2l * ncol) return;
@@ -664,6 +665,7 @@ __global__ void __launch_bounds__(64) k_thomas_df(Geo g, float *__restrict__ S, 
       sk[(long)q * sst] = rh;
     }
   };
+  auto out = [&]() { return fmaf(rh, iah, fmaf(rh, ial, rl * iah)) * fscale; };
   auto bwd = [&](int slot, int k0) {
     float *sk = s + (long)k0 * sst;
 #pragma unroll
@@ -672,7 +674,7 @@ __global__ void __launch_bounds__(64) k_thomas_df(Geo g, float *__restrict__ S, 
       float h, l;
       df_mul(c[slot][q].x, c[slot][q].y, rh, rl, h, l);
       df_add(v[slot][q], 0.f, -h, -l, rh, rl);
-      sk[-(long)q * sst] = fmaf(rh, osh, fmaf(rh, osl, rl * osh));
+      sk[-(long)q * sst] = out();
     }
   };
   load(0, 0, 1);
@@ -684,7 +686,7 @@ __global__ void __launch_bounds__(64) k_thomas_df(Geo g, float *__restrict__ S, 
     fwd(1, k0 + PF);
   }
   // the last plane is final, and goes on unrounded
-  s[(long)(K - 1) * sst] = fmaf(rh, osh, fmaf(rh, osl, rl * osh));
+  s[(long)(K - 1) * sst] = out();
   load(0, K - 2, -1);
   for (int k0 = K - 2; k0 >= 0; k0 -= 2 * PF) {
     if (k0 - PF >= 0) load(1, k0 - PF, -1);
@@ -744,8 +746,10 @@ void launch_thomas(cudaStream_t s, const Geo &g, typename cpx<T>::t *S, const do
   const unsigned nb = (unsigned)((n + bs - 1) / bs);
   const double oscale = 1.0 / ((double)(g.I / 2) * g.J) / (g.dzi * g.dzi);
   if constexpr (sizeof(T) == 4) {
-    const float osh = (float)oscale;
-    k_thomas_df<<<nb, bs, 0, s>>>(g, (float *)S, thomas_df, osh, (float)(oscale - (double)osh));
+    const double ia = 1.0 / (g.dzi * g.dzi);
+    const float iah = (float)ia;
+    k_thomas_df<<<nb, bs, 0, s>>>(g, (float *)S, thomas_df, iah, (float)(ia - (double)iah),
+                                  (float)(1.0 / ((double)(g.I / 2) * g.J)));
   } else if (g.zper) {
     k_thomas<true><<<nb, bs, 0, s>>>(g, (double *)S, zt, oscale);
   } else {
@@ -764,14 +768,17 @@ void launch_poisson(cudaStream_t s, const Geo &g, const FftPlan &plx, const FftP
   const int rows = g.I <= 256 ? 4 : 2;
   const int nrow = g.J * g.K;
   const size_t smx = (size_t)2 * rows * M * sizeof(C);
-  // the radix kernels take every transform they have a plan for; the
+  // the passes in registers take every transform they have a plan for; the
   // divergence residual (res64) keeps its own first transform
-  const bool radix = fft_radix_ok<T>(g);
+  bool plan;
+  if constexpr (sizeof(T) == 4) plan = fft_stage_ok(g);
+  else plan = fft_radix_ok<T>(g);
   bool done = false;
   hook(0, 1);
   if constexpr (sizeof(TIn) == sizeof(T)) {
-    if (radix && !res64) {
-      fft_radix_fillps_x<T>(s, g, fu, fv, fw, spec, twM, twN, dtidxi, dtidyi, dtidzi);
+    if (plan && !res64) {
+      if constexpr (sizeof(T) == 4) fft_stage_fillps_x(s, g, fu, fv, fw, spec, twM, twN, dtidxi, dtidyi, dtidzi);
+      else fft_radix_fillps_x<T>(s, g, fu, fv, fw, spec, twM, twN, dtidxi, dtidyi, dtidzi);
       done = true;
     }
   }
@@ -796,8 +803,9 @@ void launch_poisson(cudaStream_t s, const Geo &g, const FftPlan &plx, const FftP
   const size_t smy = (size_t)2 * (g.J + 1) * cols * sizeof(C);
   const dim3 gy((g.MX + cols - 1) / cols, g.K);
   auto ffty = [&](int inv) {
-    if (radix) fft_radix_y<T>(s, g, spec, twJ, inv);
-    else k_ffty<T><<<gy, 256, smy, s>>>(g, ply, S, (const C *)twJ, cols, inv);
+    if (!plan) k_ffty<T><<<gy, 256, smy, s>>>(g, ply, S, (const C *)twJ, cols, inv);
+    else if constexpr (sizeof(T) == 4) fft_stage_y(s, g, spec, twJ, inv);
+    else fft_radix_y<T>(s, g, spec, twJ, inv);
   };
   hook(1, 1);
   ffty(0);
@@ -809,8 +817,9 @@ void launch_poisson(cudaStream_t s, const Geo &g, const FftPlan &plx, const FftP
   ffty(1);
   hook(3, 0);
   hook(4, 1);
-  if (radix) {
-    fft_radix_ix<T>(s, g, spec, phi, twM, twN);
+  if (plan) {
+    if constexpr (sizeof(T) == 4) fft_stage_ix(s, g, spec, phi, twM, twN);
+    else fft_radix_ix<T>(s, g, spec, phi, twM, twN);
   } else {
     const size_t smi = (size_t)(2 * rows * M + rows * (M + 1)) * sizeof(C);
     k_ifftx<T><<<(nrow + rows - 1) / rows, 128, smi, s>>>(g, plx, S, phi, (const C *)twM, (const C *)twN, rows);
@@ -821,7 +830,10 @@ void launch_poisson(cudaStream_t s, const Geo &g, const FftPlan &plx, const FftP
 
 template <typename T>
 int poisson_set_smem_limits() {
-  if (fft_radix_set_smem_limits<T>() != 0) return -1;
+  int st;
+  if constexpr (sizeof(T) == 4) st = fft_stage_set_smem_limits();
+  else st = fft_radix_set_smem_limits<T>();
+  if (st != 0) return -1;
   cudaError_t e[4];
   e[0] = cudaFuncSetAttribute(k_fillps_fftx<T, T, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   if (sizeof(T) == 4)

@@ -1,7 +1,7 @@
-// fft_radix_kernels.cu -- the transforms of the pressure solve for lengths
+// fft_radix_kernels.cu -- the FP64 transforms of the pressure solve for lengths
 // that factor into two or three radices of {2, 3, 4, 6, 8, 9, 12, 16}: fillps
-// + real FFT along x, complex FFT along y, inverse real FFT along x, FP32 and
-// FP64, every length up to about a thousand with factors 2 and 3.
+// + real FFT along x, complex FFT along y, inverse real FFT along x, every
+// length up to about a thousand with factors 2 and 3.  (FP32: fft_stage_kernels.cu.)
 //
 // Stockham order, each butterfly a small DFT in registers.  The first pass
 // takes its elements from global memory (fillps: the divergence formed on the
@@ -10,18 +10,12 @@
 // stages of fft_smem cross it once per stage plus staging (five to seven
 // times for 384 and 768).  The first pass has no twiddles and the last one's
 // index is the butterfly's own, so neither divides.
-// FP32 is bound by L2/HBM traffic and latency (all loads of a butterfly are
-// issued together), FP64 by FP64 issue: a radix-16 butterfly is 160 FP64
-// instructions, ten per element for four binary levels, twiddles 4 each; the
-// real-transform (un)packing forms bins k and M - k together.
-// Measured, us a launch, radix-4/2/3 stages (or the four-step kernels they
-// replaced at powers of two) -> these:
-//   FP32 512 x 512 x 256: fillps+x 584 -> 294, y 433 -> 133, inverse x 399 -> 134
-//   FP32 384 x 384 x 192: fillps+x 254 -> 114, y 146 -> 57, inverse x 178 -> 58
-//   FP32 256^3 (four-step): fillps+x 73 -> 70, y 44 -> 25, inverse x 37.5 -> 36.4
-//   FP64 384 x 192 x 128: fillps+x 445 -> 421, y 287 -> 211, inverse x 331 -> 308
-// (a spectrum read and written once at the copy rate: 79 us at 512 x 512 x 256;
-// the FP64 ones run at 0.48 T FP64 instructions/s, the pipe's rate).
+// Bound by FP64 issue: a radix-16 butterfly is 160 FP64 instructions, ten per
+// element for four binary levels, twiddles 4 each; the real-transform
+// (un)packing forms bins k and M - k together.
+// Measured, us a launch, radix-4/2/3 stages -> these: 384 x 192 x 128: fillps+x
+// 445 -> 421, y 287 -> 211, inverse x 331 -> 308 (0.48 T FP64 instructions/s,
+// the pipe's rate).
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -31,7 +25,6 @@ namespace {
 
 template <typename T> struct cpx;
 template <> struct cpx<double> { typedef double2 t; };
-template <> struct cpx<float> { typedef float2 t; };
 template <typename C> using real_of = decltype(C().x);
 
 template <typename C> __device__ __forceinline__ C mk(real_of<C> a, real_of<C> b) { C r; r.x = a; r.y = b; return r; }
@@ -279,8 +272,8 @@ __device__ __forceinline__ void pass_last(int N, int t, int T, const C *__restri
 }
 
 // Complex FFT along y of COLS neighbouring kx-columns of one plane, in place:
-// COLS neighbours of 8 or 16 bytes make each access of a butterfly a full
-// 64 or 128 bytes, in global and (element-major, columns fastest) shared memory.
+// COLS neighbours of 16 bytes make each access of a butterfly a full 64 or
+// 128 bytes, in global and (element-major, columns fastest) shared memory.
 template <typename C, int MAXR, int INV, int COLS>
 __global__ void __launch_bounds__(MAXR > 9 ? 256 : 512) k_ffty_radix(Geo g, RadixPlan pl, C *__restrict__ S,
                                                                      const C *__restrict__ tw, int T) {
@@ -410,42 +403,24 @@ __global__ void __launch_bounds__(256) k_ifftx_radix(Geo g, RadixPlan pl, const 
     const C D = mk<C>(xk.x - xc.x, xk.y + xc.y), h = mk<C>((T)0.5 * wn.x, (T)0.5 * wn.y);
     O = mk<C>(fma(D.y, h.y, D.x * h.x), fma(-D.x, h.y, D.y * h.x));
   };
-  if constexpr (sizeof(T) == 4) {
-    // FP32, bound by traffic: the first butterflies form their elements from
-    // the spectrum (each bin is read twice, the second time from cache)
-    if (row < nrow) {
-      const C *x = S + (long)row * g.MX;
-      with_radix<MAXR>(pl.r[0], [&](auto R) {
-        pass_first<R.value, 1, C>(
-            M, t, T_,
-            [&](int m) {
-              C E, O;
-              half(x[m], x[M - m], __ldg(&twN[m]), E, O);
-              return mk<C>(E.x - O.y, E.y + O.x);
-            },
-            [&](int m, C v) { b[xpad<C>(m)] = v; });
-      });
-    }
-  } else {
-    // FP64, bound by its instructions: k and M - k together, staged
-    const int H = M / 2 + 1;
-    for (int e = threadIdx.x; e < rows * H; e += blockDim.x) {
-      const int rr = e / H, q = e - rr * H;
-      if (row0 + rr >= nrow) break;
-      const C *x = S + (long)(row0 + rr) * g.MX;
-      C *z = A + rr * RS;
-      C E, O;
-      half(x[q], x[M - q], __ldg(&twN[q]), E, O);
-      z[xpad<C>(q)] = mk<C>(E.x - O.y, E.y + O.x);
-      if (q != 0 && M - q != q) z[xpad<C>(M - q)] = mk<C>(E.x + O.y, O.x - E.y);
-    }
-    __syncthreads();
-    if (row < nrow)
-      with_radix<MAXR>(pl.r[0], [&](auto R) {
-        pass_first<R.value, 1, C>(M, t, T_, [&](int m) { return a[xpad<C>(m)]; },
-                                  [&](int m, C x) { b[xpad<C>(m)] = x; });
-      });
+  // FP64, bound by its instructions: k and M - k together, staged
+  const int H = M / 2 + 1;
+  for (int e = threadIdx.x; e < rows * H; e += blockDim.x) {
+    const int rr = e / H, q = e - rr * H;
+    if (row0 + rr >= nrow) break;
+    const C *x = S + (long)(row0 + rr) * g.MX;
+    C *z = A + rr * RS;
+    C E, O;
+    half(x[q], x[M - q], __ldg(&twN[q]), E, O);
+    z[xpad<C>(q)] = mk<C>(E.x - O.y, E.y + O.x);
+    if (q != 0 && M - q != q) z[xpad<C>(M - q)] = mk<C>(E.x + O.y, O.x - E.y);
   }
+  __syncthreads();
+  if (row < nrow)
+    with_radix<MAXR>(pl.r[0], [&](auto R) {
+      pass_first<R.value, 1, C>(M, t, T_, [&](int m) { return a[xpad<C>(m)]; },
+                                [&](int m, C x) { b[xpad<C>(m)] = x; });
+    });
   __syncthreads();
   if (pl.n == 3) {
     if (row < nrow)
@@ -565,7 +540,6 @@ template <typename T> int fft_radix_set_smem_limits() {
   template void fft_radix_y<T>(cudaStream_t, const Geo &, void *, const void *, int);                              \
   template void fft_radix_ix<T>(cudaStream_t, const Geo &, const void *, T *, const void *, const void *);         \
   template int fft_radix_set_smem_limits<T>();
-FFT_RADIX_INST(float)
 FFT_RADIX_INST(double)
 
 }  // namespace ibmk

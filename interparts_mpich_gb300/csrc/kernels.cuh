@@ -76,7 +76,7 @@ void launch_poisson(cudaStream_t s, const Geo &g, const FftPlan &plx, const FftP
 template <typename T> int poisson_set_smem_limits();
 // tables of the cyclic sweep (periodic z) from the eigenvalues xrt[MX], yrt[J/2+1]
 void launch_cyclic_tables(cudaStream_t s, const Geo &g, const double *xrt, const double *yrt, double *tab);
-// fft_radix_kernels.cu: the transforms of grids whose I/2 and J are products
+// fft_radix_kernels.cu: the FP64 transforms of grids whose I/2 and J are products
 // of two or three small radices (fft_radix_ok)
 template <typename T> bool fft_radix_ok(const Geo &g);
 template <typename T>
@@ -86,6 +86,14 @@ template <typename T> void fft_radix_y(cudaStream_t s, const Geo &g, void *spec,
 template <typename T>
 void fft_radix_ix(cudaStream_t s, const Geo &g, const void *spec, T *phi, const void *twM, const void *twN);
 template <typename T> int fft_radix_set_smem_limits();
+// fft_stage_kernels.cu: the FP32 transforms of grids whose I/2 and J have at
+// most six radix-4/2/3 stages (fft_stage_ok)
+bool fft_stage_ok(const Geo &g);
+void fft_stage_fillps_x(cudaStream_t s, const Geo &g, const float *fu, const float *fv, float *fw, void *spec,
+                        const void *twM, const void *twN, double sx, double sy, double sz);
+void fft_stage_y(cudaStream_t s, const Geo &g, void *spec, const void *twJ, int inv);
+void fft_stage_ix(cudaStream_t s, const Geo &g, const void *spec, float *phi, const void *twM, const void *twN);
+int fft_stage_set_smem_limits();
 
 // ibm_kernels.cu
 // rows (y, z) of a particle's box with a recorded x extent; boxes with more

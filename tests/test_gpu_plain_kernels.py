@@ -87,6 +87,24 @@ def test_projection_divergence(gpu_lib, grid):
     assert s.chkdiv()[1] < 1e-11
 
 
+# FP32 transforms: every pair of stages a pass is made of (4x4, 4x2, 4x3, 2x3,
+# 3x3, single ones), two and three passes, the four-step lengths, and lengths
+# left to the general stages.  Divergence after the projection: terms of up to
+# 32 x 2, six a cell, rounded at 2^-24 in about 20 steps: 5e-4 with room for all
+# of one sign
+@pytest.mark.parametrize("grid", [(32, 16, 4), (64, 256, 4), (128, 64, 4), (512, 128, 4), (16, 12, 4), (48, 36, 5),
+                                  (54, 27, 4), (192, 108, 4), (324, 162, 4), (384, 243, 4), (768, 486, 4), (8, 384, 4),
+                                  (16, 512, 4), (12, 8, 6)])
+def test_projection_fp32(gpu_lib, grid):
+    nx, ny, nz = grid
+    case = Case(name="fft32", itot=nx, jtot=ny, ktot=nz, lx=nx / 32, ly=ny / 32, lz=nz / 32, visc=1e-2)
+    s = IBMSolver(case, mode=_abi.IBM_MODE_MIXED)
+    s.setup(fields=_state(case, 7))
+    s.rk(1, 1e-3)
+    s.project(1, 1e-3)
+    assert s.chkdiv()[1] < 5e-4
+
+
 # radius in cells, particles, grid: below two cells (the reference's inner
 # test reaches past the surface), one sphere shared by several blocks, a box
 # of one slab, of several, of node planes too large for shared memory, and
