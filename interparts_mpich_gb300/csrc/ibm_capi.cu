@@ -535,7 +535,7 @@ int alloc_all(ibm_ctx *c) {
     const int nt = c->pg.ntab;  // entries of each point table (nl, or the sum of the point counts)
     if ((st = dalloc(c, &c->pb.off, (size_t)3 * nt))) return st;
     if ((st = dalloc(c, &c->pb.err, 8))) return st;
-    if ((st = dalloc(c, &c->pb.red, (size_t)(1 + 9 * SI_SLICES) * np))) return st;
+    if ((st = dalloc(c, &c->pb.red, (size_t)(1 + 9 * sphere_slices(np)) * np))) return st;
     if ((st = dalloc(c, &c->pb.pos4, (size_t)2 * np))) return st;
     const size_t ncell = (size_t)c->pg.ncx * c->pg.ncy * c->pg.ncz;
     if ((st = dalloc(c, &c->pb.cstart, ncell + 1))) return st;

@@ -236,7 +236,13 @@ size_t mlp_norm_scratch();
 int launch_mlp_norm(cudaStream_t s, int n, const float *feat, const float *targ, double *scratch, float *norm);
 
 // particle_kernels.cu
-constexpr int SI_SLICES = 8;  // blocks that share one (particle, component) of the sphere integrals, at most
+// blocks that share one (particle, component) of the sphere integrals: two an
+// SM in all, 24 at most (a plane of cells each for a sphere of 20 cells; one
+// sphere of 16 dx in FP64: 36 us with 8, 31 with 24)
+inline int sphere_slices(int np) {
+  const int n = 304 / (3 * (np > 0 ? np : 1));
+  return n < 1 ? 1 : (n > 24 ? 24 : n);
+}
 int sphere_set_smem_limits();
 struct PartBuffers {
   double *pf;     // [PF_N*np]
@@ -249,7 +255,7 @@ struct PartBuffers {
   double *rkp;    // [RK_N*np]
   double *off;    // [3*ntab]: force-point offsets from the centre, x, y, z
   int *err;       // [8] error flags ([4]: learned-forcing MMA wait timeout)
-  double *red;    // [(1 + 9 SI_SLICES) np]: volume [np], sphere-integral partials [np][slice][3][3]
+  double *red;    // [(1 + 9 slices) np]: volume [np], sphere-integral partials [np][slice][3][3]
   float4 *pos4;   // [2][np] FP32 positions (w: master flag) of both iterations' snapshots, for the collision filter
   int *cstart;    // [ncell+1] cell list of the snapshot positions: first item of each cell
   int *cfill;     // [ncell] scatter cursors

@@ -368,22 +368,21 @@ __global__ void __launch_bounds__(SI_T, 5) k_sphere_int_d(Geo g, PartGeo pg, Par
     const int nb = nbz / nzs, zs = nbz - nb * nzs;
     if (nb > 0 && nbf[nb] != 1) continue;
     __syncthreads();  // previous copy done with the tables and the box
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 3) {  // an axis each: in one thread's chain the set-up of one sphere took 31 us, so 27
+      const int ax = threadIdx.x;
       int nbrecv = nb;
       if (nb > 0) { nbrecv = nb + 4; if (nbrecv > 8) nbrecv -= 8; }
       double cx = PF(PF_X), cy = PF(PF_Y);
       const double cz = PF(PF_Z) + (zs == 1 ? -pg.lz : (zs == 2 ? pg.lz : 0.));
       if (nb > 0) copy_shift_sphere(nbrecv, g.lx, g.ly, cx, cy);
-      const int ilow = max(fnint((cx - radius) * g.dxi - 2.), 1), ihigh = min(fnint((cx + radius) * g.dxi + 2.), g.I);
-      const int jlow = max(fnint((cy - radius) * g.dyi - 2.), 1), jhigh = min(fnint((cy + radius) * g.dyi + 2.), g.J);
-      const int klow = max(fnint((cz - radius) * g.dzi - 2.), 1), khigh = min(fnint((cz + radius) * g.dzi + 2.), g.K);
-      s_c[0] = cx; s_c[1] = cy; s_c[2] = cz;
-      s_box[0] = ilow; s_box[1] = ihigh - ilow + 1;
-      s_box[2] = jlow; s_box[3] = jhigh - jlow + 1;
-      s_box[4] = klow; s_box[5] = khigh - klow + 1;
+      const double c = ax == 0 ? cx : (ax == 1 ? cy : cz), di = ax == 0 ? g.dxi : (ax == 1 ? g.dyi : g.dzi);
+      const int low = max(fnint((c - radius) * di - 2.), 1);
+      const int high = min(fnint((c + radius) * di + 2.), ax == 0 ? g.I : (ax == 1 ? g.J : g.K));
+      s_c[ax] = c;
+      s_box[2 * ax] = low;
+      s_box[2 * ax + 1] = high - low + 1;
     }
     __syncthreads();
-    const double cx = s_c[0], cy = s_c[1], cz = s_c[2];
     const int ilow = s_box[0], ni = s_box[1], jlow = s_box[2], nj = s_box[3], klow = s_box[4], nk = s_box[5];
     if (ni <= 0 || nj <= 0 || nk <= 0) continue;
     if (ni > SI_AX || nj > SI_AX || nk > SI_AX) {  // sphere wider than the axis tables: flag, skip
@@ -393,27 +392,18 @@ __global__ void __launch_bounds__(SI_T, 5) k_sphere_int_d(Geo g, PartGeo pg, Par
     // squared distances of the node planes and cell-centre offsets, in the
     // reference's expressions (intgr_over_sphere.f90:335-508); a cell's upper
     // face and the next one's lower face have the same expression's value
-    for (int t = threadIdx.x; t <= SI_AX; t += blockDim.x) {
-      if (t <= ni) {
-        const int i = ilow + t;
-        const double q = (comp == 0 ? 0. + (i - 0.5) * dx : 0. + (i - 1) * dx) - cx;
-        sx2[t] = q * q;
-        fx[t] = (float)sx2[t];
-        if (t < ni) srx[t] = 0. + (i - 0.5) * dx - cx;
-      }
-      if (t <= nj) {
-        const int j = jlow + t;
-        const double q = (comp == 1 ? 0. + (j - 0.5) * dy : 0. + (j - 1) * dy) - cy;
-        sy2[t] = q * q;
-        fy[t] = (float)sy2[t];
-        if (t < nj) sry[t] = 0. + (j - 0.5) * dy - cy;
-      }
-      if (t <= nk) {
-        const int k = klow + t;
-        const double q = (comp < 2 ? (k - 1) * dz : (k - 0.5) * dz) - cz;
-        sz2[t] = q * q;
-        fz[t] = (float)sz2[t];
-        if (t < nk) srz[t] = (k - 0.5) * dz - cz;
+    // (warp ax those of axis ax)
+    if (wid < 3) {
+      const double c = s_c[wid], d = wid == 0 ? dx : (wid == 1 ? dy : dz);
+      const int low = s_box[2 * wid], n = s_box[2 * wid + 1];
+      double *x2 = wid == 0 ? sx2 : (wid == 1 ? sy2 : sz2), *rc = wid == 0 ? srx : (wid == 1 ? sry : srz);
+      float *f2 = wid == 0 ? fx : (wid == 1 ? fy : fz);
+      for (int t = lane; t <= n; t += 32) {
+        const double xc = f2d_rn((float)(low + t) - 0.5f) * d;  // cell centre
+        const double q = (comp == wid ? xc : f2d_rn((float)(low + t - 1)) * d) - c;
+        x2[t] = q * q;
+        f2[t] = (float)x2[t];
+        if (t < n) rc[t] = xc - c;
       }
     }
     const int per = (nk + nsl - 1) / nsl, z0 = blockIdx.z * per, z1 = min(nk, z0 + per);
@@ -596,7 +586,7 @@ void launch_sphere_integrals(cudaStream_t s, const Geo &g, const PartGeo &pg, Pa
   const bool unit = type == 1;  // volume: integrate w = 1 (F == nullptr)
   u = unit ? nullptr : u; v = unit ? nullptr : v; w = unit ? nullptr : w;
   // few particles: several blocks share a (particle, component)
-  const int nsl = std::max(1, std::min(SI_SLICES, 304 / (3 * pg.np)));
+  const int nsl = sphere_slices(pg.np);
   const dim3 grid(pg.np, 3, nsl);
   if constexpr (sizeof(T) == 4) {
     k_sphere_int<<<grid, SF_T, 0, s>>>(g, pg, b, u, v, w);
