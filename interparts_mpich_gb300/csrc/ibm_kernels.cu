@@ -340,9 +340,15 @@ __global__ void __launch_bounds__(1024) k_ibm_res_gate(int n, const double *__re
   }
   if ((threadIdx.x & 31) == 0) { sm[0][threadIdx.x >> 5] = acc; sm[1][threadIdx.x >> 5] = acc0; }
   __syncthreads();
+  if (threadIdx.x >= 32) return;
+  // the 32 warps' sums by a warp (not one thread's chain of 64 FP64 adds)
+  double tot = sm[0][threadIdx.x], tot0 = sm[1][threadIdx.x];
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    tot += __shfl_down_sync(0xffffffffu, tot, d);
+    tot0 += __shfl_down_sync(0xffffffffu, tot0, d);
+  }
   if (threadIdx.x != 0) return;
-  double tot = 0., tot0 = 0.;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { tot += sm[0][w]; tot0 += sm[1][w]; }
   const double R = npts ? sqrt(tot / (double)npts) : 0., R0 = npts ? sqrt(tot0 / (double)npts) : 0.;
   const int cs = stage == 0 ? 1 : 10 + stage, ns = 13 + stage;
   if (plain) {  // the plain passes' reduction of the slip on the current state

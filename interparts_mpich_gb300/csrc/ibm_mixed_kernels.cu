@@ -171,11 +171,7 @@ __global__ void __launch_bounds__(256) k_ibm_box_geom(Geo g, PartGeo pg, IbmBuff
       }
       if (masks) {
         const int x0 = s.b[0] - mn[0], y0 = s.b[1] - mn[1], z0 = s.b[2] - mn[2];
-        const unsigned bits = 7u << x0;  // cells x0 .. x0 + 2 (x0 + 2 < nbx <= 32)
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-          for (int j = 0; j < 3; ++j) atomicOr(&rm[(z0 + k) * nby + y0 + j], bits);
+        atomicOr(&rm[z0 * nby + y0], 7u << x0);  // cells x0 .. x0 + 2 (x0 + 2 < nbx <= 32) of the first row
       }
     }
   __syncthreads();
@@ -198,7 +194,18 @@ __global__ void __launch_bounds__(256) k_ibm_box_geom(Geo g, PartGeo pg, IbmBuff
   }
   if (masks) {
     unsigned *rx = b.rowm + ((long)p * 3 + c) * IBM_BOX_ROWS;
-    for (int q = threadIdx.x; q < nby * nbz; q += blockDim.x) rx[q] = rm[q];
+    // a stencil's nine rows take the same cells (nine shared-memory atomics a
+    // point, many of them on one row: 26 us for 1000 spheres of 16 dx, 23 so)
+    for (int q = threadIdx.x; q < nby * nbz; q += blockDim.x) {
+      const int z = q / nby, y = q - z * nby;
+      unsigned m = 0u;
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          if (z >= k && y >= j) m |= rm[q - k * nby - j];
+      rx[q] = m;
+    }
   }
   if (threadIdx.x < 8) {
     int v = 0;
