@@ -197,10 +197,11 @@ TRAFFIC = {
 LEARNED_SETTLE_STEPS = 12
 
 
-# FP64 flops per cell of the FP64 predictor (momxad/momyad/momzad 3 x 54,
-# pressure gradient 6, RK combination 12-18): the plain form's predictor is
+# FP64 flops per cell of the FP64 predictor with every face flux formed once
+# (three diagonal fluxes 15, three shared pairs 27, their differences 27,
+# pressure gradient 9, RK combination 12-18): the plain form's predictor is
 # bound by the FP64 pipe, not by HBM
-PREDICT_FP64_FLOPS = 183
+PREDICT_FP64_FLOPS = 93
 
 
 def kernel_model(case, w: int) -> dict:
