@@ -15,7 +15,9 @@
 // (un)packing forms bins k and M - k together.
 // Measured, us a launch, radix-4/2/3 stages -> these: 384 x 192 x 128: fillps+x
 // 445 -> 421, y 287 -> 211, inverse x 331 -> 308 (0.48 T FP64 instructions/s,
-// the pipe's rate).
+// the pipe's rate); 256^3: fillps+x 833 -> 703 and inverse x 642 -> 487 with the
+// threads of a row chosen so that both passes use every lane.
+#include <cmath>
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -202,8 +204,24 @@ RadixPlan radix_plan(int N) {
         if (a * b * c == N) take(3, a, b, c);
   return best;
 }
-// threads per sequence: one butterfly each in the pass with the most of them
-int plan_threads(const RadixPlan &pl, int N) {
+// Threads per sequence, lo..hi of them: those that leave the fewest lanes idle.
+// A pass of N/R butterflies takes ceil(N/R / T) turns of all T lanes, and FP64
+// instructions cost the same with half of the lanes (8 x 16 = 128 elements: a
+// quarter is lost with 16 threads, nothing with 8).  Of equal ones the most.
+int plan_threads(const RadixPlan &pl, int N, int lo, int hi) {
+  int best = 1;
+  double least = 1e30;
+  for (int t = lo; t <= hi; ++t) {
+    double cost = 0.;
+    for (int q = 0; q < pl.n; ++q) {
+      const int R = pl.r[q], nb = N / R;
+      cost += (double)((nb + t - 1) / t) * t * R * (4. + 2.5 * std::log2((double)R));
+    }
+    if (cost <= least * (1. + 1e-9)) { least = cost < least ? cost : least; best = t; }
+  }
+  return best;
+}
+int plan_most(const RadixPlan &pl, int N) {  // one butterfly each in the pass with the most of them
   int t = 0;
   for (int q = 0; q < pl.n; ++q) t = N / pl.r[q] > t ? N / pl.r[q] : t;
   return t;
@@ -446,12 +464,17 @@ template <typename C> constexpr int ycols(int passes) { return (passes == 2 ? 12
 template <typename C> size_t ysmem(const RadixPlan &pl, int N) {
   return (size_t)(pl.n == 2 ? 1 : 2) * N * ycols<C>(pl.n) * sizeof(C);
 }
-// rows of a block of the x transforms: about 128 threads, 256 at most
+// rows of a block of the x transforms: about 128 threads, 256 at most; three
+// blocks an SM where there is a choice
 template <typename C> void xshape(const RadixPlan &pl, int M, int &rows, int &T, size_t &smem) {
-  T = plan_threads(pl, M);
-  if (T > 256) T = 256;
+  int hi = plan_most(pl, M);
+  if (hi > 256) hi = 256;
+  auto need = [&](int t) { return (size_t)2 * (t >= 128 ? 1 : 128 / t) * xrow<C>(M) * sizeof(C); };
+  int lo = hi;
+  while (lo > 1 && need(lo - 1) <= 72 * 1024) --lo;
+  T = plan_threads(pl, M, lo, hi);
   rows = T >= 128 ? 1 : 128 / T;
-  smem = (size_t)2 * rows * xrow<C>(M) * sizeof(C);
+  smem = need(T);
 }
 template <typename C> bool radix_fits(const Geo &g, RadixPlan &px, RadixPlan &py) {
   px = radix_plan(g.I / 2);
@@ -465,7 +488,7 @@ template <typename C> bool radix_fits(const Geo &g, RadixPlan &px, RadixPlan &py
 
 template <typename C, int MAXR, int INV, int COLS>
 void ffty_go(cudaStream_t s, const Geo &g, const RadixPlan &pl, C *S, const C *tw) {
-  const int cap = (MAXR > 9 ? 256 : 512) / COLS, t = plan_threads(pl, g.J), T = t < cap ? t : cap;
+  const int cap = (MAXR > 9 ? 256 : 512) / COLS, t = plan_most(pl, g.J), T = t < cap ? t : cap;
   k_ffty_radix<C, MAXR, INV, COLS><<<dim3((g.MX + COLS - 1) / COLS, g.K), COLS * T, ysmem<C>(pl, g.J), s>>>(g, pl, S,
                                                                                                           tw, T);
 }
