@@ -320,8 +320,8 @@ __global__ void __launch_bounds__(SF_T, 8) k_sphere_int(Geo g, PartGeo pg, PartB
 // time (ncap doubles of shared memory, small enough for five blocks an SM: the
 // phases of one overlap the others'; a sphere too wide for two node planes
 // forms its corner distances cell by cell).  1000 spheres of 16 dx: 1063 ->
-// 542 us (a warp per row of cells in place of a thread per line: 682); one
-// sphere, 8 slices: 82 -> 35 us.
+// 542 us (a warp per row of cells in place of a thread per line: 682), 519 with
+// the set-up spread over lanes and warps; one sphere 82 -> 27 us.
 constexpr int SI_T = 128, SI_AX = 128, SI_QCAP = 1024, SI_NODES = 16384;
 __global__ void __launch_bounds__(SI_T, 5) k_sphere_int_d(Geo g, PartGeo pg, PartBuffers b, const double *__restrict__ u,
                                                       const double *__restrict__ v, const double *__restrict__ w,
