@@ -167,28 +167,28 @@ __global__ void __launch_bounds__(FT_T + 32) k_ibm_force_torque(PartGeo pg, IbmB
       const double phi = b.pf[PF_PHI * np + p];
       trig[threadIdx.x - FT_T] = threadIdx.x == FT_T ? cos(phi) : sin(phi);
     }
-    __syncthreads();
-    return;
-  }
-  const double px = b.pf[PF_X * np + p], py = b.pf[PF_Y * np + p], pz = b.pf[PF_Z * np + p];
-  double s[6] = {0., 0., 0., 0., 0., 0.};
+  } else {
+    const double px = b.pf[PF_X * np + p], py = b.pf[PF_Y * np + p], pz = b.pf[PF_Z * np + p];
+    double s[6] = {0., 0., 0., 0., 0., 0.};
 #pragma unroll 3
-  for (int l = threadIdx.x; l < nla; l += FT_T) {
-    const long t = (long)p * pg.nl + l;
-    const double fx = b.fxl[t], fy = b.fyl[t], fz = b.fzl[t];
-    const double rx = b.xfp[t] - px, ry = b.yfp[t] - py, rz = b.zfp[t] - pz;
-    s[0] += fx; s[1] += fy; s[2] += fz;
-    s[3] = fma(-rz, fy, fma(ry, fz, s[3]));
-    s[4] = fma(-rx, fz, fma(rz, fx, s[4]));
-    s[5] = fma(-ry, fx, fma(rx, fy, s[5]));
-  }
+    for (int l = threadIdx.x; l < nla; l += FT_T) {
+      const long t = (long)p * pg.nl + l;
+      const double fx = b.fxl[t], fy = b.fyl[t], fz = b.fzl[t];
+      const double rx = b.xfp[t] - px, ry = b.yfp[t] - py, rz = b.zfp[t] - pz;
+      s[0] += fx; s[1] += fy; s[2] += fz;
+      s[3] = fma(-rz, fy, fma(ry, fz, s[3]));
+      s[4] = fma(-rx, fz, fma(rz, fx, s[4]));
+      s[5] = fma(-ry, fx, fma(rx, fy, s[5]));
+    }
 #pragma unroll
-  for (int q = 0; q < 6; ++q) {
+    for (int q = 0; q < 6; ++q) {
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) s[q] += __shfl_down_sync(0xffffffffu, s[q], d);
-    if ((threadIdx.x & 31) == 0) red[q][threadIdx.x >> 5] = s[q];
+      for (int d = 16; d > 0; d >>= 1) s[q] += __shfl_down_sync(0xffffffffu, s[q], d);
+      if ((threadIdx.x & 31) == 0) red[q][threadIdx.x >> 5] = s[q];
+    }
   }
   __syncthreads();
+  if (threadIdx.x >= 32) return;
   if (threadIdx.x < 6) {
     const int q = threadIdx.x;
     const double v = ((red[q][0] + red[q][1]) + (red[q][2] + red[q][3])) * p_dvl(pg, p);
