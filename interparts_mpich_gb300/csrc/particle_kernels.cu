@@ -1241,6 +1241,7 @@ __global__ void __launch_bounds__(256) k_ne_finalize(PartGeo pg, PartBuffers b, 
   __shared__ double sx, sy, sz, su, sv, sw, somx, somy, somz;
   __shared__ int wcount[32];
   __shared__ int base;
+  __shared__ int edge[4];  // high words of the planes where the periodic image changes, x and y
   // init: 0 = after Newton-Euler, 1 = initial set-up (initparticles +
   // coordsfp), 2 = Lagrangian points only (restart with given flags)
   if (threadIdx.x == 0) {
@@ -1284,6 +1285,10 @@ __global__ void __launch_bounds__(256) k_ne_finalize(PartGeo pg, PartBuffers b, 
     }
     sx = x; sy = y; sz = PF(PF_Z); su = PF(PF_U); sv = PF(PF_V); sw = PF(PF_W);
     somx = PF(PF_OMX); somy = PF(PF_OMY); somz = PF(PF_OMZ);
+    edge[0] = __double2hiint(0.5 * pg.dx);
+    edge[1] = __double2hiint(pg.lx + 0.5 * pg.dx);
+    edge[2] = __double2hiint(0.5 * pg.dy);
+    edge[3] = __double2hiint(pg.ly + 0.5 * pg.dy);
     base = 0;
   }
   __syncthreads();
@@ -1292,11 +1297,18 @@ __global__ void __launch_bounds__(256) k_ne_finalize(PartGeo pg, PartBuffers b, 
   const int nl = pg.nl, nlp = p_nl(pg, p), nt = pg.ntab;
   const double *off3 = b.off + p_toff(pg, p);
   const int wid = threadIdx.x / 32, lane = threadIdx.x % 32;
-  // isout (periodic image outside 1..I, 1..J) is impossible for points within
-  // half a domain of it: a screen of the whole sphere decides that, else the
-  // reference's FP64 test point by point
+  // isout (periodic image outside 1..I, 1..J): a point within half a domain of it
+  // can only be so by a rounding next to one of the two planes 0.5 dx and lx +
+  // 0.5 dx, where the image changes.  So the reference's FP64 test is for points
+  // within about 2^-20 of such a plane, by the high words of the coordinates (which
+  // order like the integers; a negative coordinate is far from both), and for all
+  // points of spheres farther out.
   const double rs = 1.01 * p_rad(pg, p);
   const bool inside = sx - rs > -0.4 * pg.lx && sx + rs < 1.4 * pg.lx && sy - rs > -0.4 * pg.ly && sy + rs < 1.4 * pg.ly;
+  auto at_plane = [](double x, const int *h) {
+    const unsigned q = (unsigned)__double2hiint(x) + 1u;
+    return q - (unsigned)h[0] <= 2u || q - (unsigned)h[1] <= 2u;
+  };
   const bool spin = !(somx == 0. && somy == 0. && somz == 0.);
   for (int l0 = 0; l0 < nlp; l0 += blockDim.x) {
     const int l = l0 + threadIdx.x;
@@ -1312,7 +1324,7 @@ __global__ void __launch_bounds__(256) k_ne_finalize(PartGeo pg, PartBuffers b, 
       yfploc = sy + ry;
       zfploc = sz + rz;
       bool isout = false;
-      if (!inside) {
+      if (!inside || at_plane(xfploc, edge) || at_plane(yfploc, edge + 2)) {
         double isperiodx = 0., isperiody = 0.;
         if (xfploc < 0. + 0.5 * pg.dx) isperiodx = 1.;
         if (xfploc >= pg.lx + 0.5 * pg.dx) isperiodx = -1.;

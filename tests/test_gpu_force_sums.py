@@ -48,3 +48,23 @@ def test_force_and_torque_sums(gpu_lib, r, points, passes):
     for q in ("torqxltot", "torqyltot", "torqzltot", "torqtheta"):
         assert np.max(np.abs(getattr(a, q) - getattr(b, q))) <= 2 * shell * tol, q
     assert np.max(np.abs(b.torqtheta)) > 1e6 * shell * tol
+
+
+# the reference leaves out a point whose periodic image rounds to a cell outside
+# the grid: next to the planes half a cell inside the domain and beyond it.  The
+# first point of the table lies level with its sphere's centre in y
+@pytest.mark.parametrize("ny", [32, 48, 108])
+def test_points_at_the_image_planes(gpu_lib, ny):
+    h = 1.0 / ny
+    half = 0.5 / float(ny)
+    y = [np.nextafter(half, 0), half, np.nextafter(half, 1), np.nextafter(1 + half, 0), 1 + half, 0.37, 0.0, 1.0]
+    case = Case(name="planes", itot=32, jtot=ny, ktot=24, lx=32 * h, ly=1.0, lz=24 * h, visc=1e-2, radius=3.3 * h,
+                np=len(y), centres=np.stack([np.full(len(y), 9.3 * h), y, np.full(len(y), 11.7 * h)], 1))
+    got = []
+    for s in (IBMSolver(case), OracleSolver(case)):
+        s.setup()
+        got.append(s.get_particles())
+    kept = [int(np.count_nonzero(p.zfp.reshape(len(y), -1)[0])) for p in got]
+    assert kept[0] == kept[1] and (ny == 108 or kept[1] == case.nl - 1)
+    for q in ("xfp", "yfp", "zfp", "ul"):
+        assert np.array_equal(getattr(got[0], q), getattr(got[1], q)), q
