@@ -382,7 +382,7 @@ void derived(ibm_ctx *c) {
   // quads that cover them; at most 160 KB of shared memory
   auto ext = [&](double di) { return (long)std::floor(2. * (pg.rmax - 0.3 / g.dxi) * di) + 5; };
   const long row = P.np > 0 ? (ext(g.dxi) + 3 + 3) / 4 * 4 : 0;
-  pg.box_cap = P.np > 0 ? (int)std::min(40960L, std::max(8192L, row * ext(g.dyi) * ext(g.dzi))) : 8192;
+  pg.box_cap = P.np > 0 ? (int)std::min((long)IBM_BOX_MOST, std::max(8192L, row * ext(g.dyi) * ext(g.dzi))) : 8192;
 }
 
 // twiddles and the Thomas pivots (initsolver.f90:10-66)
@@ -1120,7 +1120,8 @@ ibm_ctx *ibm_create(const ibm_params *P) {
   int st = alloc_all(c);
   if (st == IBM_OK) st = build_solver_tables(c);
   if (st == IBM_OK && (poisson_set_smem_limits<double>() != 0 || poisson_set_smem_limits<float>() != 0 ||
-                       mlp_set_smem_limits() != 0 || sphere_set_smem_limits() != 0 || ibm_set_smem_limits(c->pg) != 0))
+                       mlp_set_smem_limits() != 0 || sphere_set_smem_limits() != 0 ||
+                       (c->mixed && c->pg.np > 0 && ibm_set_smem_limits() != 0)))
     st = set_err(c, IBM_E_CUDA, "cudaFuncSetAttribute failed");
   if (st == IBM_OK) st = cuda_err(c, cudaStreamSynchronize(c->stream), "create");
   if (st != IBM_OK) {

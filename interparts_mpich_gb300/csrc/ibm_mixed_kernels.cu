@@ -932,15 +932,13 @@ void launch_ibm_features_f(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmB
                                         first_force);
 }
 
-// the box kernels' dynamic shared memory, raised (never lowered: other
-// contexts may use larger boxes) to a context's boxes
-int ibm_set_smem_limits(const PartGeo &pg) {
-  static int cur = 0;
-  const int need = (int)interp_smem(pg);
-  if (need <= cur) return 0;
+// the box kernels' dynamic shared memory: as much as any context uses.  Set at
+// every create, since the attributes belong to the current device's context
+int ibm_set_smem_limits() {
+  constexpr int bytes = (IBM_BOX_MOST + SPREAD_PRE) * (int)sizeof(float);
   cudaError_t e = cudaSuccess;
   auto set = [&](auto k) {
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   };
   auto all = [&](auto many) {
     constexpr int NT = decltype(many)::value ? NT_MANY : NT_FEW, MB = decltype(many)::value ? MB_MANY : MB_FEW;
@@ -956,9 +954,7 @@ int ibm_set_smem_limits(const PartGeo &pg) {
   };
   all(std::true_type{});
   all(std::false_type{});
-  if (e != cudaSuccess) return -1;
-  cur = need;
-  return 0;
+  return e == cudaSuccess ? 0 : -1;
 }
 
 }  // namespace ibmk

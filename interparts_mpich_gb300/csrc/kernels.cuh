@@ -99,6 +99,7 @@ int fft_stage_set_smem_limits();
 // rows (y, z) of a particle's box with a recorded x extent; boxes with more
 // rows are read whole
 constexpr int IBM_BOX_ROWS = 1024;
+constexpr int IBM_BOX_MOST = 40960;  // cells of the largest box (PartGeo::box_cap)
 constexpr int IBM_BST = 36;  // entries of IbmBuffers::bst per (particle, component)
 // fields of IbmBuffers::sw: the weights of three nodes along an axis, of the
 // staggered origin (nearest face) and of the centred one (H)
@@ -190,7 +191,7 @@ struct MlpTrainBuffers {
 };
 int mlp_nparam();
 size_t mlp_part_floats(int nb);
-int ibm_set_smem_limits(const PartGeo &pg);
+int ibm_set_smem_limits();
 int mlp_set_smem_limits();
 void launch_mlp_refresh(cudaStream_t s, const float *params, __nv_bfloat16 *w1b, __nv_bfloat16 *w2b);
 void launch_mlp_infer(cudaStream_t s, const __nv_bfloat16 *x, int n, const __nv_bfloat16 *w1b,
