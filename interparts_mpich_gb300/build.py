@@ -47,7 +47,7 @@ def _stale(target: Path, deps: list[Path]) -> bool:
 def build(verbose: bool = False, force: bool = False, extra_flags: list[str] | None = None) -> Path:
     """Compile every .cu under csrc/ for sm_103a and link libibm_rk3.so."""
     BUILD.mkdir(exist_ok=True)
-    headers = list(CSRC.glob("*.cuh")) + list(INCLUDE.glob("*.h"))
+    headers = [*CSRC.glob("*.cuh"), *CSRC.glob("*.h"), *INCLUDE.glob("*.h")]
     exe = nvcc()
     jobs = []
     for src in sources():

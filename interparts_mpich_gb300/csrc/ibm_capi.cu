@@ -377,12 +377,9 @@ void derived(ibm_ctx *c) {
     pg.ciy = (float)(pg.ncy / P.ly);
     pg.ciz = (float)(pg.ncz / P.lz);
   }
-  // the largest (particle, component) box of the mixed form, per axis the
-  // shell's extent and the 3-point stencils, its rows padded to the aligned
-  // quads that cover them; at most 160 KB of shared memory
-  auto ext = [&](double di) { return (long)std::floor(2. * (pg.rmax - 0.3 / g.dxi) * di) + 5; };
-  const long row = P.np > 0 ? (ext(g.dxi) + 3 + 3) / 4 * 4 : 0;
-  pg.box_cap = P.np > 0 ? (int)std::min((long)IBM_BOX_MOST, std::max(8192L, row * ext(g.dyi) * ext(g.dzi))) : 8192;
+  // the (particle, component) boxes of the mixed form
+  const double shell = 2. * (pg.rmax - 0.3 / g.dxi), span[3] = {shell * g.dxi, shell * g.dyi, shell * g.dzi};
+  pg.box_cap = P.np > 0 ? box_capacity(span) : BOX_LEAST;
 }
 
 // twiddles and the Thomas pivots (initsolver.f90:10-66)

@@ -103,35 +103,10 @@ __global__ void __launch_bounds__(256) k_ibm_points(Geo g, PartGeo pg, IbmBuffer
 // cz*nby + cy] = the cells the stencils touch in that row (bit cx): a
 // sphere's shell touches about 40 % of its box, and a row through the
 // sphere only its two ends.
-// Its copy in shared memory: with I a multiple of 4 the rows hold the aligned
-// quads of x-cells that cover them (a quad never straddles the periodic wrap),
-// so that whole quads move; else the rows alone.
-struct BoxLay {
-  int x0, y0, z0, nbx, nby, nbz;  // first cell (x, y not wrapped) and extents
-  int sh, pitch, cells;           // cells before x0 in a row, row length, size
-  __device__ __forceinline__ BoxLay(const int *bg, int I) {
-    x0 = bg[0] + bg[2]; y0 = bg[1] + bg[3]; z0 = bg[4];
-    nbx = bg[5]; nby = bg[6]; nbz = bg[7];
-    const bool quads = (I & 3) == 0;
-    sh = quads ? x0 & 3 : 0;
-    pitch = quads ? (sh + nbx + 3) & ~3 : nbx;
-    cells = pitch * nby * nbz;
-  }
-  // usable: fits cap and narrower than half the periodic domain (so relative
-  // indices are unambiguous)
-  __device__ __forceinline__ bool ok(long cap, int I, int J) const {
-    return nbx > 0 && (long)pitch * nby * nbz <= cap && nbx < I / 2 && nby < J / 2;
-  }
-  // offset of tap (0,0,0) of a point (make_cs origin, relative in x and y)
-  __device__ __forceinline__ int off(const CompStencil &s, const int *bg) const {
-    return ((s.b[2] - bg[4]) * nby + (s.b[1] - bg[3])) * pitch + (s.b[0] - bg[2]) + sh;
-  }
-};
 // Points of particle p, component c by the bank of their first tap:
 // order[(p*3 + c)*nl + bst[q] ..bst[q+1]) = those of bank q, bst[33] = the most
 // of any bank (bst: IBM_BST entries per (p, c)); -1 there where the points are
 // not ordered (box not usable, or more than SPREAD_PRE of them).
-constexpr int SPREAD_PRE = 2048;
 __global__ void __launch_bounds__(256) k_ibm_box_geom(Geo g, PartGeo pg, IbmBuffers b) {
   const int p = blockIdx.x, c = blockIdx.y, K = g.K;
   const int nla = b.nla[p];
@@ -935,22 +910,22 @@ void launch_ibm_features_f(cudaStream_t s, const Geo &g, const PartGeo &pg, IbmB
 // the box kernels' dynamic shared memory: as much as any context uses.  Set at
 // every create, since the attributes belong to the current device's context
 int ibm_set_smem_limits() {
-  constexpr int bytes = (IBM_BOX_MOST + SPREAD_PRE) * (int)sizeof(float);
+  constexpr int boxes = BOX_MOST * (int)sizeof(float), values = SPREAD_PRE * (int)sizeof(float);
   cudaError_t e = cudaSuccess;
-  auto set = [&](auto k) {
+  auto set = [&](auto k, int bytes) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   };
   auto all = [&](auto many) {
     constexpr int NT = decltype(many)::value ? NT_MANY : NT_FEW, MB = decltype(many)::value ? MB_MANY : MB_FEW;
-    set(k_ibm_spread_f<false, NT, MB>);
-    set(k_ibm_spread_f<true, NT, MB>);
+    set(k_ibm_spread_f<false, NT, MB>, boxes);
+    set(k_ibm_spread_f<true, NT, MB>, boxes);
     for (auto k : {k_ibm_interp_comp_f<1, false, false, NT, MB>, k_ibm_interp_comp_f<0, false, false, NT, MB>,
                    k_ibm_interp_comp_f<1, false, true, NT, MB>, k_ibm_interp_comp_f<0, false, true, NT, MB>,
                    k_ibm_interp_comp_f<1, true, false, NT, MB>, k_ibm_interp_comp_f<0, true, false, NT, MB>,
                    k_ibm_interp_comp_f<1, true, true, NT, MB>, k_ibm_interp_comp_f<0, true, true, NT, MB>,
                    k_ibm_interp_comp_f<-1, false, false, NT, MB>, k_ibm_interp_comp_f<-1, true, false, NT, MB>,
                    k_ibm_interp_comp_f<-2, false, false, NT, MB>, k_ibm_interp_comp_f<-2, true, false, NT, MB>})
-      set(k);
+      set(k, boxes + values);
   };
   all(std::true_type{});
   all(std::false_type{});

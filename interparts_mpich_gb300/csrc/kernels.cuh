@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_bf16.h>
 
+#include "ibm_box.h"
 #include "ibm_common.cuh"
 
 struct FftPlan {
@@ -99,7 +100,6 @@ int fft_stage_set_smem_limits();
 // rows (y, z) of a particle's box with a recorded x extent; boxes with more
 // rows are read whole
 constexpr int IBM_BOX_ROWS = 1024;
-constexpr int IBM_BOX_MOST = 40960;  // cells of the largest box (PartGeo::box_cap)
 constexpr int IBM_BST = 36;  // entries of IbmBuffers::bst per (particle, component)
 // fields of IbmBuffers::sw: the weights of three nodes along an axis, of the
 // staggered origin (nearest face) and of the centred one (H)

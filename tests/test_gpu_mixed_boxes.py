@@ -52,3 +52,32 @@ def test_forcing_boxes(gpu_lib, d, n, grid, rotation):
         got.append(f)
     for q in got[0]:
         assert rel_l2(got[0][q], got[1][q]) < TOL, q
+
+
+# the largest boxes: spheres of up to 32 cells (rows padded to quads take more
+# cells than the rows), of 34, the last that fit, of 35, and spheres whose boxes
+# are far beyond the shared memory beside smaller ones
+@pytest.mark.parametrize("d", [(31.5, 24.0), (34.0,), (35.0,), (42.0, 14.0)])
+@pytest.mark.parametrize("unequal", [False, True])
+def test_forcing_largest_boxes(gpu_lib, d, unequal):
+    nx, ny, nz = 144, 96, 64
+    h = 1.0 / 64
+    rng = np.random.default_rng(6)
+    n = len(d)
+    d = np.array(d) if unequal else np.full(n, d[0])
+    c = np.array([[(q + 0.03) * nx * h / n, (q + 0.4) * ny * h / n, rng.uniform(22.5, 41.5) * h] for q in range(n)])
+    case = Case(name="boxes", itot=nx, jtot=ny, ktot=nz, lx=nx * h, ly=ny * h, lz=nz * h, visc=1e-3,
+                radius=d[0] * h / 2, np=n, centres=c, radii=d * h / 2 if unequal else None)
+    ps = case.initial_particles(lagrangian=False)
+    ps.u[:], ps.v[:], ps.w[:] = rng.uniform(-0.1, 0.1, (3, n))
+    got = []
+    for s in (IBMSolver(case, mode=IBM_MODE_MIXED), OracleSolver(case)):
+        s.setup(particles=ps)
+        s.rk(1, 1e-3)
+        s.forcing_loop(1e-3, 3)
+        f = {q: interior(a) for q, a in s.get_intermediate().items()}
+        p = s.get_particles(lagrangian=False)
+        f["force"] = np.stack([p.fxltot, p.fyltot, p.fzltot])
+        got.append(f)
+    for q in got[0]:
+        assert rel_l2(got[0][q], got[1][q]) < TOL, q
