@@ -1323,7 +1323,7 @@ int ibm_set_particles(ibm_ctx *c, const ibm_particles *s) {
   if (np == 0) { c->have_particles = true; c->particles_ready = true; return IBM_OK; }
   const double *arr[31];
   pf_host_ptrs(s, arr);
-  std::vector<double> pf((size_t)PF_N * np, 0.);
+  std::vector<double> pf((size_t)PF_STATE * np, 0.);
   for (int f = 0; f < 31; ++f) {
     if (!arr[f]) return set_err(c, IBM_E_INVALID, "particle array missing");
     std::memcpy(&pf[(size_t)f * np], arr[f], np * sizeof(double));
@@ -1413,7 +1413,7 @@ int ibm_get_particles(ibm_ctx *c, ibm_particles *s) {
   if (!c || !s) return IBM_E_INVALID;
   const int np = c->pg.np, nq = c->nq, nl = c->pg.nl;
   if (np == 0) return IBM_OK;
-  std::vector<double> pf((size_t)PF_N * np);
+  std::vector<double> pf((size_t)PF_STATE * np);
   CK(cudaMemcpyAsync(pf.data(), c->pb.pf, pf.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   std::vector<double> cf((size_t)CF_N * np * nq);
   CK(cudaMemcpyAsync(cf.data(), c->pb.cf, cf.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));

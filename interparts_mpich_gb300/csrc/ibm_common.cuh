@@ -28,9 +28,10 @@ enum PField {
   PF_OX, PF_OY, PF_OZ, PF_OTHETA, PF_OPHI, PF_OU, PF_OV, PF_OW, PF_OOMX, PF_OOMY, PF_OOMZ, PF_OOMTHETA,
   PF_OINTU, PF_OINTV, PF_OINTW, PF_OINTOMX, PF_OINTOMY, PF_OINTOMZ,
   PF_OCOLFX, PF_OCOLFY, PF_OCOLFZ, PF_OCOLTX, PF_OCOLTY, PF_OCOLTZ,
+  PF_STATE,  // fields up to here cross the interface
   // snapshots of the collision pass (anb(:,0)), x,y,z,u,v,w,omx,omy,omz, of
-  // both iterations in turn
-  PF_SX, PF_S_LAST = PF_SX + 2 * 9 - 1,
+  // both iterations in turn, each taken before it is read in every substep
+  PF_SX = PF_STATE, PF_S_LAST = PF_SX + 2 * 9 - 1,
   PF_N
 };
 // contact arrays: current and old
