@@ -40,7 +40,7 @@ struct ibm_ctx {
   int nq = 0;
   // derived (init.f90:74-243)
   double offset = 0, volp = 0, mominert = 0, rkab[3] = {0, 0, 0};
-  // FP64 fields
+  // FP64 fields (plain form)
   double *u = nullptr, *v = nullptr, *w = nullptr, *p = nullptr;
   double *ru = nullptr, *rv = nullptr, *rw = nullptr;
   double *fu = nullptr, *fv = nullptr, *fw = nullptr, *phi = nullptr;
@@ -48,7 +48,7 @@ struct ibm_ctx {
   // mixed form: FP32 predictor, RHS, Poisson work arrays
   bool mixed = false;
   float *u32 = nullptr, *v32 = nullptr, *w32 = nullptr, *p32 = nullptr;  // FP32 state
-  float *plo32 = nullptr;  // pnew = p32 + plo32 (double-float); p is the FP64 staging copy
+  float *plo32 = nullptr;  // pnew = p32 + plo32 (double-float)
   float *ru32 = nullptr, *rv32 = nullptr, *rw32 = nullptr;
   float *fu32 = nullptr, *fv32 = nullptr, *fw32 = nullptr, *phi32 = nullptr;
   float *phi32b = nullptr;  // second (defect-correction) Poisson solution
@@ -1204,6 +1204,7 @@ static int upload_any(ibm_ctx *c, const double *h, T *d, float *lo = nullptr) {
   const size_t n = (size_t)(c->g.I + 2) * (c->g.J + 2) * (c->g.K + 2);
   if (!h) {
     CK(cudaMemsetAsync(d, 0, (size_t)c->g.nfield * sizeof(T), c->stream));
+    if (lo) CK(cudaMemsetAsync(lo, 0, (size_t)c->g.nfield * sizeof(float), c->stream));
     return IBM_OK;
   }
   const double *src = static_cast<const double *>(device_view(h));
