@@ -151,17 +151,16 @@ __device__ C *fft_smem1(C *a, C *b, int M, int nseq, int ss, const FftPlan &pl, 
 }
 
 // ---------------------------------------------------------------------------
-// Register four-step FFT (FP32 path).  N = N1*N2 with N1 = N2 or 2*N2 and
-// N1 <= 16: a group of N2 threads holds a sequence, thread t the elements
+// Register four-step FFT of the FP32 divergence residual (forward).  N = N1*N2
+// with N1 = N2 or 2*N2 and N1 <= 16: a group of N2 threads holds a sequence, thread t the elements
 // x[t + N2*n1]; an N1-point DFT in registers, the twiddle W_N^(t*k1), one
 // exchange through a padded shared buffer (group-private, __syncwarp only),
 // then N2-point DFTs in registers (N1/N2 per thread), written back in
 // natural order.  Same DFT as the Stockham stages, other summation order.
 // ---------------------------------------------------------------------------
-// multiply by exp(-+2 pi i m/den) given cos, sin of 2 pi m/den
-template <typename C>
-__device__ __forceinline__ C cmulcs(C x, float c, float s, int inv) {
-  return inv ? cmk<C>(x.x * c - x.y * s, x.y * c + x.x * s) : cmk<C>(x.x * c + x.y * s, x.y * c - x.x * s);
+// multiply by exp(-2 pi i m/den) given cos, sin of 2 pi m/den
+__device__ __forceinline__ float2 cmulcs(float2 x, float c, float s) {
+  return make_float2(x.x * c + x.y * s, x.y * c - x.x * s);
 }
 // cos, sin of 2 pi m / 16, m = 0..9
 __device__ __forceinline__ void w16(int m, float &c, float &s) {
@@ -170,29 +169,28 @@ __device__ __forceinline__ void w16(int m, float &c, float &s) {
   const float sn[10] = {0.f, S1, R2, C1, 1.f, C1, R2, S1, 0.f, -S1};
   c = cs[m]; s = sn[m];
 }
-template <int N, typename C> __device__ __forceinline__ void dft_reg(C *v, int inv);
-template <> __device__ __forceinline__ void dft_reg<2, float2>(float2 *v, int) { dft2(v); }
-template <> __device__ __forceinline__ void dft_reg<4, float2>(float2 *v, int inv) { dft4(v, inv); }
-template <> __device__ __forceinline__ void dft_reg<8, float2>(float2 *v, int inv) {
+template <int N> __device__ __forceinline__ void dft_reg(float2 *v);
+template <> __device__ __forceinline__ void dft_reg<4>(float2 *v) { dft4(v, 0); }
+template <> __device__ __forceinline__ void dft_reg<8>(float2 *v) {
   // n = n2 + 2 n1, k = k1 + 4 k2
   float2 a0[4] = {v[0], v[2], v[4], v[6]}, a1[4] = {v[1], v[3], v[5], v[7]};
-  dft4(a0, inv);
-  dft4(a1, inv);
+  dft4(a0, 0);
+  dft4(a1, 0);
   float c, s;
-  w16(2, c, s); a1[1] = cmulcs(a1[1], c, s, inv);
-  a1[2] = cmi(a1[2], inv);
-  w16(6, c, s); a1[3] = cmulcs(a1[3], c, s, inv);
+  w16(2, c, s); a1[1] = cmulcs(a1[1], c, s);
+  a1[2] = cmi(a1[2], 0);
+  w16(6, c, s); a1[3] = cmulcs(a1[3], c, s);
 #pragma unroll
   for (int k1 = 0; k1 < 4; ++k1) { v[k1] = cadd(a0[k1], a1[k1]); v[k1 + 4] = csub(a0[k1], a1[k1]); }
 }
-template <> __device__ __forceinline__ void dft_reg<16, float2>(float2 *v, int inv) {
+template <> __device__ __forceinline__ void dft_reg<16>(float2 *v) {
   // n = n2 + 4 n1, k = k1 + 4 k2
   float2 a[4][4];
 #pragma unroll
   for (int n2 = 0; n2 < 4; ++n2) {
 #pragma unroll
     for (int n1 = 0; n1 < 4; ++n1) a[n2][n1] = v[n2 + 4 * n1];
-    dft4(a[n2], inv);
+    dft4(a[n2], 0);
   }
 #pragma unroll
   for (int n2 = 1; n2 < 4; ++n2)
@@ -200,12 +198,12 @@ template <> __device__ __forceinline__ void dft_reg<16, float2>(float2 *v, int i
     for (int k1 = 1; k1 < 4; ++k1) {
       float c, s;
       w16(n2 * k1, c, s);
-      a[n2][k1] = cmulcs(a[n2][k1], c, s, inv);
+      a[n2][k1] = cmulcs(a[n2][k1], c, s);
     }
 #pragma unroll
   for (int k1 = 0; k1 < 4; ++k1) {
     float2 b[4] = {a[0][k1], a[1][k1], a[2][k1], a[3][k1]};
-    dft4(b, inv);
+    dft4(b, 0);
 #pragma unroll
     for (int k2 = 0; k2 < 4; ++k2) v[k1 + 4 * k2] = b[k2];
   }
@@ -214,37 +212,27 @@ template <> __device__ __forceinline__ void dft_reg<16, float2>(float2 *v, int i
 // ex: group-private exchange buffer of N1*(N2+1) elements.  Every thread of
 // the warp must call it (it synchronises the warp).
 template <int N1, int N2>
-__device__ __forceinline__ void fft_group(float2 *row, float2 *ex, int t, const float2 *__restrict__ tw, int inv,
-                                          bool active) {
+__device__ __forceinline__ void fft_group(float2 *row, float2 *ex, int t, const float2 *__restrict__ tw) {
   constexpr int N = N1 * N2;
   float2 v[N1];
-  if (active) {
 #pragma unroll
-    for (int r = 0; r < N1; ++r) v[r] = row[t + N2 * r];
-    dft_reg<N1, float2>(v, inv);
+  for (int r = 0; r < N1; ++r) v[r] = row[t + N2 * r];
+  dft_reg<N1>(v);
 #pragma unroll
-    for (int k1 = 1; k1 < N1; ++k1) {
-      if (t > 0) {
-        float2 w = __ldg(&tw[(t * k1) % N]);
-        if (inv) w.y = -w.y;
-        v[k1] = cmul(v[k1], w);
-      }
-    }
+  for (int k1 = 1; k1 < N1; ++k1)
+    if (t > 0) v[k1] = cmul(v[k1], __ldg(&tw[(t * k1) % N]));
 #pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) ex[k1 * (N2 + 1) + t] = v[k1];
-  }
+  for (int k1 = 0; k1 < N1; ++k1) ex[k1 * (N2 + 1) + t] = v[k1];
   __syncwarp();
-  if (active) {
 #pragma unroll
-    for (int q = 0; q < N1 / N2; ++q) {
-      const int k1 = t + q * N2;
-      float2 w[N2];
+  for (int q = 0; q < N1 / N2; ++q) {
+    const int k1 = t + q * N2;
+    float2 w[N2];
 #pragma unroll
-      for (int n2 = 0; n2 < N2; ++n2) w[n2] = ex[k1 * (N2 + 1) + n2];
-      dft_reg<N2, float2>(w, inv);
+    for (int n2 = 0; n2 < N2; ++n2) w[n2] = ex[k1 * (N2 + 1) + n2];
+    dft_reg<N2>(w);
 #pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2) row[k1 + N1 * k2] = w[k2];
-    }
+    for (int k2 = 0; k2 < N2; ++k2) row[k1 + N1 * k2] = w[k2];
   }
   __syncwarp();
 }
@@ -345,7 +333,7 @@ __global__ void __launch_bounds__(128) k_fillps_fftx_r(Geo g, const float *__res
   }
   __syncthreads();
   const int grp = threadIdx.x / N2, t = threadIdx.x - grp * N2;
-  fft_group<N1, N2>(A + grp * RS, EX + grp * ES, t, twM, 0, true);
+  fft_group<N1, N2>(A + grp * RS, EX + grp * ES, t, twM);
   __syncthreads();
   // 2. unpack to X_k, k = 0..M  (X_k = E_k + W_N^k O_k)
   for (int q = threadIdx.x; q < ROWS * (M + 1); q += blockDim.x) {

@@ -104,9 +104,9 @@ __global__ void __launch_bounds__(256) k_ibm_points(Geo g, PartGeo pg, IbmBuffer
 // sphere's shell touches about 40 % of its box, and a row through the
 // sphere only its two ends.
 // Points of particle p, component c by the bank of their first tap:
-// order[(p*3 + c)*nl + bst[q] ..bst[q+1]) = those of bank q, bst[33] = the most
-// of any bank (bst: IBM_BST entries per (p, c)); -1 there where the points are
-// not ordered (box not usable, or more than SPREAD_PRE of them).
+// order[(p*3 + c)*nl + bst[q] ..bst[q+1]) = those of bank q (bst: IBM_BST entries
+// per (p, c)); bst[33] = 0, or -1 where the points are not ordered (box not
+// usable, or more than SPREAD_PRE of them).
 __global__ void __launch_bounds__(256) k_ibm_box_geom(Geo g, PartGeo pg, IbmBuffers b) {
   const int p = blockIdx.x, c = blockIdx.y, K = g.K;
   const int nla = b.nla[p];
@@ -159,12 +159,11 @@ __global__ void __launch_bounds__(256) k_ibm_box_geom(Geo g, PartGeo pg, IbmBuff
       const int o = __shfl_up_sync(0xffffffffu, sum, d);
       if (q >= d) sum += o;
     }
-    const int most = __reduce_max_sync(0xffffffffu, n);
     cur[q] = sum - n;
     bst[q] = (short)(sum - n);
     if (q == 31) {
       bst[32] = (short)sum;
-      bst[33] = sorted ? (short)most : (short)-1;
+      bst[33] = sorted ? (short)0 : (short)-1;
     }
   }
   if (masks) {
