@@ -20,8 +20,9 @@
 // (its force sums in the last pass only), box geometry 22 -> 26 / 36 -> 47.
 //
 // Origins come from the FP64 point coordinates exactly as the FP64 form
-// computes them; delta weights, interpolation sums and spreading are FP32;
-// point forces F_l and the per-particle force/torque sums stay FP64.
+// computes them; delta weights, interpolation sums, point forces F_l and
+// spreading are FP32; the per-particle force/torque sums are FP32 per thread and
+// pairs of FP32 across a block, FP64 from there on.
 #include <cuda_bf16.h>
 
 #include <type_traits>
@@ -419,7 +420,7 @@ __global__ void __launch_bounds__(NT, MB) k_ibm_interp_comp_f(Geo g, PartGeo pg,
     __syncthreads();
   }
   // per-thread force and lever-arm sums in FP32 (a few points per thread),
-  // the block's sums in FP64
+  // the block's sums in pairs of FP32
   float sF = 0.f, sa = 0.f, sb = 0.f;
   float r2 = 0.f, r0 = 0.f;
   int pass = 0;
@@ -449,7 +450,7 @@ __global__ void __launch_bounds__(NT, MB) k_ibm_interp_comp_f(Geo g, PartGeo pg,
     }
     slip[t] = sd;  // the spreading's increment (U - u~)/dt, FP32
     if constexpr (FIRST == 1) r0 = fmaf(sd, sd, r0);  // first-pass slip, for the learned loop's gate reference
-    float ff;  // the point force, FP32 (its sums below, FP64 across the block)
+    float ff;  // the point force, FP32 (its sums below, pairs of FP32 across the block)
     if constexpr (FIRST == 1) ff = sd * dtif;
     else ff = fmaf(sd, dtif, pass == 0 ? fl[0] : (pass == 1 ? fl[1] : (pass == 2 ? fl[2] : (pass == 3 ? fl[3] : Fl[t]))));
     Fl[t] = ff;
@@ -624,7 +625,7 @@ __global__ void __launch_bounds__(NT, MB) k_ibm_spread_f(Geo g, PartGeo pg, IbmB
   float *__restrict__ Fl = c == 0 ? b.fxs : (c == 1 ? b.fys : b.fzs);
   const int4 ref = b.pref[p];
   const PointRec *rp = b.rec + t0;
-  // per-thread force and lever-arm sums in FP32, the block's sums in FP64
+  // per-thread force and lever-arm sums in FP32, the block's sums in pairs of FP32
   float sF = 0.f, sa = 0.f, sb = 0.f;
   float4 cf = make_float4(0.f, 0.f, 0.f, 0.f);
   float ysig = 0.f, ymu = 0.f, dtif = 0.f, dtf = 0.f;
@@ -642,7 +643,7 @@ __global__ void __launch_bounds__(NT, MB) k_ibm_spread_f(Geo g, PartGeo pg, IbmB
   // shared-memory adds to one address in one instruction serialise).
   const int nq = (nla + 31) >> 5;
   float asum = 0.f, r0 = 0.f;
-  if (!LY && staged) {  // the plain passes: the slips of up to six points, loaded together
+  if (!LY && staged) {  // the plain passes: a thread's slips (8 of 256 threads, 4 of 512) loaded together
     float sv[(SPREAD_PRE + NT - 1) / NT];
 #pragma unroll
     for (int q = 0; q < (SPREAD_PRE + NT - 1) / NT; ++q) {
@@ -709,7 +710,7 @@ __global__ void __launch_bounds__(NT, MB) k_ibm_spread_f(Geo g, PartGeo pg, IbmB
     }
   }
   if (!boxed) return;
-  // fixed point: scale 2^(29 - e) with bound < 2^e, so that bound * scale < 2^30
+  // fixed point: scale 2^(29 - e) with bound < 2^e, so that bound * scale < 2^29
   float scale = 0.f;
   if (staged) {
     const float bound = block_sum_all(asum);  // also orders spre before its reads

@@ -1217,8 +1217,11 @@ __global__ void __launch_bounds__(32 * COLL_WARPS) k_collide_update(PartGeo pg, 
 int launch_collide_update(cudaStream_t s, const PartGeo &pg, PartBuffers b, int iter, int rkiter, double dt) {
   if (pg.np == 0) return 0;
   int n = 1;
-  // the search over all particles costs np^2 / 32 FP32 tests in place of the
-  // cell list's one-block kernel (9 us at 1000 particles): even at about 4000
+  // The search over all particles costs np^2 / 32 FP32 tests, the cell list a
+  // one-block kernel over particles and cells.  A whole update, all / cell list:
+  // spheres of 16 dx at 256^3 (3375 cells) 1000: 140 / 148 us, 1728: 233 / 221,
+  // 2197: 282 / 260; of 3.6 dx at 128^3 (35937 cells) 1000: 142 / 258, 2197: 304 /
+  // 388, 4096: 615 / 588.  The line lies between the two break-evens.
   const int scan = pg.np <= 2048 || pg.ncx < 3 || pg.ncy < 3;
   if (!scan) { k_cell_build<<<1, 1024, 0, s>>>(pg, b, iter); ++n; }
   const double rkab = pg.rkab[rkiter - 1], f = 1. - (1. / pg.ratiorho);
